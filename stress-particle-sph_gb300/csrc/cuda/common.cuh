@@ -235,6 +235,19 @@ struct Dev {
   // has column k (stress-points) or NT - NN + k (nodes), so a warp reads its targets' list
   // entries as one contiguous run per slot.
   int32_t* lcol;
+  // One launch per RK4 stage (Ctx::fused): the particle of every list column, and what a step
+  // keeps per column or particle while positions, lists and densities do not change (see
+  // plain_fused.cu): list constants hW (k * NT + col), hG (stress-points, k * ns + col), a
+  // target's interpolation norm and its reciprocal, its CSPM moments (5 rows of NT), a
+  // stress-point's stress at the start of the step and its RK sum (4 doubles a column)
+  int32_t* colid;
+  double* hW;
+  double2* hG;
+  double *norm, *rnorm, *AE, *st0c, *rkc;
+  // the values a stage reads from its neighbours, double buffered over the stages: node
+  // velocity (2 a node), stress-point stress (4) and {stress / rho^2 (3), mass}
+  double *pv[2], *ps[2], *pa[2];
+  double *rho2, *rinv2;  // rho * rho and its reciprocal, per particle
   // get_nodes_on_free_surface: normal (module FP64), subset (1 surface, 2 inside), f_int
   double *nrmx, *nrmy;
   int8_t* subset;
@@ -910,6 +923,9 @@ int launch_pair_build(Ctx& c);
 int launch_plain_step(Ctx& c);
 int launch_fast_step(Ctx& c);
 void launch_vol(Ctx& c, int lo, int hi);
+void launch_pprep(Ctx& c);
+void launch_pstage(Ctx& c, int stage);
+void launch_pfinish(Ctx& c);
 void launch_finterp(Ctx& c);
 void launch_fderivs(Ctx& c, int stage);
 void launch_fsp_tail(Ctx& c, int stage);

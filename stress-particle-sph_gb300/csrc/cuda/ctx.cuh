@@ -90,6 +90,21 @@ struct Ctx {
     return precision == SPS_PREC_FP32_FAST && !surf_every && d.sle != 2 &&
            2 * d.capC * 32 * 4 <= 49152;
   }
+  // one launch per RK4 stage: the positions, lists and densities do not change within a step
+  // and nothing between the two halves of a stage needs the whole field (the continuity
+  // equation's densities, artificial stress, the traction-free BC's normals do)
+  bool fused() const {
+    return precision == SPS_PREC_FP64_PLAIN && d.sp_sph && !d.cont_density && !d.art_stress &&
+           !(d.no_bcs > 0 && d.ifsigman == 1);
+  }
+  // the block size for n threads: at most `most`, halved while fewer than two blocks an SM
+  // would leave SMs idle
+  static int block_for(int64_t n, int most) {
+    int b = most;
+    while (b > 32 && n < (int64_t)b * 304) b >>= 1;
+    return b;
+  }
+  int split_max = 60000;  // largest NT whose stage kernels split a target's sums over lanes
   // the last pair build left the half lists unwritten (k_fgather): sps_dump_pairs and the
   // keyed lists of the exact detection build them first (set by enqueue_step for every
   // step, since a replayed graph runs no host code)

@@ -1222,9 +1222,11 @@ __global__ void k_target_scatter(Dev D) {
   if (D.tflag[s]) {
     D.tgtS[a] = s;
     col = a;
+    D.colid[col] = D.sorted[s];
   } else if (D.tflag[D.N2 + s]) {
     D.tgtN[b] = s;
     col = (D.NT - D.NN) + b;
+    D.colid[col] = D.sorted[s];
   } else {
     col = D.NT + (s - a - b);
   }

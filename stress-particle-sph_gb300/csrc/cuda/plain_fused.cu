@@ -1,0 +1,821 @@
+// plain_fused.cu -- the RK4 stages of the FP64 plain form as one launch per stage (compiled
+// with -fmad=false).
+//
+// Within a step the positions, the neighbour lists and (without the continuity equation) the
+// densities are constant, so everything a pair sum takes from them alone is formed once, by
+// k_pprep, with the operations the reference repeats in every stage:
+//   hW   (m/rho) W of every entry (a stress-point's wall entry: 1 - beta of the wall velocity)
+//   hG   (G m)/rho of a stress-point's entries, both components
+//   norm the sum of W m / rho of a target, and its reciprocal
+//   AE   the CSPM moments of a target
+// A stage then reads them instead of recomputing: 4 + 10 FP64 operations an entry on the
+// stress-point side and 8 + 21 on the node side, against 12 + 22 and 18 + 21.
+//
+// k_pstage runs a whole stage of both kinds (blocks of stress-points first, then blocks of
+// nodes): stress_point_update, adapt_stress2 and the BCs, get_derivatives, the rates, their
+// RK accumulation, and the state of the next stage.  The values a stage reads from its
+// neighbours (node velocities pv, stress-point stresses ps and stress/rho^2 pa) are double
+// buffered, so the two kinds need no order between them.  k_pfinish interpolates the final
+// state and moves the particles.  Results are bit-identical to the separate kernels of
+// plain_step.cu, which remain for the options that change densities or node stresses between
+// the two halves of a stage (Ctx::fused).
+//
+// What bounds it: the FP64 pipe (2 lanes a clock and SM) at large sizes; at small ones the
+// serial chain of a target's sums, which LS and LN lanes a target share by component (one
+// velocity component a lane, one stress component a lane), each component still summed in
+// list order by one lane.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "ctx.cuh"
+#include "stage_tail.cuh"
+
+namespace sps {
+
+namespace {
+
+struct alignas(32) d4 {
+  double a, b, c, d;
+};
+__device__ __forceinline__ d4 ld4(const double* p) {
+  d4 v;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(v.a), "=d"(v.b), "=d"(v.c), "=d"(v.d)
+               : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void st4(double* p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d)
+               : "memory");
+}
+
+// adapt_stress2 (the plain form's stress_return of plain_step.cu)
+__device__ __forceinline__ void ret(const Real& M, double& a, double& b, double& c, double& d) {
+  if (M.ncrit != 12) return;
+  if (inside_cone_f32(M.alpha2f, M.kcf, a, b, c, d)) return;
+  adapt_stress(M.alpha2, M.kc, a, b, c, d);
+}
+
+// a / b with y = RN(1/b): the corrected product for a numerator of ordinary exponent (the
+// range in which no step of div_rcp leaves the normal numbers, |b| within 2^+-200), else the
+// IEEE division
+__device__ __forceinline__ double div_pre(double a, double b, double y) {
+  const int ex = (int)((__double_as_longlong(a) >> 52) & 0x7FF);
+  if (ex > 400 && ex < 1640) return div_rcp(a, b, y);
+  if ((__double_as_longlong(a) << 1) == 0) return a * y;  // a signed zero
+  return a / b;
+}
+
+__device__ __forceinline__ void load_real(const Dev& D, int t, const Real*& M,
+                                          const StepScalars*& sc) {
+  const int r = D.R == 1 ? 0 : D.rid[t];
+  M = &real_of(D, t);
+  sc = D.cur + r;
+}
+
+// the state of a stress-point at the start of a stage from its rates' result (a, b, c, d):
+// return and BCs; that is what the nodes interpolate (ps), and returned once more (the
+// reference returns every stress again after the interpolation) it enters get_derivatives
+// (pa = sigma / rho^2)
+__device__ __forceinline__ void sp_publish(const Dev& D, const Real& M, const StepScalars& sc,
+                                           int t, int buf, double a, double b, double c, double d,
+                                           bool with_pa, double* fin) {
+  double vx = 0.0, vy = 0.0;
+  ret(M, a, b, c, d);
+  apply_bcs(D, sc, t, vx, vy, a, b, c, d);
+  const size_t i = (size_t)(t - D.NN);
+  st4(D.ps[buf] + 4 * i, a, b, c, d);
+  ret(M, a, b, c, d);
+  apply_bcs(D, sc, t, vx, vy, a, b, c, d);
+  if (with_pa) {
+    const double r2 = D.rho2[t], y = D.rinv2[t];
+    st4(D.pa[buf] + 4 * i, div_pre(a, r2, y), div_pre(b, r2, y), div_pre(c, r2, y), D.mass[t]);
+  }
+  if (fin) {
+    fin[0] = a;
+    fin[1] = b;
+    fin[2] = c;
+    fin[3] = d;
+  }
+}
+
+// Once per step, per target: the constants of its list entries (file comment), the boundary
+// force of a node (boundary_forces, over its list's innermost dummies as k_bound), and the
+// state of stage 0.  Bound by the FP64 pipe (22 operations a stress-point entry, 8 a node's).
+__global__ void __launch_bounds__(128) k_pprep(Dev D) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= D.NT) return;
+  const int ns = D.NT - D.NN;
+  const int t = D.colid[k];
+  const Real* Mp;
+  const StepScalars* scp;
+  load_real(D, t, Mp, scp);
+  const Real& M = *Mp;
+  const int deg = D.degC[k];
+  const double xt = D.px[t], yt = D.py[t];
+  double norm = 0.0;
+  double AE[4] = {0.0, 0.0, 0.0, 0.0};
+  if (k < ns) {
+    for (int j = 0; j < deg; j++) {
+      const int4 e = D.cross[ell(j, k, D.N2)];
+      const int u = e.x;
+      const bool wall = e.y < 0;
+      const double Gx = f64_of(__int_as_float(e.z)), Gy = f64_of(__int_as_float(e.w));
+      const double mu = D.mass[u], ru = D.rho[u], iu = D.rinv[u];
+      double h, h1, h2;
+      if (!wall) {
+        const double w = f64_of(__int_as_float(e.y));
+        h = D.vol[u] * w;
+        norm = norm + div_rcp(w * mu, ru, iu);
+        h1 = div_rcp(Gx * mu, ru, iu);
+        h2 = div_rcp(Gy * mu, ru, iu);
+        if (D.cspm) {
+          const double xu = D.px[u] - xt, yu = D.py[u] - yt;
+          AE[0] = AE[0] + xu * h1;
+          AE[1] = AE[1] + yu * h1;
+          AE[2] = AE[2] + xu * h2;
+          AE[3] = AE[3] + yu * h2;
+        }
+      } else {
+        const double wp = (double)D.wallpos[u];
+        double da, db;
+        if (D.horiz[u] == 1.0f) {
+          da = fabs(yt - wp);
+          db = fabs(D.py[u] - wp);
+        } else {
+          da = fabs(xt - wp);
+          db = fabs(D.px[u] - wp);
+        }
+        const double bq = 1.0 + db / da;
+        const double beta = 1.5 < bq ? 1.5 : bq;
+        h = 1.0 - beta;
+        h1 = div_rcp(-Gx * mu, ru, iu);
+        h2 = div_rcp(-Gy * mu, ru, iu);
+      }
+      D.hW[(size_t)j * D.NT + k] = h;
+      D.hG[(size_t)j * ns + k] = make_double2(h1, h2);
+    }
+  } else {
+    constexpr int K = 8;
+    int ids[K];
+    float tx[K], ty[K];
+    int n = 0, bc_int = 0;
+    const int j0 = M.dum0, j1 = M.dum0 + M.ndum2;
+    for (int j = 0; j < deg; j++) {
+      const int4 e = D.cross[ell(j, k, D.N2)];
+      const int u = e.x;
+      if (e.y >= 0) {
+        const double w = f64_of(__int_as_float(e.y));
+        const double mu = D.mass[u], ru = D.rho[u], iu = D.rinv[u];
+        D.hW[(size_t)j * D.NT + k] = D.vol[u] * w;
+        norm = norm + div_rcp(w * mu, ru, iu);
+        if (D.cspm) {
+          const double dwx = -f64_of(__int_as_float(e.z)), dwy = -f64_of(__int_as_float(e.w));
+          const double h1b = -div_rcp(dwx * mu, ru, iu), h2b = -div_rcp(dwy * mu, ru, iu);
+          const double xu = D.px[u] - xt, yu = D.py[u] - yt;
+          AE[0] = AE[0] + xu * h1b;
+          AE[1] = AE[1] + yu * h1b;
+          AE[2] = AE[2] + xu * h2b;
+          AE[3] = AE[3] + yu * h2b;
+        }
+      } else {
+        bc_int = 1;
+        float fx, fy;
+        if (D.inside && D.bound_from_lists && u >= j0 && u < j1 && bound_term(D, M, t, u, fx, fy)) {
+          if (n < K) {
+            int p = n++;
+            while (p > 0 && ids[p - 1] > u) {
+              ids[p] = ids[p - 1];
+              tx[p] = tx[p - 1];
+              ty[p] = ty[p - 1];
+              p--;
+            }
+            ids[p] = u;
+            tx[p] = fx;
+            ty[p] = fy;
+          } else {
+            atomicOr(D.err, ERR_BOUND);
+          }
+        }
+      }
+    }
+    double bx = 0.0, by = 0.0;
+    if (D.inside && !D.bound_from_lists) {
+      for (int j = j0; j < j1; j++) {
+        float fx, fy;
+        if (!bound_term(D, M, t, j, fx, fy)) continue;
+        bx = bx + (double)fx;
+        by = by + (double)fy;
+      }
+    } else {
+      for (int j = 0; j < n; j++) {
+        bx = bx + f64_of(tx[j]);
+        by = by + f64_of(ty[j]);
+      }
+    }
+    D.fbx[t] = bx;
+    D.fby[t] = by;
+    D.bc_int[t] = bc_int;
+  }
+  D.norm[k] = norm;
+  D.rnorm[k] = norm != 0.0 ? 1.0 / norm : 0.0;
+  if (D.cspm) {
+    double A4 = AE[0] * AE[3] - AE[1] * AE[2];
+    if (fabs(A4) < D.cspm_det) {
+      A4 = 1;
+      AE[0] = 1;
+      AE[1] = 0;
+      AE[2] = 0;
+      AE[3] = 1;
+    } else {
+      A4 = 1.0 / A4;
+    }
+    for (int q = 0; q < 4; q++) D.AE[(size_t)q * D.NT + k] = AE[q];
+    D.AE[(size_t)4 * D.NT + k] = A4;
+  }
+  // the state of stage 0 (RK4 starts from zero rates)
+  if (k < ns) {
+    const double a = D.s0[t], b = D.s1[t], c = D.s2[t], d = D.s3[t];
+    st4(D.st0c + 4 * (size_t)k, a, b, c, d);
+    sp_publish(D, M, *scp, t, 0, a + 0.0, b + 0.0, c + 0.0, d + 0.0, true, nullptr);
+  } else {
+    const double v0x = D.vx[t], v0y = D.vy[t];
+    D.vx0[t] = v0x;
+    D.vy0[t] = v0y;
+    double vx = v0x + 0.0, vy = v0y + 0.0, a = 0.0, b = 0.0, c = 0.0, d = 0.0;
+    if (norm == 0.0) {  // no stress-point in reach: RK4 clears the stress, nothing sets it
+      ret(M, a, b, c, d);
+      apply_bcs(D, *scp, t, vx, vy, a, b, c, d);
+      D.s0[t] = a;
+      D.s1[t] = b;
+      D.s2[t] = c;
+      D.s3[t] = d;
+      vx = 0.0;
+      vy = 0.0;
+    }
+    apply_bcs(D, *scp, t, vx, vy, a, b, c, d);
+    reinterpret_cast<double2*>(D.pv[0])[t] = make_double2(vx, vy);
+  }
+}
+
+// entries a pass whose list words and neighbour records are loaded before any is summed
+constexpr int kP = 4;
+
+// One stage of a stress-point; LS = 2: lane d of the pair sums velocity component d
+template <int LS>
+__device__ __forceinline__ void sp_stage(const Dev& D, int stage, int k, bool act, int q) {
+  const int ns = D.NT - D.NN, cur = stage & 1, nxt = cur ^ 1;
+  const int t = D.colid[k];
+  const double2* __restrict__ pv = reinterpret_cast<const double2*>(D.pv[cur]);
+  const int deg = act ? D.degC[k] : 0;
+  const double norm = D.norm[k], rn = D.rnorm[k];
+  const Real* Mp;
+  const StepScalars* scp;
+  load_real(D, t, Mp, scp);
+  const Real& M = *Mp;
+  double v0 = 0.0, v1 = 0.0;
+  for (int j = 0; j < deg; j += kP) {
+    int4 e[kP];
+    double h[kP];
+    double2 v[kP];
+#pragma unroll
+    for (int i = 0; i < kP; i++) {
+      e[i] = j + i < deg ? D.cross[ell(j + i, k, D.N2)] : make_int4(0, -1, 0, 0);
+      h[i] = e[i].y >= 0 ? D.hW[(size_t)(j + i) * D.NT + k] : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < kP; i++) v[i] = e[i].y >= 0 ? pv[e[i].x] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int i = 0; i < kP; i++)
+      if (e[i].y >= 0) {
+        if (LS == 1) {
+          v0 = v0 + v[i].x * h[i];
+          v1 = v1 + v[i].y * h[i];
+        } else {
+          v0 = v0 + (q ? v[i].y : v[i].x) * h[i];
+        }
+      }
+  }
+  double vt0 = 0.0, vt1 = 0.0;  // RK4 clears the velocity; no node in reach leaves it so
+  if (norm != 0.0) {
+    vt0 = div_pre(v0, norm, rn);
+    if (LS == 1) vt1 = div_pre(v1, norm, rn);
+  }
+  if (LS == 2) {
+    const double o = __shfl_xor_sync(0xffffffffu, vt0, 1);
+    vt1 = q ? vt0 : o;
+    vt0 = q ? o : vt0;
+  }
+  const d4 own = ld4(D.ps[cur] + 4 * (size_t)(t - D.NN));
+  double st[4] = {own.a, own.b, own.c, own.d};
+  ret(M, st[0], st[1], st[2], st[3]);
+  apply_bcs(D, *scp, t, vt0, vt1, st[0], st[1], st[2], st[3]);
+  double g[4] = {0.0, 0.0, 0.0, 0.0};  // grad1(a,b) at a + 2b
+  const double vtq = LS == 2 && q ? vt1 : vt0;
+  for (int j = 0; j < deg; j += kP) {
+    int4 e[kP];
+    double2 h[kP], v[kP];
+#pragma unroll
+    for (int i = 0; i < kP; i++) {
+      e[i] = j + i < deg ? D.cross[ell(j + i, k, D.N2)] : make_int4(0, 0, 0, 0);
+      h[i] = j + i < deg ? D.hG[(size_t)(j + i) * ns + k] : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for (int i = 0; i < kP; i++) {
+      v[i] = make_double2(0.0, 0.0);
+      if (j + i < deg) {
+        if (e[i].y >= 0) v[i] = pv[e[i].x];
+        else v[i].x = D.hW[(size_t)(j + i) * D.NT + k];  // 1 - beta
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kP; i++)
+      if (j + i < deg) {
+        const bool wall = e[i].y < 0;
+        // a wall's velocity seen by the stress-point: v (1 - beta) + beta 0
+        if (LS == 1) {
+          const double du0 = wall ? vt0 - (vt0 * v[i].x + 0.0) : v[i].x - vt0;
+          const double du1 = wall ? vt1 - (vt1 * v[i].x + 0.0) : v[i].y - vt1;
+          g[0] = g[0] + du0 * h[i].x;
+          g[2] = g[2] + du0 * h[i].y;
+          g[1] = g[1] + du1 * h[i].x;
+          g[3] = g[3] + du1 * h[i].y;
+        } else {
+          const double du = wall ? vtq - (vtq * v[i].x + 0.0) : (q ? v[i].y : v[i].x) - vtq;
+          g[0] = g[0] + du * h[i].x;
+          g[2] = g[2] + du * h[i].y;
+        }
+      }
+  }
+  if (LS == 2) {
+    g[1] = __shfl_xor_sync(0xffffffffu, g[0], 1);
+    g[3] = __shfl_xor_sync(0xffffffffu, g[2], 1);
+    if (q) return;
+  }
+  if (!act) return;
+  if (D.cspm) {
+    double A[5];
+    for (int i = 0; i < 5; i++) A[i] = D.AE[(size_t)i * D.NT + k];
+    for (int d = 0; d < 2; d++) {
+      g[d] = A[4] * (A[0] * g[d] + A[1] * g[d + 2]);
+      g[d + 2] = A[4] * (A[2] * g[d] + A[3] * g[d + 2]);
+    }
+  }
+  double rhs[4], der;
+  sp_rates_f64(D, M, *scp, t, g, st, rhs, der);
+  const double f2 = (stage == 1 || stage == 2) ? 2.0 : 1.0;  // RK4 weights 1, 2, 2, 1
+  double rk[4] = {0.0, 0.0, 0.0, 0.0}, rd = 0.0;
+  double* rks = D.rkc + 4 * (size_t)k;
+  if (stage > 0) {
+    const d4 o = ld4(rks);
+    rk[0] = o.a;
+    rk[1] = o.b;
+    rk[2] = o.c;
+    rk[3] = o.d;
+    rd = D.RKd[k];
+  }
+  for (int i = 0; i < 4; i++) rk[i] = rk[i] + f2 * rhs[i];
+  rd = rd + der * f2;
+  const d4 s0 = ld4(D.st0c + 4 * (size_t)k);
+  if (stage < 3) {
+    st4(rks, rk[0], rk[1], rk[2], rk[3]);
+    D.RKd[k] = rd;
+    const double f1dt = (stage == 2 ? 1.0 : 0.5) * M.dt;  // RK4 nodes 1/2, 1/2, 1
+    sp_publish(D, M, *scp, t, nxt, s0.a + f1dt * rhs[0], s0.b + f1dt * rhs[1],
+               s0.c + f1dt * rhs[2], s0.d + f1dt * rhs[3], true, nullptr);
+  } else {  // the end of RK4 (2_SPH_main_2018.f90:784-799) and update_strain
+    const double dt6 = M.dt6;
+    double f[4];
+    sp_publish(D, M, *scp, t, nxt, s0.a + dt6 * rk[0], s0.b + dt6 * rk[1], s0.c + dt6 * rk[2],
+               s0.d + dt6 * rk[3], false, f);
+    D.s0[t] = f[0];
+    D.s1[t] = f[1];
+    D.s2[t] = f[2];
+    D.s3[t] = f[3];
+    const int ex = (int)((__double_as_longlong(rd) >> 52) & 0x7FF);
+    const double dd = (ex > 64 && ex < 1980) ? div_rcp(rd, 6.0, 1.0 / 6.0) : rd / 6.0;
+    D.Ddev[t] = dd;
+    D.iv1[t] = D.iv1[t] + M.dt * dd;
+  }
+}
+
+// artificial_viscosity's pair value for target t and neighbour u (2_SPH_main_2018.f90:
+// 826-904): the FP32 products visc dW; the quotient by the pair's density uses the
+// reciprocal of the last density met (the pairs of a uniform material share one)
+struct ViscT {
+  double xt, yt, vtx, vty, ht, rt, a600, beta;
+  float hf, rf;
+  double yrho;
+  float yfor;
+};
+__device__ __forceinline__ float2 visc_pair(const Dev& D, ViscT& T, const int4& e, double2 vu) {
+  const int u = e.x;
+  const float xij = f32_rn(T.xt - D.px[u]), yij = f32_rn(T.yt - D.py[u]);
+  const double hu = D.hsml[u], ru = D.rho[u];
+  // 0.5 (h + h) = h exactly
+  const float h = __double_as_longlong(hu) == __double_as_longlong(T.ht) ? T.hf
+                                                                          : (float)(0.5 * (T.ht + hu));
+  const float rho2 = __double_as_longlong(ru) == __double_as_longlong(T.rt)
+                         ? T.rf
+                         : (float)(0.5 * (T.rt + ru));
+  float div_u = f32_rn(f64_of(xij) * (T.vtx - vu.x));
+  div_u = f32_rn(f64_of(div_u) + f64_of(yij) * (T.vty - vu.y));
+  const float sq = sqrtf(xij * xij + yij * yij);
+  const float theta = (h * div_u) / (sq * sq + 0.01f * (h * h));
+  float visc = 0.0f;
+  if (div_u < 0) {
+    if (rho2 != T.yfor) {
+      T.yfor = rho2;
+      T.yrho = 1.0 / f64_of(rho2);
+    }
+    const double num = -(T.a600 * f64_of(theta)) + T.beta * f64_of(theta * theta);
+    visc = div_rcp_f32(num, f64_of(rho2), T.yrho);
+  }
+  return make_float2(visc * __int_as_float(e.z), visc * __int_as_float(e.w));
+}
+
+// One stage of a node; LN = 4: lane q of the group sums stress component q, then the
+// derivative sums of component q (q < 3)
+template <int LN>
+__device__ __forceinline__ void node_stage(const Dev& D, int stage, int k, bool act, int q) {
+  const int cur = stage & 1, nxt = cur ^ 1;
+  const int t = D.colid[k];
+  const double* __restrict__ ps = D.ps[cur];
+  const double* __restrict__ pa = D.pa[cur];
+  const int deg = act ? D.degC[k] : 0;
+  const double norm = D.norm[k], rn = D.rnorm[k];
+  const Real* Mp;
+  const StepScalars* scp;
+  load_real(D, t, Mp, scp);
+  const Real& M = *Mp;
+  const int b0 = LN == 4 ? (threadIdx.x & 31 & ~3) : 0;
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int j = 0; j < deg; j += kP) {
+    int4 e[kP];
+    double h[kP];
+    d4 v[kP];
+    double vq[kP];
+#pragma unroll
+    for (int i = 0; i < kP; i++) {
+      e[i] = j + i < deg ? D.cross[ell(j + i, k, D.N2)] : make_int4(0, -1, 0, 0);
+      h[i] = e[i].y >= 0 ? D.hW[(size_t)(j + i) * D.NT + k] : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < kP; i++)
+      if (e[i].y >= 0) {
+        const double* p = ps + 4 * (size_t)(e[i].x - D.NN);
+        if (LN == 1) v[i] = ld4(p);
+        else vq[i] = p[q];
+      }
+#pragma unroll
+    for (int i = 0; i < kP; i++)
+      if (e[i].y >= 0) {
+        if (LN == 1) {
+          s[0] = s[0] + v[i].a * h[i];
+          s[1] = s[1] + v[i].b * h[i];
+          s[2] = s[2] + v[i].c * h[i];
+          s[3] = s[3] + v[i].d * h[i];
+        } else {
+          s[0] = s[0] + vq[i] * h[i];
+        }
+      }
+  }
+  if (norm != 0.0) {
+    if (LN == 1) {
+      for (int i = 0; i < 4; i++) s[i] = div_pre(s[i], norm, rn);
+    } else {
+      s[0] = div_pre(s[0], norm, rn);
+    }
+  }
+  if (LN == 4) {
+    const double o = s[0];
+    for (int i = 0; i < 4; i++) s[i] = __shfl_sync(0xffffffffu, o, b0 + i);
+  }
+  double2 v = reinterpret_cast<const double2*>(D.pv[cur])[t];
+  if (norm == 0.0) {  // the stress of the last return, returned again at the stage's start
+    s[0] = D.s0[t];
+    s[1] = D.s1[t];
+    s[2] = D.s2[t];
+    s[3] = D.s3[t];
+    if (stage > 0) {
+      ret(M, s[0], s[1], s[2], s[3]);
+      apply_bcs(D, *scp, t, v.x, v.y, s[0], s[1], s[2], s[3]);
+    }
+  }
+  ret(M, s[0], s[1], s[2], s[3]);
+  apply_bcs(D, *scp, t, v.x, v.y, s[0], s[1], s[2], s[3]);
+  const double r2 = D.rho2[t], y2 = D.rinv2[t];
+  double at[3];
+  if (LN == 1) {
+    for (int i = 0; i < 3; i++) at[i] = div_pre(s[i], r2, y2);
+  } else {
+    at[0] = div_pre(q == 0 ? s[0] : q == 1 ? s[1] : s[2], r2, y2);
+  }
+  double g2[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // grad2(s,b) at s + 3b
+  const double sq = q == 0 ? s[0] : q == 1 ? s[1] : s[2];
+  const int qa = LN == 4 ? (q < 3 ? q : 2) : 0;
+  for (int j = 0; j < deg; j += kP) {
+    int4 e[kP];
+    d4 v4[kP];
+    double aq[kP], mu[kP];
+#pragma unroll
+    for (int i = 0; i < kP; i++)
+      e[i] = j + i < deg ? D.cross[ell(j + i, k, D.N2)] : make_int4(0, 0, 0, 0);
+#pragma unroll
+    for (int i = 0; i < kP; i++)
+      if (j + i < deg && e[i].y >= 0) {
+        const double* p = pa + 4 * (size_t)(e[i].x - D.NN);
+        if (LN == 1) {
+          v4[i] = ld4(p);
+          mu[i] = v4[i].d;
+        } else {
+          aq[i] = p[qa];
+          mu[i] = p[3];
+        }
+      }
+#pragma unroll
+    for (int i = 0; i < kP; i++)
+      if (j + i < deg) {
+        const double dwx = -f64_of(__int_as_float(e[i].z)), dwy = -f64_of(__int_as_float(e[i].w));
+        if (e[i].y < 0) {  // a dummy carries the node's stress
+          const int u = e[i].x;
+          const double ru2 = D.rho2[u], yu2 = D.rinv2[u];
+          mu[i] = D.mass[u];
+          if (LN == 1) {
+            v4[i].a = div_pre(s[0], ru2, yu2);
+            v4[i].b = div_pre(s[1], ru2, yu2);
+            v4[i].c = div_pre(s[2], ru2, yu2);
+          } else {
+            aq[i] = div_pre(sq, ru2, yu2);
+          }
+        }
+        if (LN == 1) {
+          const double au[3] = {v4[i].a, v4[i].b, v4[i].c};
+#pragma unroll
+          for (int p = 0; p < 3; p++) {
+            const double sum = at[p] + au[p];
+            g2[p] = g2[p] - mu[i] * (dwx * sum);
+            g2[p + 3] = g2[p + 3] - mu[i] * (dwy * sum);
+          }
+        } else {
+          const double sum = at[0] + aq[i];
+          g2[0] = g2[0] - mu[i] * (dwx * sum);
+          g2[3] = g2[3] - mu[i] * (dwy * sum);
+        }
+      }
+  }
+  if (LN == 4) {
+    const double a = g2[0], b = g2[3];
+    for (int i = 0; i < 3; i++) {
+      g2[i] = __shfl_sync(0xffffffffu, a, b0 + i);
+      g2[i + 3] = __shfl_sync(0xffffffffu, b, b0 + i);
+    }
+  }
+  double avx = 0.0, avy = 0.0;
+  if (M.alpha > 0 || M.beta > 0) {
+    // artificial_viscosity (2_SPH_main_2018.f90:826-904): FP32 accumulators.  LN = 4: the
+    // group's lanes evaluate four pairs together, then add them in list order
+    float ax = 0.0f, ay = 0.0f;
+    const int degs = act ? D.degS[k] : 0;
+    const double2* __restrict__ pv = reinterpret_cast<const double2*>(D.pv[cur]);
+    ViscT T;
+    T.xt = D.px[t];
+    T.yt = D.py[t];
+    T.vtx = v.x;
+    T.vty = v.y;
+    T.ht = D.hsml[t];
+    T.rt = D.rho[t];
+    T.hf = f32_rn(T.ht);
+    T.rf = f32_rn(T.rt);
+    T.a600 = M.alpha * 600.0;
+    T.beta = M.beta;
+    T.yfor = 0.0f;
+    T.yrho = 0.0;
+    int nmax = degs;
+    if (LN == 4) nmax = __reduce_max_sync(0xffffffffu, degs);  // every lane meets the shuffles
+    for (int j = 0; j < nmax; j += LN) {
+      double px = 0.0, py = 0.0;
+      const int jj = j + (LN == 4 ? q : 0);
+      if (jj < degs) {
+        const int4 e = D.same[ell(jj, k, D.N2)];
+        const float2 p = visc_pair(D, T, e, pv[e.x]);
+        const double mu = D.mass[e.x];
+        px = f64_of(p.x) * mu;
+        py = f64_of(p.y) * mu;
+      }
+      if (LN == 1) {
+        ax = f32_rn(f64_of(ax) + px);
+        ay = f32_rn(f64_of(ay) + py);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const double qx = __shfl_sync(0xffffffffu, px, b0 + i);
+          const double qy = __shfl_sync(0xffffffffu, py, b0 + i);
+          if (j + i < degs) {
+            ax = f32_rn(f64_of(ax) + qx);
+            ay = f32_rn(f64_of(ay) + qy);
+          }
+        }
+      }
+    }
+    avx = -f64_of(ax);
+    avy = -f64_of(ay);
+  }
+  if (LN == 4 && q) return;
+  if (!act) return;
+  if (D.cspm) {
+    double A[5];
+    for (int i = 0; i < 5; i++) A[i] = D.AE[(size_t)i * D.NT + k];
+    for (int d = 0; d < 2; d++) {
+      g2[d] = A[4] * (A[0] * g2[d] + A[1] * g2[d + 3]);
+      g2[d + 3] = A[4] * (A[2] * g2[d] + A[3] * g2[d + 3]);
+    }
+  }
+  double rx, ry;
+  node_rhs_f64(D, M, *scp, t, g2, v.x, v.y, avx, avy, 0.0, 0.0, rx, ry);
+  const double f2 = (stage == 1 || stage == 2) ? 2.0 : 1.0;
+  double kx = 0.0, ky = 0.0;
+  if (stage > 0) {
+    kx = D.RKv[0][t];
+    ky = D.RKv[1][t];
+  }
+  kx = kx + f2 * rx;
+  ky = ky + f2 * ry;
+  const double v0x = D.vx0[t], v0y = D.vy0[t];
+  double nx, ny, a = 0.0, b = 0.0, c = 0.0, d = 0.0;
+  if (stage < 3) {
+    D.RKv[0][t] = kx;
+    D.RKv[1][t] = ky;
+    const double f1dt = (stage == 2 ? 1.0 : 0.5) * M.dt;
+    nx = v0x + f1dt * rx;
+    ny = v0y + f1dt * ry;
+  } else {
+    nx = v0x + M.dt6 * kx;
+    ny = v0y + M.dt6 * ky;
+  }
+  if (norm == 0.0) {
+    D.s0[t] = s[0];
+    D.s1[t] = s[1];
+    D.s2[t] = s[2];
+    D.s3[t] = s[3];
+    nx = 0.0;
+    ny = 0.0;
+  }
+  apply_bcs(D, *scp, t, nx, ny, a, b, c, d);
+  reinterpret_cast<double2*>(D.pv[nxt])[t] = make_double2(nx, ny);
+}
+
+// RK4 stage (2_SPH_main_2018.f90:700-777): blocks [0, nbs) the stress-points, the rest the
+// nodes
+template <int LS, int LN>
+__global__ void __launch_bounds__(128) k_pstage(Dev D, int stage, int nbs) {
+  const int ns = D.NT - D.NN;
+  if ((int)blockIdx.x < nbs) {
+    const int g = (blockIdx.x * blockDim.x + threadIdx.x) / LS;
+    const bool act = g < ns;
+    if (LS == 1 && !act) return;
+    sp_stage<LS>(D, stage, act ? g : 0, act, threadIdx.x & (LS - 1));
+  } else {
+    const int g = ((blockIdx.x - nbs) * blockDim.x + threadIdx.x) / LN;
+    const bool act = g < D.NN;
+    if (LN == 1 && !act) return;
+    node_stage<LN>(D, stage, ns + (act ? g : 0), act, threadIdx.x & (LN - 1));
+  }
+}
+
+// the final interpolation, return and BCs (2_SPH_main_2018.f90:130-135), then the position
+// update (:140-146, without XSPH) and the displacements (:166-180)
+__global__ void __launch_bounds__(128) k_pfinish(Dev D) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= D.N2) return;
+  if (k >= D.NT) {  // dummies: their place in the step's pair build
+    D.x0x[k] = D.px[k];
+    D.x0y[k] = D.py[k];
+    return;
+  }
+  const int ns = D.NT - D.NN;
+  const int t = D.colid[k];
+  const int deg = D.degC[k];
+  const double norm = D.norm[k], rn = D.rnorm[k];
+  const Real* Mp;
+  const StepScalars* scp;
+  load_real(D, t, Mp, scp);
+  const Real& M = *Mp;
+  double vx, vy, vx0, vy0;
+  if (k < ns) {
+    const double2* __restrict__ pv = reinterpret_cast<const double2*>(D.pv[0]);
+    double v0 = 0.0, v1 = 0.0;
+    for (int j = 0; j < deg; j += kP) {
+      int4 e[kP];
+      double h[kP];
+      double2 v[kP];
+#pragma unroll
+      for (int i = 0; i < kP; i++) {
+        e[i] = j + i < deg ? D.cross[ell(j + i, k, D.N2)] : make_int4(0, -1, 0, 0);
+        h[i] = e[i].y >= 0 ? D.hW[(size_t)(j + i) * D.NT + k] : 0.0;
+      }
+#pragma unroll
+      for (int i = 0; i < kP; i++) v[i] = e[i].y >= 0 ? pv[e[i].x] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int i = 0; i < kP; i++)
+        if (e[i].y >= 0) {
+          v0 = v0 + v[i].x * h[i];
+          v1 = v1 + v[i].y * h[i];
+        }
+    }
+    vx0 = D.vx[t];
+    vy0 = D.vy[t];
+    vx = vy = 0.0;
+    if (norm != 0.0) {
+      vx = div_pre(v0, norm, rn);
+      vy = div_pre(v1, norm, rn);
+    }
+    double a = 0.0, b = 0.0, c = 0.0, d = 0.0;
+    apply_bcs(D, *scp, t, vx, vy, a, b, c, d);
+    D.vx0[t] = vx0;
+    D.vy0[t] = vy0;
+  } else {
+    const double* __restrict__ ps = D.ps[0];
+    double s[4] = {0.0, 0.0, 0.0, 0.0}, iv = 0.0;
+    for (int j = 0; j < deg; j += kP) {
+      int4 e[kP];
+      double h[kP], w[kP];
+      d4 v[kP];
+#pragma unroll
+      for (int i = 0; i < kP; i++) {
+        e[i] = j + i < deg ? D.cross[ell(j + i, k, D.N2)] : make_int4(0, -1, 0, 0);
+        h[i] = e[i].y >= 0 ? D.hW[(size_t)(j + i) * D.NT + k] : 0.0;
+      }
+#pragma unroll
+      for (int i = 0; i < kP; i++)
+        if (e[i].y >= 0) {
+          v[i] = ld4(ps + 4 * (size_t)(e[i].x - D.NN));
+          w[i] = D.iv1[e[i].x];
+        }
+#pragma unroll
+      for (int i = 0; i < kP; i++)
+        if (e[i].y >= 0) {
+          s[0] = s[0] + v[i].a * h[i];
+          s[1] = s[1] + v[i].b * h[i];
+          s[2] = s[2] + v[i].c * h[i];
+          s[3] = s[3] + v[i].d * h[i];
+          iv = iv + w[i] * h[i];
+        }
+    }
+    const double2 v = reinterpret_cast<const double2*>(D.pv[0])[t];
+    vx = v.x;
+    vy = v.y;
+    if (norm != 0.0) {
+      for (int i = 0; i < 4; i++) s[i] = div_pre(s[i], norm, rn);
+      D.iv1[t] = div_pre(iv, norm, rn);
+    } else {  // RK4's last return and BCs, then no interpolated stress
+      s[0] = D.s0[t];
+      s[1] = D.s1[t];
+      s[2] = D.s2[t];
+      s[3] = D.s3[t];
+      ret(M, s[0], s[1], s[2], s[3]);
+      apply_bcs(D, *scp, t, vx, vy, s[0], s[1], s[2], s[3]);
+      vx = 0.0;
+      vy = 0.0;
+    }
+    ret(M, s[0], s[1], s[2], s[3]);
+    apply_bcs(D, *scp, t, vx, vy, s[0], s[1], s[2], s[3]);
+    D.s0[t] = s[0];
+    D.s1[t] = s[1];
+    D.s2[t] = s[2];
+    D.s3[t] = s[3];
+    vx0 = D.vx0[t];
+    vy0 = D.vy0[t];
+  }
+  D.vx[t] = vx;
+  D.vy[t] = vy;
+  move_particle(D, M, t, k >= ns, vx0, vy0, vx, vy);
+}
+
+}  // namespace
+
+void launch_pprep(Ctx& c) {
+  const int b = c.block_for(c.d.NT, 128);
+  k_pprep<<<(c.d.NT + b - 1) / b, b, 0, c.stream>>>(c.d);
+}
+
+// Lanes a target: split by component while one lane a target leaves most of the chip's 608
+// FP64 pipes with a warp or less
+void launch_pstage(Ctx& c, int stage) {
+  const Dev& D = c.d;
+  const int ns = D.NT - D.NN;
+  const bool split = D.NT <= c.split_max;
+  const int ls = split ? 2 : 1, ln = split ? 4 : 1;
+  const int b = c.block_for(ns * ls + D.NN * ln, std::min(c.blk[TK_DERIVS], 128));
+  const int nbs = (ns * ls + b - 1) / b, nbn = (D.NN * ln + b - 1) / b;
+  if (split) k_pstage<2, 4><<<nbs + nbn, b, 0, c.stream>>>(D, stage, nbs);
+  else k_pstage<1, 1><<<nbs + nbn, b, 0, c.stream>>>(D, stage, nbs);
+}
+
+void launch_pfinish(Ctx& c) {
+  const int b = c.block_for(c.d.N2, 128);
+  k_pfinish<<<(c.d.N2 + b - 1) / b, b, 0, c.stream>>>(c.d);
+}
+
+}  // namespace sps

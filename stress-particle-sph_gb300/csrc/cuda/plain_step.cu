@@ -137,32 +137,6 @@ __global__ void k_step_init(Dev D) {
   }
 }
 
-// boundary_forces, test == 2 (2_SPH_main_2018.f90:1117-1161): FP32 locals.  Only innermost
-// dummies closer than 0.75 dx give a non-zero term; they are summed in ascending id.
-__device__ __forceinline__ bool bound_term(const Dev& D, const Real& M, int i, int j, float& fx,
-                                           float& fy) {
-  const float cc = 20.0f;
-  const float d0 = (float)(M.dx / 2.0);
-  float r0 = (float)(D.px[i] - D.px[j]);
-  float r1 = (float)(D.py[i] - D.py[j]);
-  float r2 = sqrtf(r0 * r0 + r1 * r1);
-  float h = (float)(0.5 * (D.hsml[i] + D.hsml[j]));
-  float r_bound = r2 / (0.75f * h);
-  float f2;
-  if (r2 > 0 && r2 < 1.5f * d0) f2 = 1.0f - (r2 / (1.5f * d0));
-  else f2 = 0.0f;
-  float f;
-  if (0 < r_bound && r_bound <= 2.0f / 3.0f) f = 2.0f / 3.0f;
-  else if (2.0f / 3.0f < r_bound && r_bound <= 1) f = 2.0f * r_bound - 1.5f * (r_bound * r_bound);
-  else if (1 < r_bound && r_bound < 2) f = 0.5f * ((2.0f - r_bound) * (2.0f - r_bound));
-  else f = 0.0f;
-  if (f2 == 0.0f || f == 0.0f) return false;
-  float k = ((0.01f * (cc * cc)) * f2) * f;
-  fx = k * (r0 / (r2 * r2));
-  fy = k * (r1 / (r2 * r2));
-  return true;
-}
-
 // boundary_forces (2_SPH_main_2018.f90:1039-1165), test 2: the wall force on every node
 // from the innermost dummy row, once per step (positions are frozen within a step)
 __global__ void k_bound(Dev D) {
@@ -429,6 +403,11 @@ __global__ void k_vol(Dev D, int lo, int hi) {
   double r = D.rho[i];
   D.vol[i] = D.mass[i] / r;
   D.rinv[i] = 1.0 / r;
+  if (D.rho2) {
+    const double r2 = r * r;
+    D.rho2[i] = r2;
+    D.rinv2[i] = 1.0 / r2;
+  }
   if (D.fast) {
     D.recV[i] = split2(D.vx[i], D.vy[i]);
     D.recI[i] = make_float4(i < D.NT ? (float)D.iv1[i] : 0.0f, (float)D.vol[i], (float)r,
@@ -946,27 +925,12 @@ void launch_pderivs(Ctx& c, int stage) {
   k_derivs<2><<<(D.NN + b - 1) / b, b, 0, c.stream>>>(D, stage, D.tgtN, D.NN);
 }
 
-int launch_plain_step(Ctx& c) {
+// RK4, the final interpolation and the position update as separate kernels
+void launch_stages(Ctx& c) {
   Dev& D = c.d;
   cudaStream_t st = c.stream;
   int nbT = (D.NT + kBlock - 1) / kBlock;
   int nbN = (D.NN + kBlock - 1) / kBlock;
-  c.mark("load_scalars");
-  k_load_scalars<<<1, 128, 0, st>>>(D);
-  launch_pair_build(c);
-  if (c.step_variant & 1) {
-    // the outside approach re-interpolates after a shift: stress_point_update and
-    // adapt_stress2 (2_SPH_main_2018.f90:99-108)
-    c.mark("interp");
-    if (D.fast) launch_finterp(c);
-    else launch_pinterp(c);
-    if (D.cont_density) {
-      c.mark("node_rho");
-      k_node_rho<<<nbN, kBlock, 0, st>>>(D);
-    }
-    c.mark("adapt_bc");
-    k_adapt_bc<<<c.grid_of(TK_ADAPT, D.NT), c.blk[TK_ADAPT], 0, st>>>(D, 0, 0);
-  }
   c.mark("step_init");
   k_step_init<<<(D.N2 + kBlock - 1) / kBlock, kBlock, 0, st>>>(D);
   if (D.inside) {
@@ -1018,6 +982,44 @@ int launch_plain_step(Ctx& c) {
     c.mark("trapezoid");
     k_trapezoid<<<nbT, kBlock, 0, st>>>(D);
   }
+}
+
+int launch_plain_step(Ctx& c) {
+  Dev& D = c.d;
+  cudaStream_t st = c.stream;
+  int nbN = (D.NN + kBlock - 1) / kBlock;
+  c.mark("load_scalars");
+  k_load_scalars<<<1, 128, 0, st>>>(D);
+  launch_pair_build(c);
+  if (c.step_variant & 1) {
+    // the outside approach re-interpolates after a shift: stress_point_update and
+    // adapt_stress2 (2_SPH_main_2018.f90:99-108)
+    c.mark("interp");
+    if (D.fast) launch_finterp(c);
+    else launch_pinterp(c);
+    if (D.cont_density) {
+      c.mark("node_rho");
+      k_node_rho<<<nbN, kBlock, 0, st>>>(D);
+    }
+    c.mark("adapt_bc");
+    k_adapt_bc<<<c.grid_of(TK_ADAPT, D.NT), c.blk[TK_ADAPT], 0, st>>>(D, 0, 0);
+  }
+  if (c.fused()) {
+    c.mark("prep");
+    launch_pprep(c);
+    for (int stage = 0; stage < 4; stage++) {
+      c.mark("stage");
+      launch_pstage(c, stage);
+    }
+    c.mark("finish");
+    launch_pfinish(c);
+    if (D.update_x && D.xsph) {
+      c.mark("xsph");
+      k_xsph<<<c.grid_of(TK_XSPH, D.N2), c.blk[TK_XSPH], 0, st>>>(D);
+    }
+  } else {
+    launch_stages(c);
+  }
   // get_nodes_on_free_surface after the position update (2_SPH_main_2018.f90:153); on
   // demand instead when no later step reads it (Ctx::surf_every)
   if (D.update_x && c.surf_every) launch_surface(c);
@@ -1025,8 +1027,10 @@ int launch_plain_step(Ctx& c) {
     c.mark("shift");
     k_shift<<<nbN, kBlock, 0, st>>>(D, (c.step_variant & 2) ? 1 : 0);
   }
-  c.mark("displ");
-  k_displ<<<nbN, kBlock, 0, st>>>(D);
+  if (!c.fused() || (D.update_x && D.xsph)) {  // k_pfinish forms it otherwise
+    c.mark("displ");
+    k_displ<<<nbN, kBlock, 0, st>>>(D);
+  }
   c.mark("next_step");
   k_next_step<<<1, 1, 0, st>>>(D);
   return 0;

@@ -723,6 +723,22 @@ int sps_create_batch(int32_t nreal, const sps_params* ps, sps_ctx** out) {
     D.tflag = dalloc<int32_t>(c, 2 * N2);
     D.toff = dalloc<int32_t>(c, 2 * N2 + 2);
     D.lcol = dalloc<int32_t>(c, N2);
+    D.colid = dalloc<int32_t>(c, NT);
+    if (c.fused()) {
+      const size_t ns = NT - NN_;
+      D.norm = dalloc<double>(c, NT);
+      D.rnorm = dalloc<double>(c, NT);
+      D.AE = p->cspm ? dalloc<double>(c, 5 * NT) : nullptr;
+      D.st0c = dalloc<double>(c, 4 * ns);
+      D.rkc = dalloc<double>(c, 4 * ns);
+      for (int k = 0; k < 2; k++) {
+        D.pv[k] = dalloc<double>(c, 2 * NN_);
+        D.ps[k] = dalloc<double>(c, 4 * ns);
+        D.pa[k] = dalloc<double>(c, 4 * ns);
+      }
+      D.rho2 = dalloc<double>(c, N2);
+      D.rinv2 = dalloc<double>(c, N2);
+    }
     if (D.fast) {
       D.recV = dalloc<float4>(c, N2);
       D.recS = dalloc<float4>(c, NT);
@@ -997,6 +1013,10 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
         D.same = dalloc<int4>(c, (size_t)D.N2 * rows);
         D.crossW = c.precision == SPS_PREC_FP32_FAST ? dalloc<int2>(c, (size_t)D.N2 * rows)
                                                      : nullptr;
+        if (c.fused()) {
+          D.hW = dalloc<double>(c, (size_t)D.NT * (size_t)capn);
+          D.hG = dalloc<double2>(c, (size_t)(D.NT - D.NN) * (size_t)capn);
+        }
         D.keyC = dalloc<int32_t>(c, (size_t)D.N2 * (size_t)capn);
         D.keyS = dalloc<int32_t>(c, (size_t)D.N2 * (size_t)capn);
         D.capH = D.capC = D.capS = capn;
@@ -1723,8 +1743,10 @@ int sps_autotune(sps_ctx* h, int32_t nsteps, int32_t* blocks) {
       copy(false);
       for (int k = 0; k < sps::TK_N; k++)
         for (size_t q = 0; q < kn.size(); q++)
-          // the FP32 form's direct list gather takes the pair search's block size
-          if ((kn[q] == sps::kTunedNames[k] || (k == sps::TK_HALF && kn[q] == "gather")) &&
+          // the FP32 form's direct list gather takes the pair search's block size, the
+          // one-launch stages the derivative sums'
+          if ((kn[q] == sps::kTunedNames[k] || (k == sps::TK_HALF && kn[q] == "gather") ||
+               (k == sps::TK_DERIVS && kn[q] == "stage")) &&
               kms[q] < best_ms[k]) {
             best_ms[k] = kms[q];
             best[k] = c.blk[k];

@@ -88,6 +88,50 @@ __device__ __forceinline__ void tail_sp_grad(const Dev& D, int t, double* g, con
     gu[3] = g[3];
 }
 
+// stress-point rates of the plain form from the gradient g and the stage stress st: D : grad(v),
+// plastic_terms / drucker_prager (updates f_drucker), Jaumann spin; rhs(4) and the plastic
+// strain rate
+__device__ __forceinline__ void sp_rates_f64(const Dev& D, const Real& M, const StepScalars& sc,
+                                             int t, const double* g, const double* st,
+                                             double* rhs, double& der) {
+  const double g11 = g[0], g21 = g[1], g12 = g[2], g22 = g[3];
+  double div1[4];
+  div1[0] = -(M.D11 * g11 + M.D12 * g22);
+  div1[1] = -(M.D12 * g11 + M.D22 * g22);
+  div1[2] = -(M.D33 * g21 + M.D33 * g12);
+  div1[3] = -(M.D41 * g11 + M.D42 * g22);
+  // plastic_terms (3_SPH_material_2018.f90:1884-1954)
+  double Gs[4] = {0.0, 0.0, 0.0, 0.0};
+  der = 0.0;
+  if (M.ntype_eco > 1) {
+    double s2v[4] = {st[0], st[1], st[2], st[3]};
+    if (M.ntype_solid == 1) s2v[3] = M.poiss * (s2v[0] + s2v[1]);
+    double vivel[4] = {0.0, 0.0, 0.0, 0.0}, G2[4];
+    if (M.ncrit <= 4) {
+      viscoplastic(M, s2v, D.iv1[t], vivel, Gs);
+    } else if (M.ncrit == 12) {
+      double f = D.fdp[t];
+      drucker_prager(M, sc.time_sph, s2v, g, &f, G2, vivel);
+      D.fdp[t] = f;
+      for (int k = 0; k < 4; k++) Gs[k] = -G2[k];
+      if (D.cap_buf && (G2[0] != 0.0 || G2[1] != 0.0 || G2[2] != 0.0 || G2[3] != 0.0))
+        capture_tuple(D, t, s2v, g, Gs);
+    }
+    der = sqrt((2.0 * ((vivel[0] * vivel[0] + vivel[1] * vivel[1]) + vivel[3] * vivel[3]) +
+                vivel[2] * vivel[2]) /
+               3.0);
+  }
+  double spin[4] = {0.0, 0.0, 0.0, 0.0};
+  if (D.update_x) {
+    double om1 = 0.5 * (g12 - g21);
+    double om2 = -0.5 * (g12 - g21);
+    spin[0] = 2.0 * om1 * st[2];
+    spin[1] = 2.0 * om2 * st[2];
+    spin[2] = om2 * st[0] + om1 * st[1];
+  }
+  for (int k = 0; k < 4; k++) rhs[k] = (-div1[k] + spin[k]) + Gs[k];
+}
+
 // stress-point rates after the gradient: D : grad(v), plastic_terms / drucker_prager,
 // Jaumann spin, RHS and RK4 accumulation.  Gs_net (may be null): a plastic source from the
 // learned surrogate that replaces the exact one (with its plastic strain rate der_net)
@@ -102,38 +146,38 @@ __device__ __forceinline__ void tail_sp_rates(const Dev& D, const StepScalars& s
                                               double der_net = 0.0,
                                               const double* dp = nullptr) {
     const Real& M = real_of(D, t);
-    const double g11 = g[0], g21 = g[1], g12 = g[2], g22 = g[3];
-    double div1[4];
-    if (!FAST) {
-      div1[0] = -(M.D11 * g11 + M.D12 * g22);
-      div1[1] = -(M.D12 * g11 + M.D22 * g22);
-      div1[2] = -(M.D33 * g21 + M.D33 * g12);
-      div1[3] = -(M.D41 * g11 + M.D42 * g22);
-    }
-    // plastic_terms (3_SPH_material_2018.f90:1884-1954)
     double st[4] = {D.s0[t], D.s1[t], D.s2[t], D.s3[t]};
-    double Gs[4] = {0.0, 0.0, 0.0, 0.0}, der = 0.0;
-    if (M.ntype_eco > 1) {
-      double s2v[4] = {st[0], st[1], st[2], st[3]};
-      if (M.ntype_solid == 1) s2v[3] = M.poiss * (s2v[0] + s2v[1]);
-      double vivel[4] = {0.0, 0.0, 0.0, 0.0}, G2[4];
-      if (M.ncrit <= 4) {
-        viscoplastic(M, s2v, D.iv1[t], vivel, Gs);
-      } else if (M.ncrit == 12) {
-        double f;
-        if (dp) {
-          for (int k = 0; k < 4; k++) {
-            G2[k] = dp[k];
-            vivel[k] = dp[4 + k];
+    double der = 0.0;
+    if (!FAST) {
+      double rhs[4];
+      sp_rates_f64(D, M, sc, t, g, st, rhs, der);
+      for (int k = 0; k < 4; k++) {
+        D.RHS1[k][t] = rhs[k];
+        D.RKs[k][t] = D.RKs[k][t] + f2 * rhs[k];
+      }
+    } else {
+      const double g11 = g[0], g21 = g[1], g12 = g[2], g22 = g[3];
+      // plastic_terms (3_SPH_material_2018.f90:1884-1954)
+      double Gs[4] = {0.0, 0.0, 0.0, 0.0};
+      if (M.ntype_eco > 1) {
+        double s2v[4] = {st[0], st[1], st[2], st[3]};
+        if (M.ntype_solid == 1) s2v[3] = M.poiss * (s2v[0] + s2v[1]);
+        double vivel[4] = {0.0, 0.0, 0.0, 0.0}, G2[4];
+        if (M.ncrit <= 4) {
+          viscoplastic(M, s2v, D.iv1[t], vivel, Gs);
+        } else if (M.ncrit == 12) {
+          double f;
+          if (dp) {
+            for (int k = 0; k < 4; k++) {
+              G2[k] = dp[k];
+              vivel[k] = dp[4 + k];
+            }
+            f = dp[8];
+          } else {
+            f = D.fdp[t];
+            drucker_prager_f32(M, sc.time_sph, s2v, g, &f, G2, vivel);
           }
-          f = dp[8];
-        } else {
-          f = D.fdp[t];
-          if (FAST) drucker_prager_f32(M, sc.time_sph, s2v, g, &f, G2, vivel);
-          else drucker_prager(M, sc.time_sph, s2v, g, &f, G2, vivel);
-        }
-        D.fdp[t] = f;
-        if (FAST) {
+          D.fdp[t] = f;
           // negation and the non-zero test on the integer pipe (sign bit; magnitude bits)
           bool nz = false;
           for (int k = 0; k < 4; k++) {
@@ -142,29 +186,17 @@ __device__ __forceinline__ void tail_sp_rates(const Dev& D, const StepScalars& s
             nz = nz || (b << 1) != 0;
           }
           if (D.cap_buf && nz) capture_tuple(D, t, s2v, g, Gs);
-        } else {
-          for (int k = 0; k < 4; k++) Gs[k] = -G2[k];
-          if (D.cap_buf && (G2[0] != 0.0 || G2[1] != 0.0 || G2[2] != 0.0 || G2[3] != 0.0))
-            capture_tuple(D, t, s2v, g, Gs);
         }
-      }
-      if (FAST) {
         float v0 = f32_rn(vivel[0]), v1 = f32_rn(vivel[1]), v2 = f32_rn(vivel[2]),
               v3 = f32_rn(vivel[3]);
         // explicit fmaf: the same rounding in every kernel that inlines this tail
         float q = fmaf(2.0f, fmaf(v0, v0, fmaf(v1, v1, __fmul_rn(v3, v3))), __fmul_rn(v2, v2));
         der = f64_of(sqrtf(__fmul_rn(q, 1.0f / 3.0f)));
-      } else {
-        der = sqrt((2.0 * ((vivel[0] * vivel[0] + vivel[1] * vivel[1]) + vivel[3] * vivel[3]) +
-                    vivel[2] * vivel[2]) /
-                   3.0);
       }
-    }
-    if (Gs_net) {
-      for (int k = 0; k < 4; k++) Gs[k] = Gs_net[k];
-      der = der_net;
-    }
-    if (FAST) {
+      if (Gs_net) {
+        for (int k = 0; k < 4; k++) Gs[k] = Gs_net[k];
+        der = der_net;
+      }
       // the FP32 form: the elastic rate, the spin and the right-hand side in FP32 (the
       // gradient comes from FP32 neighbour sums and carries their accuracy), conversions on
       // the integer pipe; only the RK accumulation stays FP64
@@ -185,20 +217,6 @@ __device__ __forceinline__ void tail_sp_rates(const Dev& D, const StepScalars& s
         const double rhs = f64_of(r[k] + f32_rn(Gs[k]));
         D.RHS1[k][t] = rhs;
         D.RKs[k][t] = fma(f2, rhs, D.RKs[k][t]);
-      }
-    } else {
-      double spin[4] = {0.0, 0.0, 0.0, 0.0};
-      if (D.update_x) {
-        double om1 = 0.5 * (g12 - g21);
-        double om2 = -0.5 * (g12 - g21);
-        spin[0] = 2.0 * om1 * st[2];
-        spin[1] = 2.0 * om2 * st[2];
-        spin[2] = om2 * st[0] + om1 * st[1];
-      }
-      for (int k = 0; k < 4; k++) {
-        double rhs = (-div1[k] + spin[k]) + Gs[k];
-        D.RHS1[k][t] = rhs;
-        D.RKs[k][t] = D.RKs[k][t] + f2 * rhs;
       }
     }
     D.RKd[t] = D.RKd[t] + der * f2;
@@ -244,6 +262,22 @@ __device__ __forceinline__ void art_force_node(const Dev& D, int col, int t, dou
   *afy = T[2][0] + T[1][1];
 }
 
+// node right-hand side from the (CSPM-corrected) sums g2 = grad2(s,b) at s + 3b: divergence,
+// gravity with damping, artificial viscosity, wall and artificial force
+__device__ __forceinline__ void node_rhs_f64(const Dev& D, const Real& M, const StepScalars& sc,
+                                             int t, const double* g2, double vtx, double vty,
+                                             double avx, double avy, double afx, double afy,
+                                             double& rhsx, double& rhsy) {
+  double div2x = -(g2[0] + g2[2 + 3]);
+  double div2y = -(g2[2] + g2[1 + 3]);
+  double gx = (M.ic_grav == 1) ? sc.factg * M.cgrav[0] : 0.0;
+  double gy = (M.ic_grav == 1) ? sc.factg * M.cgrav[1] : 0.0;
+  gx = gx - M.damping * vtx;
+  gy = gy - M.damping * vty;
+  rhsx = (((-div2x + gx) + avx) + D.fbx[t]) + afx;
+  rhsy = (((-div2y + gy) + avy) + D.fby[t]) + afy;
+}
+
 // node tail: g2 = grad2(s,b) at s + 3b, AE = CSPM moments, av = artificial viscosity,
 // af = artificial force
 __device__ __forceinline__ void tail_node(const Dev& D, const StepScalars& sc, int t, double* g2,
@@ -267,20 +301,65 @@ __device__ __forceinline__ void tail_node(const Dev& D, const StepScalars& sc, i
       g2[d + 3] = A4 * (A2 * g2[d] + A3 * g2[d + 3]);
     }
   }
-  const Real& M = real_of(D, t);
-  double div2x = -(g2[0] + g2[2 + 3]);
-  double div2y = -(g2[2] + g2[1 + 3]);
-  const double vtx = D.vx[t], vty = D.vy[t];
-  double gx = (M.ic_grav == 1) ? sc.factg * M.cgrav[0] : 0.0;
-  double gy = (M.ic_grav == 1) ? sc.factg * M.cgrav[1] : 0.0;
-  gx = gx - M.damping * vtx;
-  gy = gy - M.damping * vty;
-  double rhsx = (((-div2x + gx) + avx) + D.fbx[t]) + afx;
-  double rhsy = (((-div2y + gy) + avy) + D.fby[t]) + afy;
+  double rhsx, rhsy;
+  node_rhs_f64(D, real_of(D, t), sc, t, g2, D.vx[t], D.vy[t], avx, avy, afx, afy, rhsx, rhsy);
   D.RHS2[0][t] = rhsx;
   D.RHS2[1][t] = rhsy;
   D.RKv[0][t] = D.RKv[0][t] + f2 * rhsx;
   D.RKv[1][t] = D.RKv[1][t] + f2 * rhsy;
+}
+
+// boundary_forces, test == 2 (2_SPH_main_2018.f90:1117-1161): FP32 locals.  Only innermost
+// dummies closer than 0.75 dx give a non-zero term; they are summed in ascending id.
+__device__ __forceinline__ bool bound_term(const Dev& D, const Real& M, int i, int j, float& fx,
+                                           float& fy) {
+  const float cc = 20.0f;
+  const float d0 = (float)(M.dx / 2.0);
+  float r0 = (float)(D.px[i] - D.px[j]);
+  float r1 = (float)(D.py[i] - D.py[j]);
+  float r2 = sqrtf(r0 * r0 + r1 * r1);
+  float h = (float)(0.5 * (D.hsml[i] + D.hsml[j]));
+  float r_bound = r2 / (0.75f * h);
+  float f2;
+  if (r2 > 0 && r2 < 1.5f * d0) f2 = 1.0f - (r2 / (1.5f * d0));
+  else f2 = 0.0f;
+  float f;
+  if (0 < r_bound && r_bound <= 2.0f / 3.0f) f = 2.0f / 3.0f;
+  else if (2.0f / 3.0f < r_bound && r_bound <= 1) f = 2.0f * r_bound - 1.5f * (r_bound * r_bound);
+  else if (1 < r_bound && r_bound < 2) f = 0.5f * ((2.0f - r_bound) * (2.0f - r_bound));
+  else f = 0.0f;
+  if (f2 == 0.0f || f == 0.0f) return false;
+  float k = ((0.01f * (cc * cc)) * f2) * f;
+  fx = k * (r0 / (r2 * r2));
+  fy = k * (r1 / (r2 * r2));
+  return true;
+}
+
+// The end of a step for particle t: its place in the step's pair build kept in x0x, x0y, then
+// the position update without XSPH (2_SPH_main_2018.f90:145-146): x = x0 + vel_half dt with
+// vel_half = 0.5 (v0 + v) rounded to FP32, and a node's displacement (:166-180).  With XSPH
+// both follow in their own kernels.  Explicit roundings: the same in every unit.
+__device__ __forceinline__ void move_particle(const Dev& D, const Real& M, int t, bool node,
+                                              double vx0, double vy0, double vx, double vy) {
+  double x = D.px[t], y = D.py[t];
+  D.x0x[t] = x;
+  D.x0y[t] = y;
+  if (D.update_x) {
+    if (D.xsph) return;
+    // the conversions on the integer pipe (the same bits as the hardware's)
+    const float hx = f32_rn(0.5 * __dadd_rn(vx0, vx)), hy = f32_rn(0.5 * __dadd_rn(vy0, vy));
+    x = __dadd_rn(x, __dmul_rn(f64_of(hx), M.dt));
+    y = __dadd_rn(y, __dmul_rn(f64_of(hy), M.dt));
+    D.px[t] = x;
+    D.py[t] = y;
+    if (node) {
+      D.dispx[t] = __dsub_rn(x, D.x00x[t]);
+      D.dispy[t] = __dsub_rn(y, D.x00y[t]);
+    }
+  } else if (node) {
+    D.dispx[t] = __dadd_rn(D.dispx[t], __dmul_rn(0.5 * __dadd_rn(vx0, vx), M.dt));
+    D.dispy[t] = __dadd_rn(D.dispy[t], __dmul_rn(0.5 * __dadd_rn(vy0, vy), M.dt));
+  }
 }
 
 }  // namespace sps

@@ -27,6 +27,7 @@ CUDA_UNITS = [
     ("cuda/sps_api.cu", []),
     ("cuda/neighbours.cu", ["-fmad=false"]),
     ("cuda/plain_step.cu", ["-fmad=false"]),
+    ("cuda/plain_fused.cu", ["-fmad=false"]),
     ("cuda/fast_step.cu", []),
     ("cuda/surface.cu", ["-fmad=false"]),
     ("cuda/mlp_train.cu", []),
