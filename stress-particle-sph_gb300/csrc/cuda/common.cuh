@@ -244,10 +244,20 @@ struct Dev {
   double* hW;
   double2* hG;
   double *norm, *rnorm, *AE, *st0c, *rkc;
+  double* stc;  // FP32 form: a stress-point's stress of the stage (4 doubles a column)
   // the values a stage reads from its neighbours, double buffered over the stages: node
   // velocity (2 a node), stress-point stress (4) and {stress / rho^2 (3), mass}
   double *pv[2], *ps[2], *pa[2];
-  double *rho2, *rinv2;  // rho * rho and its reciprocal, per particle
+  double *rho2, *rinv2;  // rho * rho and its reciprocal, per particle (plain form)
+  // FP32 form: the second buffers of the neighbour records recV, recS, recA, recAl; the
+  // list constants hGf (k * NT + col): a stress-point's {Gx m/rho, Gy m/rho}, a node's {-m
+  // Gx, -m Gy}; hB (k * ns + col): 1 - beta of a stress-point's wall entries; {norm, 1/norm}
+  // and the node's sums of m dW (hi, lo of x and y) per column
+  float4 *recV1, *recS1, *recA1, *recAl1;
+  float2* hGf;
+  double* hB;
+  float2* normf;
+  float4* msum;
   // get_nodes_on_free_surface: normal (module FP64), subset (1 surface, 2 inside), f_int
   double *nrmx, *nrmy;
   int8_t* subset;
@@ -615,7 +625,7 @@ static __device__ __noinline__ void adapt_stress_fast_return(double alpha2, doub
 __device__ __forceinline__ void adapt_stress_fast(double alpha2, double kc, double shift,
                                                   double& a, double& b, double& c, double& d) {
   const double third = 1.0 / 3.0;
-  const double smean = ((a + b) + d) * third;
+  const double smean = __dmul_rn((a + b) + d, third);  // never fused into the differences
   const double d0 = a - smean, d1 = b - smean, d2 = c, d3 = d - smean;
   const double varj2 = fma(d2, d2, 0.5 * fma(d0, d0, fma(d1, d1, d3 * d3)));
   const double yield = fma(-3.0 * alpha2, smean, kc);
@@ -626,7 +636,7 @@ static __device__ __noinline__ void adapt_stress_fast_return(double alpha2, doub
                                                              double shift, double& a,
                                                              double& b, double& c, double& d) {
   const double third = 1.0 / 3.0;
-  double smean = ((a + b) + d) * third;
+  double smean = __dmul_rn((a + b) + d, third);
   double d0 = a - smean, d1 = b - smean, d2 = c, d3 = d - smean;
   double varj2 = fma(d2, d2, 0.5 * fma(d0, d0, fma(d1, d1, d3 * d3)));
   double yield = fma(-3.0 * alpha2, smean, kc);
@@ -634,7 +644,7 @@ static __device__ __noinline__ void adapt_stress_fast_return(double alpha2, doub
     a = (a - smean) + shift;
     b = (b - smean) + shift;
     d = (d - smean) + shift;
-    smean = ((a + b) + d) * third;
+    smean = __dmul_rn((a + b) + d, third);
     d0 = a - smean;
     d1 = b - smean;
     d2 = c;
@@ -825,9 +835,10 @@ __device__ __forceinline__ float two_sum_f(float a, float b, float& e) {
 // drucker_prager: the updated f, the plastic source G and vivel.
 // the body, with its outputs as the FP32 values they are (G, vivel); returns whether the
 // point is loading (G non-zero)
-__device__ __forceinline__ bool drucker_prager_f32v(const Real& M, double time_sph,
-                                                    const double* s, const double* gu,
-                                                    double* fdp, float* G, float* vivel) {
+__device__ __forceinline__ bool drucker_prager_f32g(const Real& M, double time_sph,
+                                                    const double* s, float g11, float g21,
+                                                    float g12, float g22, double* fdp, float* G,
+                                                    float* vivel) {
   const double f0 = *fdp;
   float s0h, s0l, s1h, s1l, s3h, s3l;
   f32_split(s[0], s0h, s0l);
@@ -846,9 +857,9 @@ __device__ __forceinline__ bool drucker_prager_f32v(const Real& M, double time_s
   const float dv2 = f32_rn(s[2]);
   const float varj2 = fmaf(dv2, dv2, 0.5f * fmaf(dv0, dv0, fmaf(dv1, dv1, dv3 * dv3)));
   const float vari1 = 3.0f * smean;
-  const float eps11 = f32_rn(gu[0]);
-  const float eps12 = 0.5f * (f32_rn(gu[2]) + f32_rn(gu[1]));
-  const float eps22 = f32_rn(gu[3]);
+  const float eps11 = g11;
+  const float eps12 = 0.5f * (g12 + g21);
+  const float eps22 = g22;
   const float emean = eps11 + eps22;
   const float alpha2 = M.dpf_alpha2, kc = M.dpf_kc;
   const float yield = kc - alpha2 * vari1;
@@ -876,6 +887,14 @@ __device__ __forceinline__ bool drucker_prager_f32v(const Real& M, double time_s
   G[0] = G[1] = G[2] = G[3] = 0.0f;
   vivel[0] = vivel[1] = vivel[2] = vivel[3] = 0.0f;
   return false;
+}
+
+// the same from the FP64 gradient
+__device__ __forceinline__ bool drucker_prager_f32v(const Real& M, double time_sph,
+                                                    const double* s, const double* gu,
+                                                    double* fdp, float* G, float* vivel) {
+  return drucker_prager_f32g(M, time_sph, s, f32_rn(gu[0]), f32_rn(gu[1]), f32_rn(gu[2]),
+                             f32_rn(gu[3]), fdp, G, vivel);
 }
 
 // the same with FP64 outputs (exact conversions of the FP32 values)
@@ -926,9 +945,13 @@ void launch_vol(Ctx& c, int lo, int hi);
 void launch_pprep(Ctx& c);
 void launch_pstage(Ctx& c, int stage);
 void launch_pfinish(Ctx& c);
+void launch_fprep(Ctx& c);
+void launch_fstage(Ctx& c, int stage);
+void launch_ffinish(Ctx& c);
 void launch_finterp(Ctx& c);
 void launch_fderivs(Ctx& c, int stage);
 void launch_fsp_tail(Ctx& c, int stage);
+void launch_fsp_cand(Ctx& c, int stage, bool by_col);
 void launch_surface(Ctx& c);
 void launch_surface_f32(Ctx& c);
 void launch_lists_keys(Ctx& c);

@@ -94,8 +94,7 @@ struct Ctx {
   // and nothing between the two halves of a stage needs the whole field (the continuity
   // equation's densities, artificial stress, the traction-free BC's normals do)
   bool fused() const {
-    return precision == SPS_PREC_FP64_PLAIN && d.sp_sph && !d.cont_density && !d.art_stress &&
-           !(d.no_bcs > 0 && d.ifsigman == 1);
+    return d.sp_sph && !d.cont_density && !d.art_stress && !(d.no_bcs > 0 && d.ifsigman == 1);
   }
   // the block size for n threads: at most `most`, halved while fewer than two blocks an SM
   // would leave SMs idle

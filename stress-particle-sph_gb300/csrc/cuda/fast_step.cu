@@ -22,43 +22,11 @@
 #include <string>
 
 #include "ctx.cuh"
-#include "stage_tail.cuh"
+#include "fast_sums.cuh"
 
 namespace sps {
 
 namespace {
-
-struct Kahan {
-  float s = 0.0f, c = 0.0f;
-  __device__ __forceinline__ void add(float x) {
-    float y = x - c;
-    float t = s + y;
-    c = (t - s) - y;
-    s = t;
-  }
-  __device__ __forceinline__ double val() const { return (double)s - (double)c; }
-  // the compensated sum rounded to FP32
-  __device__ __forceinline__ float fval() const { return s - c; }
-};
-
-// sum of exact FP32 products: p = RN(a b) and e = a b - p (exact, by one FMA: the
-// error-free product transformation of Ogita, Rump and Oishi, "Accurate sum and dot
-// product", SIAM J. Sci. Comput. 26(6), 2005); p is Kahan-summed, e summed plainly
-struct ProdSum {
-  Kahan hi;
-  float lo = 0.0f;
-  __device__ __forceinline__ void add(float a, float b) {
-    float p = a * b;
-    float e = fmaf(a, b, -p);
-    hi.add(p);
-    lo += e;
-  }
-};
-
-// difference of two double-float values (hi + lo) in FP32
-__device__ __forceinline__ float dfdiff(float ah, float al, float bh, float bl) {
-  return (ah - bh) + (al - bl);
-}
 
 // The node tail of get_derivatives / RK4 (tail_node without CSPM) in FP32: the divergence,
 // gravity with damping and the right-hand side carry the FP32 accuracy of the sums they
@@ -93,73 +61,6 @@ __device__ __forceinline__ void tail_node_f32(const Dev& D, const StepScalars& s
   D.RKv[0][t] = fma(f2, rx, D.RKv[0][t]);
   D.RKv[1][t] = fma(f2, ry, D.RKv[1][t]);
 }
-
-// Walks entries 0 .. deg of list column col, KP entries a pass, software-pipelined: the
-// next pass's entries are loaded while the current pass's records are gathered and summed,
-// so that the entry loads (streamed from DRAM) overlap the record gathers (mostly L2 hits)
-// instead of adding their latency to them.  load(e) returns the records of entry e (called
-// only for entries below deg), sum(e, rec) adds one term; terms are added in list order,
-// so the result does not depend on KP.
-template <int KP, typename Rec, typename Load, typename Sum>
-__device__ __forceinline__ void walk_list(const int4* __restrict__ list, int col, int N2,
-                                          int deg, Load&& load, Sum&& sum) {
-  int4 nxt[KP];
-#pragma unroll
-  for (int q = 0; q < KP; q++)
-    nxt[q] = q < deg ? list[ell(q, col, N2)] : make_int4(0, 0, 0, 0);
-  for (int k = 0; k < deg; k += KP) {
-    int4 cur[KP];
-    Rec rec[KP] = {};
-#pragma unroll
-    for (int q = 0; q < KP; q++) {
-      cur[q] = nxt[q];
-      if (k + q < deg) rec[q] = load(cur[q]);
-    }
-#pragma unroll
-    for (int q = 0; q < KP; q++)
-      nxt[q] = k + KP + q < deg ? list[ell(k + KP + q, col, N2)] : make_int4(0, 0, 0, 0);
-#pragma unroll
-    for (int q = 0; q < KP; q++)
-      if (k + q < deg) sum(cur[q], rec[q]);
-  }
-}
-
-// the same walk over the compact {id, W} entries (crossW: entry k of column col at
-// k * N2 + col)
-template <int KP, typename Rec, typename Load, typename Sum>
-__device__ __forceinline__ void walk_compact(const int2* __restrict__ list, int col, int N2,
-                                             int deg, Load&& load, Sum&& sum) {
-  int2 nxt[KP];
-#pragma unroll
-  for (int q = 0; q < KP; q++) nxt[q] = q < deg ? list[(size_t)q * N2 + col] : make_int2(0, 0);
-  for (int k = 0; k < deg; k += KP) {
-    int2 cur[KP];
-    Rec rec[KP] = {};
-#pragma unroll
-    for (int q = 0; q < KP; q++) {
-      cur[q] = nxt[q];
-      if (k + q < deg) rec[q] = load(cur[q]);
-    }
-#pragma unroll
-    for (int q = 0; q < KP; q++)
-      nxt[q] = k + KP + q < deg ? list[(size_t)(k + KP + q) * N2 + col] : make_int2(0, 0);
-#pragma unroll
-    for (int q = 0; q < KP; q++)
-      if (k + q < deg) sum(cur[q], rec[q]);
-  }
-}
-
-// records of one neighbour, as the four sums read them
-struct RecVI {  // velocity (hi, lo) and m / rho
-  float4 v;
-  float vol;
-};
-struct RecSI {  // stress and {intvar1, m / rho, rho, m}
-  float4 s, i;
-};
-struct RecA {  // sigma / rho^2 (hi with m, lo)
-  float4 a, l;
-};
 
 // stress_point_update (2_SPH_main_2018.f90:403-482), FP32 sums.  A stress-point's velocity
 // is the weighted mean of its nodes' velocities; it is formed as the first node's velocity
@@ -505,143 +406,41 @@ __global__ void __launch_bounds__(256, KIND == 1 ? 4 : 3) k_fderivs(Dev D, int s
 // copies); FP64 only for the state's RK accumulation.
 __device__ __forceinline__ void tail_sp_f32(const Dev& D, const StepScalars& sc, int t,
                                             double f2) {
-  const Real& M = real_of(D, t);
   const double* gu = D.grad_u + 4 * (size_t)t;
-  const double g[4] = {gu[0], gu[1], gu[2], gu[3]};
   const double st[4] = {D.s0[t], D.s1[t], D.s2[t], D.s3[t]};
-  double f = D.fdp[t];
-  float G[4], vv[4];
-  drucker_prager_f32v(M, sc.time_sph, st, g, &f, G, vv);  // (no capture: see lean_tail)
-  D.fdp[t] = f;
-  // explicit fmaf: the same rounding as tail_sp_rates<true>
-  const float q = fmaf(2.0f, fmaf(vv[0], vv[0], fmaf(vv[1], vv[1], __fmul_rn(vv[3], vv[3]))),
-                       __fmul_rn(vv[2], vv[2]));
-  const double der = f64_of(sqrtf(__fmul_rn(q, 1.0f / 3.0f)));
-  const float h11 = f32_rn(g[0]), h21 = f32_rn(g[1]), h12 = f32_rn(g[2]), h22 = f32_rn(g[3]);
-  float r[4];
-  r[0] = fmaf(M.D11f, h11, M.D12f * h22);
-  r[1] = fmaf(M.D12f, h11, M.D22f * h22);
-  r[2] = M.D33f * (h21 + h12);
-  r[3] = fmaf(M.D41f, h11, M.D42f * h22);
-  if (D.update_x) {
-    const float om1 = 0.5f * (h12 - h21);
-    const float t0 = f32_rn(st[0]), t1 = f32_rn(st[1]), t2 = f32_rn(st[2]);
-    r[0] = fmaf(2.0f * om1, t2, r[0]);
-    r[1] = fmaf(-2.0f * om1, t2, r[1]);
-    r[2] = fmaf(om1, t1 - t0, r[2]);
-  }
+  double rhs[4], der;
+  sp_rates_lean(D, real_of(D, t), sc, t, f32_rn(gu[0]), f32_rn(gu[1]), f32_rn(gu[2]),
+                f32_rn(gu[3]), st, rhs, der);
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    const double rhs = f64_of(r[k] + -G[k]);
-    D.RHS1[k][t] = rhs;
-    D.RKs[k][t] = fma(f2, rhs, D.RKs[k][t]);
+    D.RHS1[k][t] = rhs[k];
+    D.RKs[k][t] = fma(f2, rhs[k], D.RKs[k][t]);
   }
   D.RKd[t] = D.RKd[t] + der * f2;
 }
 
-// The surrogate's view of stress-point t: the exact rule (drucker_prager, whose results dp
-// = {G, vivel, f} the tail reuses), whether it is loading, and for a loading point the
-// network's inputs x, their output scale and whether they lie in the training envelope.
-// Deterministic, so k_fsp_cand and k_fsp_tail<true> reach the same decisions.
-__device__ __forceinline__ void surr_front(const Dev& D, const Real& M, const StepScalars& sc,
-                                           int t, double* g, double* s2v, float* x,
-                                           double& scale, bool& loading, bool& cand,
-                                           double* dp) {
-  const double* gu = D.grad_u + 4 * (size_t)t;
-  for (int k = 0; k < 4; k++) g[k] = gu[k];
-  s2v[0] = D.s0[t];
-  s2v[1] = D.s1[t];
-  s2v[2] = D.s2[t];
-  s2v[3] = D.s3[t];
-  if (M.ntype_solid == 1) s2v[3] = M.poiss * (s2v[0] + s2v[1]);
-  double f = D.fdp[t], G2[4], vivel[4];
-  drucker_prager_f32(M, sc.time_sph, s2v, g, &f, G2, vivel);  // the exact rule
-  loading = G2[0] != 0.0 || G2[1] != 0.0 || G2[2] != 0.0 || G2[3] != 0.0;
-  for (int k = 0; k < 4; k++) {
-    dp[k] = G2[k];
-    dp[4 + k] = vivel[k];
-  }
-  dp[8] = f;
-  scale = 0.0;
-  cand = false;
-  if (loading) {
-    scale = mlp_features(s2v, g, M.tanfi, M.coh, M.young, M.poiss, D.rho[t], x);
-    cand = scale > 0.0;
-    for (int k = 0; k < MLP_NIN && cand; k++) cand = x[k] >= D.env_lo[k] && x[k] <= D.env_hi[k];
-  }
-}
-
 // One stress-point (index i among the stress-points) of k_fsp_tail; the warp's 32 lanes
-// call it together.  SURR: the network's prediction for a candidate is the row that
-// k_fsp_cand appended for it this stage, computed by the tensor-core kernel in between.
+// call it together.  SURR: with the network's answer (surr_answer).
 template <bool SURR, bool LEAN = false>
 __device__ __forceinline__ void fsp_tail_one(const Dev& D, int stage, int i) {
-  const int lane = threadIdx.x & 31;
   const bool act = i < D.NT - D.NN;
   const int t = D.NN + (act ? i : 0);
   const double f2 = (stage == 1 || stage == 2) ? 2.0 : 1.0;  // RK4 weights 1, 2, 2, 1
   const Real& M = real_of(D, t);
   const StepScalars& sc = D.cur[D.R == 1 ? 0 : D.rid[t]];
-  double g[4] = {0.0, 0.0, 0.0, 0.0}, s2v[4] = {0.0, 0.0, 0.0, 0.0};
-  float x[16];
-  double scale = 0.0;
-  bool loading = false, cand = false;
+  double g[4] = {0.0, 0.0, 0.0, 0.0}, Gnet[4], der = 0.0;
   // drucker_prager's results (G, vivel, f), handed to the tail, which would repeat them
   double dp[9];
-  bool have_dp = false;
-  if (SURR && act && M.ntype_eco > 1 && M.ncrit == 12) {
-    surr_front(D, M, sc, t, g, s2v, x, scale, loading, cand, dp);
-    have_dp = true;
-  }
-  double Gnet[4];
-  bool accept = false;
-  if (SURR && cand) {
-    const float* y = D.ycand + 4 * (size_t)D.cand_row[i];
-    bool inside = true;
-    for (int k = 0; k < MLP_NOUT; k++) {
-      const float yk = y[k];
-      inside = inside && fabsf(yk) <= 1.5f * D.out_max;
-      Gnet[k] = (double)yk * scale;
-    }
-    if (inside) {
-      // drift test in FP64
-      double sm = ((s2v[0] + s2v[1]) + s2v[3]) / 3.0;
-      double d0 = s2v[0] - sm, d1 = s2v[1] - sm, d2 = s2v[2], d3 = s2v[3] - sm;
-      double sj = sqrt(d2 * d2 + 0.5 * ((d0 * d0 + d1 * d1) + d3 * d3));
-      double e0 = M.D11 * g[0] + M.D12 * g[3] + Gnet[0];
-      double e1 = M.D12 * g[0] + M.D22 * g[3] + Gnet[1];
-      double e2 = M.D33 * g[1] + M.D33 * g[2] + Gnet[2];
-      double e3 = M.D41 * g[0] + M.D42 * g[3] + Gnet[3];
-      double df = (d0 * e0 + d1 * e1 + d3 * e3 + 2.0 * d2 * e2) / (2.0 * sj) +
-                  M.alpha2 * (e0 + e1 + e3);
-      accept = sj > 0.0 && M.dt * fabs(df) <= D.surr_tol * sj;
-    } else {
-      cand = false;  // counted as outside the envelope
-    }
-  }
-  // counters: loading, answered, outside the envelope, drift-rejected
+  bool have_dp = false, accept = false;
   if (SURR) {
-    unsigned ml = __ballot_sync(0xffffffffu, loading), ma = __ballot_sync(0xffffffffu, accept),
-             mc = __ballot_sync(0xffffffffu, cand);
-    if (lane == 0 && ml) {
-      atomicAdd(&D.surr_cnt[0], (unsigned long long)__popc(ml));
-      atomicAdd(&D.surr_cnt[1], (unsigned long long)__popc(ma));
-      atomicAdd(&D.surr_cnt[2], (unsigned long long)(__popc(ml) - __popc(mc)));
-      atomicAdd(&D.surr_cnt[3], (unsigned long long)(__popc(mc) - __popc(ma)));
-    }
+    const double st[4] = {D.s0[t], D.s1[t], D.s2[t], D.s3[t]};
+    accept = surr_answer(D, M, sc, act, i, t, st, g, Gnet, der, dp, have_dp);
   }
   if (!act) return;
-  if (accept) {
-    // plastic strain rate of the predicted source: e_p = G / (2 G_mod), shear G / G_mod
-    const double gm = M.young / (2.0 * (1.0 + M.poiss));
-    double v0 = -Gnet[0] / (2.0 * gm), v1 = -Gnet[1] / (2.0 * gm), v2 = -Gnet[2] / gm,
-           v3 = -Gnet[3] / (2.0 * gm);
-    double der = sqrt((2.0 * ((v0 * v0 + v1 * v1) + v3 * v3) + v2 * v2) / 3.0);
-    tail_sp_rates<true>(D, sc, t, D.grad_u + 4 * (size_t)t, f2, Gnet, der, have_dp ? dp : nullptr);
-  } else if (LEAN) {
+  if (LEAN) {
     tail_sp_f32(D, sc, t, f2);
   } else {
-    tail_sp_rates<true>(D, sc, t, D.grad_u + 4 * (size_t)t, f2, nullptr, 0.0,
+    tail_sp_rates<true>(D, sc, t, D.grad_u + 4 * (size_t)t, f2, accept ? Gnet : nullptr, der,
                         have_dp ? dp : nullptr);
   }
 }
@@ -668,20 +467,31 @@ __global__ void __launch_bounds__(128) k_fsp_tail(Dev D, int stage) {
 // stress-point whose inputs lie in the training envelope appends its inputs (16 floats) as
 // one row of xcand; cand_row[i] holds the row of stress-point i, or -1.  The rows of a warp
 // are reserved with one atomic on the stage's count (reset at the start of every step).
+template <bool COL>
 __global__ void __launch_bounds__(128) k_fsp_cand(Dev D, int stage) {
   if (!D.surr || D.surr_gate->on == 0) return;
   const int ns = D.NT - D.NN, lane = threadIdx.x & 31;
   for (int base = blockIdx.x * blockDim.x; base < ns; base += gridDim.x * blockDim.x) {
     const int i = base + threadIdx.x;
     const bool act = i < ns;
-    const int t = D.NN + (act ? i : 0);
+    // the one-launch stages number the stress-points by list column
+    const int t = COL ? D.colid[act ? i : 0] : D.NN + (act ? i : 0);
     const Real& M = real_of(D, t);
     const StepScalars& sc = D.cur[D.R == 1 ? 0 : D.rid[t]];
     double g[4], s2v[4], scale, dp[9];
     float x[16];
     bool loading = false, cand = false;
-    if (act && M.ntype_eco > 1 && M.ncrit == 12)
-      surr_front(D, M, sc, t, g, s2v, x, scale, loading, cand, dp);
+    if (act && M.ntype_eco > 1 && M.ncrit == 12) {
+      double st[4] = {D.s0[t], D.s1[t], D.s2[t], D.s3[t]};
+      if (COL) {
+        const d4 o = ld4(D.stc + 4 * (size_t)i);
+        st[0] = o.a;
+        st[1] = o.b;
+        st[2] = o.c;
+        st[3] = o.d;
+      }
+      surr_front(D, M, sc, t, st, g, s2v, x, scale, loading, cand, dp);
+    }
     const unsigned m = __ballot_sync(0xffffffffu, cand);
     int row0 = 0;
     if (lane == 0 && m) row0 = atomicAdd(&D.cand_count[stage], __popc(m));
@@ -772,18 +582,26 @@ void launch_fderivs(Ctx& c, int stage) {
     default: launch_fderivs_kp<2>(c, stage);
   }
 }
+// the network's rows of this stage: candidates, then the tensor-core forward pass over as many
+// 128-row tiles as there are candidates (a grid of at most two CTAs per SM).  Stress-points
+// by list column (by_col: the one-launch stages) or by id.
+void launch_fsp_cand(Ctx& c, int stage, bool by_col) {
+  const int ns = c.d.NT - c.d.NN;
+  const int nb = std::min((ns + 127) / 128, kTailBlocks);
+  c.kernels_launched += 2;
+  if (by_col) k_fsp_cand<true><<<nb, 128, 0, c.stream>>>(c.d, stage);
+  else k_fsp_cand<false><<<nb, 128, 0, c.stream>>>(c.d, stage);
+  SPS_CUDA_CHECK(mlp_tc_forward(c.d.tc_img, c.d.tc_bias, c.d.xcand, 16, MLP_NIN,
+                                c.d.cand_count + stage, ns, c.d.ycand, MLP_NOUT, c.d.err,
+                                kErrTensorCore, c.tc_grid, c.stream));
+}
 void launch_fsp_tail(Ctx& c, int stage) {
   int ns = c.d.NT - c.d.NN;
   if (ns <= 0) return;
   const int nb = std::min((ns + 127) / 128, kTailBlocks);
   if (c.d.surr) {
-    // the network's rows of this stage: candidates, then the tensor-core forward pass over
-    // as many 128-row tiles as there are candidates (a grid of at most two CTAs per SM)
-    c.kernels_launched += 3;
-    k_fsp_cand<<<nb, 128, 0, c.stream>>>(c.d, stage);
-    SPS_CUDA_CHECK(mlp_tc_forward(c.d.tc_img, c.d.tc_bias, c.d.xcand, 16, MLP_NIN,
-                                  c.d.cand_count + stage, ns, c.d.ycand, MLP_NOUT, c.d.err,
-                                  kErrTensorCore, c.tc_grid, c.stream));
+    c.kernels_launched += 1;
+    launch_fsp_cand(c, stage, false);
     k_fsp_tail<true><<<nb, 128, 0, c.stream>>>(c.d, stage);
   }
   // the variant without the network over one block per 128 stress-points: when it runs

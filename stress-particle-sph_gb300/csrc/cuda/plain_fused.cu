@@ -35,21 +35,6 @@ namespace sps {
 
 namespace {
 
-struct alignas(32) d4 {
-  double a, b, c, d;
-};
-__device__ __forceinline__ d4 ld4(const double* p) {
-  d4 v;
-  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
-               : "=d"(v.a), "=d"(v.b), "=d"(v.c), "=d"(v.d)
-               : "l"(p));
-  return v;
-}
-__device__ __forceinline__ void st4(double* p, double a, double b, double c, double d) {
-  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d)
-               : "memory");
-}
-
 // adapt_stress2 (the plain form's stress_return of plain_step.cu)
 __device__ __forceinline__ void ret(const Real& M, double& a, double& b, double& c, double& d) {
   if (M.ncrit != 12) return;
@@ -65,13 +50,6 @@ __device__ __forceinline__ double div_pre(double a, double b, double y) {
   if (ex > 400 && ex < 1640) return div_rcp(a, b, y);
   if ((__double_as_longlong(a) << 1) == 0) return a * y;  // a signed zero
   return a / b;
-}
-
-__device__ __forceinline__ void load_real(const Dev& D, int t, const Real*& M,
-                                          const StepScalars*& sc) {
-  const int r = D.R == 1 ? 0 : D.rid[t];
-  M = &real_of(D, t);
-  sc = D.cur + r;
 }
 
 // the state of a stress-point at the start of a stage from its rates' result (a, b, c, d):
@@ -221,18 +199,9 @@ __global__ void __launch_bounds__(128) k_pprep(Dev D) {
   D.norm[k] = norm;
   D.rnorm[k] = norm != 0.0 ? 1.0 / norm : 0.0;
   if (D.cspm) {
-    double A4 = AE[0] * AE[3] - AE[1] * AE[2];
-    if (fabs(A4) < D.cspm_det) {
-      A4 = 1;
-      AE[0] = 1;
-      AE[1] = 0;
-      AE[2] = 0;
-      AE[3] = 1;
-    } else {
-      A4 = 1.0 / A4;
-    }
-    for (int q = 0; q < 4; q++) D.AE[(size_t)q * D.NT + k] = AE[q];
-    D.AE[(size_t)4 * D.NT + k] = A4;
+    double A[5];
+    cspm_moments<false>(D, AE, A);
+    for (int q = 0; q < 5; q++) D.AE[(size_t)q * D.NT + k] = A[q];
   }
   // the state of stage 0 (RK4 starts from zero rates)
   if (k < ns) {
@@ -261,6 +230,10 @@ __global__ void __launch_bounds__(128) k_pprep(Dev D) {
 
 // entries a pass whose list words and neighbour records are loaded before any is summed
 constexpr int kP = 4;
+
+// A wall's velocity seen by a stress-point: v - (v (1 - beta) + beta 0).  Rare, and out of line:
+// as predicated instructions it would take the FP64 pipe for every entry.
+static __device__ __noinline__ double wall_du64(double v, double ob) { return v - (v * ob + 0.0); }
 
 // One stage of a stress-point; LS = 2: lane d of the pair sums velocity component d
 template <int LS>
@@ -332,19 +305,19 @@ __device__ __forceinline__ void sp_stage(const Dev& D, int stage, int k, bool ac
 #pragma unroll
     for (int i = 0; i < kP; i++)
       if (j + i < deg) {
-        const bool wall = e[i].y < 0;
-        // a wall's velocity seen by the stress-point: v (1 - beta) + beta 0
+        double du0, du1 = 0.0;
+        if (e[i].y >= 0) {
+          du0 = LS == 1 ? v[i].x - vt0 : (q ? v[i].y : v[i].x) - vtq;
+          if (LS == 1) du1 = v[i].y - vt1;
+        } else {
+          du0 = wall_du64(vtq, v[i].x);
+          if (LS == 1) du1 = wall_du64(vt1, v[i].x);
+        }
+        g[0] = g[0] + du0 * h[i].x;
+        g[2] = g[2] + du0 * h[i].y;
         if (LS == 1) {
-          const double du0 = wall ? vt0 - (vt0 * v[i].x + 0.0) : v[i].x - vt0;
-          const double du1 = wall ? vt1 - (vt1 * v[i].x + 0.0) : v[i].y - vt1;
-          g[0] = g[0] + du0 * h[i].x;
-          g[2] = g[2] + du0 * h[i].y;
           g[1] = g[1] + du1 * h[i].x;
           g[3] = g[3] + du1 * h[i].y;
-        } else {
-          const double du = wall ? vtq - (vtq * v[i].x + 0.0) : (q ? v[i].y : v[i].x) - vtq;
-          g[0] = g[0] + du * h[i].x;
-          g[2] = g[2] + du * h[i].y;
         }
       }
   }
@@ -357,10 +330,7 @@ __device__ __forceinline__ void sp_stage(const Dev& D, int stage, int k, bool ac
   if (D.cspm) {
     double A[5];
     for (int i = 0; i < 5; i++) A[i] = D.AE[(size_t)i * D.NT + k];
-    for (int d = 0; d < 2; d++) {
-      g[d] = A[4] * (A[0] * g[d] + A[1] * g[d + 2]);
-      g[d + 2] = A[4] * (A[2] * g[d] + A[3] * g[d + 2]);
-    }
+    cspm_correct<2, false>(A, g);
   }
   double rhs[4], der;
   sp_rates_f64(D, M, *scp, t, g, st, rhs, der);
@@ -394,7 +364,8 @@ __device__ __forceinline__ void sp_stage(const Dev& D, int stage, int k, bool ac
     D.s2[t] = f[2];
     D.s3[t] = f[3];
     const int ex = (int)((__double_as_longlong(rd) >> 52) & 0x7FF);
-    const double dd = (ex > 64 && ex < 1980) ? div_rcp(rd, 6.0, 1.0 / 6.0) : rd / 6.0;
+    const double dd = (ex > 64 && ex < 1980) ? div_rcp(rd, 6.0, 1.0 / 6.0)
+                      : (__double_as_longlong(rd) << 1) == 0 ? rd : rd / 6.0;
     D.Ddev[t] = dd;
     D.iv1[t] = D.iv1[t] + M.dt * dd;
   }
@@ -434,6 +405,9 @@ __device__ __forceinline__ float2 visc_pair(const Dev& D, ViscT& T, const int4& 
   }
   return make_float2(visc * __int_as_float(e.z), visc * __int_as_float(e.w));
 }
+
+// sigma / rho_d^2 of a node's dummy partner (out of line as wall_du64)
+static __device__ __noinline__ double wall_A(double s, double r2, double y) { return div_pre(s, r2, y); }
 
 // One stage of a node; LN = 4: lane q of the group sums stress component q, then the
 // derivative sums of component q (q < 3)
@@ -543,11 +517,11 @@ __device__ __forceinline__ void node_stage(const Dev& D, int stage, int k, bool 
           const double ru2 = D.rho2[u], yu2 = D.rinv2[u];
           mu[i] = D.mass[u];
           if (LN == 1) {
-            v4[i].a = div_pre(s[0], ru2, yu2);
-            v4[i].b = div_pre(s[1], ru2, yu2);
-            v4[i].c = div_pre(s[2], ru2, yu2);
+            v4[i].a = wall_A(s[0], ru2, yu2);
+            v4[i].b = wall_A(s[1], ru2, yu2);
+            v4[i].c = wall_A(s[2], ru2, yu2);
           } else {
-            aq[i] = div_pre(sq, ru2, yu2);
+            aq[i] = wall_A(sq, ru2, yu2);
           }
         }
         if (LN == 1) {
@@ -627,10 +601,7 @@ __device__ __forceinline__ void node_stage(const Dev& D, int stage, int k, bool 
   if (D.cspm) {
     double A[5];
     for (int i = 0; i < 5; i++) A[i] = D.AE[(size_t)i * D.NT + k];
-    for (int d = 0; d < 2; d++) {
-      g2[d] = A[4] * (A[0] * g2[d] + A[1] * g2[d + 3]);
-      g2[d + 3] = A[4] * (A[2] * g2[d] + A[3] * g2[d + 3]);
-    }
+    cspm_correct<3, false>(A, g2);
   }
   double rx, ry;
   node_rhs_f64(D, M, *scp, t, g2, v.x, v.y, avx, avy, 0.0, 0.0, rx, ry);

@@ -1006,16 +1006,20 @@ int launch_plain_step(Ctx& c) {
   }
   if (c.fused()) {
     c.mark("prep");
-    launch_pprep(c);
+    if (D.fast) launch_fprep(c);
+    else launch_pprep(c);
     for (int stage = 0; stage < 4; stage++) {
       c.mark("stage");
-      launch_pstage(c, stage);
+      if (D.fast) launch_fstage(c, stage);
+      else launch_pstage(c, stage);
     }
     c.mark("finish");
-    launch_pfinish(c);
+    if (D.fast) launch_ffinish(c);
+    else launch_pfinish(c);
     if (D.update_x && D.xsph) {
       c.mark("xsph");
-      k_xsph<<<c.grid_of(TK_XSPH, D.N2), c.blk[TK_XSPH], 0, st>>>(D);
+      if (D.fast) launch_fxsph(c);
+      else k_xsph<<<c.grid_of(TK_XSPH, D.N2), c.blk[TK_XSPH], 0, st>>>(D);
     }
   } else {
     launch_stages(c);

@@ -726,18 +726,29 @@ int sps_create_batch(int32_t nreal, const sps_params* ps, sps_ctx** out) {
     D.colid = dalloc<int32_t>(c, NT);
     if (c.fused()) {
       const size_t ns = NT - NN_;
-      D.norm = dalloc<double>(c, NT);
-      D.rnorm = dalloc<double>(c, NT);
       D.AE = p->cspm ? dalloc<double>(c, 5 * NT) : nullptr;
       D.st0c = dalloc<double>(c, 4 * ns);
       D.rkc = dalloc<double>(c, 4 * ns);
-      for (int k = 0; k < 2; k++) {
-        D.pv[k] = dalloc<double>(c, 2 * NN_);
-        D.ps[k] = dalloc<double>(c, 4 * ns);
-        D.pa[k] = dalloc<double>(c, 4 * ns);
+      if (D.fast) {
+        D.stc = dalloc<double>(c, 4 * ns);
+        if (p->cspm) D.pv[0] = dalloc<double>(c, 2 * NN_);
+        D.recV1 = dalloc<float4>(c, NN_);
+        D.recS1 = dalloc<float4>(c, NT);
+        D.recA1 = dalloc<float4>(c, NT);
+        D.recAl1 = dalloc<float4>(c, NT);
+        D.normf = dalloc<float2>(c, NT);
+        D.msum = dalloc<float4>(c, NN_);
+      } else {
+        D.norm = dalloc<double>(c, NT);
+        D.rnorm = dalloc<double>(c, NT);
+        for (int k = 0; k < 2; k++) {
+          D.pv[k] = dalloc<double>(c, 2 * NN_);
+          D.ps[k] = dalloc<double>(c, 4 * ns);
+          D.pa[k] = dalloc<double>(c, 4 * ns);
+        }
+        D.rho2 = dalloc<double>(c, N2);
+        D.rinv2 = dalloc<double>(c, N2);
       }
-      D.rho2 = dalloc<double>(c, N2);
-      D.rinv2 = dalloc<double>(c, N2);
     }
     if (D.fast) {
       D.recV = dalloc<float4>(c, N2);
@@ -1013,7 +1024,10 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
         D.same = dalloc<int4>(c, (size_t)D.N2 * rows);
         D.crossW = c.precision == SPS_PREC_FP32_FAST ? dalloc<int2>(c, (size_t)D.N2 * rows)
                                                      : nullptr;
-        if (c.fused()) {
+        if (c.fused() && D.fast) {
+          D.hGf = dalloc<float2>(c, (size_t)D.NT * (size_t)capn);
+          D.hB = dalloc<double>(c, (size_t)(D.NT - D.NN) * (size_t)capn);
+        } else if (c.fused()) {
           D.hW = dalloc<double>(c, (size_t)D.NT * (size_t)capn);
           D.hG = dalloc<double2>(c, (size_t)(D.NT - D.NN) * (size_t)capn);
         }
@@ -1775,7 +1789,7 @@ int sps_autotune(sps_ctx* h, int32_t nsteps, int32_t* blocks) {
         copy(false);
         for (int g = 0; g < 2; g++)
           for (size_t q = 0; q < kn.size(); q++)
-            if (kn[q] == names[g] && kms[q] < best_la_ms[g]) {
+            if ((kn[q] == names[g] || (c.fused() && kn[q] == "stage")) && kms[q] < best_la_ms[g]) {
               best_la_ms[g] = kms[q];
               best_la[g] = v[g];
             }

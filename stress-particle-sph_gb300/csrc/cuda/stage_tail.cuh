@@ -11,6 +11,30 @@
 
 namespace sps {
 
+// four doubles of one 32-byte sector, loaded and stored together
+struct alignas(32) d4 {
+  double a, b, c, d;
+};
+__device__ __forceinline__ d4 ld4(const double* p) {
+  d4 v;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(v.a), "=d"(v.b), "=d"(v.c), "=d"(v.d)
+               : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void st4(double* p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d)
+               : "memory");
+}
+
+// the constants and the step's scalars of particle t's realisation
+__device__ __forceinline__ void load_real(const Dev& D, int t, const Real*& M,
+                                          const StepScalars*& sc) {
+  const int r = D.R == 1 ? 0 : D.rid[t];
+  M = &real_of(D, t);
+  sc = D.cur + r;
+}
+
 // BCs (3_SPH_material_2018.f90:1640-1660) for one particle: Normal_BCs (:1665-1770), then
 // with ifsigman = 1 apply_stress_free (:1775-1858): a free-surface node away from the walls
 // keeps only the stress component along the surface (zero normal and shear traction)
@@ -59,6 +83,38 @@ __device__ __forceinline__ void capture_tuple(const Dev& D, int t, const double*
   float* o = D.cap_buf + (size_t)k * MLP_TUPLE;
   for (int j = 0; j < MLP_NIN; j++) o[j] = x[j];
   for (int j = 0; j < MLP_NOUT; j++) o[MLP_NIN + j] = (float)(Gs[j] / scale);
+}
+
+// a b + c d: both products rounded (the plain form, as the reference), or the first one fused
+// with the sum (FMA: the FP32 form, as its separate kernels are compiled)
+template <bool FMA>
+__device__ __forceinline__ double dot2(double a, double b, double c, double d) {
+  return FMA ? fma(a, b, __dmul_rn(c, d)) : __dadd_rn(__dmul_rn(a, b), __dmul_rn(c, d));
+}
+// CSPM: the moments AE as the correction uses them (identity below the determinant's
+// threshold) and A[4] = 1 / determinant
+template <bool FMA>
+__device__ __forceinline__ void cspm_moments(const Dev& D, const double* AE, double* A) {
+  double A4 = dot2<FMA>(AE[0], AE[3], -AE[1], AE[2]);
+  for (int k = 0; k < 4; k++) A[k] = AE[k];
+  if (fabs(A4) < D.cspm_det) {
+    A4 = 1;
+    A[0] = 1;
+    A[1] = 0;
+    A[2] = 0;
+    A[3] = 1;
+  } else {
+    A4 = 1.0 / A4;
+  }
+  A[4] = A4;
+}
+// the correction of a gradient whose components (., 1) and (., 2) are `half` apart
+template <int half, bool FMA>
+__device__ __forceinline__ void cspm_correct(const double* A, double* g) {
+  for (int d = 0; d < 2; d++) {
+    g[d] = __dmul_rn(A[4], dot2<FMA>(A[0], g[d], A[1], g[d + half]));
+    g[d + half] = __dmul_rn(A[4], dot2<FMA>(A[3], g[d + half], A[2], g[d]));
+  }
 }
 
 // stress-point gradient: CSPM correction of g = grad1(a,b) (at a + 2b) with the moments AE,
@@ -132,6 +188,76 @@ __device__ __forceinline__ void sp_rates_f64(const Dev& D, const Real& M, const 
   for (int k = 0; k < 4; k++) rhs[k] = (-div1[k] + spin[k]) + Gs[k];
 }
 
+// stress-point rates of the FP32 form: drucker_prager in FP32 (or the FP64 viscoplastic laws),
+// the plastic strain-rate norm, the elastic rate and the spin in FP32; rhs(4) and the plastic
+// strain rate.  Gs_net (may be null): a plastic source from the learned surrogate that replaces
+// the exact one (with its plastic strain rate der_net); dp (may be null): drucker_prager's
+// results for this stress-point, already evaluated on the same inputs by the caller: G (4),
+// vivel (4), the updated f
+__device__ __forceinline__ void sp_rates_fast(const Dev& D, const Real& M, const StepScalars& sc,
+                                              int t, const double* g, const double* st,
+                                              const double* Gs_net, double der_net,
+                                              const double* dp, double* rhs, double& der) {
+  const double g11 = g[0], g21 = g[1], g12 = g[2], g22 = g[3];
+  // plastic_terms (3_SPH_material_2018.f90:1884-1954)
+  double Gs[4] = {0.0, 0.0, 0.0, 0.0};
+  if (M.ntype_eco > 1) {
+    double s2v[4] = {st[0], st[1], st[2], st[3]};
+    if (M.ntype_solid == 1) s2v[3] = M.poiss * (s2v[0] + s2v[1]);
+    double vivel[4] = {0.0, 0.0, 0.0, 0.0}, G2[4];
+    if (M.ncrit <= 4) {
+      viscoplastic(M, s2v, D.iv1[t], vivel, Gs);
+    } else if (M.ncrit == 12) {
+      double f;
+      if (dp) {
+        for (int k = 0; k < 4; k++) {
+          G2[k] = dp[k];
+          vivel[k] = dp[4 + k];
+        }
+        f = dp[8];
+      } else {
+        f = D.fdp[t];
+        drucker_prager_f32(M, sc.time_sph, s2v, g, &f, G2, vivel);
+      }
+      D.fdp[t] = f;
+      // negation and the non-zero test on the integer pipe (sign bit; magnitude bits)
+      bool nz = false;
+      for (int k = 0; k < 4; k++) {
+        const long long b = __double_as_longlong(G2[k]);
+        Gs[k] = __longlong_as_double(b ^ (long long)0x8000000000000000ull);
+        nz = nz || (b << 1) != 0;
+      }
+      if (D.cap_buf && nz) capture_tuple(D, t, s2v, g, Gs);
+    }
+    float v0 = f32_rn(vivel[0]), v1 = f32_rn(vivel[1]), v2 = f32_rn(vivel[2]),
+          v3 = f32_rn(vivel[3]);
+    // explicit fmaf: the same rounding in every kernel that inlines this tail
+    float q = fmaf(2.0f, fmaf(v0, v0, fmaf(v1, v1, __fmul_rn(v3, v3))), __fmul_rn(v2, v2));
+    der = f64_of(sqrtf(__fmul_rn(q, 1.0f / 3.0f)));
+  }
+  if (Gs_net) {
+    for (int k = 0; k < 4; k++) Gs[k] = Gs_net[k];
+    der = der_net;
+  }
+  // the FP32 form: the elastic rate, the spin and the right-hand side in FP32 (the
+  // gradient comes from FP32 neighbour sums and carries their accuracy), conversions on
+  // the integer pipe; only the RK accumulation stays FP64
+  const float h11 = f32_rn(g11), h21 = f32_rn(g21), h12 = f32_rn(g12), h22 = f32_rn(g22);
+  float r[4];
+  r[0] = fmaf(M.D11f, h11, M.D12f * h22);
+  r[1] = fmaf(M.D12f, h11, M.D22f * h22);
+  r[2] = M.D33f * (h21 + h12);
+  r[3] = fmaf(M.D41f, h11, M.D42f * h22);
+  if (D.update_x) {
+    const float om1 = 0.5f * (h12 - h21);
+    const float t0 = f32_rn(st[0]), t1 = f32_rn(st[1]), t2 = f32_rn(st[2]);
+    r[0] = fmaf(2.0f * om1, t2, r[0]);
+    r[1] = fmaf(-2.0f * om1, t2, r[1]);
+    r[2] = fmaf(om1, t1 - t0, r[2]);
+  }
+  for (int k = 0; k < 4; k++) rhs[k] = f64_of(r[k] + f32_rn(Gs[k]));
+}
+
 // stress-point rates after the gradient: D : grad(v), plastic_terms / drucker_prager,
 // Jaumann spin, RHS and RK4 accumulation.  Gs_net (may be null): a plastic source from the
 // learned surrogate that replaces the exact one (with its plastic strain rate der_net)
@@ -156,67 +282,11 @@ __device__ __forceinline__ void tail_sp_rates(const Dev& D, const StepScalars& s
         D.RKs[k][t] = D.RKs[k][t] + f2 * rhs[k];
       }
     } else {
-      const double g11 = g[0], g21 = g[1], g12 = g[2], g22 = g[3];
-      // plastic_terms (3_SPH_material_2018.f90:1884-1954)
-      double Gs[4] = {0.0, 0.0, 0.0, 0.0};
-      if (M.ntype_eco > 1) {
-        double s2v[4] = {st[0], st[1], st[2], st[3]};
-        if (M.ntype_solid == 1) s2v[3] = M.poiss * (s2v[0] + s2v[1]);
-        double vivel[4] = {0.0, 0.0, 0.0, 0.0}, G2[4];
-        if (M.ncrit <= 4) {
-          viscoplastic(M, s2v, D.iv1[t], vivel, Gs);
-        } else if (M.ncrit == 12) {
-          double f;
-          if (dp) {
-            for (int k = 0; k < 4; k++) {
-              G2[k] = dp[k];
-              vivel[k] = dp[4 + k];
-            }
-            f = dp[8];
-          } else {
-            f = D.fdp[t];
-            drucker_prager_f32(M, sc.time_sph, s2v, g, &f, G2, vivel);
-          }
-          D.fdp[t] = f;
-          // negation and the non-zero test on the integer pipe (sign bit; magnitude bits)
-          bool nz = false;
-          for (int k = 0; k < 4; k++) {
-            const long long b = __double_as_longlong(G2[k]);
-            Gs[k] = __longlong_as_double(b ^ (long long)0x8000000000000000ull);
-            nz = nz || (b << 1) != 0;
-          }
-          if (D.cap_buf && nz) capture_tuple(D, t, s2v, g, Gs);
-        }
-        float v0 = f32_rn(vivel[0]), v1 = f32_rn(vivel[1]), v2 = f32_rn(vivel[2]),
-              v3 = f32_rn(vivel[3]);
-        // explicit fmaf: the same rounding in every kernel that inlines this tail
-        float q = fmaf(2.0f, fmaf(v0, v0, fmaf(v1, v1, __fmul_rn(v3, v3))), __fmul_rn(v2, v2));
-        der = f64_of(sqrtf(__fmul_rn(q, 1.0f / 3.0f)));
-      }
-      if (Gs_net) {
-        for (int k = 0; k < 4; k++) Gs[k] = Gs_net[k];
-        der = der_net;
-      }
-      // the FP32 form: the elastic rate, the spin and the right-hand side in FP32 (the
-      // gradient comes from FP32 neighbour sums and carries their accuracy), conversions on
-      // the integer pipe; only the RK accumulation stays FP64
-      const float h11 = f32_rn(g11), h21 = f32_rn(g21), h12 = f32_rn(g12), h22 = f32_rn(g22);
-      float r[4];
-      r[0] = fmaf(M.D11f, h11, M.D12f * h22);
-      r[1] = fmaf(M.D12f, h11, M.D22f * h22);
-      r[2] = M.D33f * (h21 + h12);
-      r[3] = fmaf(M.D41f, h11, M.D42f * h22);
-      if (D.update_x) {
-        const float om1 = 0.5f * (h12 - h21);
-        const float t0 = f32_rn(st[0]), t1 = f32_rn(st[1]), t2 = f32_rn(st[2]);
-        r[0] = fmaf(2.0f * om1, t2, r[0]);
-        r[1] = fmaf(-2.0f * om1, t2, r[1]);
-        r[2] = fmaf(om1, t1 - t0, r[2]);
-      }
+      double rhs[4];
+      sp_rates_fast(D, M, sc, t, g, st, Gs_net, der_net, dp, rhs, der);
       for (int k = 0; k < 4; k++) {
-        const double rhs = f64_of(r[k] + f32_rn(Gs[k]));
-        D.RHS1[k][t] = rhs;
-        D.RKs[k][t] = fma(f2, rhs, D.RKs[k][t]);
+        D.RHS1[k][t] = rhs[k];
+        D.RKs[k][t] = fma(f2, rhs[k], D.RKs[k][t]);
       }
     }
     D.RKd[t] = D.RKd[t] + der * f2;
@@ -311,21 +381,22 @@ __device__ __forceinline__ void tail_node(const Dev& D, const StepScalars& sc, i
 
 // boundary_forces, test == 2 (2_SPH_main_2018.f90:1117-1161): FP32 locals.  Only innermost
 // dummies closer than 0.75 dx give a non-zero term; they are summed in ascending id.
+// Explicit roundings: the same in every unit.
 __device__ __forceinline__ bool bound_term(const Dev& D, const Real& M, int i, int j, float& fx,
                                            float& fy) {
   const float cc = 20.0f;
   const float d0 = (float)(M.dx / 2.0);
   float r0 = (float)(D.px[i] - D.px[j]);
   float r1 = (float)(D.py[i] - D.py[j]);
-  float r2 = sqrtf(r0 * r0 + r1 * r1);
+  float r2 = sqrtf(__fadd_rn(__fmul_rn(r0, r0), __fmul_rn(r1, r1)));
   float h = (float)(0.5 * (D.hsml[i] + D.hsml[j]));
   float r_bound = r2 / (0.75f * h);
   float f2;
-  if (r2 > 0 && r2 < 1.5f * d0) f2 = 1.0f - (r2 / (1.5f * d0));
+  if (r2 > 0 && r2 < 1.5f * d0) f2 = __fsub_rn(1.0f, r2 / (1.5f * d0));
   else f2 = 0.0f;
   float f;
   if (0 < r_bound && r_bound <= 2.0f / 3.0f) f = 2.0f / 3.0f;
-  else if (2.0f / 3.0f < r_bound && r_bound <= 1) f = 2.0f * r_bound - 1.5f * (r_bound * r_bound);
+  else if (2.0f / 3.0f < r_bound && r_bound <= 1) f = __fsub_rn(2.0f * r_bound, __fmul_rn(1.5f, __fmul_rn(r_bound, r_bound)));
   else if (1 < r_bound && r_bound < 2) f = 0.5f * ((2.0f - r_bound) * (2.0f - r_bound));
   else f = 0.0f;
   if (f2 == 0.0f || f == 0.0f) return false;

@@ -29,6 +29,7 @@ CUDA_UNITS = [
     ("cuda/plain_step.cu", ["-fmad=false"]),
     ("cuda/plain_fused.cu", ["-fmad=false"]),
     ("cuda/fast_step.cu", []),
+    ("cuda/fast_fused.cu", []),
     ("cuda/surface.cu", ["-fmad=false"]),
     ("cuda/mlp_train.cu", []),
     ("cuda/mlp_tc.cu", []),
