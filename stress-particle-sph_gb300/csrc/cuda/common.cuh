@@ -202,7 +202,12 @@ struct Dev {
   const void* tc_img;   // the network as the tensor-core kernel's shared-memory image
   const float* tc_bias;
   // cells
-  int32_t *cell_of, *cell_cnt, *cell_start, *cell_cursor, *sorted, *spos;
+  int32_t *cell_of, *cell_cnt, *cell_start, *sorted, *spos;
+  // counts of a cell by kind (nodes << 32 | stress-points; dummies) and the scans of the
+  // counts, in two parts (k_scan_cells)
+  unsigned long long *cntK, *cell_locK, *cell_bsK;
+  int32_t *cntD, *cell_loc, *cell_bs;
+  unsigned* tick;  // tickets of the kernels whose last block finishes the work
   float *xr, *yr, *hr;
   float *xrl, *yrl;  // FP32 form: low parts of the cell-relative offsets
   float4* srec;       // by sorted position: (xr, yr, hr, 0) of the particle there
@@ -215,7 +220,8 @@ struct Dev {
   int32_t* half_cnt;
   int4* half_meta;    // per creator (sorted position): group starts 1-4 (16 bits each),
                       // pair count, id
-  int64_t* half_off;  // exclusive scan of half_cnt over sorted positions (size N2+1)
+  // exclusive scan of half_cnt over sorted positions (size N2 + 1), in two parts (k_scan_half)
+  int64_t *half_off, *half_bs;
   int4 *cross, *same;
   // FP32 form with gathered lists: the cross lists' {neighbour id, W} again, 8 bytes an
   // entry at k * N2 + col (a warp reads entry k of its columns as one contiguous run): the
@@ -229,7 +235,8 @@ struct Dev {
   int l2_prefetch;  // FP32 form: bulk L2 prefetch of list entries (bit 0 interp, bit 1 derivs)
   // sorted positions of the stress-point and of the node targets (each in sorted order), so
   // that the gathers run one kind per warp
-  int32_t *tgtS, *tgtN, *tflag, *toff;
+  int32_t *tgtS, *tgtN;
+  int32_t* tflag;  // the cells' particles before they are in id order
   // list column of every sorted position: the stress-points first, then the nodes (each in
   // sorted order, as tgtS and tgtN), then the rest.  The k-th target of a one-kind launch
   // has column k (stress-points) or NT - NN + k (nodes), so a warp reads its targets' list
@@ -270,8 +277,6 @@ struct Dev {
   int* step_idx;
   StepScalars* cur;
   int* err;
-  // scan scratch
-  int64_t* scan_tmp;
 };
 
 // Index of entry k of list column col in the per-target lists (cross, same).  Entries 2j and

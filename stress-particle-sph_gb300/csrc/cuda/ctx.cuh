@@ -118,8 +118,6 @@ struct Ctx {
   // FP32 form: every realisation is Drucker-Prager (ncrit 12, ntype_eco > 1) in plane strain
   // without continuity density, so the stress-point tail takes its lean kernel
   bool lean_tail = false;
-  // scratch for scans
-  int scan_blocks = 0;
   // per-kernel event timing (sps_profile_step)
   bool profiling = false;
   std::vector<std::pair<const char*, cudaEvent_t>> prof_events;
@@ -164,10 +162,6 @@ struct Ctx {
     prof_events.push_back({name, e});
   }
 };
-
-// generic exclusive scans on the context stream
-void scan_i32_to_i32(Ctx& c, const int32_t* in, int32_t* out, int n);
-void scan_i32_to_i64(Ctx& c, const int32_t* in, int64_t* out, int n);
 
 }  // namespace sps
 

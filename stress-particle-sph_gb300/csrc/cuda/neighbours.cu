@@ -3,9 +3,10 @@
 // Restates grid_find_NEW (example_problems/soil_failure_bui_et_al_2008/
 // 2_SPH_main_2018.f90:1199-1435), kernel (:1440) and Pint_Update
 // (3_SPH_material_2018.f90:1574) as a GB300 pipeline:
-//   k_bbox      Check_Out_Domain (:1170) + bounding box / max h over active particles
-//   k_grid      grid parameters with the reference's arithmetic (:1245-1258)
-//   k_cell_*    counting sort by cell, stable in particle id (the order list_picell holds)
+//   k_bbox      Check_Out_Domain (:1170) + bounding box / max h over active particles; its last
+//               block forms the grid parameters with the reference's arithmetic (:1245-1258)
+//   k_cell_*    counting sort by cell and kind, then by particle id (the order list_picell
+//               holds), with the list column of every particle
 //   k_half      pairs created by each particle over the half stencil (self, +x, row
 //               above), in the reference's creation order, with FP32-stored W and dW
 //   k_lists     per-target neighbour lists in the reference's linked-list walk order
@@ -92,13 +93,47 @@ __device__ __forceinline__ double unkey(unsigned long long k) {
 }
 constexpr unsigned long long kNoKey = ~0ull;  // no active particle
 
+// true for every thread of the block that is the last of its grid to get here, once all
+// blocks' earlier global writes are visible to it (read them past L1: __ldcg); the ticket is
+// back at zero for the next launch
+__device__ __forceinline__ bool last_block(unsigned* ticket) {
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (last) {
+      *ticket = 0u;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  return last;
+}
+
 // Check_Out_Domain (2_SPH_main_2018.f90:1170) + the bounding box of the active particles of
 // every realisation: keys of (minx, miny, -maxx, -maxy, -maxh, minh), reduced over the warp
 // (or the block) when it holds one realisation, then atomicMin per realisation
-__global__ void k_bbox(Dev D) {
+// The step's first kernel: it also loads the step's scalars, clears the cell counts, and its
+// last block forms the grids (one launch instead of five: each of the small ones took about
+// 5 us of a step that lasts 300 at 10,000 particles).
+__device__ void grid_block(const Dev& D);
+__global__ void __launch_bounds__(kBlock) k_bbox(Dev D) {
   __shared__ unsigned long long sh[kBlock / 32][6];
   __shared__ int shr[kBlock / 32];
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.x == 0) {
+    const int k = *D.step_idx;
+    if (D.surr && threadIdx.x < 4) D.cand_count[threadIdx.x] = 0;  // the network's rows
+    for (int r = threadIdx.x; r < D.R; r += blockDim.x)
+      D.cur[r] = D.scal_table[(size_t)k * D.R + r];
+    __syncthreads();
+    if (threadIdx.x == 0) *D.step_idx = k + 1;
+  }
+  for (int c = i; c < D.cell_cap + 2; c += gridDim.x * blockDim.x) {
+    D.cntK[c] = 0ull;
+    D.cntD[c] = 0;
+  }
   unsigned long long v[6] = {kNoKey, kNoKey, kNoKey, kNoKey, kNoKey, kNoKey};
   int r = -1;
   if (i < D.N2) {
@@ -167,11 +202,13 @@ __global__ void k_bbox(Dev D) {
           for (int k = 0; k < 6; k++) atomicMin(&D.bbox[6 * (size_t)shr[w] + k], sh[w][k]);
     }
   }
+  if (last_block(D.tick)) grid_block(D);
 }
 
 // grid parameters of every realisation (2_SPH_main_2018.f90:1230-1260) and the numbering
-// of their cells (one block; the bounding-box keys are reset for the next step)
-__global__ void k_grid(Dev D) {
+// of their cells (one block of kBlock threads; the bounding-box keys are reset for the next
+// step)
+__device__ void grid_block(const Dev& D) {
   __shared__ int sc[kBlock];
   __shared__ int carry, bad;
   const int tid = threadIdx.x;
@@ -187,7 +224,7 @@ __global__ void k_grid(Dev D) {
     if (r < D.R) {
       double red[6];
       for (int k = 0; k < 6; k++) {
-        unsigned long long key = D.bbox[6 * (size_t)r + k];
+        unsigned long long key = __ldcg(&D.bbox[6 * (size_t)r + k]);
         D.bbox[6 * (size_t)r + k] = kNoKey;
         red[k] = key == kNoKey ? 1e300 : unkey(key);
       }
@@ -306,7 +343,9 @@ __device__ __forceinline__ int cell_index(const Grid& g, double x, double y) {
 }
 
 // Task 2 of grid_find_NEW (2_SPH_main_2018.f90:1275-1286): the cell of every particle
-// inside the domain, and the cells' counts
+// inside the domain, and the cells' counts by kind: cntK (nodes in the high word, stress-points
+// in the low one) and cntD (dummies).  A particle's place in the count is its slot among its
+// cell's particles of its kind (spos, until k_cell_rank), so the fill needs no second atomic.
 __global__ void k_cell_count(Dev D) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= D.N2) return;
@@ -337,45 +376,155 @@ __global__ void k_cell_count(Dev D) {
     c = g.cell0 + cl;
   }
   D.cell_of[i] = c;
-  atomicAdd(&D.cell_cnt[c], 1);
+  if (i < D.NN) D.spos[i] = (int)(atomicAdd(&D.cntK[c], 1ull << 32) >> 32);
+  else if (i < D.NT) D.spos[i] = (int)(unsigned)atomicAdd(&D.cntK[c], 1ull);
+  else D.spos[i] = atomicAdd(&D.cntD[c], 1);
 }
 
-// the cells' particle lists (list_picell, 2_SPH_main_2018.f90:1288-1305), filled in any
-// order here and put in ascending id order by k_cell_sort
-__global__ void k_cell_fill(Dev D) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= D.N2) return;
-  int c = D.cell_of[i];
-  int slot = atomicAdd(&D.cell_cursor[c], 1);
-  D.spos[D.cell_start[c] + slot] = i;  // spos used as scratch here
-}
-
-// per cell: sort the ids ascending (list_picell order, 2_SPH_main_2018.f90:1299-1305),
-// write sorted[] and spos[]
-__global__ void k_cell_sort(Dev D) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const GridTotal g = *D.gtot;
-  if (c > g.ncells) return;
-  int st = D.cell_start[c], n = D.cell_cnt[c];
-  for (int a = 0; a < n; a++) {
-    int v = D.spos[st + a];
-    int b = a - 1;
-    while (b >= 0 && D.sorted[st + b] > v) {
-      D.sorted[st + b + 1] = D.sorted[st + b];
-      b--;
-    }
-    D.sorted[st + b + 1] = v;
+// Exclusive scans of the cells' counts (total and by kind), kScan cells a block: the scan
+// within the block (cell_loc, cell_locK) and, by the last block, of the blocks' sums (cell_bs,
+// cell_bsK); readers add the two.  Blocks past the last cell only take their ticket.
+constexpr int kScan = kBlock * 16;
+template <typename T>
+__device__ __forceinline__ T block_exclusive(T v, T* sh, T& total) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  T s = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const T u = __shfl_up_sync(0xffffffffu, s, o);
+    if (lane >= o) s += u;
   }
-  if (c == g.ncells) D.gtot->nactive = st;
+  __syncthreads();
+  if (lane == 31) sh[w] = s;
+  __syncthreads();
+  T before = 0;
+  total = 0;
+#pragma unroll
+  for (int k = 0; k < kBlock / 32; k++) {
+    if (k < w) before += sh[k];
+    total += sh[k];
+  }
+  return before + s - v;
+}
+// in place, by one block: exclusive scan of the nb sums
+template <typename T>
+__device__ __forceinline__ T scan_sums(T* bs, int nb, T* sh) {
+  T carry = 0;
+  for (int base = 0; base < nb; base += kBlock) {
+    const int i = base + threadIdx.x;
+    const T v = i < nb ? __ldcg(&bs[i]) : (T)0;
+    T total;
+    const T e = block_exclusive(v, sh, total);
+    if (i < nb) bs[i] = carry + e;
+    carry += total;
+  }
+  return carry;
+}
+__global__ void __launch_bounds__(kBlock) k_scan_cells(Dev D) {
+  __shared__ int shT[kBlock / 32];
+  __shared__ unsigned long long shK[kBlock / 32];
+  const int n = D.gtot->ncells + 1;  // the out-of-domain bucket is the last
+  const int base = blockIdx.x * kScan;
+  if (base < n) {
+    const int i0 = base + threadIdx.x * 16;
+    int lt = 0;
+    unsigned long long lk = 0;
+    for (int q = 0; q < 16; q++) {
+      const int c = i0 + q;
+      if (c >= n) break;
+      const unsigned long long k = D.cntK[c];
+      const int t = (int)(k >> 32) + (int)(unsigned)k + D.cntD[c];
+      D.cell_cnt[c] = t;
+      lt += t;
+      lk += k;
+    }
+    int totT;
+    unsigned long long totK;
+    int rt = block_exclusive(lt, shT, totT);
+    unsigned long long rk = block_exclusive(lk, shK, totK);
+    for (int q = 0; q < 16; q++) {
+      const int c = i0 + q;
+      if (c >= n) break;
+      D.cell_loc[c] = rt;
+      D.cell_locK[c] = rk;
+      rt += D.cell_cnt[c];
+      rk += D.cntK[c];
+    }
+    if (threadIdx.x == 0) {
+      D.cell_bs[blockIdx.x] = totT;
+      D.cell_bsK[blockIdx.x] = totK;
+    }
+  }
+  if (last_block(D.tick + 1)) {
+    const int nb = (n + kScan - 1) / kScan;
+    scan_sums(D.cell_bs, nb, shT);
+    scan_sums(D.cell_bsK, nb, shK);
+  }
+}
+__device__ __forceinline__ int cell_first(const Dev& D, int c) {
+  return D.cell_loc[c] + D.cell_bs[c / kScan];
 }
 
-// sorted position of every particle, and the pair search's per-particle values in sorted
-// order (the candidates of a cell are then read contiguously)
-__global__ void k_spos(Dev D) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= D.N2) return;
-  const int t = D.sorted[s];
+// the cells' particle lists (list_picell, 2_SPH_main_2018.f90:1288-1305): nodes, stress-points
+// and dummies of a cell one after the other (ids ascend from kind to kind), each kind in any
+// order (tflag, put in ascending id order by k_cell_rank); and the cells' starts
+__global__ void k_cell_fill(Dev D) {
+  const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nc = D.gtot->ncells;
+  for (int c = i0; c <= nc; c += gridDim.x * blockDim.x) {
+    const int st = cell_first(D, c);
+    D.cell_start[c] = st;
+    if (c == nc) D.gtot->nactive = st;
+  }
+  if (i0 >= D.N2) return;
+  const int c = D.cell_of[i0];
+  const unsigned long long k = D.cntK[c];
+  const int nn = (int)(k >> 32), ns = (int)(unsigned)k;
+  const int off = i0 < D.NN ? 0 : i0 < D.NT ? nn : nn + ns;
+  D.tflag[cell_first(D, c) + off + D.spos[i0]] = i0;
+}
+
+// per sorted position: the particle's rank by id among its cell's particles of its kind
+// (list_picell order, 2_SPH_main_2018.f90:1299-1305), hence its sorted position; its list
+// column (stress-points, then nodes, then dummies, each in sorted order); and the pair
+// search's per-particle values in sorted order (the candidates of a cell are then read
+// contiguously).  A cell holds a handful of each kind, so a particle counts the smaller ids
+// itself: 6 us at 10,000 particles where one thread a cell sorting by insertion, the sorted
+// copy and the eight launches that compacted the kinds took 72.  The order of the
+// out-of-domain particles, which have no pairs, is left as it is.
+__global__ void k_cell_rank(Dev D) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= D.N2) return;
+  const int t = D.tflag[p];
+  const int c = D.cell_of[t];
+  const unsigned long long k = D.cntK[c];
+  const int nn = (int)(k >> 32), ns = (int)(unsigned)k;
+  const int first = D.cell_start[c];
+  const bool node = t < D.NN, sp = !node && t < D.NT;
+  const int seg = first + (node ? 0 : sp ? nn : nn + ns);
+  const int len = node ? nn : sp ? ns : D.cntD[c];
+  int rank = 0;
+  if (c == D.gtot->ncells) rank = p - seg;
+  else
+    for (int j = 0; j < len; j++) rank += D.tflag[seg + j] < t;
+  const int s = seg + rank;
+  D.sorted[s] = t;
   D.spos[t] = s;
+  const unsigned long long before = D.cell_locK[c] + D.cell_bsK[c / kScan];
+  const int bn = (int)(before >> 32), bsp = (int)(unsigned)before;
+  int col;
+  if (sp) {
+    col = bsp + rank;
+    D.tgtS[col] = s;
+    D.colid[col] = t;
+  } else if (node) {
+    D.tgtN[bn + rank] = s;
+    col = (D.NT - D.NN) + bn + rank;
+    D.colid[col] = t;
+  } else {
+    col = D.NT + (first - bn - bsp) + rank;
+  }
+  D.lcol[s] = col;
   D.srec[s] = make_float4(D.xr[t], D.yr[t], D.hr[t], __int_as_float(D.itype[t]));
   if (D.fast) D.srecl[s] = make_float2(D.xrl[t], D.yrl[t]);
 }
@@ -743,24 +892,17 @@ __device__ __forceinline__ bool gather_accept(const Dev& D, int a, float xa, flo
 // FP32 form: Task 3 of grid_find_NEW (2_SPH_main_2018.f90:1307-1403), kernel (:1440-1538)
 // and Pint_Update (3_SPH_material_2018.f90:1574-1634) per target, gathering its entries
 // from the 3 x 3 cell stencil directly in creation order.
-// KIND 1: the stress-point targets tgt[0..n), 2: the node targets.  SAME: the same-kind
-// entries are written too (the steps that read them: XSPH, artificial viscosity or stress,
+// SAME: the same-kind entries are written too (the steps that read them: XSPH, artificial viscosity or stress,
 // the FP32 free-surface detection); without them degS holds 0 unless the outside approach
 // reads the counts.  Phase 1 tests the stencil's candidates and keeps the
 // accepted ones (sorted position and cell offset) in shared memory; phase 2 evaluates the
 // kernel values, so that a warp's lanes evaluate together.  Dynamic shared memory:
 // (capC + SAME capS) ints per thread, entry k of thread j at k * blockDim + j.
-template <int KIND, bool SAME>
-__global__ void __launch_bounds__(512, 2) k_fgather(Dev D, const int32_t* __restrict__ tgt,
-                                                    int ntgt) {
-  extern __shared__ int gbuf[];
-  const int k0 = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k0 >= ntgt) return;
+template <bool SAME>
+__device__ __forceinline__ void gather_target(const Dev& D, int s, int col, int* gbuf) {
   const int bd = blockDim.x, tid = threadIdx.x;
   int* bufC = gbuf;
   int* bufS = gbuf + (size_t)D.capC * bd;
-  const int s = tgt[k0];
-  const int col = list_col<KIND>(D, k0, s);
   int nC = 0, nS = 0, nHalf = 0;
   if (s < D.gtot->nactive) {
     const int a = D.sorted[s];
@@ -868,11 +1010,8 @@ __global__ void __launch_bounds__(512, 2) k_fgather(Dev D, const int32_t* __rest
 // every sorted position that is not a stress-point or node target: the half-list length
 // of an active dummy (its pairs with the particles after it in its half stencil), zero
 // counts for inactive positions and dummies' list columns
-__global__ void k_fgather_rest(Dev D) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= D.N2) return;
-  const int a = D.sorted[s];
-  if (a < D.NT) return;  // a stress-point or node target: k_fgather
+__device__ __forceinline__ void gather_rest(const Dev& D, int a) {
+  const int s = D.spos[a];
   const int col = D.lcol[s];
   D.degC[col] = 0;
   D.degS[col] = 0;
@@ -903,15 +1042,58 @@ __global__ void k_fgather_rest(Dev D) {
   D.half_cnt[s] = k;
 }
 
-// pair counts of every realisation (its pairs are the half lists of its sorted range)
-__global__ void k_pair_meta(Dev D) {
+// the stress-point targets [0, bs blocks), the node targets [bs, bn), the dummies: one launch
+template <bool SAME>
+__global__ void __launch_bounds__(512, 2) k_fgather(Dev D, int bs, int bn) {
+  extern __shared__ int gbuf[];
+  const int ns = D.NT - D.NN, b = blockIdx.x;
+  if (b < bs) {
+    const int k = b * blockDim.x + threadIdx.x;
+    if (k < ns) gather_target<SAME>(D, D.tgtS[k], k, gbuf);
+  } else if (b < bn) {
+    const int k = (b - bs) * blockDim.x + threadIdx.x;
+    if (k < D.NN) gather_target<SAME>(D, D.tgtN[k], ns + k, gbuf);
+  } else {
+    const int k = (b - bn) * blockDim.x + threadIdx.x;
+    if (D.NT + k < D.N2) gather_rest(D, D.NT + k);
+  }
+}
+
+// Pair counts: half_off, the exclusive scan of the half-list lengths within kScan sorted
+// positions, and half_bs, the scan of the blocks' sums (readers add the two: half_first), then
+// the pair bookkeeping of every realisation (its pairs are the half lists of its sorted
+// range), both by the last block
+__device__ __forceinline__ int64_t half_first(const Dev& D, int s) {
+  return D.half_off[s] + D.half_bs[s / kScan];
+}
+__global__ void __launch_bounds__(kBlock) k_scan_half(Dev D) {
+  __shared__ long long sh[kBlock / 32];
+  const int base = blockIdx.x * kScan, i0 = base + threadIdx.x * 16;
+  long long l = 0;
+  for (int q = 0; q < 16; q++)
+    if (i0 + q < D.N2) l += D.half_cnt[i0 + q];
+  long long tot;
+  long long run = block_exclusive(l, sh, tot);
+  for (int q = 0; q < 16; q++)
+    if (i0 + q <= D.N2) {  // one past the end: the total
+      D.half_off[i0 + q] = run;
+      if (i0 + q < D.N2) run += D.half_cnt[i0 + q];
+    }
+  if (threadIdx.x == 0) D.half_bs[blockIdx.x] = tot;
+  if (!last_block(D.tick + 2)) return;
+  const long long all = scan_sums(reinterpret_cast<long long*>(D.half_bs), (int)gridDim.x, sh);
+  __syncthreads();
+  auto first = [&](int s) -> int64_t {
+    return (int64_t)__ldcg((const long long*)&D.half_off[s]) +
+           (int64_t)__ldcg((const long long*)&D.half_bs[s / kScan]);
+  };
   const GridTotal gt = *D.gtot;
   for (int r = threadIdx.x; r < D.R; r += blockDim.x) {
     const Grid& g = D.grid[r];
     int64_t lo = 0, hi = 0;
     if (!gt.overflow) {
-      lo = D.half_off[D.cell_start[g.cell0]];
-      hi = D.half_off[D.cell_start[g.cell0 + g.ncells]];
+      lo = first(D.cell_start[g.cell0]);
+      hi = first(D.cell_start[g.cell0 + g.ncells]);
     }
     PairMeta m = D.meta[r];
     m.m_prev = m.m;
@@ -921,7 +1103,7 @@ __global__ void k_pair_meta(Dev D) {
     D.meta[r] = m;
   }
   // walk-order keys hold 2 x position in 32 bits
-  if (threadIdx.x == 0 && D.half_off[D.N2] > 1073741823LL) atomicOr(D.err, ERR_NPAIRS);
+  if (threadIdx.x == 0 && all > 1073741823LL) atomicOr(D.err, ERR_NPAIRS);
 }
 
 template <bool KEYS>
@@ -1075,7 +1257,7 @@ __device__ __forceinline__ void lists_target(const Dev& D, int s, int4& pendC, i
             const int4 e = D.half[(size_t)as[q] * D.capH + pos[q]];
             if ((int)((unsigned)e.x & kHalfIdMask) == t)
               push(cid[q], (int)((unsigned)e.x >> kHalfTypeShift), e.y,
-                   -__int_as_float(e.z), -__int_as_float(e.w), D.half_off[as[q]] + pos[q], false);
+                   -__int_as_float(e.z), -__int_as_float(e.w), half_first(D, as[q]) + pos[q], false);
           }
       }
       {
@@ -1084,7 +1266,7 @@ __device__ __forceinline__ void lists_target(const Dev& D, int s, int4& pendC, i
         for (int k = 0; k < n; k++) {
           int4 e = h[k];
           push((int)((unsigned)e.x & kHalfIdMask), (int)((unsigned)e.x >> kHalfTypeShift), e.y,
-               __int_as_float(e.z), __int_as_float(e.w), D.half_off[s] + k, true);
+               __int_as_float(e.z), __int_as_float(e.w), half_first(D, s) + k, true);
         }
       }
       {
@@ -1127,111 +1309,7 @@ __global__ void k_lists(Dev D) {
     lists_target<KEYS>(D, s, lists_pend[threadIdx.x], lists_pend[blockDim.x + threadIdx.x]);
 }
 
-// ------------------------------------------------------------------------ scans
-template <typename TI, typename TO>
-__global__ void k_scan_blocks(const TI* in, TO* out, TO* bsum, int n, int per_block) {
-  // each block scans per_block elements (per_block = blockDim.x * items)
-  __shared__ TO sh[kBlock];
-  int base = blockIdx.x * per_block;
-  int items = per_block / blockDim.x;
-  int i0 = base + threadIdx.x * items;
-  TO local = 0;
-  for (int k = 0; k < items; k++) {
-    int i = i0 + k;
-    if (i < n) local += (TO)in[i];
-  }
-  sh[threadIdx.x] = local;
-  __syncthreads();
-  for (int o = 1; o < blockDim.x; o <<= 1) {
-    TO v = threadIdx.x >= o ? sh[threadIdx.x - o] : 0;
-    __syncthreads();
-    sh[threadIdx.x] += v;
-    __syncthreads();
-  }
-  TO run = sh[threadIdx.x] - local;  // exclusive prefix of this thread
-  for (int k = 0; k < items; k++) {
-    int i = i0 + k;
-    if (i < n) {
-      out[i] = run;
-      run += (TO)in[i];
-    }
-  }
-  if (threadIdx.x == blockDim.x - 1) bsum[blockIdx.x] = sh[threadIdx.x];
-}
-
-template <typename TO>
-__global__ void k_scan_top(TO* bsum, int nb, TO* total) {
-  // single block: exclusive scan of block sums (sequential chunks of blockDim)
-  __shared__ TO sh[kBlock];
-  __shared__ TO carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int base = 0; base < nb; base += blockDim.x) {
-    int i = base + threadIdx.x;
-    TO v = i < nb ? bsum[i] : 0;
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = 1; o < blockDim.x; o <<= 1) {
-      TO u = threadIdx.x >= o ? sh[threadIdx.x - o] : 0;
-      __syncthreads();
-      sh[threadIdx.x] += u;
-      __syncthreads();
-    }
-    if (i < nb) bsum[i] = sh[threadIdx.x] - v + carry;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry += sh[threadIdx.x];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *total = carry;
-}
-
-template <typename TO>
-__global__ void k_scan_add(TO* out, const TO* bsum, int n, int per_block) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] += bsum[i / per_block];
-}
-
-template <typename TI, typename TO>
-void scan_impl(Ctx& c, const TI* in, TO* out, int n) {
-  const int per_block = kBlock * 16;
-  int nb = (n + per_block - 1) / per_block;
-  TO* bsum = reinterpret_cast<TO*>(c.d.scan_tmp);
-  k_scan_blocks<TI, TO><<<nb, kBlock, 0, c.stream>>>(in, out, bsum, n, per_block);
-  k_scan_top<TO><<<1, kBlock, 0, c.stream>>>(bsum, nb, out + n);
-  k_scan_add<TO><<<(n + kBlock - 1) / kBlock, kBlock, 0, c.stream>>>(out, bsum, n, per_block);
-}
-
 }  // namespace
-
-void scan_i32_to_i32(Ctx& c, const int32_t* in, int32_t* out, int n) { scan_impl(c, in, out, n); }
-void scan_i32_to_i64(Ctx& c, const int32_t* in, int64_t* out, int n) { scan_impl(c, in, out, n); }
-
-// flags (stress-point, node) of every sorted position, for the compaction below
-__global__ void k_target_flags(Dev D) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= D.N2) return;
-  int t = D.sorted[s];
-  D.tflag[s] = (t >= D.NN && t < D.NT) ? 1 : 0;
-  D.tflag[D.N2 + s] = t < D.NN ? 1 : 0;
-}
-__global__ void k_target_scatter(Dev D) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= D.N2) return;
-  const int a = D.toff[s], b = D.toff[D.N2 + 1 + s];  // stress-points, nodes before s
-  int col;
-  if (D.tflag[s]) {
-    D.tgtS[a] = s;
-    col = a;
-    D.colid[col] = D.sorted[s];
-  } else if (D.tflag[D.N2 + s]) {
-    D.tgtN[b] = s;
-    col = (D.NT - D.NN) + b;
-    D.colid[col] = D.sorted[s];
-  } else {
-    col = D.NT + (s - a - b);
-  }
-  D.lcol[s] = col;
-}
 
 // per-target lists (k_lists), one thread per sorted position; keys: with the walk-order
 // keys (and the same-kind entries); same: the same-kind entries even when no step kernel
@@ -1239,90 +1317,61 @@ __global__ void k_target_scatter(Dev D) {
 void launch_lists(Ctx& c, bool keys, bool same = false) {
   Dev D = c.d;
   if (same) D.same_entries = 1;
-  const size_t pend = 2 * sizeof(int4) * (size_t)c.blk[TK_LISTS];
-  if (keys) k_lists<true><<<c.grid_of(TK_LISTS, D.N2), c.blk[TK_LISTS], pend, c.stream>>>(D);
-  else k_lists<false><<<c.grid_of(TK_LISTS, D.N2), c.blk[TK_LISTS], pend, c.stream>>>(D);
+  const int b = Ctx::block_for(D.N2, c.blk[TK_LISTS]), nb = (D.N2 + b - 1) / b;
+  const size_t pend = 2 * sizeof(int4) * (size_t)b;
+  if (keys) k_lists<true><<<nb, b, pend, c.stream>>>(D);
+  else k_lists<false><<<nb, b, pend, c.stream>>>(D);
 }
 
-// the targets split by kind: their sorted positions (tgtS, tgtN) and every position's list
-// column (lcol)
-void split_targets(Ctx& c) {
-  const Dev& D = c.d;
-  const int nb = (D.N2 + kBlock - 1) / kBlock;
-  k_target_flags<<<nb, kBlock, 0, c.stream>>>(D);
-  scan_i32_to_i32(c, D.tflag, D.toff, D.N2);
-  scan_i32_to_i32(c, D.tflag + D.N2, D.toff + D.N2 + 1, D.N2);
-  k_target_scatter<<<nb, kBlock, 0, c.stream>>>(D);
-}
-
-// FP32 form: the lists straight from the cell stencil (k_fgather, one launch per target
-// kind) and the remaining positions' counts; the block size is the tuned pair-search size,
-// lowered until each thread's candidate lists fit 48 KB of shared memory
+// FP32 form: the lists straight from the cell stencil and the remaining positions' counts; the
+// block size is the tuned pair-search size, lowered until each thread's candidate lists fit
+// 48 KB of shared memory and until two blocks an SM have work
 void launch_gather(Ctx& c, bool same, const Dev& D) {
   const size_t per_thread = sizeof(int) * (size_t)(D.capC + (same ? D.capS : 0));
-  int b = std::min(c.blk[TK_HALF], 512);  // k_fgather's launch bounds
+  int b = Ctx::block_for(D.NT, std::min(c.blk[TK_HALF], 512));  // k_fgather's launch bounds
   while (b > 32 && per_thread * (size_t)b > 49152) b >>= 1;
   const size_t sm = per_thread * (size_t)b;
-  const int ns = D.NT - D.NN;
-  c.kernels_launched += 2;
-  if (same) {
-    if (ns > 0) k_fgather<1, true><<<(ns + b - 1) / b, b, sm, c.stream>>>(D, D.tgtS, ns);
-    if (D.NN > 0) k_fgather<2, true><<<(D.NN + b - 1) / b, b, sm, c.stream>>>(D, D.tgtN, D.NN);
-  } else {
-    if (ns > 0) k_fgather<1, false><<<(ns + b - 1) / b, b, sm, c.stream>>>(D, D.tgtS, ns);
-    if (D.NN > 0) k_fgather<2, false><<<(D.NN + b - 1) / b, b, sm, c.stream>>>(D, D.tgtN, D.NN);
-  }
-  k_fgather_rest<<<(D.N2 + kBlock - 1) / kBlock, kBlock, 0, c.stream>>>(D);
+  const int bs = (D.NT - D.NN + b - 1) / b, bn = bs + (D.NN + b - 1) / b;
+  const int nb = bn + (D.N2 - D.NT + b - 1) / b;
+  if (same) k_fgather<true><<<nb, b, sm, c.stream>>>(D, bs, bn);
+  else k_fgather<false><<<nb, b, sm, c.stream>>>(D, bs, bn);
 }
 
 int launch_pair_build(Ctx& c) {
   Dev& D = c.d;
   cudaStream_t st = c.stream;
-  int nb = (D.N2 + kBlock - 1) / kBlock;
+  const int nb = (D.N2 + kBlock - 1) / kBlock;
+  const int b = Ctx::block_for(D.N2, kBlock), nbs = (D.N2 + b - 1) / b;
   c.mark("bbox");
   k_bbox<<<nb, kBlock, 0, st>>>(D);
-  c.mark("grid");
-  k_grid<<<1, kBlock, 0, st>>>(D);
   c.mark("cell_count");
-  cudaMemsetAsync(D.cell_cnt, 0, sizeof(int32_t) * (D.cell_cap + 2), st);
-  cudaMemsetAsync(D.cell_cursor, 0, sizeof(int32_t) * (D.cell_cap + 2), st);
-  k_cell_count<<<nb, kBlock, 0, st>>>(D);
-  c.mark("scan_cells", 3);
-  scan_i32_to_i32(c, D.cell_cnt, D.cell_start, D.cell_cap + 1);
+  k_cell_count<<<nbs, b, 0, st>>>(D);
+  c.mark("scan_cells");
+  k_scan_cells<<<(D.cell_cap + 1 + kScan - 1) / kScan, kBlock, 0, st>>>(D);
   c.mark("cell_fill");
-  k_cell_fill<<<nb, kBlock, 0, st>>>(D);
-  c.mark("cell_sort");
-  k_cell_sort<<<(D.cell_cap + 1 + kBlock - 1) / kBlock, kBlock, 0, st>>>(D);
-  c.mark("spos");
-  k_spos<<<nb, kBlock, 0, st>>>(D);
+  k_cell_fill<<<nbs, b, 0, st>>>(D);
+  c.mark("cell_rank");
+  k_cell_rank<<<nbs, b, 0, st>>>(D);
   // variant bit 2: a download follows most steps; the exact detection wants the keys, the
   // FP32 detection only the same-kind entries
   const bool want = (c.step_variant & 4) != 0;
-  if (c.lists_direct()) {
-    c.mark("split_targets", 8);
-    split_targets(c);
+  const bool direct = c.lists_direct();
+  if (direct) {
     c.mark("gather");
     launch_gather(c, D.same_entries || want, D);
-    c.mark("scan_half", 3);
-    scan_i32_to_i64(c, D.half_cnt, D.half_off, D.N2);
-    c.mark("pair_meta");
-    k_pair_meta<<<1, 128, 0, st>>>(D);
-    c.half_stale = true;
-    return 0;
+  } else {
+    c.mark("half");
+    const int h = Ctx::block_for(D.N2, c.blk[TK_HALF]);
+    if (c.precision == SPS_PREC_FP32_FAST) k_half<true><<<(D.N2 + h - 1) / h, h, 0, st>>>(D);
+    else k_half<false><<<(D.N2 + h - 1) / h, h, 0, st>>>(D);
   }
-  c.mark("half");
-  if (c.precision == SPS_PREC_FP32_FAST)
-    k_half<true><<<c.grid_of(TK_HALF, D.N2), c.blk[TK_HALF], 0, st>>>(D);
-  else k_half<false><<<c.grid_of(TK_HALF, D.N2), c.blk[TK_HALF], 0, st>>>(D);
-  c.mark("scan_half", 3);
-  scan_i32_to_i64(c, D.half_cnt, D.half_off, D.N2);
-  c.mark("pair_meta");
-  k_pair_meta<<<1, 128, 0, st>>>(D);
-  c.mark("split_targets", 8);
-  split_targets(c);
-  c.mark("lists");
-  launch_lists(c, c.surf_every || (want && !c.surface_f32()), want);
-  c.half_stale = false;
+  c.mark("scan_half");
+  k_scan_half<<<(D.N2 + 1 + kScan - 1) / kScan, kBlock, 0, st>>>(D);
+  if (!direct) {
+    c.mark("lists");
+    launch_lists(c, c.surf_every || (want && !c.surface_f32()), want);
+  }
+  c.half_stale = direct;
   return 0;
 }
 

@@ -60,16 +60,8 @@ __device__ __forceinline__ void write_records(const Dev& D, int i, bool rec_i, d
     D.recI[i] = make_float4(f32_rn(D.iv1[i]), f32_rn(D.vol[i]), f32_rn(D.rho[i]), f32_rn(D.mass[i]));
 }
 
-__global__ void k_load_scalars(Dev D) {
-  int k = *D.step_idx;
-  if (D.surr && threadIdx.x < 4) D.cand_count[threadIdx.x] = 0;  // the network's rows
-  for (int r = threadIdx.x; r < D.R; r += blockDim.x) D.cur[r] = D.scal_table[(size_t)k * D.R + r];
-}
-
-// end of a step: the step counter, and the surrogate's gate for the next step
+// end of a step with the surrogate installed: its gate for the next step
 __global__ void k_next_step(Dev D) {
-  *D.step_idx += 1;
-  if (!D.surr) return;
   SurrGate& g = *D.surr_gate;
   const unsigned long long l = D.surr_cnt[0], a = D.surr_cnt[1];
   if (g.on) {
@@ -988,8 +980,6 @@ int launch_plain_step(Ctx& c) {
   Dev& D = c.d;
   cudaStream_t st = c.stream;
   int nbN = (D.NN + kBlock - 1) / kBlock;
-  c.mark("load_scalars");
-  k_load_scalars<<<1, 128, 0, st>>>(D);
   launch_pair_build(c);
   if (c.step_variant & 1) {
     // the outside approach re-interpolates after a shift: stress_point_update and
@@ -1035,8 +1025,10 @@ int launch_plain_step(Ctx& c) {
     c.mark("displ");
     k_displ<<<nbN, kBlock, 0, st>>>(D);
   }
-  c.mark("next_step");
-  k_next_step<<<1, 1, 0, st>>>(D);
+  if (D.surr) {
+    c.mark("next_step");
+    k_next_step<<<1, 1, 0, st>>>(D);
+  }
   return 0;
 }
 

@@ -720,8 +720,9 @@ int sps_create_batch(int32_t nreal, const sps_params* ps, sps_ctx** out) {
     // stress-point and node targets in sorted order (both forms)
     D.tgtS = dalloc<int32_t>(c, NT - NN_ + 1);
     D.tgtN = dalloc<int32_t>(c, NN_ + 1);
-    D.tflag = dalloc<int32_t>(c, 2 * N2);
-    D.toff = dalloc<int32_t>(c, 2 * N2 + 2);
+    D.tflag = dalloc<int32_t>(c, N2);
+    D.tick = dalloc<unsigned>(c, 4);
+    SPS_CUDA_CHECK(cudaMemsetAsync(D.tick, 0, 4 * sizeof(unsigned), c.stream));
     D.lcol = dalloc<int32_t>(c, N2);
     D.colid = dalloc<int32_t>(c, NT);
     if (c.fused()) {
@@ -773,13 +774,13 @@ int sps_create_batch(int32_t nreal, const sps_params* ps, sps_ctx** out) {
     D.half_cnt = dalloc<int32_t>(c, N2);
     D.half_meta = dalloc<int4>(c, N2);
     D.half_off = dalloc<int64_t>(c, N2 + 1);
+    D.half_bs = dalloc<int64_t>(c, N2 / 4096 + 2);
     D.degC = dalloc<int32_t>(c, N2);
     D.degS = dalloc<int32_t>(c, N2);
     D.meta = dalloc<sps::PairMeta>(c, nreal);
     D.step_idx = dalloc<int>(c, 1);
     D.cur = dalloc<sps::StepScalars>(c, nreal);
     D.err = dalloc<int>(c, 1);
-    D.scan_tmp = dalloc<int64_t>(c, (N2 + 4096) / 4096 + 64);
     // upload staging: x, vel, x00 (2 each), stress (4), mass, rho, hsml, intvars1,
     // f_drucker (1 each) as doubles, itype as int32
     c.stage = dalloc<double>(c, 16 * (size_t)N2);
@@ -996,10 +997,13 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
     if (cap > D.cell_cap) {
       D.cell_cnt = dalloc<int32_t>(c, (size_t)cap + 2);
       D.cell_start = dalloc<int32_t>(c, (size_t)cap + 2);
-      D.cell_cursor = dalloc<int32_t>(c, (size_t)cap + 2);
+      D.cntD = dalloc<int32_t>(c, (size_t)cap + 2);
+      D.cell_loc = dalloc<int32_t>(c, (size_t)cap + 2);
+      D.cntK = dalloc<unsigned long long>(c, (size_t)cap + 2);
+      D.cell_locK = dalloc<unsigned long long>(c, (size_t)cap + 2);
+      D.cell_bs = dalloc<int32_t>(c, (size_t)cap / 4096 + 2);
+      D.cell_bsK = dalloc<unsigned long long>(c, (size_t)cap / 4096 + 2);
       D.cell_cap = cap;
-      size_t nscan = std::max<size_t>((size_t)D.N2, (size_t)cap + 2);
-      D.scan_tmp = dalloc<int64_t>(c, nscan / 4096 + 64);
       drop_graphs(c);
     }
     // neighbour capacities: one species holds about pi (scale_k h / dx)^2 partners in the
