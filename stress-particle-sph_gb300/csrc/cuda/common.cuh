@@ -74,6 +74,9 @@ struct PairMeta {
   int64_t m_prev;  // list nodes before this step (m_pairs)
   int64_t m;       // list nodes after this step
   int64_t base;    // global creation index of the realisation's first pair this step
+  // direct lists with new list nodes (n > m_prev): the first new pair's creator and partner
+  // (sorted positions)
+  int newc, newo;
 };
 
 // constants of one realisation (a batch packs problems that share the solver flags but
@@ -169,6 +172,7 @@ struct Dev {
   int same_entries;    // k_lists writes the same-kind lists' entries only when a step kernel
                       // reads them (XSPH, artificial viscosity or stress) or with keys;
                       // their lengths (degS) always
+  int walk_order;  // directly gathered lists are put in walk order (put_walk_order)
   double* artR;        // its per-node rotated tensile stresses R(3) of the stage, (3, NN)
   double *vol, *rinv;  // m / rho and 1 / rho per particle (refreshed when rho changes)
   double* A[3];        // sigma_k / (rho * rho) of the stage, per particle

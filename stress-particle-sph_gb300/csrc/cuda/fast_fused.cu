@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(128) k_fprep(Dev D) {
   load_real(D, t, Mp, scp);
   const Real& M = *Mp;
   const int deg = D.degC[k];
+  if (D.walk_order) put_target_walk_order(D, k, t, k >= ns);
   Kahan nm;
   Kahan e0, e1, e2, e3;
   const double xt = D.px[t], yt = D.py[t];

@@ -640,6 +640,86 @@ __device__ __forceinline__ void cubic_mixed(const Grid& g, dfl dx, dfl dy, float
   }
 }
 
+// RN32(v.hi + v.lo) is certainly the float nearest to every value within |v| rel of it: true
+// when the rest of v and that error stay inside half an ulp of v.hi (a power of two, whose
+// lower neighbour is closer, and values off the ordinary exponents are left undecided)
+__device__ __forceinline__ bool rounds_to_hi(dfl v, float rel) {
+  const unsigned b = __float_as_uint(v.hi), e = (b >> 23) & 0xFFu;
+  if (e < 40u || e > 250u || (b & 0x7FFFFFu) == 0u) return false;
+  return fabsf(v.lo) + fabsf(v.hi) * rel < __uint_as_float((e - 24u) << 23);
+}
+
+// The reference's cubic kernel for a uniform h as the plain form stores it -- the FP64 values of
+// cubic_uniform rounded to FP32 -- from double-float arithmetic, without the FP64 pipe (the
+// separation dx, dy apart): the values are formed to a relative E and kept when no float
+// boundary lies within E of them, so that the FP64 evaluation, which lies within E of them too,
+// rounds to the same floats.  Returns false when undecided (about one pair in a thousand): the
+// caller evaluates in FP64.
+// Bounds, u = 2^-24.  dx, dy split into hi + lo: 2^-48.  The squared sum, its square root and
+// q = r / h in double-float: each step below 2^-44, together below 2^-42.  For q <= 1 the
+// polynomials stay above 1/6 of their largest term: 2^-39.  For q > 1, t = 2 - q carries
+// 2^-41 / t, so t^2 and t^3 carry 3 2^-41 / t + 2^-43.  The FP64 evaluation's own error is
+// below 2^-49 + 2^-49 / t.  E = 2^-38 (q <= 1) and 2^-38 (1 + 1 / t) covers the sums; q
+// within 2^-36 of 1 and t below 2^-9 stay undecided.
+__device__ __forceinline__ bool cubic_certified(const Grid& g, double dxd, double dyd, float* w,
+                                                float* dw0, float* dw1) {
+  dfl dx, dy;
+  f32_split(dxd, dx.hi, dx.lo);
+  f32_split(dyd, dy.hi, dy.lo);
+  const dfl r2 = df_sumsq(dx, dy);
+  if (!(r2.hi > 1e-25f && r2.hi < 1e25f)) return false;
+  const dfl r = df_sqrt(r2);
+  const dfl q = df_mul(r, g.df_yh);
+  const float q1 = (q.hi - 1.0f) + q.lo;
+  dfl W, a;
+  float E;
+  if (q1 < -1.4551915e-11f) {  // -2^-36
+    const dfl q2 = df_mul(q, q), q3 = df_mul(q2, q);
+    dfl b = df_2sum(2.0f / 3.0f, -q2.hi);
+    b = df_fast2sum(b.hi, b.lo - q2.lo);
+    dfl c = df_2sum(b.hi, 0.5f * q3.hi);
+    c = df_fast2sum(c.hi, (c.lo + b.lo) + 0.5f * q3.lo);
+    W = df_mul(g.df_factor, c);
+    const float p = 1.5f * q.hi, pe = fmaf(1.5f, q.hi, -p);
+    dfl m = df_2sum(-2.0f, p);
+    m = df_fast2sum(m.hi, m.lo + fmaf(1.5f, q.lo, pe));
+    a = df_mul(df_mul(g.df_factor, m), g.df_yhh);
+    E = 3.637979e-12f;  // 2^-38
+  } else if (q1 > 1.4551915e-11f) {
+    const dfl t = df_fast2sum(2.0f - q.hi, -q.lo);  // 2 - q.hi is exact
+    if (!(t.hi >= 0.001953125f)) return false;
+    const dfl t2 = df_mul(t, t);
+    W = df_mul(g.df_factor6, df_mul(t2, t));
+    // 1 / r: a Newton step in double-float from the FP32 reciprocal
+    const float y0 = __frcp_rn(r.hi);
+    const float e = fmaf(-r.hi, y0, 1.0f) - r.lo * y0;
+    const dfl y = df_fast2sum(y0, y0 * e);
+    a = df_mul(df_mul(df_mul(g.df_c3, t2), g.df_yh), y);
+    a.hi = -a.hi;
+    a.lo = -a.lo;
+    E = 3.637979e-12f * (1.0f + __frcp_rn(t.hi));
+  } else {
+    return false;
+  }
+  const dfl g0 = df_mul(a, dx), g1 = df_mul(a, dy);
+  *w = W.hi;
+  // a zero separation component: a is negative, so the product is a zero of the other sign
+  *dw0 = dx.hi == 0.0f ? -dx.hi : g0.hi;
+  *dw1 = dy.hi == 0.0f ? -dy.hi : g1.hi;
+  return rounds_to_hi(W, E) && (dx.hi == 0.0f || rounds_to_hi(g0, E)) &&
+         (dy.hi == 0.0f || rounds_to_hi(g1, E));
+}
+
+// the FP64 evaluation of a pair's stored kernel values (out of line: the rare case where h is
+// uniform)
+static __device__ __noinline__ float3 pair_values_f64(const Dev& D, const Grid& g, int a, int b) {
+  double r, dx, dy, mh, w, dw0, dw1;
+  exact_test(D, a, b, r, dx, dy, mh);
+  if (g.uniform_h) cubic_uniform(g, r, dx, dy, &w, &dw0, &dw1);
+  else sph_kernel(D.skf, D.pi, r, dx, dy, mh, &w, &dw0, &dw1);
+  return make_float3(f32_rn(w), f32_rn(dw0), f32_rn(dw1));
+}
+
 // Pairs created by the particle at sorted position s, in the reference's creation order:
 // the rest of its own cell, the cell to its right, then the three cells of the row above.
 // FAST = false: W and dW from the reference's FP64 kernel, stored in FP32 (the plain
@@ -658,16 +738,15 @@ __device__ __forceinline__ int4 half_entry(const Dev& D, const Grid& g, int a, i
   const float cx = (float)qx * cw, cy = (float)qy * ch;
   const float4 rb = D.srec[bs];
   const float fx = (xa - rb.x) - cx, fy = (ya - rb.y) - cy;
-  double r, dx, dy, mh;
-  if (!FAST) exact_test(D, a, b, r, dx, dy, mh);
   float wf, d0f, d1f;
   if (!FAST) {
-    double w, dw0, dw1;
-    if (g.uniform_h) cubic_uniform(g, r, dx, dy, &w, &dw0, &dw1);
-    else sph_kernel(D.skf, D.pi, r, dx, dy, mh, &w, &dw0, &dw1);
-    wf = f32_rn(w);  // the same bits as (float), on the integer pipe
-    d0f = f32_rn(dw0);
-    d1f = f32_rn(dw1);
+    if (!(g.uniform_h &&
+          cubic_certified(g, D.px[a] - D.px[b], D.py[a] - D.py[b], &wf, &d0f, &d1f))) {
+      const float3 v = pair_values_f64(D, g, a, b);
+      wf = v.x;
+      d0f = v.y;
+      d1f = v.z;
+    }
   } else if (g.uniform_h) {
     // separation as double-float from the cell-relative hi/lo offsets
     // x_a - x_b = (offset_a - offset_b) - (cell shift) with every term in double-float
@@ -829,15 +908,15 @@ __device__ __forceinline__ void store_pair(int4* dst, int4 a, int4 b) {
                : "memory");
 }
 
-// ---------------------------------------------------------------- FP32 form: direct lists
-// The FP32 form builds each target's lists straight from its 3 x 3 cell stencil, without
-// the half lists and the search through them.  Scanning the stencil's cells in ascending
+// -------------------------------------------------------------------------- direct lists
+// Where no walk-order keys are wanted, each target's lists are built straight from its 3 x 3
+// cell stencil, without the half lists and the search through them.  Scanning the stencil's cells in ascending
 // sorted position visits a target's partners in the reference's creation order of their
 // pairs: first the creators before it (the row below, the cell to its left, its own cell
 // up to it), one pair each, then its own half list (the rest of its cell, the cell to its
-// right, the row above).  The lists hold that order; the FP32 form's sums use it in every
-// step (the plain form's walk order reverses the newest pairs in steps where the pair
-// count reaches a new maximum).
+// right, the row above).  The lists hold that order.  The FP32 form's sums use it in every
+// step; the plain form's walk order reverses the newest pairs in steps where the pair count
+// reaches a new maximum (put_walk_order, from the first new pair that k_scan_half finds).
 // The pair test is the same symmetric test (prefilter and exact FP64 band test), and the
 // kernel values are evaluated with the target in the creator's role: the separation is
 // negated exactly (double-float additions and the cell shift are sign-symmetric), so W is
@@ -850,13 +929,22 @@ __device__ __forceinline__ void store_pair(int4* dst, int4 a, int4 b) {
 // bit set for a dummy partner), dW/dx, dW/dy} with the gradient with respect to the target.
 // f32: the kernel values in FP32 from the FP32 separation (same-kind entries that only the
 // FP32 free-surface detection reads), otherwise r and r/h in double-float (cubic_mixed)
-__device__ __forceinline__ int4 gather_entry(const Dev& D, const Grid& g, int ta, float xa,
+template <bool PLAIN>
+__device__ __forceinline__ int4 gather_entry(const Dev& D, const Grid& g, int a, int ta, float xa,
                                              float ya, float ha, float xal, float yal, int bs,
                                              int qx, int qy, bool f32 = false) {
   const int b = D.sorted[bs];
   const float4 rb = D.srec[bs];
   float wf, d0f, d1f;
-  if (g.uniform_h && !f32) {
+  if (PLAIN) {
+    if (!(g.uniform_h &&
+          cubic_certified(g, D.px[a] - D.px[b], D.py[a] - D.py[b], &wf, &d0f, &d1f))) {
+      const float3 v = pair_values_f64(D, g, a, b);
+      wf = v.x;
+      d0f = v.y;
+      d1f = v.z;
+    }
+  } else if (g.uniform_h && !f32) {
     const float2 rl = D.srecl[bs];
     cubic_mixed(g, df_sep(xa, xal, rb.x, rl.x, qx, g.df_cell[0]),
                 df_sep(ya, yal, rb.y, rl.y, qy, g.df_cell[1]), &wf, &d0f, &d1f);
@@ -898,7 +986,7 @@ __device__ __forceinline__ bool gather_accept(const Dev& D, int a, float xa, flo
 // accepted ones (sorted position and cell offset) in shared memory; phase 2 evaluates the
 // kernel values, so that a warp's lanes evaluate together.  Dynamic shared memory:
 // (capC + SAME capS) ints per thread, entry k of thread j at k * blockDim + j.
-template <bool SAME>
+template <bool SAME, bool PLAIN>
 __device__ __forceinline__ void gather_target(const Dev& D, int s, int col, int* gbuf) {
   const int bd = blockDim.x, tid = threadIdx.x;
   int* bufC = gbuf;
@@ -981,15 +1069,15 @@ __device__ __forceinline__ void gather_target(const Dev& D, int s, int col, int*
       nC = min(nC, D.capC);
       nS = min(nS, D.capS);
     }
-    const float xal = D.xrl[a], yal = D.yrl[a];
+    const float xal = PLAIN ? 0.0f : D.xrl[a], yal = PLAIN ? 0.0f : D.yrl[a];
     // phase 2: the entries, stored in pairs (whole 32-byte sectors)
     auto finish = [&](const int* buf, int n, int4* list, int2* compact, bool f32) {
       int4 pend = make_int4(0, 0, 0, 0);
       for (int k = 0; k < n; k++) {
         const unsigned v = (unsigned)buf[(size_t)k * bd + tid];
         const int code = (int)(v >> kHalfTypeShift);
-        const int4 e = gather_entry(D, g, ta, xa, ya, ha, xal, yal, (int)(v & kHalfIdMask),
-                                    code % 3 - 1, code / 3 - 1, f32);
+        const int4 e = gather_entry<PLAIN>(D, g, a, ta, xa, ya, ha, xal, yal,
+                                           (int)(v & kHalfIdMask), code % 3 - 1, code / 3 - 1, f32);
         if (k & 1) store_pair(list + ell(k - 1, col, D.N2), pend, e);
         else pend = e;
         // the lanes of a warp write entry k of adjacent columns together: whole sectors
@@ -1043,20 +1131,43 @@ __device__ __forceinline__ void gather_rest(const Dev& D, int a) {
 }
 
 // the stress-point targets [0, bs blocks), the node targets [bs, bn), the dummies: one launch
-template <bool SAME>
+template <bool SAME, bool PLAIN>
 __global__ void __launch_bounds__(512, 2) k_fgather(Dev D, int bs, int bn) {
   extern __shared__ int gbuf[];
   const int ns = D.NT - D.NN, b = blockIdx.x;
   if (b < bs) {
     const int k = b * blockDim.x + threadIdx.x;
-    if (k < ns) gather_target<SAME>(D, D.tgtS[k], k, gbuf);
+    if (k < ns) gather_target<SAME, PLAIN>(D, D.tgtS[k], k, gbuf);
   } else if (b < bn) {
     const int k = (b - bs) * blockDim.x + threadIdx.x;
-    if (k < D.NN) gather_target<SAME>(D, D.tgtN[k], ns + k, gbuf);
+    if (k < D.NN) gather_target<SAME, PLAIN>(D, D.tgtN[k], ns + k, gbuf);
   } else {
     const int k = (b - bn) * blockDim.x + threadIdx.x;
     if (D.NT + k < D.N2) gather_rest(D, D.NT + k);
   }
+}
+
+// The sorted position of the K-th partner (from 0) of the creator at sorted position s: its
+// half stencil in ascending sorted position, which is its creation order
+__device__ __forceinline__ int creator_partner(const Dev& D, int s, int64_t K) {
+  const int a = D.sorted[s];
+  const Grid& g = D.grid[D.rid[a]];
+  const int c = D.cell_of[a] - g.cell0, nx = g.ndiv[0], ny = g.ndiv[1];
+  const int ix = c % nx, iy = c / nx;
+  const float xa = D.xr[a], ya = D.yr[a], ha = D.hr[a];
+  const float cw = (float)g.deltx[0], ch = (float)g.deltx[1];
+  for (int q = 0; q < 5; q++) {
+    const int dx = (q == 1 || q == 4) ? 1 : (q == 2 ? -1 : 0), dy = q >= 2 ? 1 : 0;
+    const int jx = ix + dx, jy = iy + dy;
+    if (jx < 0 || jx >= nx || jy >= ny) continue;
+    const int cc = g.cell0 + jy * nx + jx;
+    const int lo = q == 0 ? s + 1 : D.cell_start[cc], hi = D.cell_start[cc] + D.cell_cnt[cc];
+    for (int bs = lo; bs < hi; bs++)
+      if (gather_accept(D, a, xa, ya, ha, D.srec[bs], bs, (float)dx * cw, (float)dy * ch, g.tau) &&
+          K-- == 0)
+        return bs;
+  }
+  return D.N2;
 }
 
 // Pair counts: half_off, the exclusive scan of the half-list lengths within kScan sorted
@@ -1100,6 +1211,19 @@ __global__ void __launch_bounds__(kBlock) k_scan_half(Dev D) {
     m.n = hi - lo;
     m.base = lo;
     if (m.n > m.m) m.m = m.n;
+    if (D.walk_order && m.n > m.m_prev) {
+      // the first new pair: its creator is the last sorted position whose pairs start at or
+      // before it
+      const int64_t B = m.base + m.m_prev;
+      int a = D.cell_start[g.cell0], b = D.cell_start[g.cell0 + g.ncells];
+      while (b - a > 1) {
+        const int mid = a + (b - a) / 2;
+        if (first(mid) <= B) a = mid;
+        else b = mid;
+      }
+      m.newc = a;
+      m.newo = creator_partner(D, a, B - first(a));
+    }
     D.meta[r] = m;
   }
   // walk-order keys hold 2 x position in 32 bits
@@ -1333,8 +1457,13 @@ void launch_gather(Ctx& c, bool same, const Dev& D) {
   const size_t sm = per_thread * (size_t)b;
   const int bs = (D.NT - D.NN + b - 1) / b, bn = bs + (D.NN + b - 1) / b;
   const int nb = bn + (D.N2 - D.NT + b - 1) / b;
-  if (same) k_fgather<true><<<nb, b, sm, c.stream>>>(D, bs, bn);
-  else k_fgather<false><<<nb, b, sm, c.stream>>>(D, bs, bn);
+  if (D.fast) {
+    if (same) k_fgather<true, false><<<nb, b, sm, c.stream>>>(D, bs, bn);
+    else k_fgather<false, false><<<nb, b, sm, c.stream>>>(D, bs, bn);
+  } else {
+    if (same) k_fgather<true, true><<<nb, b, sm, c.stream>>>(D, bs, bn);
+    else k_fgather<false, true><<<nb, b, sm, c.stream>>>(D, bs, bn);
+  }
 }
 
 int launch_pair_build(Ctx& c) {
@@ -1355,7 +1484,7 @@ int launch_pair_build(Ctx& c) {
   // variant bit 2: a download follows most steps; the exact detection wants the keys, the
   // FP32 detection only the same-kind entries
   const bool want = (c.step_variant & 4) != 0;
-  const bool direct = c.lists_direct();
+  const bool direct = c.step_direct();
   if (direct) {
     c.mark("gather");
     launch_gather(c, D.same_entries || want, D);
@@ -1387,11 +1516,13 @@ Dev build_view(const Ctx& c) {
   return D;
 }
 
-// the half lists of the last pair build, when it gathered the lists directly (the FP32
-// form): the same pairs, counts and creation order
+// the half lists of the last pair build, when it gathered the lists directly: the same pairs,
+// counts and creation order
 void ensure_half_lists(Ctx& c) {
   if (!c.half_stale) return;
-  k_half<true><<<c.grid_of(TK_HALF, c.d.N2), c.blk[TK_HALF], 0, c.stream>>>(build_view(c));
+  const int nb = c.grid_of(TK_HALF, c.d.N2), b = c.blk[TK_HALF];
+  if (c.d.fast) k_half<true><<<nb, b, 0, c.stream>>>(build_view(c));
+  else k_half<false><<<nb, b, 0, c.stream>>>(build_view(c));
   c.half_stale = false;
 }
 
@@ -1404,8 +1535,12 @@ void launch_lists_keys(Ctx& c) {
 
 // the lists of the last step again with the same-kind entries (the FP32 detection)
 void launch_lists_same(Ctx& c) {
-  if (c.lists_direct() && c.half_stale) launch_gather(c, true, build_view(c));
-  else launch_lists(c, false, true);
+  if (c.lists_direct() && c.half_stale && !c.d.walk_order) {
+    launch_gather(c, true, build_view(c));
+  } else {
+    ensure_half_lists(c);
+    launch_lists(c, false, true);
+  }
 }
 
 }  // namespace sps

@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(128) k_pprep(Dev D) {
   load_real(D, t, Mp, scp);
   const Real& M = *Mp;
   const int deg = D.degC[k];
+  if (D.walk_order) put_target_walk_order(D, k, t, k >= ns);
   const double xt = D.px[t], yt = D.py[t];
   double norm = 0.0;
   double AE[4] = {0.0, 0.0, 0.0, 0.0};

@@ -324,10 +324,10 @@ int variant_of(const sps::Ctx& c, int64_t it) {
 void enqueue_step(sps::Ctx& c) {
   c.itimestep += 1;
   c.step_variant = variant_of(c, c.itimestep) | (c.keys_in_step ? 4 : 0);
-  c.keys_written = (c.keys_in_step && !c.surface_f32() && !c.lists_direct()) || c.surf_every;
+  c.keys_written = (c.keys_in_step && !c.surface_f32() && !c.step_direct()) || c.surf_every;
   c.same_written = c.keys_in_step || c.surf_every || c.d.same_entries;
   // set here, on the host, for every step: a replayed graph runs no host code
-  c.half_stale = c.lists_direct();
+  c.half_stale = c.step_direct();
   if (c.use_graph && !c.profiling) {
     if (!c.graphs[c.step_variant]) build_graph(c);
     SPS_CUDA_CHECK(cudaGraphLaunch(c.graphs[c.step_variant], c.stream));
@@ -1050,6 +1050,9 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
     D.bound_from_lists = bfl;
     // the FP32 form's interpolation reads the compact {id, W} entries that the gathered
     // lists also write
+    const int wo = c.lists_direct() && (!D.fast || D.sle == 2) ? 1 : 0;
+    if (wo != D.walk_order) drop_graphs(c);
+    D.walk_order = wo;
     const int uw = c.lists_direct() && D.crossW ? 1 : 0;
     if (uw != D.use_crossW) drop_graphs(c);
     D.use_crossW = uw;

@@ -35,6 +35,38 @@ __device__ __forceinline__ void load_real(const Dev& D, int t, const Real*& M,
   sc = D.cur + r;
 }
 
+// The walk order of a directly gathered list (column col, n entries in creation order) in a step
+// whose pair count passed the list length: the new pairs -- those created from the pair
+// (m.newc, m.newo) on, a suffix of the list -- newest first, then the others.  s: the target's
+// sorted position.
+__device__ __forceinline__ void put_walk_order(const Dev& D, const PairMeta& m, int4* list, int s,
+                                               int col, int n) {
+  int fresh = 0;
+  for (int j = n - 1; j >= 0; j--) {
+    const int p = D.spos[list[ell(j, col, D.N2)].x];
+    const int cr = p < s ? p : s, o = p < s ? s : p;
+    if (cr < m.newc || (cr == m.newc && o < m.newo)) break;
+    fresh++;
+  }
+  auto reverse = [&](int lo, int hi) {
+    for (hi--; lo < hi; lo++, hi--) {
+      const int4 t = list[ell(lo, col, D.N2)];
+      list[ell(lo, col, D.N2)] = list[ell(hi, col, D.N2)];
+      list[ell(hi, col, D.N2)] = t;
+    }
+  };
+  if (fresh == 0) return;
+  reverse(0, n);
+  reverse(fresh, n);
+}
+__device__ __forceinline__ void put_target_walk_order(const Dev& D, int col, int t, bool node) {
+  const PairMeta m = D.meta[D.R == 1 ? 0 : D.rid[t]];
+  if (m.n <= m.m_prev) return;
+  const int s = node ? D.tgtN[col - (D.NT - D.NN)] : D.tgtS[col];
+  put_walk_order(D, m, D.cross, s, col, D.degC[col]);
+  if (D.same_entries) put_walk_order(D, m, D.same, s, col, D.degS[col]);
+}
+
 // BCs (3_SPH_material_2018.f90:1640-1660) for one particle: Normal_BCs (:1665-1770), then
 // with ifsigman = 1 apply_stress_free (:1775-1858): a free-surface node away from the walls
 // keeps only the stress component along the surface (zero normal and shear traction)
