@@ -172,6 +172,7 @@ struct Dev {
   int same_entries;    // k_lists writes the same-kind lists' entries only when a step kernel
                       // reads them (XSPH, artificial viscosity or stress) or with keys;
                       // their lengths (degS) always
+  int same_f32;    // the gathered same-kind entries serve the FP32 detection only
   int walk_order;  // directly gathered lists are put in walk order (put_walk_order)
   double* artR;        // its per-node rotated tensile stresses R(3) of the stage, (3, NN)
   double *vol, *rinv;  // m / rho and 1 / rho per particle (refreshed when rho changes)
@@ -951,7 +952,7 @@ int launch_pair_build(Ctx& c);
 int launch_plain_step(Ctx& c);
 int launch_fast_step(Ctx& c);
 void launch_vol(Ctx& c, int lo, int hi);
-void launch_pprep(Ctx& c);
+void launch_pprep(Ctx& c);  // (both preparations put the lists in walk order)
 void launch_pstage(Ctx& c, int stage);
 void launch_pfinish(Ctx& c);
 void launch_fprep(Ctx& c);

@@ -81,20 +81,20 @@ struct Ctx {
   bool surface_exact = false;
   bool surface_f32() const { return precision == SPS_PREC_FP32_FAST && !surface_exact; }
   int64_t last_refresh = -1;   // steps_done at the last on-demand detection
-  // the steps build their lists straight from the cell stencil (k_fgather) unless every step
-  // runs the exact free-surface detection (its keyed lists come from the half lists), the
+  // the steps build their lists straight from the cell stencil (k_fgather) unless the
   // smoothing lengths evolve (sle 2 with the continuity equation: a rebuild after the step
   // could not repeat the build's band test) or the list capacity leaves no room for the
   // gather's shared memory (two lists of capC ints for each of 32 threads within 48 KB).
   // Where the walk order matters the fused stages' preparation restores it (Dev::walk_order):
-  // always in the plain form, and in the FP32 form with sle 2, whose sums have followed it.
+  // always in the plain form, and in the FP32 form with sle 2 or an exact free-surface
+  // detection in every step, whose sums have followed it.
+  bool walks() const { return precision == SPS_PREC_FP64_PLAIN || d.sle == 2 || surf_every; }
   bool lists_direct() const {
-    const bool walk = precision == SPS_PREC_FP64_PLAIN || d.sle == 2;
-    return !surf_every && !(d.sle == 2 && d.cont_density) && (!walk || fused()) &&
+    return !(d.sle == 2 && d.cont_density) && (!walks() || fused()) &&
            2 * d.capC * 32 * 4 <= 49152;
   }
-  // ... and the plain form's (and sle 2's) steps with keys write the keyed lists instead
-  bool step_direct() const { return lists_direct() && !(d.walk_order && keys_in_step); }
+  // whether this step writes the same-kind lists
+  bool same_now() const { return d.same_entries || surf_every || (step_variant & 4); }
   // one launch per RK4 stage: the positions, lists and densities do not change within a step
   // and nothing between the two halves of a stage needs the whole field (the continuity
   // equation's densities, artificial stress, the traction-free BC's normals do)

@@ -773,7 +773,9 @@ void launch_fstage_kp(Ctx& c, int stage) {
 
 void launch_fprep(Ctx& c) {
   const int b = c.block_for(c.d.NT, 128);
-  k_fprep<<<(c.d.NT + b - 1) / b, b, 0, c.stream>>>(c.d);
+  Dev D = c.d;
+  D.same_entries = c.same_now();  // the lists to put in walk order
+  k_fprep<<<(D.NT + b - 1) / b, b, 0, c.stream>>>(D);
 }
 
 // The look-ahead of the interpolation (ahead[0]) sets the pair; the node derivative sums'

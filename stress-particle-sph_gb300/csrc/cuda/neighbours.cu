@@ -19,6 +19,7 @@
 #include <stdexcept>
 
 #include "ctx.cuh"
+#include "stage_tail.cuh"
 
 namespace sps {
 
@@ -54,6 +55,15 @@ __device__ __forceinline__ dfl df_sqrt(dfl x) {
   float p = s * s;
   float e = fmaf(s, s, -p);
   float r = ((x.hi - p) - e) + x.lo;
+  return df_fast2sum(s, r * (0.5f * __frcp_rn(s)));
+}
+// the same from the correctly rounded FP32 root: its error of 2^-25 leaves a correction that FP32
+// carries to 2^-47 (the FP32 form keeps df_sqrt, and with it its kernel values' last bits)
+__device__ __forceinline__ dfl df_sqrt_rn(dfl x) {
+  const float s = __fsqrt_rn(x.hi);
+  const float p = s * s;
+  const float e = fmaf(s, s, -p);
+  const float r = ((x.hi - p) - e) + x.lo;
   return df_fast2sum(s, r * (0.5f * __frcp_rn(s)));
 }
 // x^2 + y^2 of two double-float values, accurate to a few units of 2^-44: the exact
@@ -653,14 +663,14 @@ __device__ __forceinline__ bool rounds_to_hi(dfl v, float rel) {
 // cubic_uniform rounded to FP32 -- from double-float arithmetic, without the FP64 pipe (the
 // separation dx, dy apart): the values are formed to a relative E and kept when no float
 // boundary lies within E of them, so that the FP64 evaluation, which lies within E of them too,
-// rounds to the same floats.  Returns false when undecided (about one pair in a thousand): the
+// rounds to the same floats.  Returns false when undecided (about one pair in ten thousand): the
 // caller evaluates in FP64.
-// Bounds, u = 2^-24.  dx, dy split into hi + lo: 2^-48.  The squared sum, its square root and
-// q = r / h in double-float: each step below 2^-44, together below 2^-42.  For q <= 1 the
-// polynomials stay above 1/6 of their largest term: 2^-39.  For q > 1, t = 2 - q carries
-// 2^-41 / t, so t^2 and t^3 carry 3 2^-41 / t + 2^-43.  The FP64 evaluation's own error is
-// below 2^-49 + 2^-49 / t.  E = 2^-38 (q <= 1) and 2^-38 (1 + 1 / t) covers the sums; q
-// within 2^-36 of 1 and t below 2^-9 stay undecided.
+// Bounds: dx, dy split into hi + lo, the squared sum and its root to 2^-47, q = r / h to 2^-45.
+// For q > 1, t = 2 - q carries 2^-44 / t, so t^2 and t^3 3 2^-44 / t; for q <= 1 the
+// polynomials lose at most a factor 8 to cancellation.  The FP64 evaluation's own error is below
+// 2^-49 (1 + 1 / t).  E = 2^-41 (1 + 1 / t), 2^-41 for q <= 1; the largest errors met in 2.4e7
+// random pairs (h 3e-4 .. 3, all directions) were 2^-43.1 (1 + 1 / t) and 2^-44.  q within
+// 2^-36 of 1 and t below 2^-9 stay undecided.
 __device__ __forceinline__ bool cubic_certified(const Grid& g, double dxd, double dyd, float* w,
                                                 float* dw0, float* dw1) {
   dfl dx, dy;
@@ -668,7 +678,7 @@ __device__ __forceinline__ bool cubic_certified(const Grid& g, double dxd, doubl
   f32_split(dyd, dy.hi, dy.lo);
   const dfl r2 = df_sumsq(dx, dy);
   if (!(r2.hi > 1e-25f && r2.hi < 1e25f)) return false;
-  const dfl r = df_sqrt(r2);
+  const dfl r = df_sqrt_rn(r2);
   const dfl q = df_mul(r, g.df_yh);
   const float q1 = (q.hi - 1.0f) + q.lo;
   dfl W, a;
@@ -684,7 +694,7 @@ __device__ __forceinline__ bool cubic_certified(const Grid& g, double dxd, doubl
     dfl m = df_2sum(-2.0f, p);
     m = df_fast2sum(m.hi, m.lo + fmaf(1.5f, q.lo, pe));
     a = df_mul(df_mul(g.df_factor, m), g.df_yhh);
-    E = 3.637979e-12f;  // 2^-38
+    E = 4.5474735e-13f;  // 2^-41
   } else if (q1 > 1.4551915e-11f) {
     const dfl t = df_fast2sum(2.0f - q.hi, -q.lo);  // 2 - q.hi is exact
     if (!(t.hi >= 0.001953125f)) return false;
@@ -697,7 +707,7 @@ __device__ __forceinline__ bool cubic_certified(const Grid& g, double dxd, doubl
     a = df_mul(df_mul(df_mul(g.df_c3, t2), g.df_yh), y);
     a.hi = -a.hi;
     a.lo = -a.lo;
-    E = 3.637979e-12f * (1.0f + __frcp_rn(t.hi));
+    E = 4.5474735e-13f * (1.0f + __frcp_rn(t.hi));
   } else {
     return false;
   }
@@ -1088,7 +1098,7 @@ __device__ __forceinline__ void gather_target(const Dev& D, int s, int col, int*
     finish(bufC, nC, D.cross, D.use_crossW ? D.crossW : nullptr, false);
     // same-kind entries that no step kernel reads serve the FP32 free-surface detection
     // only: FP32 kernel values
-    if (SAME) finish(bufS, nS, D.same, nullptr, !D.same_entries);
+    if (SAME) finish(bufS, nS, D.same, nullptr, D.same_f32);
   }
   D.degC[col] = nC;
   D.degS[col] = nS;
@@ -1484,10 +1494,10 @@ int launch_pair_build(Ctx& c) {
   // variant bit 2: a download follows most steps; the exact detection wants the keys, the
   // FP32 detection only the same-kind entries
   const bool want = (c.step_variant & 4) != 0;
-  const bool direct = c.step_direct();
+  const bool direct = c.lists_direct();
   if (direct) {
     c.mark("gather");
-    launch_gather(c, D.same_entries || want, D);
+    launch_gather(c, c.same_now(), D);
   } else {
     c.mark("half");
     const int h = Ctx::block_for(D.N2, c.blk[TK_HALF]);
@@ -1502,6 +1512,13 @@ int launch_pair_build(Ctx& c) {
   }
   c.half_stale = direct;
   return 0;
+}
+
+// both lists of every target from creation order to walk order (a rebuild after the step; in
+// the step the fused stages' preparation does it)
+__global__ void k_walk_order(Dev D) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < D.NT) put_target_walk_order(D, k, D.colid[k], k >= D.NT - D.NN);
 }
 
 // The device view of the last pair build for a rebuild after the step: the FP64 positions
@@ -1535,10 +1552,12 @@ void launch_lists_keys(Ctx& c) {
 
 // the lists of the last step again with the same-kind entries (the FP32 detection)
 void launch_lists_same(Ctx& c) {
-  if (c.lists_direct() && c.half_stale && !c.d.walk_order) {
-    launch_gather(c, true, build_view(c));
+  if (c.lists_direct()) {
+    Dev D = build_view(c);
+    launch_gather(c, true, D);
+    D.same_entries = 1;
+    if (D.walk_order) k_walk_order<<<(D.NT + kBlock - 1) / kBlock, kBlock, 0, c.stream>>>(D);
   } else {
-    ensure_half_lists(c);
     launch_lists(c, false, true);
   }
 }

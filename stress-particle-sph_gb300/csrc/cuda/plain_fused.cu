@@ -769,7 +769,9 @@ __global__ void __launch_bounds__(128) k_pfinish(Dev D) {
 
 void launch_pprep(Ctx& c) {
   const int b = c.block_for(c.d.NT, 128);
-  k_pprep<<<(c.d.NT + b - 1) / b, b, 0, c.stream>>>(c.d);
+  Dev D = c.d;
+  D.same_entries = c.same_now();  // the lists to put in walk order
+  k_pprep<<<(D.NT + b - 1) / b, b, 0, c.stream>>>(D);
 }
 
 // Lanes a target: split by component while one lane a target leaves most of the chip's 608

@@ -324,10 +324,10 @@ int variant_of(const sps::Ctx& c, int64_t it) {
 void enqueue_step(sps::Ctx& c) {
   c.itimestep += 1;
   c.step_variant = variant_of(c, c.itimestep) | (c.keys_in_step ? 4 : 0);
-  c.keys_written = (c.keys_in_step && !c.surface_f32() && !c.step_direct()) || c.surf_every;
+  c.keys_written = !c.d.walk_order && ((c.keys_in_step && !c.surface_f32() && !c.lists_direct()) || c.surf_every);
   c.same_written = c.keys_in_step || c.surf_every || c.d.same_entries;
   // set here, on the host, for every step: a replayed graph runs no host code
-  c.half_stale = c.step_direct();
+  c.half_stale = c.lists_direct();
   if (c.use_graph && !c.profiling) {
     if (!c.graphs[c.step_variant]) build_graph(c);
     SPS_CUDA_CHECK(cudaGraphLaunch(c.graphs[c.step_variant], c.stream));
@@ -845,7 +845,12 @@ void refresh_surface(sps::Ctx& c, bool sync = true) {
     if (!c.same_written) sps::launch_lists_same(c);
     sps::launch_surface_f32(c);
   } else {
-    if (!c.keys_written) sps::launch_lists_keys(c);
+    // directly gathered lists in walk order need no keys, but their same-kind entries
+    if (c.d.walk_order) {
+      if (!c.same_written) sps::launch_lists_same(c);
+    } else if (!c.keys_written) {
+      sps::launch_lists_keys(c);
+    }
     sps::launch_surface(c);
   }
   SPS_CUDA_CHECK(cudaGetLastError());
@@ -1050,9 +1055,10 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
     D.bound_from_lists = bfl;
     // the FP32 form's interpolation reads the compact {id, W} entries that the gathered
     // lists also write
-    const int wo = c.lists_direct() && (!D.fast || D.sle == 2) ? 1 : 0;
+    const int wo = c.lists_direct() && c.walks() ? 1 : 0;
     if (wo != D.walk_order) drop_graphs(c);
     D.walk_order = wo;
+    D.same_f32 = D.fast && !D.same_entries && !c.surf_every;
     const int uw = c.lists_direct() && D.crossW ? 1 : 0;
     if (uw != D.use_crossW) drop_graphs(c);
     D.use_crossW = uw;

@@ -23,46 +23,85 @@ namespace {
 
 constexpr int kBlock = 256;
 
+// Where the lists were gathered directly (SP) a target's entries need no stored keys: its pairs
+// are created in ascending sorted position of the partner, so that position orders them, the
+// new pairs (a suffix, when the pair count passed the list length) newest first before the
+// others; and the target created the pairs with partners after it.
+struct WalkOrder {
+  int s;  // the target's sorted position
+  bool grown;
+  int newc, newo;
+};
+__device__ __forceinline__ WalkOrder walk_order_of(const Dev& D, int s, int t) {
+  const PairMeta& m = D.meta[D.R == 1 ? 0 : D.rid[t]];
+  WalkOrder w;
+  w.s = s;
+  w.grown = m.n > m.m_prev;
+  w.newc = m.newc;
+  w.newo = m.newo;
+  return w;
+}
+__device__ __forceinline__ int walk_key(const WalkOrder& w, int p) {
+  if (!w.grown) return p;
+  const int cr = min(p, w.s), o = max(p, w.s);
+  return cr > w.newc || (cr == w.newc && o >= w.newo) ? -1 - p : p;
+}
+
 // the merged walk over a target's node--stress-point (cross, non-dummy neighbour) and
-// same-type entries, in ascending key; f(u, gx, gy, is_pair_i)
-template <typename F>
-__device__ __forceinline__ void walk_123(const Dev& D, int col, F&& f) {
+// same-type entries, in ascending key; f(u, gx, gy, is_pair_i); sp: the target is a
+// stress-point
+template <bool SP, typename F>
+__device__ __forceinline__ void walk_123(const Dev& D, int col, const WalkOrder& W, bool sp,
+                                         F&& f) {
   const int nC = D.degC[col], nS = D.degS[col];
   int a = 0, b = 0;
   int32_t ka = 0, kb = 0;
+  bool ia = false, ib = false;  // is_pair_i
   int4 ea = make_int4(0, 0, 0, 0), eb = make_int4(0, 0, 0, 0);
   auto next_cross = [&]() {
     while (a < nC) {
       ea = D.cross[ell(a, col, D.N2)];
       if (ea.y >= 0) {  // not a dummy partner (sign bit of W)
-        ka = D.keyC[(size_t)a * D.N2 + col];
+        if (SP) {
+          ka = walk_key(W, D.spos[ea.x]);
+          ia = sp;
+        } else {
+          ka = D.keyC[(size_t)a * D.N2 + col];
+          ia = (ka & 1) != 0;
+        }
         return;
       }
       a++;
     }
   };
-  next_cross();
-  if (b < nS) {
+  auto next_same = [&]() {
+    if (b >= nS) return;
     eb = D.same[ell(b, col, D.N2)];
-    kb = D.keyS[(size_t)b * D.N2 + col];
-  }
+    if (SP) {
+      const int p = D.spos[eb.x];
+      kb = walk_key(W, p);
+      ib = p > W.s;
+    } else {
+      kb = D.keyS[(size_t)b * D.N2 + col];
+      ib = (kb & 1) != 0;
+    }
+  };
+  next_cross();
+  next_same();
   while (a < nC || b < nS) {
     // one call site for both lists, so that a warp whose lanes take different lists runs
     // the body once
     const bool takeC = (a < nC) && (b >= nS || ka < kb);
     const int u = takeC ? ea.x : eb.x;
     const int gx = takeC ? ea.z : eb.z, gy = takeC ? ea.w : eb.w;
-    const int32_t key = takeC ? ka : kb;
-    f(u, __int_as_float(gx), __int_as_float(gy), (key & 1) != 0);
+    const bool pair_i = takeC ? ia : ib;
+    f(u, __int_as_float(gx), __int_as_float(gy), pair_i);
     if (takeC) {
       a++;
       next_cross();
     } else {
       b++;
-      if (b < nS) {
-        eb = D.same[ell(b, col, D.N2)];
-        kb = D.keyS[(size_t)b * D.N2 + col];
-      }
+      next_same();
     }
   }
 }
@@ -81,24 +120,47 @@ __device__ __forceinline__ float acc_f64(float acc, double d, float h) {
   return f32_rn(f64_of(acc) + d * f64_of(h));
 }
 
+// L = 4: lane q of a target's four sums component q of the renormalisation matrix (each still
+// in walk order by one lane), for problems too small to fill the chip with one lane a target
+template <bool SP, int L>
 __global__ void k_fs_normal0(Dev D) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= D.N2) return;
-  const int t = D.sorted[s];
-  if (t >= D.NT) return;
+  const int s = (blockIdx.x * blockDim.x + threadIdx.x) / L, q = threadIdx.x & (L - 1);
+  const bool act = s < D.N2 && D.sorted[s < D.N2 ? s : 0] < D.NT;
+  if (L == 1 && !act) return;
+  const int t = act ? D.sorted[s] : 0;
   const double xt = D.px[t], yt = D.py[t];
   float A0 = 0.0f, A1 = 0.0f, A2 = 0.0f, A3 = 0.0f, f0 = 0.0f, f1 = 0.0f;
-  walk_123(D, D.lcol[s], [&](int u, float gx, float gy, bool) {
-    const double m = D.mass[u], rho = D.rho[u], ri = D.rinv[u];
-    float h1 = hf_of(m, rho, ri, gx), h2 = hf_of(m, rho, ri, gy);
-    double dx = D.px[u] - xt, dy = D.py[u] - yt;
-    A0 = acc_f64(A0, dx, h1);
-    A1 = acc_f64(A1, dy, h1);
-    A2 = acc_f64(A2, dx, h2);
-    A3 = acc_f64(A3, dy, h2);
-    f0 = f0 + h1;
-    f1 = f1 + h2;
-  });
+  if (act)
+    walk_123<SP>(D, D.lcol[s], walk_order_of(D, s, t), t >= D.NN,
+                 [&](int u, float gx, float gy, bool) {
+      const double m = D.mass[u], rho = D.rho[u], ri = D.rinv[u];
+      if (L == 1) {
+        float h1 = hf_of(m, rho, ri, gx), h2 = hf_of(m, rho, ri, gy);
+        double dx = D.px[u] - xt, dy = D.py[u] - yt;
+        A0 = acc_f64(A0, dx, h1);
+        A1 = acc_f64(A1, dy, h1);
+        A2 = acc_f64(A2, dx, h2);
+        A3 = acc_f64(A3, dy, h2);
+        f0 = f0 + h1;
+        f1 = f1 + h2;
+      } else {
+        const float h = hf_of(m, rho, ri, q < 2 ? gx : gy);
+        const double d = (q & 1) ? D.py[u] - yt : D.px[u] - xt;
+        A0 = acc_f64(A0, d, h);
+        f0 = f0 + h;
+      }
+    });
+  if (L == 4) {
+    const int b0 = threadIdx.x & 31 & ~3;
+    const float a = A0, f = f0;
+    A0 = __shfl_sync(0xffffffffu, a, b0);
+    A1 = __shfl_sync(0xffffffffu, a, b0 + 1);
+    A2 = __shfl_sync(0xffffffffu, a, b0 + 2);
+    A3 = __shfl_sync(0xffffffffu, a, b0 + 3);
+    f0 = __shfl_sync(0xffffffffu, f, b0);
+    f1 = __shfl_sync(0xffffffffu, f, b0 + 2);
+    if (q || !act) return;
+  }
   if (fabsf(A0) <= 1.e-8f) A0 = 0.0f;
   if (fabsf(A1) <= 1.e-8f) A1 = 0.0f;
   if (fabsf(A2) <= 1.e-8f) A2 = 0.0f;
@@ -149,23 +211,37 @@ __device__ __forceinline__ bool in_scan_region(const ScanRegion& R, double xb, d
   return false;  // a NaN distance lies in neither part of the region
 }
 
+// L lanes a target look at its neighbours together (any order: one in the region decides)
+template <int L>
 __global__ void k_fs_scan(Dev D) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= D.N2) return;
-  const int t = D.sorted[s];
-  if (t >= D.NT) return;
+  const int s = (blockIdx.x * blockDim.x + threadIdx.x) / L, q = threadIdx.x & (L - 1);
+  const bool act = s < D.N2 && D.sorted[s < D.N2 ? s : 0] < D.NT;
+  if (L == 1 && !act) return;
+  const int t = act ? D.sorted[s] : 0;
   bool inside = false;
-  const int col = D.lcol[s];
-  const int nS = D.degS[col], nC = D.degC[col];
+  const int col = act ? D.lcol[s] : 0;
+  const int nS = act ? D.degS[col] : 0, nC = act ? D.degC[col] : 0;
   const ScanRegion R = scan_region(D, t);
-  for (int k = 0; k < nS && !inside; k++) {
-    int u = D.same[ell(k, col, D.N2)].x;
-    inside = in_scan_region(R, D.px[u], D.py[u]);
+  // every lane of a group agrees to stop
+  const unsigned grp = L == 1 ? 0u : (L == 32 ? ~0u : ((1u << L) - 1u) << (threadIdx.x & 31 & ~(L - 1)));
+  auto any = [&](bool b) { return L == 1 ? b : __any_sync(grp, b) != 0; };
+  for (int k = 0; k < nS && !inside; k += L) {
+    bool in = false;
+    if (k + q < nS) {
+      const int u = D.same[ell(k + q, col, D.N2)].x;
+      in = in_scan_region(R, D.px[u], D.py[u]);
+    }
+    inside = any(in);
   }
-  for (int k = 0; k < nC && !inside; k++) {
-    const int4 e = D.cross[ell(k, col, D.N2)];
-    if (e.y < 0) inside = in_scan_region(R, D.px[e.x], D.py[e.x]);  // dummy partners
+  for (int k = 0; k < nC && !inside; k += L) {
+    bool in = false;
+    if (k + q < nC) {
+      const int4 e = D.cross[ell(k + q, col, D.N2)];
+      if (e.y < 0) in = in_scan_region(R, D.px[e.x], D.py[e.x]);  // dummy partners
+    }
+    inside = any(in);
   }
+  if (q || !act) return;
   int sub = inside ? 2 : 1;
   D.fint[t] = inside ? -1.0f : 0.0f;
   int bc = D.bc_or_not[t];
@@ -175,18 +251,26 @@ __global__ void k_fs_scan(Dev D) {
   D.subset[t] = (int8_t)sub;
 }
 
+// A particle inside the body has no normal (0): its sums would only decide the sign of one, so
+// they are formed for the surface particles alone.
+template <bool SP>
 __global__ void k_fs_normal(Dev D) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= D.N2) return;
   const int t = D.sorted[s];
   if (t >= D.NT) return;
-  const bool surf = D.subset[t] == 1;
+  if (D.subset[t] != 1) {
+    D.nrmx[t] = 0.0;
+    D.nrmy[t] = 0.0;
+    return;
+  }
   const float ft = D.fint[t];
   const float xtf = (float)D.px[t], ytf = (float)D.py[t];
   double nx = 0.0, ny = 0.0;
   float nb = 0.0f, g0 = 0.0f, g1 = 0.0f;
-  walk_123(D, D.lcol[s], [&](int u, float gx, float gy, bool pair_i) {
-    if (surf && D.subset[u] == 1) {
+  walk_123<SP>(D, D.lcol[s], walk_order_of(D, s, t), t >= D.NN,
+               [&](int u, float gx, float gy, bool pair_i) {
+    if (D.subset[u] == 1) {
       // the reference adds the same vector x_j - x_i to both particles of the pair
       float xu = (float)D.px[u], yu = (float)D.py[u];
       float xv = pair_i ? xu - xtf : xtf - xu;
@@ -201,17 +285,15 @@ __global__ void k_fs_normal(Dev D) {
     g0 = g0 + df * h1;
     g1 = g1 + df * h2;
   });
-  if (surf) {
-    nx = nx / (double)nb;
-    ny = ny / (double)nb;
-    float nv = (float)sqrt(nx * nx + ny * ny);
-    nx = nx / (double)nv;
-    ny = ny / (double)nv;
-    float p = (float)((double)g0 * nx + (double)g1 * ny);
-    if (p < 0) {
-      nx = -nx;
-      ny = -ny;
-    }
+  nx = nx / (double)nb;
+  ny = ny / (double)nb;
+  float nv = (float)sqrt(nx * nx + ny * ny);
+  nx = nx / (double)nv;
+  ny = ny / (double)nv;
+  float p = (float)((double)g0 * nx + (double)g1 * ny);
+  if (p < 0) {
+    nx = -nx;
+    ny = -ny;
   }
   D.nrmx[t] = nx;
   D.nrmy[t] = ny;
@@ -312,7 +394,11 @@ __global__ void k_fs_normal_f32(Dev D) {
   if (s >= D.N2) return;
   const int t = D.sorted[s];
   if (t >= D.NT) return;
-  const bool surf = D.subset[t] == 1;
+  if (D.subset[t] != 1) {  // no normal inside the body (as k_fs_normal)
+    D.nrmx[t] = 0.0;
+    D.nrmy[t] = 0.0;
+    return;
+  }
   const bool t_sp = is_sp(D.itype[t]);
   const float ft = D.fint[t];
   const double xt = D.px[t], yt = D.py[t];
@@ -337,7 +423,7 @@ __global__ void k_fs_normal_f32(Dev D) {
   Sum nx, ny, g0, g1;
   float nb = 0.0f;
   walk_123_f32(D, D.lcol[s], [&](int u, float gx, float gy, bool same) {
-    if (surf && D.subset[u] == 1) {
+    if (D.subset[u] == 1) {
       // the reference adds the same vector x_j - x_i to both particles of the pair
       const bool pair_i = same ? s < D.spos[u] : t_sp;
       const float xv = f32_rn(pair_i ? D.px[u] - xt : xt - D.px[u]);
@@ -351,18 +437,14 @@ __global__ void k_fs_normal_f32(Dev D) {
     g0.add_prod(df, v * gx);
     g1.add_prod(df, v * gy);
   });
-  double dnx = 0.0, dny = 0.0;
-  if (surf) {
-    dnx = nx.val() / (double)nb;
-    dny = ny.val() / (double)nb;
-    const float nv = (float)sqrt(dnx * dnx + dny * dny);
-    dnx = dnx / (double)nv;
-    dny = dny / (double)nv;
-    const float p = (float)(g0.val() * dnx + g1.val() * dny);
-    if (p < 0) {
-      dnx = -dnx;
-      dny = -dny;
-    }
+  double dnx = nx.val() / (double)nb, dny = ny.val() / (double)nb;
+  const float nv = (float)sqrt(dnx * dnx + dny * dny);
+  dnx = dnx / (double)nv;
+  dny = dny / (double)nv;
+  const float p = (float)(g0.val() * dnx + g1.val() * dny);
+  if (p < 0) {
+    dnx = -dnx;
+    dny = -dny;
   }
   D.nrmx[t] = dnx;
   D.nrmy[t] = dny;
@@ -371,19 +453,31 @@ __global__ void k_fs_normal_f32(Dev D) {
 }  // namespace
 
 void launch_surface_f32(Ctx& c) {
-  const int nb = (c.d.N2 + kBlock - 1) / kBlock;
+  const int b = Ctx::block_for(c.d.N2, kBlock), nb = (c.d.N2 + b - 1) / b;
   c.mark("surface", 3);
   k_fs_vol32<<<(c.d.NT + kBlock - 1) / kBlock, kBlock, 0, c.stream>>>(c.d);
-  k_fs_normal_scan_f32<<<nb, kBlock, 0, c.stream>>>(c.d);
-  k_fs_normal_f32<<<nb, kBlock, 0, c.stream>>>(c.d);
+  k_fs_normal_scan_f32<<<nb, b, 0, c.stream>>>(c.d);
+  k_fs_normal_f32<<<nb, b, 0, c.stream>>>(c.d);
 }
 
 void launch_surface(Ctx& c) {
-  const int nb = (c.d.N2 + kBlock - 1) / kBlock;
+  const Dev& D = c.d;
+  const int b = Ctx::block_for(D.N2, kBlock), nb = (D.N2 + b - 1) / b;
+  const bool direct = D.walk_order;  // lists gathered directly, in walk order
   c.mark("surface", 3);
-  k_fs_normal0<<<nb, kBlock, 0, c.stream>>>(c.d);
-  k_fs_scan<<<nb, kBlock, 0, c.stream>>>(c.d);
-  k_fs_normal<<<nb, kBlock, 0, c.stream>>>(c.d);
+  if (D.NT <= c.split_max) {
+    const int b4 = Ctx::block_for(4 * (int64_t)D.N2, kBlock);
+    const int n4 = (int)((4 * (int64_t)D.N2 + b4 - 1) / b4), n8 = (int)((8 * (int64_t)D.N2 + b4 - 1) / b4);
+    if (direct) k_fs_normal0<true, 4><<<n4, b4, 0, c.stream>>>(D);
+    else k_fs_normal0<false, 4><<<n4, b4, 0, c.stream>>>(D);
+    k_fs_scan<8><<<n8, b4, 0, c.stream>>>(D);
+  } else {
+    if (direct) k_fs_normal0<true, 1><<<nb, b, 0, c.stream>>>(D);
+    else k_fs_normal0<false, 1><<<nb, b, 0, c.stream>>>(D);
+    k_fs_scan<1><<<nb, b, 0, c.stream>>>(D);
+  }
+  if (direct) k_fs_normal<true><<<nb, b, 0, c.stream>>>(D);
+  else k_fs_normal<false><<<nb, b, 0, c.stream>>>(D);
 }
 
 }  // namespace sps
