@@ -48,11 +48,20 @@ struct Ctx {
   cudaStream_t stream = nullptr;
   int device = 0;
   std::vector<void*> allocs;
+  // the context's arrays are cut from a few large allocations (dalloc): what is left of the
+  // last one
+  char* arena = nullptr;
+  size_t arena_left = 0, arena_chunk = 0;
   StepScalars* d_scal_table = nullptr;
   int scal_cap = 0;  // steps
   std::vector<StepScalars> h_scal;
-  int* h_err = nullptr;  // pinned
-  unsigned long long* h_chk = nullptr;  // pinned: upload checks and extents
+  // pinned: the error word, the upload checks and extents, and the packed fields of small
+  // realisations on their way to or from the caller's arrays (kPackBytes at most)
+  char* h_pin = nullptr;
+  int* h_err = nullptr;
+  unsigned long long* h_chk = nullptr;
+  char* h_pack = nullptr;
+  size_t pack_cap = 0;
   unsigned long long* d_chk = nullptr;
   double* stage = nullptr;  // device staging for interleaved host arrays (10 x ntotal2)
   bool uploaded = false;

@@ -43,13 +43,34 @@ std::string g_create_error;
 
 constexpr int kBlock = 256;
 
+// n elements of device memory for the life of the context.  Small requests are cut from a
+// chunk (a context holds about ninety arrays, and an allocation call costs about 10 us); one
+// that would waste much of a chunk is an allocation of its own.
 template <typename T>
 T* dalloc(sps::Ctx& c, size_t n) {
+  const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~(size_t)255;
   void* p = nullptr;
-  SPS_CUDA_CHECK(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)));
+  if (bytes > c.arena_left && bytes <= c.arena_chunk / 4) {
+    SPS_CUDA_CHECK(cudaMalloc(&p, c.arena_chunk));
+    c.allocs.push_back(p);
+    c.arena = static_cast<char*>(p);
+    c.arena_left = c.arena_chunk;
+  }
+  if (bytes <= c.arena_left) {
+    p = c.arena;
+    c.arena += bytes;
+    c.arena_left -= bytes;
+    return reinterpret_cast<T*>(p);
+  }
+  SPS_CUDA_CHECK(cudaMalloc(&p, bytes));
   c.allocs.push_back(p);
   return static_cast<T*>(p);
 }
+
+// realisations whose packed fields are at most this long cross the bus as one copy through
+// pinned memory: eight copies into the caller's pageable arrays cost about 8 us each, the host
+// copy of 1 MB about 60
+constexpr size_t kPackBytes = 1 << 20;
 
 double tcurve_value(const sps::HostReal& h, int it, double t) {
   int nc = h.p.ntcurves;
@@ -112,21 +133,6 @@ void segments(const sps::Ctx& c, int r, Seg* s) {
   s[0] = {0, M.nnode, M.node0};
   s[1] = {M.nnode, M.nsp, M.sp0};
   s[2] = {(int64_t)M.nnode + M.nsp, M.ndum, M.dum0};
-}
-
-__global__ void k_aos_to_soa2(const double* in, double* a, double* b, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    a[i] = in[2 * (size_t)i];
-    b[i] = in[2 * (size_t)i + 1];
-  }
-}
-__global__ void k_soa_to_aos2(double* out, const double* a, const double* b, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    out[2 * (size_t)i] = a[i];
-    out[2 * (size_t)i + 1] = b[i];
-  }
 }
 
 // ordered key of a double: unsigned order of the keys = numeric order of the values
@@ -270,23 +276,96 @@ __global__ void k_snap_pack(sps::Dev D, char* out, const int64_t* roff) {
     s[2 * l + 1] = make_double2(0.0, 0.0);
   }
 }
-__global__ void k_aos_to_soa4(const double* in, double* a, double* b, double* c, double* d, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    a[i] = in[4 * (size_t)i];
-    b[i] = in[4 * (size_t)i + 1];
-    c[i] = in[4 * (size_t)i + 2];
-    d[i] = in[4 * (size_t)i + 3];
+// realisation r's fields, one thread a local particle, in the layout of snap_block
+__global__ void k_pack_real(sps::Dev D, int r, char* base) {
+  const sps::Real& M = D.real[r];
+  const int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t nn = M.nnode, nt = nn + M.nsp, n2 = nt + M.ndum;
+  if (l >= n2) return;
+  const int g = (int)(l < nn ? M.node0 + l : l < nt ? M.sp0 + (l - nn) : M.dum0 + (l - nt));
+  const SnapBlock b = snap_block(nn, nt, n2);
+  double2* s = reinterpret_cast<double2*>(base + b.stress);
+  reinterpret_cast<double2*>(base + b.x)[l] = make_double2(D.px[g], D.py[g]);
+  reinterpret_cast<double2*>(base + b.vel)[l] = make_double2(D.vx[g], D.vy[g]);
+  reinterpret_cast<double*>(base + b.rho)[l] = D.rho[g];
+  if (l >= nt) {
+    // dummy stress is pair-local in the reference; report zero like its RK4 clear (:690)
+    s[2 * l] = s[2 * l + 1] = make_double2(0.0, 0.0);
+    return;
   }
+  s[2 * l] = make_double2(D.s0[g], D.s1[g]);
+  s[2 * l + 1] = make_double2(D.s2[g], D.s3[g]);
+  reinterpret_cast<double*>(base + b.iv1)[l] = D.iv1[g];
+  reinterpret_cast<double*>(base + b.fdp)[l] = D.fdp[g];
+  reinterpret_cast<int32_t*>(base + b.bc)[l] = D.bc_or_not[g];
+  if (l < nn) reinterpret_cast<double2*>(base + b.displ)[l] = make_double2(D.dispx[g], D.dispy[g]);
 }
-__global__ void k_soa_to_aos4(double* out, const double* a, const double* b, const double* c,
-                              const double* d, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    out[4 * (size_t)i] = a[i];
-    out[4 * (size_t)i + 1] = b[i];
-    out[4 * (size_t)i + 2] = c[i];
-    out[4 * (size_t)i + 3] = d[i];
+
+// an uploaded realisation: x(2,n2) vel(2,n2) x00(2,n2) stress(4,n2) mass rho hsml(n2)
+// intvars1 f_drucker(nt) itype(n2), each field on a 256-byte boundary
+struct UpBlock {
+  size_t x, vel, x00, stress, mass, rho, hsml, iv1, fdp, itype, bytes;
+};
+__host__ __device__ inline UpBlock up_block(int64_t nt, int64_t n2) {
+  UpBlock b;
+  auto up = [](size_t v) { return (v + 255) / 256 * 256; };
+  b.x = 0;
+  b.vel = b.x + up(16 * n2);
+  b.x00 = b.vel + up(16 * n2);
+  b.stress = b.x00 + up(16 * n2);
+  b.mass = b.stress + up(32 * n2);
+  b.rho = b.mass + up(8 * n2);
+  b.hsml = b.rho + up(8 * n2);
+  b.iv1 = b.hsml + up(8 * n2);
+  b.fdp = b.iv1 + up(8 * nt);
+  b.itype = b.fdp + up(8 * nt);
+  b.bytes = b.itype + up(4 * n2);
+  return b;
+}
+// an upload's fields into the state of realisation r (one pass instead of about thirty copies,
+// transposes and clears), and the start values of its checks
+__global__ void k_unpack_real(sps::Dev D, int r, const char* base, bool iv, bool fdp,
+                              unsigned long long* chk) {
+  const sps::Real& M = D.real[r];
+  const int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (l < 8) chk[l] = l < 6 ? ~0ull : 0ull;
+  const int64_t nn = M.nnode, nt = nn + M.nsp, n2 = nt + M.ndum;
+  if (l >= n2) return;
+  const int g = (int)(l < nn ? M.node0 + l : l < nt ? M.sp0 + (l - nn) : M.dum0 + (l - nt));
+  const UpBlock b = up_block(nt, n2);
+  const double2 x = reinterpret_cast<const double2*>(base + b.x)[l];
+  const double2 v = reinterpret_cast<const double2*>(base + b.vel)[l];
+  const double2 x0 = reinterpret_cast<const double2*>(base + b.x00)[l];
+  const double2 s01 = reinterpret_cast<const double2*>(base + b.stress)[2 * l];
+  const double2 s23 = reinterpret_cast<const double2*>(base + b.stress)[2 * l + 1];
+  const double rho = reinterpret_cast<const double*>(base + b.rho)[l];
+  D.px[g] = x.x;
+  D.py[g] = x.y;
+  D.vx[g] = v.x;
+  D.vy[g] = v.y;
+  D.x00x[g] = x0.x;
+  D.x00y[g] = x0.y;
+  D.s0[g] = s01.x;
+  D.s1[g] = s01.y;
+  D.s2[g] = s23.x;
+  D.s3[g] = s23.y;
+  D.mass[g] = reinterpret_cast<const double*>(base + b.mass)[l];
+  D.rho[g] = rho;
+  D.hsml[g] = reinterpret_cast<const double*>(base + b.hsml)[l];
+  D.itype[g] = reinterpret_cast<const int32_t*>(base + b.itype)[l];
+  D.out[g] = 0;
+  if (l < nt) {
+    D.iv1[g] = iv ? reinterpret_cast<const double*>(base + b.iv1)[l] : 0.0;
+    D.fdp[g] = fdp ? reinterpret_cast<const double*>(base + b.fdp)[l] : 0.0;
+  }
+  if (l < nn) {
+    D.dispx[g] = 0.0;
+    D.dispy[g] = 0.0;
+    if (D.vel_vector) {  // Setup_Global_Arrays (3_SPH_material_2018.f90:1032)
+      D.x10x[g] = x.x;
+      D.x10y[g] = x.y;
+      D.disp10[g] = 0.0;
+    }
   }
 }
 __global__ void k_check_finite(sps::Dev D) {
@@ -620,6 +699,7 @@ int sps_create_batch(int32_t nreal, const sps_params* ps, sps_ctx** out) {
     D.pi = p->pi;
     for (int b = 0; b < p->no_bcs; b++) D.bcvar[b] = (int)p->bc_list[8 * (size_t)b + 1];
     const size_t N2 = D.N2, NT = D.NT, NN_ = D.NN;
+    c.arena_chunk = N2 * 1200 + (size_t)nreal * 1024 + (1 << 16);  // about what follows
     {
       sps::Real* rd = dalloc<sps::Real>(c, nreal);
       SPS_CUDA_CHECK(cudaMemcpyAsync(rd, c.real.data(), sizeof(sps::Real) * nreal,
@@ -781,9 +861,8 @@ int sps_create_batch(int32_t nreal, const sps_params* ps, sps_ctx** out) {
     D.step_idx = dalloc<int>(c, 1);
     D.cur = dalloc<sps::StepScalars>(c, nreal);
     D.err = dalloc<int>(c, 1);
-    // upload staging: x, vel, x00 (2 each), stress (4), mass, rho, hsml, intvars1,
-    // f_drucker (1 each) as doubles, itype as int32
-    c.stage = dalloc<double>(c, 16 * (size_t)N2);
+    // staging of an upload's or a download's packed fields
+    c.stage = dalloc<double>(c, std::max(up_block(NT, N2).bytes, snap_block(NN_, NT, N2).bytes) / 8);
     c.d_chk = dalloc<unsigned long long>(c, 8);
     SPS_CUDA_CHECK(cudaMemsetAsync(D.meta, 0, sizeof(sps::PairMeta) * nreal, c.stream));
     SPS_CUDA_CHECK(cudaMemsetAsync(D.bbox, 0xff, sizeof(unsigned long long) * 6 * nreal, c.stream));
@@ -816,8 +895,16 @@ int sps_create_batch(int32_t nreal, const sps_params* ps, sps_ctx** out) {
       SPS_CUDA_CHECK(cudaMemcpyAsync(D.horiz, ho.data(), sizeof(float) * N2, cudaMemcpyHostToDevice, c.stream));
       SPS_CUDA_CHECK(cudaStreamSynchronize(c.stream));
     }
-    SPS_CUDA_CHECK(cudaMallocHost(&c.h_err, sizeof(int)));
-    SPS_CUDA_CHECK(cudaMallocHost(&c.h_chk, 8 * sizeof(unsigned long long)));
+    c.pack_cap = std::min(kPackBytes,
+                          std::max(up_block(NT, N2).bytes, snap_block(NN_, NT, N2).bytes));
+    {
+      void* pin = nullptr;
+      SPS_CUDA_CHECK(cudaMallocHost(&pin, 512 + c.pack_cap));
+      c.h_pin = static_cast<char*>(pin);
+      c.h_err = reinterpret_cast<int*>(c.h_pin);
+      c.h_chk = reinterpret_cast<unsigned long long*>(c.h_pin + 256);
+      c.h_pack = c.h_pin + 512;
+    }
     ensure_scal(c, 256);
     D.cell_cap = 0;  // sized at upload
     c.d_dev = nullptr;
@@ -879,89 +966,41 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
   if (!x || !vel || !stress || !mass || !rho || !hsml || !itype)
     return fail(&c, SPS_ERR_ARG, "sps_upload: null array");
   const sps::Real& M = c.real[r];
-  const size_t nn = M.nnode, nt = (size_t)M.nnode + M.nsp, n2 = nt + M.ndum;
+  const size_t nt = (size_t)M.nnode + M.nsp, n2 = nt + M.ndum;
   Seg sg[3];
   segments(c, r, sg);
   try {
     // every host array is copied into the staging area on the upload stream, which may
-    // run while the previous step still computes (the state it reads is untouched); the
-    // context stream waits for the copies, transposes the interleaved arrays and moves
-    // the others into the state, reduces the checks and extents, and synchronises once
-    double* st_x = c.stage;
-    double* st_v = st_x + 2 * n2;
-    double* st_0 = st_v + 2 * n2;
-    double* st_s = st_0 + 2 * n2;
-    double* st_m = st_s + 4 * n2;
-    double* st_r = st_m + n2;
-    double* st_h = st_r + n2;
-    double* st_i = st_h + n2;
-    double* st_f = st_i + n2;
-    int32_t* st_t = reinterpret_cast<int32_t*>(st_f + n2);
+    // run while the previous step still computes (the state it reads is untouched); small
+    // realisations through one pinned buffer.  The context stream waits for the copies,
+    // moves them into the state, reduces the checks and extents, and synchronises once.
     auto nbk = [](int64_t n) { return (int)((n + kBlock - 1) / kBlock); };
-    auto h2d = [&](void* dst, const void* src, size_t bytes) {
-      if (bytes) SPS_CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c.up_stream));
+    const UpBlock ub = up_block((int64_t)nt, (int64_t)n2);
+    char* st = reinterpret_cast<char*>(c.stage);
+    const bool packed = ub.bytes <= c.pack_cap;
+    auto h2d = [&](size_t off, const void* src, size_t bytes) {
+      if (!bytes || !src) return;
+      if (packed) std::memcpy(c.h_pack + off, src, bytes);
+      else SPS_CUDA_CHECK(cudaMemcpyAsync(st + off, src, bytes, cudaMemcpyHostToDevice, c.up_stream));
     };
-    h2d(st_x, x, sizeof(double) * 2 * n2);
-    h2d(st_v, vel, sizeof(double) * 2 * n2);
-    h2d(st_0, x00 ? x00 : x, sizeof(double) * 2 * n2);
-    h2d(st_s, stress, sizeof(double) * 4 * n2);
-    h2d(st_m, mass, sizeof(double) * n2);
-    h2d(st_r, rho, sizeof(double) * n2);
-    h2d(st_h, hsml, sizeof(double) * n2);
-    h2d(st_t, itype, sizeof(int32_t) * n2);
-    if (intvars1) h2d(st_i, intvars1, sizeof(double) * nt);
-    if (f_drucker) h2d(st_f, f_drucker, sizeof(double) * nt);
+    h2d(ub.x, x, 16 * n2);
+    h2d(ub.vel, vel, 16 * n2);
+    h2d(ub.x00, x00 ? x00 : x, 16 * n2);
+    h2d(ub.stress, stress, 32 * n2);
+    h2d(ub.mass, mass, 8 * n2);
+    h2d(ub.rho, rho, 8 * n2);
+    h2d(ub.hsml, hsml, 8 * n2);
+    h2d(ub.iv1, intvars1, 8 * nt);
+    h2d(ub.fdp, f_drucker, 8 * nt);
+    h2d(ub.itype, itype, 4 * n2);
+    if (packed)
+      SPS_CUDA_CHECK(cudaMemcpyAsync(st, c.h_pack, ub.bytes, cudaMemcpyHostToDevice, c.up_stream));
     SPS_CUDA_CHECK(cudaEventRecord(c.up_ready, c.up_stream));
     SPS_CUDA_CHECK(cudaStreamWaitEvent(c.stream, c.up_ready, 0));
-    auto soa2 = [&](double* st, double* a, double* b) {
-      for (const Seg& q : sg)
-        if (q.n > 0)
-          k_aos_to_soa2<<<nbk(q.n), kBlock, 0, c.stream>>>(st + 2 * q.l, a + q.g, b + q.g, (int)q.n);
-    };
-    auto d2d = [&](void* dst, const void* src, size_t esz, int nseg) {
-      for (int k = 0; k < nseg; k++)
-        if (sg[k].n > 0)
-          SPS_CUDA_CHECK(cudaMemcpyAsync((char*)dst + esz * sg[k].g, (const char*)src + esz * sg[k].l,
-                                         esz * sg[k].n, cudaMemcpyDeviceToDevice, c.stream));
-    };
-    soa2(st_x, D.px, D.py);
-    soa2(st_v, D.vx, D.vy);
-    if (D.vel_vector && nn > 0) {  // Setup_Global_Arrays (3_SPH_material_2018.f90:1032)
-      SPS_CUDA_CHECK(cudaMemcpyAsync(D.x10x + M.node0, D.px + M.node0, sizeof(double) * nn,
-                                     cudaMemcpyDeviceToDevice, c.stream));
-      SPS_CUDA_CHECK(cudaMemcpyAsync(D.x10y + M.node0, D.py + M.node0, sizeof(double) * nn,
-                                     cudaMemcpyDeviceToDevice, c.stream));
-      SPS_CUDA_CHECK(cudaMemsetAsync(D.disp10 + M.node0, 0, sizeof(double) * nn, c.stream));
-    }
-    soa2(st_0, D.x00x, D.x00y);
-    for (const Seg& q : sg)
-      if (q.n > 0)
-        k_aos_to_soa4<<<nbk(q.n), kBlock, 0, c.stream>>>(st_s + 4 * q.l, D.s0 + q.g, D.s1 + q.g,
-                                                          D.s2 + q.g, D.s3 + q.g, (int)q.n);
-    d2d(D.mass, st_m, sizeof(double), 3);
-    d2d(D.rho, st_r, sizeof(double), 3);
-    d2d(D.hsml, st_h, sizeof(double), 3);
-    d2d(D.itype, st_t, sizeof(int32_t), 3);
-    for (int k = 0; k < 2; k++) {  // nodes and stress-points
-      const Seg& q = sg[k];
-      if (q.n == 0) continue;
-      if (intvars1)
-        SPS_CUDA_CHECK(cudaMemcpyAsync(D.iv1 + q.g, st_i + q.l, sizeof(double) * q.n, cudaMemcpyDeviceToDevice, c.stream));
-      else
-        SPS_CUDA_CHECK(cudaMemsetAsync(D.iv1 + q.g, 0, sizeof(double) * q.n, c.stream));
-      if (f_drucker)
-        SPS_CUDA_CHECK(cudaMemcpyAsync(D.fdp + q.g, st_f + q.l, sizeof(double) * q.n, cudaMemcpyDeviceToDevice, c.stream));
-      else
-        SPS_CUDA_CHECK(cudaMemsetAsync(D.fdp + q.g, 0, sizeof(double) * q.n, c.stream));
-    }
-    for (const Seg& q : sg)
-      if (q.n > 0) SPS_CUDA_CHECK(cudaMemsetAsync(D.out + q.g, 0, q.n, c.stream));
-    SPS_CUDA_CHECK(cudaMemsetAsync(D.dispx + M.node0, 0, sizeof(double) * nn, c.stream));
-    SPS_CUDA_CHECK(cudaMemsetAsync(D.dispy + M.node0, 0, sizeof(double) * nn, c.stream));
+    k_unpack_real<<<nbk(std::max<int64_t>((int64_t)n2, 8)), kBlock, 0, c.stream>>>(
+        D, r, st, intvars1 != nullptr, f_drucker != nullptr, c.d_chk);
     for (const Seg& q : sg)
       if (q.n > 0) sps::launch_vol(c, (int)q.g, (int)(q.g + q.n));
-    SPS_CUDA_CHECK(cudaMemsetAsync(c.d_chk, 0xff, 6 * sizeof(unsigned long long), c.stream));
-    SPS_CUDA_CHECK(cudaMemsetAsync(c.d_chk + 6, 0, 2 * sizeof(unsigned long long), c.stream));
     if (n2 > 0)
       k_upload_check<<<std::min(nbk((int64_t)n2), 4 * 152), kBlock, 0, c.stream>>>(
           D.itype, D.px, D.py, D.hsml, sg[0].g, sg[0].n, sg[1].g, sg[1].n, sg[2].g, sg[2].n,
@@ -1082,13 +1121,14 @@ int sps_upload_bcs(sps_ctx* h, const int32_t* bc_or_not, const int32_t* bc_info)
     if (bc_or_not)
       SPS_CUDA_CHECK(cudaMemcpyAsync(c.d.bc_or_not, bc_or_not, sizeof(int32_t) * NT, cudaMemcpyHostToDevice, c.stream));
     if (bc_info) {
+      // no early exit, so that the check vectorises (8 ints a particle)
+      const unsigned top = (unsigned)std::max(c.p.no_bcs, 0);
+      unsigned bad = 0;
       for (size_t i = 0; i < NT; i++)
-        for (int r = 2; r < 7; r++) {
-          int b = bc_info[8 * i + r];
-          if (b < 0 || b > c.p.no_bcs)
-            return fail(&c, SPS_ERR_ARG, "sps_upload_bcs: bc_info refers to a missing BC");
-        }
-      SPS_CUDA_CHECK(cudaMemcpyAsync(c.d.bc_info, bc_info, sizeof(int32_t) * 8 * NT, cudaMemcpyHostToDevice, c.stream));
+        for (int r = 2; r < 7; r++) bad |= (unsigned)((unsigned)bc_info[8 * i + r] > top);
+      if (bad) return fail(&c, SPS_ERR_ARG, "sps_upload_bcs: bc_info refers to a missing BC");
+      // without BCs nothing on the device reads it
+      if (top > 0) SPS_CUDA_CHECK(cudaMemcpyAsync(c.d.bc_info, bc_info, sizeof(int32_t) * 8 * NT, cudaMemcpyHostToDevice, c.stream));
     }
     SPS_CUDA_CHECK(cudaStreamSynchronize(c.stream));
   } catch (const std::exception& e) {
@@ -1156,51 +1196,32 @@ int sps_download_real(sps_ctx* h, int32_t r, double* x, double* vel, double* str
   if (r < 0 || r >= D.R) return fail(&c, SPS_ERR_ARG, "sps_download_real: no such realisation");
   const sps::Real& M = c.real[r];
   const size_t nn = M.nnode, nt = (size_t)M.nnode + M.nsp, n2 = nt + M.ndum;
-  Seg sg[3];
-  segments(c, r, sg);
   try {
     if (bc_or_not) refresh_surface(c, false);
-    // the interleaved outputs are transposed into the staging buffer side by side, every
-    // copy is enqueued, and the stream is synchronised once
-    double* st_x = c.stage;
-    double* st_v = st_x + 2 * n2;
-    double* st_s = st_v + 2 * n2;
-    double* st_d = st_s + 4 * n2;
-    auto nbk = [](int64_t n) { return (int)((n + kBlock - 1) / kBlock); };
-    auto down2 = [&](double* dst, double* st, const double* a, const double* b, int nseg, size_t n) {
-      for (int k = 0; k < nseg; k++)
-        if (sg[k].n > 0)
-          k_soa_to_aos2<<<nbk(sg[k].n), kBlock, 0, c.stream>>>(st + 2 * sg[k].l, a + sg[k].g,
-                                                                b + sg[k].g, (int)sg[k].n);
-      SPS_CUDA_CHECK(cudaMemcpyAsync(dst, st, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, c.stream));
-    };
-    auto down1 = [&](void* dst, const void* src, size_t esz, int nseg) {
-      for (int k = 0; k < nseg; k++)
-        if (sg[k].n > 0)
-          SPS_CUDA_CHECK(cudaMemcpyAsync((char*)dst + esz * sg[k].l, (const char*)src + esz * sg[k].g,
-                                         esz * sg[k].n, cudaMemcpyDeviceToHost, c.stream));
-    };
-    if (x) down2(x, st_x, D.px, D.py, 3, n2);
-    if (vel) down2(vel, st_v, D.vx, D.vy, 3, n2);
-    if (displ) down2(displ, st_d, D.dispx, D.dispy, 1, nn);
-    if (stress) {
-      for (int k = 0; k < 2; k++) {
-        const Seg& q = sg[k];
-        if (q.n > 0)
-          k_soa_to_aos4<<<nbk(q.n), kBlock, 0, c.stream>>>(st_s + 4 * q.l, D.s0 + q.g, D.s1 + q.g,
-                                                            D.s2 + q.g, D.s3 + q.g, (int)q.n);
-      }
-      // dummy stress is pair-local in the reference; report zero like its RK4 clear (:690)
-      if (n2 > nt)
-        SPS_CUDA_CHECK(cudaMemsetAsync(st_s + 4 * nt, 0, sizeof(double) * 4 * (n2 - nt), c.stream));
-      SPS_CUDA_CHECK(cudaMemcpyAsync(stress, st_s, sizeof(double) * 4 * n2, cudaMemcpyDeviceToHost, c.stream));
-    }
-    if (rho) down1(rho, D.rho, sizeof(double), 3);
-    if (intvars1) down1(intvars1, D.iv1, sizeof(double), 2);
-    if (bc_or_not) down1(bc_or_not, D.bc_or_not, sizeof(int32_t), 2);
-    if (f_drucker) down1(f_drucker, D.fdp, sizeof(double), 2);
+    // the fields are packed side by side in the staging buffer; a small realisation crosses
+    // as one copy through pinned memory, a larger one field by field into the caller's arrays
+    const SnapBlock b = snap_block((int64_t)nn, (int64_t)nt, (int64_t)n2);
+    char* st = reinterpret_cast<char*>(c.stage);
+    if (n2 > 0)
+      k_pack_real<<<(int)((n2 + kBlock - 1) / kBlock), kBlock, 0, c.stream>>>(D, r, st);
+    const bool packed = b.bytes <= c.pack_cap;
+    if (packed)
+      SPS_CUDA_CHECK(cudaMemcpyAsync(c.h_pack, st, b.bytes, cudaMemcpyDeviceToHost, c.stream));
+    struct Field {
+      void* dst;
+      size_t off, bytes;
+    } fields[] = {{x, b.x, 16 * n2},          {vel, b.vel, 16 * n2},  {stress, b.stress, 32 * n2},
+                  {rho, b.rho, 8 * n2},       {intvars1, b.iv1, 8 * nt}, {f_drucker, b.fdp, 8 * nt},
+                  {displ, b.displ, 16 * nn},  {bc_or_not, b.bc, 4 * nt}};
+    if (!packed)
+      for (const Field& f : fields)
+        if (f.dst && f.bytes)
+          SPS_CUDA_CHECK(cudaMemcpyAsync(f.dst, st + f.off, f.bytes, cudaMemcpyDeviceToHost, c.stream));
     SPS_CUDA_CHECK(cudaGetLastError());
     SPS_CUDA_CHECK(cudaStreamSynchronize(c.stream));
+    if (packed)
+      for (const Field& f : fields)
+        if (f.dst && f.bytes) std::memcpy(f.dst, c.h_pack + f.off, f.bytes);
   } catch (const std::exception& e) {
     return fail(&c, SPS_ERR_CUDA, e.what());
   }
@@ -1868,8 +1889,7 @@ void sps_destroy(sps_ctx* h) {
                   (void*)c.surr_cnt, c.surr_rows, c.tc_img})
     if (p) cudaFree(p);
   for (void* p : c.allocs) cudaFree(p);
-  if (c.h_err) cudaFreeHost(c.h_err);
-  if (c.h_chk) cudaFreeHost(c.h_chk);
+  if (c.h_pin) cudaFreeHost(c.h_pin);
   if (c.snap_stream) {
     cudaStreamSynchronize(c.snap_stream);
     cudaStreamDestroy(c.snap_stream);
