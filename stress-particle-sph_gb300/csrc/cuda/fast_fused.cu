@@ -657,8 +657,13 @@ __device__ __forceinline__ void nodef_stage(const Dev& D, int stage, int k) {
 
 // RK4 stage (2_SPH_main_2018.f90:700-777): blocks [0, nbs) the stress-points, the rest the
 // nodes
-template <int KP, int KD, bool LEAN>
-__global__ void __launch_bounds__(128) k_fstage(Dev D, int stage, int nbs) {
+// MINB: blocks of 128 an SM must hold.  Large problems wait on the record gathers (18 resident
+// warps of 64 issue a quarter of the cycles), so 64 registers and some spills pay: a stage at
+// 2.0M particles takes 0.409 ms at 96 registers, 0.364 at 80, 0.340 at 72, 0.327 at 64 and
+// 0.340 at 56.  Small ones cannot fill the SMs anyway and keep their registers (10k particles:
+// 25 us against 27).
+template <int KP, int KD, bool LEAN, int MINB>
+__global__ void __launch_bounds__(128, MINB) k_fstage(Dev D, int stage, int nbs) {
   const int ns = D.NT - D.NN;
   if ((int)blockIdx.x < nbs) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -763,10 +768,16 @@ void launch_fstage_kp(Ctx& c, int stage) {
   const int ns = D.NT - D.NN;
   const int b = c.block_for(D.NT, std::min(c.blk[TK_DERIVS], 128));
   const int nbs = (ns + b - 1) / b, nbn = (D.NN + b - 1) / b;
-  if (c.lean_tail && !D.cap_buf)
-    k_fstage<KP, KD, true><<<nbs + nbn, b, 0, c.stream>>>(D, stage, nbs);
-  else
-    k_fstage<KP, KD, false><<<nbs + nbn, b, 0, c.stream>>>(D, stage, nbs);
+  const int nb = nbs + nbn;
+  // up to eight blocks an SM in all, a tighter bound on the registers adds no resident block
+  const bool small = D.NT <= 152 * 8 * 128;
+  if (c.lean_tail && !D.cap_buf) {
+    if (small) k_fstage<KP, KD, true, 1><<<nb, b, 0, c.stream>>>(D, stage, nbs);
+    else k_fstage<KP, KD, true, 8><<<nb, b, 0, c.stream>>>(D, stage, nbs);
+  } else {
+    if (small) k_fstage<KP, KD, false, 1><<<nb, b, 0, c.stream>>>(D, stage, nbs);
+    else k_fstage<KP, KD, false, 8><<<nb, b, 0, c.stream>>>(D, stage, nbs);
+  }
 }
 
 }  // namespace
