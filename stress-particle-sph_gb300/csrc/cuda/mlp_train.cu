@@ -7,9 +7,15 @@
 // (N), are read as one (K + 1) x N matrix.  So
 //   forward   Z   = [A, 1] . [W; b]
 //   backward  d[W; b] = [A, 1]^T . dZ,   dA = dZ . W^T
-// with one tiled FP32 product kernel (k_gemm) for all three shapes.  The weight gradient
-// splits its long reduction (over the minibatch rows) into partial products that a
-// second kernel sums in a fixed order, so training is deterministic.
+// A minibatch is three launches:
+//   k_rows    32 rows a block: the whole forward pass, the loss and the backward pass down to
+//             every layer's dZ, the network in shared memory
+//   k_wgrad   the four layers' weight gradients, their long reductions (over the rows) split
+//             into partial products
+//   k_update  the partial products summed in a fixed order, Adam, the next forward pass's
+//             rounded weights, the loss sums
+// Every sum is one FP32 multiply-add chain in ascending index, so training is deterministic
+// and does not depend on the tiling.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -54,80 +60,6 @@ constexpr Layer kLayers[4] = {{MLP_W1, MLP_IN, MLP_H},
                               {MLP_W3, MLP_H, MLP_H},
                               {MLP_W4, MLP_H, MLP_OUT}};
 
-// C(m, n) = sum over k in this block's split of A(m, k) B(k, n);  A(m, k) = A[m sam + k sak],
-// B(k, n) = B[k sbk + n sbn], C(m, n) at C[(z M + m) ldc + n] for split z = blockIdx.z.
-// 64 x 64 tiles, 256 threads with 4 x 4 outputs each.
-__global__ void __launch_bounds__(256) k_gemm(const float* __restrict__ A, long sam, long sak,
-                                              const float* __restrict__ B, long sbk, long sbn,
-                                              float* __restrict__ C, int ldc, int M, int N,
-                                              int K, int kchunk) {
-  __shared__ float As[16][68];
-  __shared__ float Bs[16][68];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
-  float acc[4][4] = {};
-  for (int kb = kbeg; kb < kend; kb += 16) {
-    for (int e = tid; e < 1024; e += 256) {
-      int mm, kk;
-      if (sam == 1) {
-        mm = e & 63;
-        kk = e >> 6;
-      } else {
-        kk = e & 15;
-        mm = e >> 4;
-      }
-      int m = m0 + mm, k = kb + kk;
-      As[kk][mm] = (m < M && k < kend) ? A[m * sam + k * sak] : 0.0f;
-      int nn, k2;
-      if (sbn == 1) {
-        nn = e & 63;
-        k2 = e >> 6;
-      } else {
-        k2 = e & 15;
-        nn = e >> 4;
-      }
-      int n = n0 + nn, kk2 = kb + k2;
-      Bs[k2][nn] = (n < N && kk2 < kend) ? B[kk2 * sbk + n * sbn] : 0.0f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 16; kk++) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-  float* Cz = C + (size_t)blockIdx.z * M * ldc;
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    int m = m0 + ty * 4 + i;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      int n = n0 + tx * 4 + j;
-      if (n < N) Cz[(size_t)m * ldc + n] = acc[i][j];
-    }
-  }
-}
-
-// out[i] = sum over the splits of part[z n + i], in split order
-__global__ void k_sum_splits(const float* __restrict__ part, int nsplit, int n,
-                             float* __restrict__ out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float s = 0.0f;
-  for (int z = 0; z < nsplit; z++) s += part[(size_t)z * n + i];
-  out[i] = s;
-}
-
 __device__ __forceinline__ bool is_bias(int i) {
   return (i >= MLP_B1 && i < MLP_W2) || (i >= MLP_B2 && i < MLP_W3) ||
          (i >= MLP_B3 && i < MLP_W4) || i >= MLP_B4;
@@ -141,83 +73,311 @@ __global__ void k_quantize(const float* __restrict__ P, float* __restrict__ Wq, 
   Wq[i] = (quantize && !is_bias(i)) ? bf16r(v) : v;
 }
 
-// minibatch rows r < n: X = [inputs (14), 0, 0, 1] (17 columns), T = targets (4)
-__global__ void k_gather(const float* __restrict__ data, const int* __restrict__ perm,
-                         long start, int n, int quantize, float* __restrict__ X,
-                         float* __restrict__ T) {
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  const float* src = data + (size_t)perm[start + r] * MLP_TUPLE;
-  float* x = X + (size_t)r * (MLP_IN + 1);
-  for (int k = 0; k < MLP_NIN; k++) x[k] = quantize ? bf16r(src[k]) : src[k];
-  x[14] = 0.0f;
-  x[15] = 0.0f;
-  x[16] = 1.0f;
-  for (int k = 0; k < MLP_NOUT; k++) T[(size_t)r * MLP_NOUT + k] = src[MLP_NIN + k];
-}
+// ---- one minibatch ------------------------------------------------------------------------
 
-// H = [silu(Z), 1] (129 columns), BF16-rounded when quantize
-__global__ void k_act(const float* __restrict__ Z, float* __restrict__ H, int n, int quantize) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= (long)n * (MLP_H + 1)) return;
-  long r = i / (MLP_H + 1);
-  int c = (int)(i % (MLP_H + 1));
-  float v = 1.0f;
-  if (c < MLP_H) {
-    v = silu(Z[r * MLP_H + c]);
-    if (quantize) v = bf16r(v);
-  }
-  H[i] = v;
-}
+constexpr int kRows = 32;        // rows a block, four a warp
+constexpr int kHS = MLP_H + 4;   // row stride of H = [silu(Z), 1] and of W in shared memory
+constexpr int kXS = 20;          // row stride of X = [inputs (14), 0, 0, 1]
+constexpr int kWgradTiles = 2 + 6 + 6 + 3;  // 64 x 64 tiles of the four gradients
 
-// dZ = dH * silu'(Z)
-__global__ void k_act_bwd(const float* __restrict__ dH, const float* __restrict__ Z,
-                          float* __restrict__ dZ, int n) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= (long)n * MLP_H) return;
-  float z = Z[i];
-  float sg = 1.0f / (1.0f + expf(-z));
-  dZ[i] = dH[i] * (sg * (1.0f + z * (1.0f - sg)));
-}
+struct RowsSmem {
+  float w1[(MLP_IN + 1) * kHS];
+  float w2[(MLP_H + 1) * kHS], w3[(MLP_H + 1) * kHS];
+  float w4[(MLP_H + 1) * MLP_OUT];
+  float a[kRows * kHS];  // a warp's four rows: activations, then dZ
+  float dy[kRows * MLP_OUT];
+};
 
-// dY = 2 (Y - T) / (4 n) on the 4 used outputs (0 on the padding); per-block sum of the
-// squared errors into lossp[blockIdx.x]
-__global__ void k_loss(const float* __restrict__ Y, const float* __restrict__ T,
-                       float* __restrict__ dY, int n, float* __restrict__ lossp) {
-  __shared__ float sh[256];
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  float l = 0.0f;
-  if (r < n) {
-    const float sc = 2.0f / (4.0f * (float)n);
-    for (int c = 0; c < MLP_OUT; c++) {
-      float d = 0.0f;
-      if (c < MLP_NOUT) {
-        d = Y[(size_t)r * MLP_OUT + c] - T[(size_t)r * MLP_NOUT + c];
-        l += d * d;
+// z of a warp's four rows and a lane's columns lane + 32 c: the chain over k of A(row, k) W(k, n)
+// (K values of A in shared memory, then the bias row)
+template <int K>
+__device__ __forceinline__ void layer_forward(const float* __restrict__ A, int as,
+                                              const float* __restrict__ W, int lane,
+                                              float (*z)[4]) {
+#pragma unroll
+  for (int r = 0; r < 4; r++)
+#pragma unroll
+    for (int c = 0; c < 4; c++) z[r][c] = 0.0f;
+#pragma unroll 2
+  for (int k = 0; k < K; k += 4) {
+    float4 a[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) a[r] = *reinterpret_cast<const float4*>(A + r * as + k);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      float b[4];
+#pragma unroll
+      for (int c = 0; c < 4; c++) b[c] = W[(k + q) * kHS + lane + 32 * c];
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const float v = q == 0 ? a[r].x : q == 1 ? a[r].y : q == 2 ? a[r].z : a[r].w;
+#pragma unroll
+        for (int c = 0; c < 4; c++) z[r][c] = fmaf(v, b[c], z[r][c]);
       }
-      dY[(size_t)r * MLP_OUT + c] = sc * d;
     }
   }
-  sh[threadIdx.x] = l;
-  __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-    __syncthreads();
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    const float b = W[K * kHS + lane + 32 * c];
+#pragma unroll
+    for (int r = 0; r < 4; r++) z[r][c] = fmaf(1.0f, b, z[r][c]);
   }
-  if (threadIdx.x == 0) lossp[blockIdx.x] = sh[0];
+}
+// dA of the same rows and columns: the chain over the outputs j of dZ(row, j) W(n, j)
+__device__ __forceinline__ void layer_backward(const float* __restrict__ dZ,
+                                               const float* __restrict__ W, int lane,
+                                               float (*d)[4]) {
+#pragma unroll
+  for (int r = 0; r < 4; r++)
+#pragma unroll
+    for (int c = 0; c < 4; c++) d[r][c] = 0.0f;
+#pragma unroll 2
+  for (int j = 0; j < MLP_H; j += 4) {
+    float4 a[4], b[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) a[r] = *reinterpret_cast<const float4*>(dZ + r * kHS + j);
+#pragma unroll
+    for (int c = 0; c < 4; c++) b[c] = *reinterpret_cast<const float4*>(W + (lane + 32 * c) * kHS + j);
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        d[r][c] = fmaf(a[r].x, b[c].x, d[r][c]);
+        d[r][c] = fmaf(a[r].y, b[c].y, d[r][c]);
+        d[r][c] = fmaf(a[r].z, b[c].z, d[r][c]);
+        d[r][c] = fmaf(a[r].w, b[c].w, d[r][c]);
+      }
+  }
 }
 
-__global__ void k_adam(float* __restrict__ P, const float* __restrict__ G, float* __restrict__ Mo,
-                       float* __restrict__ Vo, float lr, float b1, float b2, float eps,
-                       float bc1, float bc2) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Rows r < n of a minibatch (data rows perm[start + r]): X, H = [silu(Z), 1] of the hidden
+// layers (BF16-rounded when quantize), dY = 2 (Y - T) / (4 n), dZ of the hidden layers, and the
+// rows' squared errors.  A warp owns four rows from the inputs to dZ of the first layer, so
+// warps meet only where the network is loaded; its Z stay in registers.  167 KB of shared
+// memory, one block an SM: 128 blocks for a minibatch of 4096.  Bound by the shared-memory
+// reads of the weights (4 wavefronts for 16 multiply-adds a lane).  With the other two kernels
+// a minibatch of 4096 takes three launches in place of twenty-seven.
+__global__ void __launch_bounds__(256, 1) k_rows(const float* __restrict__ data,
+                                                 const int* __restrict__ perm, long start, int n,
+                                                 int quantize, const float* __restrict__ Wq,
+                                                 float* __restrict__ X, float* __restrict__ H1,
+                                                 float* __restrict__ H2, float* __restrict__ H3,
+                                                 float* __restrict__ dY, float* __restrict__ dZ1,
+                                                 float* __restrict__ dZ2, float* __restrict__ dZ3,
+                                                 float* __restrict__ lrow) {
+  extern __shared__ __align__(16) uint8_t rows_raw[];
+  RowsSmem& S = *reinterpret_cast<RowsSmem*>(rows_raw);
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  for (int i = tid; i < (MLP_IN + 1) * MLP_H; i += 256)
+    S.w1[(i >> 7) * kHS + (i & 127)] = Wq[MLP_W1 + i];
+  for (int i = tid; i < (MLP_H + 1) * MLP_H; i += 256) {
+    S.w2[(i >> 7) * kHS + (i & 127)] = Wq[MLP_W2 + i];
+    S.w3[(i >> 7) * kHS + (i & 127)] = Wq[MLP_W3 + i];
+  }
+  for (int i = tid; i < (MLP_H + 1) * MLP_OUT; i += 256) S.w4[i] = Wq[MLP_W4 + i];
+  const int row0 = blockIdx.x * kRows + 4 * w;
+  float* A = S.a + 4 * w * kHS;
+  // inputs: lane k of a row its column k (rows past n stay zero and store nothing)
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+    float v = lane == MLP_IN ? 1.0f : 0.0f;
+    if (row0 + r < n) {
+      if (lane < MLP_NIN) {
+        v = data[(size_t)perm[start + row0 + r] * MLP_TUPLE + lane];
+        if (quantize) v = bf16r(v);
+      }
+      if (lane < kXS) X[(size_t)(row0 + r) * kXS + lane] = v;
+    }
+    if (lane < kXS) A[r * kHS + lane] = v;
+  }
+  __syncthreads();
+
+  float z1[4][4], z2[4][4], z3[4][4];
+  auto activate = [&](const float (*z)[4], float* __restrict__ H) {
+    __syncwarp();  // every lane has read the rows
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        float v = silu(z[r][c]);
+        if (quantize) v = bf16r(v);
+        A[r * kHS + lane + 32 * c] = v;
+        if (row0 + r < n) H[(size_t)(row0 + r) * kHS + lane + 32 * c] = v;
+      }
+      if (lane == 0) {
+        A[r * kHS + MLP_H] = 1.0f;
+        if (row0 + r < n) H[(size_t)(row0 + r) * kHS + MLP_H] = 1.0f;
+      }
+    }
+    __syncwarp();
+  };
+  layer_forward<MLP_IN>(A, kHS, S.w1, lane, z1);
+  activate(z1, H1);
+  layer_forward<MLP_H>(A, kHS, S.w2, lane, z2);
+  activate(z2, H2);
+  layer_forward<MLP_H>(A, kHS, S.w3, lane, z3);
+  activate(z3, H3);
+  {  // output layer and loss: lane 8 r + c holds output c of row r
+    const int r = lane >> 3, c = lane & 7, row = row0 + r;
+    float y = 0.0f;
+#pragma unroll 4
+    for (int k = 0; k <= MLP_H; k++) y = fmaf(A[r * kHS + k], S.w4[k * MLP_OUT + c], y);
+    const float sc = 2.0f / (4.0f * (float)n);
+    float d = 0.0f;
+    if (row < n && c < MLP_NOUT) d = y - data[(size_t)perm[start + row] * MLP_TUPLE + MLP_NIN + c];
+    float l = 0.0f;
+#pragma unroll
+    for (int q = 0; q < MLP_NOUT; q++) {
+      const float dq = __shfl_sync(0xffffffffu, d, (lane & 24) + q);
+      l = fmaf(dq, dq, l);
+    }
+    S.dy[(4 * w + r) * MLP_OUT + c] = sc * d;
+    if (row < n) {
+      dY[(size_t)row * MLP_OUT + c] = sc * d;
+      if (c == 0) lrow[row] = l;
+    }
+    __syncwarp();
+  }
+  // dZ = dA silu'(Z), kept as the warp's rows
+  auto through = [&](const float (*d)[4], const float (*z)[4], float* __restrict__ dZ) {
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const float zz = z[r][c];
+        const float sg = 1.0f / (1.0f + expf(-zz));
+        const float v = d[r][c] * (sg * (1.0f + zz * (1.0f - sg)));
+        A[r * kHS + lane + 32 * c] = v;
+        if (row0 + r < n) dZ[(size_t)(row0 + r) * MLP_H + lane + 32 * c] = v;
+      }
+    __syncwarp();
+  };
+  float d[4][4];
+#pragma unroll
+  for (int r = 0; r < 4; r++)
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      float v = 0.0f;
+#pragma unroll
+      for (int k = 0; k < MLP_OUT; k++)
+        v = fmaf(S.dy[(4 * w + r) * MLP_OUT + k], S.w4[(lane + 32 * c) * MLP_OUT + k], v);
+      d[r][c] = v;
+    }
+  through(d, z3, dZ3);
+  layer_backward(A, S.w3, lane, d);
+  through(d, z2, dZ2);
+  layer_backward(A, S.w2, lane, d);
+  through(d, z1, dZ1);
+}
+
+struct WgradLayer {
+  const float *A, *dZ;  // A (n x (K + 1), stride as), dZ (n x N)
+  int as, K, N, off;
+};
+struct WgradArgs {
+  WgradLayer l[4];
+};
+// part[z][i]: the weight gradient d[W; b] = [A, 1]^T . dZ of the rows of split z, every layer's at
+// its parameters' place; 64 x 64 tiles (blockIdx.x), 256 threads with 4 x 4 outputs each
+__global__ void __launch_bounds__(256) k_wgrad(WgradArgs args, int n, int kchunk,
+                                               float* __restrict__ part) {
+  __shared__ __align__(16) float As[16][68];
+  __shared__ __align__(16) float Bs[16][68];
+  int tile = blockIdx.x, li = 0;
+  if (tile >= 2) {
+    tile -= 2;
+    li = 1 + tile / 6;
+    tile = li < 3 ? tile % 6 : tile - 12;
+    if (li > 3) li = 3;
+  }
+  const WgradLayer L = args.l[li];
+  const int M = L.K + 1, N = L.N, nt = (N + 63) / 64;
+  const int m0 = tile / nt * 64, n0 = tile % nt * 64;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int kbeg = blockIdx.y * kchunk, kend = min(n, kbeg + kchunk);
+  float acc[4][4] = {};
+  const int mm = tid & 63, k4 = tid >> 6;  // a thread's column and rows k4 + 4 i of a step
+  float ra[4], rb[4];
+  auto fetch = [&](int kb) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int k = kb + k4 + 4 * i;
+      ra[i] = m0 + mm < M && k < kend ? L.A[(size_t)k * L.as + m0 + mm] : 0.0f;
+      rb[i] = n0 + mm < N && k < kend ? L.dZ[(size_t)k * N + n0 + mm] : 0.0f;
+    }
+  };
+  fetch(kbeg);
+  for (int kb = kbeg; kb < kend; kb += 16) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      As[k4 + 4 * i][mm] = ra[i];
+      Bs[k4 + 4 * i][mm] = rb[i];
+    }
+    __syncthreads();
+    if (kb + 16 < kend) fetch(kb + 16);  // the next step's rows while this one is summed
+#pragma unroll
+    for (int kk = 0; kk < 16; kk++) {
+      const float4 a = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
+      const float4 b = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
+      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    }
+    __syncthreads();
+  }
+  float* C = part + (size_t)blockIdx.y * MLP_NPARAM + L.off;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int m = m0 + ty * 4 + i;
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int c = n0 + tx * 4 + j;
+      if (c < N) C[(size_t)m * N + c] = acc[i][j];
+    }
+  }
+}
+
+// The gradient (the splits summed in order), with `adam` the update and the rounded weights of
+// the next forward pass; the blocks after the parameters' sum 256 rows' squared errors each
+// into lossp
+__global__ void __launch_bounds__(256) k_update(const float* __restrict__ part, int nsplit,
+                                                float* __restrict__ G, float* __restrict__ P,
+                                                float* __restrict__ Wq, float* __restrict__ Mo,
+                                                float* __restrict__ Vo, int adam, int quantize,
+                                                float lr, float b1, float b2, float eps, float bc1,
+                                                float bc2, const float* __restrict__ lrow, int n,
+                                                float* __restrict__ lossp) {
+  constexpr int pb = (MLP_NPARAM + 255) / 256;
+  if ((int)blockIdx.x >= pb) {
+    __shared__ float sh[256];
+    const int b = blockIdx.x - pb, r = b * 256 + threadIdx.x;
+    sh[threadIdx.x] = r < n ? lrow[r] : 0.0f;
+    __syncthreads();
+    for (int s = 128; s > 0; s >>= 1) {
+      if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) lossp[b] = sh[0];
+    return;
+  }
+  const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= MLP_NPARAM) return;
-  float g = G[i];
+  float g = 0.0f;
+#pragma unroll 4
+  for (int z = 0; z < nsplit; z++) g += part[(size_t)z * MLP_NPARAM + i];
+  G[i] = g;
+  if (!adam) return;
   float m = b1 * Mo[i] + (1.0f - b1) * g;
   float v = b2 * Vo[i] + (1.0f - b2) * (g * g);
   Mo[i] = m;
   Vo[i] = v;
-  P[i] = P[i] - lr * (m / bc1) / (sqrtf(v / bc2) + eps);
+  const float p = P[i] - lr * (m / bc1) / (sqrtf(v / bc2) + eps);
+  P[i] = p;
+  Wq[i] = (quantize && !is_bias(i)) ? bf16r(p) : p;
 }
 
 // B-operand registers of mma.m16n8k16 (row.col, BF16) for every tile and lane:
@@ -288,8 +448,8 @@ struct sps_mlp {
   cudaStream_t stream = nullptr;
   std::vector<void*> allocs;
   float *P = nullptr, *Wq = nullptr, *G = nullptr, *Mo = nullptr, *Vo = nullptr;
-  float *part = nullptr, *X = nullptr, *T = nullptr, *Y = nullptr, *dY = nullptr;
-  float *Z[3] = {}, *H[3] = {}, *dH = nullptr, *dZ = nullptr;
+  float *part = nullptr, *X = nullptr, *dY = nullptr, *lrow = nullptr;
+  float *H[3] = {}, *dZ[3] = {};
   float* lossp = nullptr;
   int lossp_cap = 0;
   float* data = nullptr;
@@ -332,51 +492,23 @@ struct sps_mlp {
     if (stream) cudaStreamDestroy(stream);
   }
 
-  void gemm(const float* A, long sam, long sak, const float* B, long sbk, long sbn, float* C,
-            int ldc, int M, int N, int K, int nsplit) {
-    int kchunk = ((K + nsplit - 1) / nsplit + 15) / 16 * 16;
-    nsplit = (K + kchunk - 1) / kchunk;
-    dim3 grid((N + 63) / 64, (M + 63) / 64, nsplit);
-    k_gemm<<<grid, 256, 0, stream>>>(A, sam, sak, B, sbk, sbn, C, ldc, M, N, K, kchunk);
-  }
-  void weight_grad(const float* Aext, int K, const float* dZ_, int N, int n, int off) {
-    // d[W; b] ((K + 1) x N) = Aext^T (n x (K + 1)) . dZ (n x N), split over rows
-    int kchunk = ((n + kSplit - 1) / kSplit + 15) / 16 * 16;
-    int nsplit = (n + kchunk - 1) / kchunk;
-    dim3 grid((N + 63) / 64, (K + 1 + 63) / 64, nsplit);
-    k_gemm<<<grid, 256, 0, stream>>>(Aext, 1, K + 1, dZ_, N, 1, part, N, K + 1, N, n, kchunk);
-    int tot = (K + 1) * N;
-    k_sum_splits<<<(tot + 255) / 256, 256, 0, stream>>>(part, nsplit, tot, G + off);
-  }
-
-  // forward + loss + backward for n gathered rows (X, T); gradient into G, per-block
-  // squared errors into lossp[lo ...]
-  void fwd_bwd(int n, int lo) {
-    const int q = cfg.quantize;
-    const float* A = X;
-    int K = MLP_IN;
-    for (int l = 0; l < 3; l++) {
-      gemm(A, K + 1, 1, Wq + kLayers[l].off, MLP_H, 1, Z[l], MLP_H, n, MLP_H, K + 1, 1);
-      long tot = (long)n * (MLP_H + 1);
-      k_act<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(Z[l], H[l], n, q);
-      A = H[l];
-      K = MLP_H;
-    }
-    gemm(A, MLP_H + 1, 1, Wq + MLP_W4, MLP_OUT, 1, Y, MLP_OUT, n, MLP_OUT, MLP_H + 1, 1);
-    k_loss<<<(n + 255) / 256, 256, 0, stream>>>(Y, T, dY, n, lossp + lo);
-    // output layer
-    weight_grad(H[2], MLP_H, dY, MLP_OUT, n, MLP_W4);
-    // dH3 = dY . W4^T (first 128 columns)
-    gemm(dY, MLP_OUT, 1, Wq + MLP_W4, 1, MLP_OUT, dH, MLP_H, n, MLP_H, MLP_OUT, 1);
-    for (int l = 2; l >= 0; l--) {
-      long tot = (long)n * MLP_H;
-      k_act_bwd<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(dH, Z[l], dZ, n);
-      const float* Ain = l > 0 ? H[l - 1] : X;
-      int Kin = l > 0 ? MLP_H : MLP_IN;
-      weight_grad(Ain, Kin, dZ, MLP_H, n, kLayers[l].off);
-      if (l > 0)  // dA = dZ . W^T
-        gemm(dZ, MLP_H, 1, Wq + kLayers[l].off, 1, MLP_H, dH, MLP_H, n, MLP_H, MLP_H, 1);
-    }
+  // forward, loss and backward of n rows (data rows perm[start ...]) with the weights Wq; the
+  // gradient into G, per-256-row squared errors into lossp[lo ...]; adam: one update of the
+  // parameters and Wq with the learning rate lr
+  void minibatch(const float* rows, const int* order, long start, int n, int lo, bool adam,
+                 float lr, float bc1, float bc2) {
+    k_rows<<<(n + kRows - 1) / kRows, 256, sizeof(RowsSmem), stream>>>(
+        rows, order, start, n, cfg.quantize, Wq, X, H[0], H[1], H[2], dY, dZ[0], dZ[1], dZ[2], lrow);
+    const int kchunk = ((n + kSplit - 1) / kSplit + 15) / 16 * 16;
+    const int nsplit = (n + kchunk - 1) / kchunk;
+    WgradArgs args = {{{X, dZ[0], kXS, MLP_IN, MLP_H, MLP_W1},
+                       {H[0], dZ[1], kHS, MLP_H, MLP_H, MLP_W2},
+                       {H[1], dZ[2], kHS, MLP_H, MLP_H, MLP_W3},
+                       {H[2], dY, kHS, MLP_H, MLP_OUT, MLP_W4}}};
+    k_wgrad<<<dim3(kWgradTiles, nsplit), 256, 0, stream>>>(args, n, kchunk, part);
+    k_update<<<(MLP_NPARAM + 255) / 256 + (n + 255) / 256, 256, 0, stream>>>(
+        part, nsplit, G, P, Wq, Mo, Vo, adam ? 1 : 0, cfg.quantize, lr, cfg.beta1, cfg.beta2,
+        cfg.eps, bc1, bc2, lrow, n, lossp + lo);
   }
   void quantize() {
     k_quantize<<<(MLP_NPARAM + 255) / 256, 256, 0, stream>>>(P, Wq, cfg.quantize);
@@ -430,17 +562,16 @@ int sps_mlp_create(const sps_mlp_config* cfg, sps_mlp** out) {
     m->G = m->alloc<float>(MLP_NPARAM);
     m->Mo = m->alloc<float>(MLP_NPARAM);
     m->Vo = m->alloc<float>(MLP_NPARAM);
-    m->part = m->alloc<float>((size_t)kSplit * (MLP_H + 1) * MLP_H);
-    m->X = m->alloc<float>((size_t)B * (MLP_IN + 1));
-    m->T = m->alloc<float>((size_t)B * MLP_NOUT);
-    m->Y = m->alloc<float>((size_t)B * MLP_OUT);
+    m->part = m->alloc<float>((size_t)kSplit * MLP_NPARAM);
+    m->X = m->alloc<float>((size_t)B * kXS);
     m->dY = m->alloc<float>((size_t)B * MLP_OUT);
+    m->lrow = m->alloc<float>(B);
     for (int l = 0; l < 3; l++) {
-      m->Z[l] = m->alloc<float>((size_t)B * MLP_H);
-      m->H[l] = m->alloc<float>((size_t)B * (MLP_H + 1));
+      m->H[l] = m->alloc<float>((size_t)B * kHS);
+      m->dZ[l] = m->alloc<float>((size_t)B * MLP_H);
     }
-    m->dH = m->alloc<float>((size_t)B * MLP_H);
-    m->dZ = m->alloc<float>((size_t)B * MLP_H);
+    MLP_CHECK(cudaFuncSetAttribute(k_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(RowsSmem)));
     m->ident = m->alloc<int>(B);
     m->gtuples = m->alloc<float>((size_t)B * MLP_TUPLE);
     m->frag = m->alloc<uint2>(MLP_FRAG_U2);
@@ -532,6 +663,7 @@ int sps_mlp_train(sps_mlp* m, int32_t epochs, float lr, float* loss) {
     m->ensure_lossp((int)(nmb * per));
     std::vector<int> perm(m->ndata);
     std::vector<float> lp;
+    if (epochs > 0) m->quantize();  // k_update keeps the rounded weights from here on
     for (int ep = 0; ep < epochs; ep++) {
       for (int64_t i = 0; i < m->ndata; i++) perm[i] = (int)i;
       for (int64_t i = m->ndata - 1; i > 0; i--) {  // Fisher-Yates
@@ -541,16 +673,10 @@ int sps_mlp_train(sps_mlp* m, int32_t epochs, float lr, float* loss) {
       MLP_CHECK(cudaMemcpyAsync(m->perm, perm.data(), sizeof(int) * m->ndata,
                                 cudaMemcpyHostToDevice, m->stream));
       for (int64_t b = 0; b < nmb; b++) {
-        m->quantize();
-        k_gather<<<(B + 255) / 256, 256, 0, m->stream>>>(m->data, m->perm, b * B, B,
-                                                         m->cfg.quantize, m->X, m->T);
-        m->fwd_bwd(B, (int)(b * per));
         m->adam_t++;
         float bc1 = (float)(1.0 - std::pow((double)m->cfg.beta1, (double)m->adam_t));
         float bc2 = (float)(1.0 - std::pow((double)m->cfg.beta2, (double)m->adam_t));
-        k_adam<<<(MLP_NPARAM + 255) / 256, 256, 0, m->stream>>>(
-            m->P, m->G, m->Mo, m->Vo, lr, m->cfg.beta1, m->cfg.beta2, m->cfg.eps, bc1,
-            bc2);
+        m->minibatch(m->data, m->perm, b * B, B, (int)(b * per), true, lr, bc1, bc2);
       }
       MLP_CHECK(cudaGetLastError());
       lp.resize(nmb * per);
@@ -573,9 +699,7 @@ int sps_mlp_grad(sps_mlp* m, const float* tuples, int32_t n, float* grad, float*
     MLP_CHECK(cudaMemcpyAsync(m->gtuples, tuples, sizeof(float) * MLP_TUPLE * n,
                               cudaMemcpyHostToDevice, m->stream));
     m->quantize();
-    k_gather<<<(n + 255) / 256, 256, 0, m->stream>>>(m->gtuples, m->ident, 0, n,
-                                                     m->cfg.quantize, m->X, m->T);
-    m->fwd_bwd(n, 0);
+    m->minibatch(m->gtuples, m->ident, 0, n, 0, false, 0.0f, 1.0f, 1.0f);
     MLP_CHECK(cudaGetLastError());
     std::vector<float> lp((n + 255) / 256);
     MLP_CHECK(cudaMemcpyAsync(grad, m->G, sizeof(float) * MLP_NPARAM, cudaMemcpyDeviceToHost, m->stream));
