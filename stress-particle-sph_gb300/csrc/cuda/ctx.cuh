@@ -117,6 +117,11 @@ struct Ctx {
     while (b > 32 && n < (int64_t)b * 304) b >>= 1;
     return b;
   }
+  // largest NT whose preparation takes eight lanes a target: every lane of a group repeats the
+  // sums, which pays while lanes are idle (us with one / eight lanes: plain slope of 29,000
+  // 52 / 41, of 40,000 64 / 51, of 80,000 86 / 91, biaxial sample of 40,000 with wall segments
+  // 58 / 110; FP32 slope of 40,000 31 / 23, of 180,000 49 / 74)
+  int group_max = 40000;
   int split_max = 60000;  // largest NT whose stage kernels split a target's sums over lanes
   // the last pair build left the half lists unwritten (k_fgather): sps_dump_pairs and the
   // keyed lists of the exact detection build them first (set by enqueue_step for every

@@ -82,141 +82,186 @@ __device__ __forceinline__ void spf_publish(const Dev& D, const Real& M, const S
   (buf ? D.recAl1 : D.recAl)[t] = l;
 }
 
-// Once per step, per target: the list constants (file comment), a node's wall force and wall
-// flag, the state of stage 0
-__global__ void __launch_bounds__(128) k_fprep(Dev D) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= D.NT) return;
+// one entry of a target: its constants, and what its sums take of it
+struct TermF {
+  bool wall, push;
+  int u;
+  float h;         // (m/rho) W
+  float m, gx, gy; // node: mass and gradient -dW (m dW summed without error)
+  float xu, yu, hx, hy;  // CSPM: separation and gradient factors
+  float fx, fy;    // a wall's force on a node
+};
+template <bool CSPM>
+__device__ __forceinline__ void spf_entry(const Dev& D, int k, int j, double xt, double yt,
+                                          TermF& T) {
   const int ns = D.NT - D.NN;
+  const int4 e = D.cross[ell(j, k, D.N2)];
+  const int u = e.x;
+  const float Gx = __int_as_float(e.z), Gy = __int_as_float(e.w);
+  const float vol = D.recI[u].y;
+  T.wall = e.y < 0;
+  if (!T.wall) {
+    T.h = vol * __int_as_float(e.y);
+    D.crossW[(size_t)j * D.N2 + k] = make_int2(u, __float_as_int(T.h));
+    T.hx = Gx * vol;
+    T.hy = Gy * vol;
+    D.hGf[(size_t)j * D.NT + k] = make_float2(T.hx, T.hy);
+    if (CSPM) {
+      T.xu = (float)(D.px[u] - xt);
+      T.yu = (float)(D.py[u] - yt);
+    }
+    return;
+  }
+  const double wall = (double)D.wallpos[u];
+  double da, db;
+  if (D.horiz[u] == 1.0f) {
+    da = fabs(yt - wall);
+    db = fabs(D.py[u] - wall);
+  } else {
+    da = fabs(xt - wall);
+    db = fabs(D.px[u] - wall);
+  }
+  const double bq = 1.0 + db / da;
+  const double beta = 1.5 < bq ? 1.5 : bq;
+  D.hB[(size_t)j * ns + k] = 1.0 - beta;
+  D.crossW[(size_t)j * D.N2 + k] = make_int2(u, (int)0x80000000u);
+  D.hGf[(size_t)j * D.NT + k] = make_float2(-Gx * vol, -Gy * vol);
+}
+template <bool CSPM>
+__device__ __forceinline__ void nodef_entry(const Dev& D, const Real& M, int t, int k, int j,
+                                            double xt, double yt, TermF& T) {
+  const int4 e = D.cross[ell(j, k, D.N2)];
+  const int u = e.x;
+  const float dwx = -__int_as_float(e.z), dwy = -__int_as_float(e.w);
+  T.u = u;
+  T.gx = dwx;
+  T.gy = dwy;
+  T.wall = e.y < 0;
+  if (!T.wall) {
+    const float4 ri = D.recI[u];
+    T.m = ri.w;
+    T.h = ri.y * __int_as_float(e.y);
+    D.crossW[(size_t)j * D.N2 + k] = make_int2(u, __float_as_int(T.h));
+    if (CSPM) {
+      const float vol = ri.y;
+      T.hx = -(dwx * vol);
+      T.hy = -(dwy * vol);
+      T.xu = (float)(D.px[u] - xt);
+      T.yu = (float)(D.py[u] - yt);
+    }
+  } else {
+    T.m = (float)D.mass[u];
+    D.crossW[(size_t)j * D.N2 + k] = make_int2(u, (int)0x80000000u);
+    T.push = D.inside && D.bound_from_lists && u >= M.dum0 && u < M.dum0 + M.ndum2 &&
+             bound_term(D, M, t, u, T.fx, T.fy);
+  }
+  D.hGf[(size_t)j * D.NT + k] = make_float2(T.m * dwx, T.m * dwy);
+}
+
+// Once per step, per target: the list constants (file comment), a node's wall force and wall
+// flag, the state of stage 0.  L = 8 as k_pprep: eight lanes form the entries' constants, each
+// adds their terms in list order (37 -> 20 us at 10,000 particles).
+template <int L, bool CSPM>
+__global__ void __launch_bounds__(128) k_fprep(Dev D) {
+  constexpr unsigned all = 0xffffffffu;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / L, q = threadIdx.x & (L - 1);
+  const bool act = i < D.NT;
+  if (L == 1 && !act) return;
+  const int k = act ? i : 0;
+  const int ns = D.NT - D.NN;
+  const bool sp = k < ns;
   const int t = D.colid[k];
   const Real* Mp;
   const StepScalars* scp;
   load_real(D, t, Mp, scp);
   const Real& M = *Mp;
-  const int deg = D.degC[k];
-  if (D.walk_order) put_target_walk_order(D, k, t, k >= ns);
+  const int deg = act ? D.degC[k] : 0;
+  if (D.walk_order && act && q == 0) put_target_walk_order(D, k, t, !sp);
+  if (L > 1) __syncwarp();
   Kahan nm;
   Kahan e0, e1, e2, e3;
+  ProdSum sx, sy;
+  WallForce F;
   const double xt = D.px[t], yt = D.py[t];
-  if (k < ns) {
-    for (int j = 0; j < deg; j++) {
-      const int4 e = D.cross[ell(j, k, D.N2)];
-      const int u = e.x;
-      const float Gx = __int_as_float(e.z), Gy = __int_as_float(e.w);
-      const float vol = D.recI[u].y;
-      if (e.y >= 0) {
-        const float w = __int_as_float(e.y);
-        const float h2 = vol * w;
-        nm.add(h2);
-        D.crossW[(size_t)j * D.N2 + k] = make_int2(u, __float_as_int(h2));
-        const float h1x = Gx * vol, h1y = Gy * vol;
-        D.hGf[(size_t)j * D.NT + k] = make_float2(h1x, h1y);
-        if (D.cspm) {
-          const float xu = (float)(D.px[u] - xt), yu = (float)(D.py[u] - yt);
-          e0.add(xu * h1x);
-          e1.add(yu * h1x);
-          e2.add(xu * h1y);
-          e3.add(yu * h1y);
-        }
-      } else {
-        const double wall = (double)D.wallpos[u];
-        double da, db;
-        if (D.horiz[u] == 1.0f) {
-          da = fabs(yt - wall);
-          db = fabs(D.py[u] - wall);
-        } else {
-          da = fabs(xt - wall);
-          db = fabs(D.px[u] - wall);
-        }
-        const double bq = 1.0 + db / da;
-        const double beta = 1.5 < bq ? 1.5 : bq;
-        D.hB[(size_t)j * ns + k] = 1.0 - beta;
-        D.crossW[(size_t)j * D.N2 + k] = make_int2(u, (int)0x80000000u);
-        D.hGf[(size_t)j * D.NT + k] = make_float2(-Gx * vol, -Gy * vol);
+  auto take = [&](const TermF& x, bool node) {
+    if (!x.wall) {
+      nm.add(x.h);
+      if (CSPM) {
+        e0.add(x.xu * x.hx);
+        e1.add(x.yu * x.hx);
+        e2.add(x.xu * x.hy);
+        e3.add(x.yu * x.hy);
+      }
+    } else if (node) {
+      F.met(D, x.push, x.u, x.fx, x.fy);
+    }
+    if (node) {
+      sx.add(x.m, x.gx);
+      sy.add(x.m, x.gy);
+    }
+  };
+  if (L == 1) {
+    if (sp) {
+      for (int j = 0; j < deg; j++) {
+        TermF T;
+        spf_entry<CSPM>(D, k, j, xt, yt, T);
+        take(T, false);
+      }
+    } else {
+      for (int j = 0; j < deg; j++) {
+        TermF T;
+        nodef_entry<CSPM>(D, M, t, k, j, xt, yt, T);
+        take(T, true);
       }
     }
   } else {
-    ProdSum sx, sy;
-    constexpr int K = 8;
-    int ids[K];
-    float tx[K], ty[K];
-    int n = 0, bc_int = 0;
-    const int j0 = M.dum0, j1 = M.dum0 + M.ndum2;
-    for (int j = 0; j < deg; j++) {
-      const int4 e = D.cross[ell(j, k, D.N2)];
-      const int u = e.x;
-      const float dwx = -__int_as_float(e.z), dwy = -__int_as_float(e.w);
-      float m;
-      if (e.y >= 0) {
-        const float4 ri = D.recI[u];
-        m = ri.w;
-        const float w = __int_as_float(e.y);
-        const float h1 = ri.y * w;
-        nm.add(h1);
-        D.crossW[(size_t)j * D.N2 + k] = make_int2(u, __float_as_int(h1));
-        if (D.cspm) {
-          const float vol = ri.y;
-          const float h1b = -(dwx * vol), h2b = -(dwy * vol);
-          const float xu = (float)(D.px[u] - xt), yu = (float)(D.py[u] - yt);
-          e0.add(xu * h1b);
-          e1.add(yu * h1b);
-          e2.add(xu * h2b);
-          e3.add(yu * h2b);
-        }
-      } else {
-        m = (float)D.mass[u];
-        bc_int = 1;
-        D.crossW[(size_t)j * D.N2 + k] = make_int2(u, (int)0x80000000u);
-        float fx, fy;
-        if (D.inside && D.bound_from_lists && u >= j0 && u < j1 && bound_term(D, M, t, u, fx, fy)) {
-          if (n < K) {
-            int p = n++;
-            while (p > 0 && ids[p - 1] > u) {
-              ids[p] = ids[p - 1];
-              tx[p] = tx[p - 1];
-              ty[p] = ty[p - 1];
-              p--;
-            }
-            ids[p] = u;
-            tx[p] = fx;
-            ty[p] = fy;
-          } else {
-            atomicOr(D.err, ERR_BOUND);
-          }
-        }
+    const int nmax = __reduce_max_sync(all, deg);
+    for (int j = 0; j < nmax; j += L) {
+      TermF T = {};
+      if (j + q < deg) {
+        if (sp) spf_entry<CSPM>(D, k, j + q, xt, yt, T);
+        else nodef_entry<CSPM>(D, M, t, k, j + q, xt, yt, T);
       }
-      D.hGf[(size_t)j * D.NT + k] = make_float2(m * dwx, m * dwy);
-      sx.add(m, dwx);
-      sy.add(m, dwy);
-    }
-    double bx = 0.0, by = 0.0;
-    if (D.inside && !D.bound_from_lists) {
-      for (int j = j0; j < j1; j++) {
-        float fx, fy;
-        if (!bound_term(D, M, t, j, fx, fy)) continue;
-        bx = bx + (double)fx;
-        by = by + (double)fy;
-      }
-    } else {
-      for (int j = 0; j < n; j++) {
-        bx = bx + f64_of(tx[j]);
-        by = by + f64_of(ty[j]);
+      const bool walls = __any_sync(all, T.wall);
+#pragma unroll
+      for (int o = 0; o < L; o++) {
+        TermF x = {};
+        x.wall = __shfl_sync(all, (int)T.wall, o, L);
+        x.h = __shfl_sync(all, T.h, o, L);
+        x.m = __shfl_sync(all, T.m, o, L);
+        x.gx = __shfl_sync(all, T.gx, o, L);
+        x.gy = __shfl_sync(all, T.gy, o, L);
+        if (CSPM) {
+          x.xu = __shfl_sync(all, T.xu, o, L);
+          x.yu = __shfl_sync(all, T.yu, o, L);
+          x.hx = __shfl_sync(all, T.hx, o, L);
+          x.hy = __shfl_sync(all, T.hy, o, L);
+        }
+        if (walls) {
+          x.push = __shfl_sync(all, (int)T.push, o, L);
+          x.u = __shfl_sync(all, T.u, o, L);
+          x.fx = __shfl_sync(all, T.fx, o, L);
+          x.fy = __shfl_sync(all, T.fy, o, L);
+        }
+        if (j + o < deg) take(x, !sp);
       }
     }
-    D.fbx[t] = bx;
-    D.fby[t] = by;
-    D.bc_int[t] = bc_int;
+  }
+  if (q || !act) return;
+  if (!sp) {
+    F.store(D, M, t);
+    D.bc_int[t] = F.bc_int;
     D.msum[k - ns] = make_float4(sx.hi.s, sx.lo - sx.hi.c, sy.hi.s, sy.lo - sy.hi.c);
   }
   const float norm = nm.fval();
   D.normf[k] = make_float2(norm, norm != 0.0f ? __frcp_rn(norm) : 0.0f);
-  if (D.cspm) {
+  if (CSPM) {
     const double AE[4] = {e0.val(), e1.val(), e2.val(), e3.val()};
     double A[5];
     cspm_moments<true>(D, AE, A);
     for (int q = 0; q < 5; q++) D.AE[(size_t)q * D.NT + k] = A[q];
   }
-  if (k < ns) {
+  if (sp) {
     double a = D.s0[t], b = D.s1[t], c = D.s2[t], d = D.s3[t];
     st4(D.st0c + 4 * (size_t)k, a, b, c, d);
     a = a + 0.0;  // RK4 starts from zero rates
@@ -241,7 +286,7 @@ __global__ void __launch_bounds__(128) k_fprep(Dev D) {
     apply_bcs(D, *scp, t, vx, vy, a, b, c, d);
     D.recV[t] = split2f(vx, vy);
     // the correction's right-hand side takes the stage velocity in FP64 (its own node's only)
-    if (D.cspm) reinterpret_cast<double2*>(D.pv[0])[t] = make_double2(vx, vy);
+    if (CSPM) reinterpret_cast<double2*>(D.pv[0])[t] = make_double2(vx, vy);
   }
 }
 
@@ -783,10 +828,13 @@ void launch_fstage_kp(Ctx& c, int stage) {
 }  // namespace
 
 void launch_fprep(Ctx& c) {
-  const int b = c.block_for(c.d.NT, 128);
   Dev D = c.d;
   D.same_entries = c.same_now();  // the lists to put in walk order
-  k_fprep<<<(D.NT + b - 1) / b, b, 0, c.stream>>>(D);
+  const bool group = D.NT <= c.group_max;
+  const int n = group ? 8 * D.NT : D.NT, b = c.block_for(n, 128), nb = (n + b - 1) / b;
+  auto k = D.cspm ? (group ? k_fprep<8, true> : k_fprep<1, true>)
+                  : (group ? k_fprep<8, false> : k_fprep<1, false>);
+  k<<<nb, b, 0, c.stream>>>(D);
 }
 
 // The look-ahead of the interpolation (ahead[0]) sets the pair; the node derivative sums'

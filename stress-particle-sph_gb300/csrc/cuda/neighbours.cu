@@ -990,17 +990,14 @@ __device__ __forceinline__ bool gather_accept(const Dev& D, int a, float xa, flo
 // FP32 form: Task 3 of grid_find_NEW (2_SPH_main_2018.f90:1307-1403), kernel (:1440-1538)
 // and Pint_Update (3_SPH_material_2018.f90:1574-1634) per target, gathering its entries
 // from the 3 x 3 cell stencil directly in creation order.
-// SAME: the same-kind entries are written too (the steps that read them: XSPH, artificial viscosity or stress,
-// the FP32 free-surface detection); without them degS holds 0 unless the outside approach
+// No same-kind lists (gather_by_group writes them): degS holds 0 unless the outside approach
 // reads the counts.  Phase 1 tests the stencil's candidates and keeps the
 // accepted ones (sorted position and cell offset) in shared memory; phase 2 evaluates the
 // kernel values, so that a warp's lanes evaluate together.  Dynamic shared memory:
-// (capC + SAME capS) ints per thread, entry k of thread j at k * blockDim + j.
-template <bool SAME, bool PLAIN>
-__device__ __forceinline__ void gather_target(const Dev& D, int s, int col, int* gbuf) {
+// capC ints per thread, entry k of thread j at k * blockDim + j.
+template <bool PLAIN>
+__device__ __forceinline__ void gather_target(const Dev& D, int s, int col, int* buf) {
   const int bd = blockDim.x, tid = threadIdx.x;
-  int* bufC = gbuf;
-  int* bufS = gbuf + (size_t)D.capC * bd;
   int nC = 0, nS = 0, nHalf = 0;
   if (s < D.gtot->nactive) {
     const int a = D.sorted[s];
@@ -1012,10 +1009,10 @@ __device__ __forceinline__ void gather_target(const Dev& D, int s, int col, int*
     const int ix = c % nx, iy = c / nx;
     const float xa = D.xr[a], ya = D.yr[a], ha = D.hr[a];
     const float cw = (float)g.deltx[0], ch = (float)g.deltx[1];
-    // same-kind partners before the target matter only for the full same-kind count
-    // (the same lists, or the outside approach's isolated-node test); otherwise only the
+    // same-kind partners before the target matter only for the outside approach's
+    // isolated-node test, which reads the full same-kind count; otherwise only the
     // ones after it are tested, for the half-list count
-    const bool all_same = SAME || D.outside;
+    const bool all_same = D.outside;
     // a uniform smoothing length makes the prefilter's bounds constant (the same FP32
     // expressions as prefilter(), so the same decisions)
     float s2lo = 0.0f, s2hi = 0.0f;
@@ -1061,10 +1058,9 @@ __device__ __forceinline__ void gather_target(const Dev& D, int s, int col, int*
         nHalf += bs > s;
         const int code = (qy + 1) * 3 + (qx + 1);  // cell offset, kept in the top 4 bits
         if (same) {
-          if (SAME && nS < D.capS) bufS[(size_t)nS * bd + tid] = bs | (code << kHalfTypeShift);
           nS++;
         } else {
-          if (nC < D.capC) bufC[(size_t)nC * bd + tid] = bs | (code << kHalfTypeShift);
+          if (nC < D.capC) buf[(size_t)nC * bd + tid] = bs | (code << kHalfTypeShift);
           nC++;
         }
       }
@@ -1081,28 +1077,137 @@ __device__ __forceinline__ void gather_target(const Dev& D, int s, int col, int*
     }
     const float xal = PLAIN ? 0.0f : D.xrl[a], yal = PLAIN ? 0.0f : D.yrl[a];
     // phase 2: the entries, stored in pairs (whole 32-byte sectors)
-    auto finish = [&](const int* buf, int n, int4* list, int2* compact, bool f32) {
-      int4 pend = make_int4(0, 0, 0, 0);
-      for (int k = 0; k < n; k++) {
-        const unsigned v = (unsigned)buf[(size_t)k * bd + tid];
-        const int code = (int)(v >> kHalfTypeShift);
-        const int4 e = gather_entry<PLAIN>(D, g, a, ta, xa, ya, ha, xal, yal,
-                                           (int)(v & kHalfIdMask), code % 3 - 1, code / 3 - 1, f32);
-        if (k & 1) store_pair(list + ell(k - 1, col, D.N2), pend, e);
-        else pend = e;
-        // the lanes of a warp write entry k of adjacent columns together: whole sectors
-        if (compact) compact[(size_t)k * D.N2 + col] = make_int2(e.x, e.y);
-      }
-      if (n & 1) list[ell(n - 1, col, D.N2)] = pend;
-    };
-    finish(bufC, nC, D.cross, D.use_crossW ? D.crossW : nullptr, false);
-    // same-kind entries that no step kernel reads serve the FP32 free-surface detection
-    // only: FP32 kernel values
-    if (SAME) finish(bufS, nS, D.same, nullptr, D.same_f32);
+    int4 pend = make_int4(0, 0, 0, 0);
+    for (int k = 0; k < nC; k++) {
+      const unsigned v = (unsigned)buf[(size_t)k * bd + tid];
+      const int code = (int)(v >> kHalfTypeShift);
+      const int4 e = gather_entry<PLAIN>(D, g, a, ta, xa, ya, ha, xal, yal,
+                                         (int)(v & kHalfIdMask), code % 3 - 1, code / 3 - 1, false);
+      if (k & 1) store_pair(D.cross + ell(k - 1, col, D.N2), pend, e);
+      else pend = e;
+      // the lanes of a warp write entry k of adjacent columns together: whole sectors
+      if (D.use_crossW) D.crossW[(size_t)k * D.N2 + col] = make_int2(e.x, e.y);
+    }
+    if (nC & 1) D.cross[ell(nC - 1, col, D.N2)] = pend;
   }
   D.degC[col] = nC;
   D.degS[col] = nS;
   D.half_cnt[s] = nHalf;
+}
+
+// The same gather by G lanes a target: they test G candidates at a time, keep the accepted ones
+// in order (their places from a ballot) and share the kernel values.  The same decisions and
+// values; all 32 lanes of a warp take part (act: the group has a target).  Two reasons to
+// take it: the serial chain of about 100 tests and up to 36 evaluations a target is G times
+// shorter where the problem cannot fill the chip, and a group's buffers are shared, so that G times
+// as many warps fit a multiprocessor where two lists are buffered (launch_gather).  SAME: the
+// same-kind entries are written too, for the steps that read them (XSPH, artificial viscosity
+// or stress, the FP32 free-surface detection; those that no step kernel reads hold FP32 kernel
+// values, Dev::same_f32).
+template <bool SAME, bool PLAIN, int G>
+__device__ __forceinline__ void gather_by_group(const Dev& D, int s, int col, bool act, int* bufC) {
+  constexpr unsigned all = 0xffffffffu;
+  const int q = threadIdx.x & (G - 1), sh = threadIdx.x & 31 & ~(G - 1);
+  const unsigned below = (1u << q) - 1u;
+  int* bufS = bufC + D.capC;
+  auto group = [&](bool b) { return (__ballot_sync(all, b) >> sh) & ((1u << G) - 1u); };
+  const bool on = act && s < D.gtot->nactive;
+  const int a = D.sorted[s];
+  const int ta = D.itype[a];
+  const Grid& g = D.grid[D.rid[a]];
+  const float tau = g.tau;
+  const int nx = g.ndiv[0], ny = g.ndiv[1];
+  const int c = on ? D.cell_of[a] - g.cell0 : 0;
+  const int ix = c % nx, iy = c / nx;
+  const float xa = D.xr[a], ya = D.yr[a], ha = D.hr[a];
+  const float cw = (float)g.deltx[0], ch = (float)g.deltx[1];
+  const bool all_same = SAME || D.outside;
+  float s2lo = 0.0f, s2hi = 0.0f;
+  if (g.uniform_h) {
+    const float sv = (float)D.scale_k * ((ha + ha) * 0.5f);
+    const float s2 = sv * sv;
+    s2lo = s2 * (1.0f - tau);
+    s2hi = s2 * (1.0f + tau);
+  }
+  int nC = 0, nS = 0, nHalf = 0;
+  for (int qy = -1; qy <= 1; qy++) {
+    const int jy = iy + qy;
+    int lo = 0, hi = 0, b0 = 0, b1 = 0;
+    if (on && jy >= 0 && jy < ny) {
+      const int row0 = g.cell0 + jy * nx;
+      const int cr = row0 + (ix + 1 < nx ? ix + 1 : ix);
+      lo = D.cell_start[row0 + (ix > 0 ? ix - 1 : 0)];
+      hi = D.cell_start[cr] + D.cell_cnt[cr];
+      b0 = D.cell_start[row0 + ix];
+      b1 = ix + 1 < nx ? D.cell_start[row0 + ix + 1] : hi;
+    }
+    const float cy = qy < 0 ? -ch : (qy > 0 ? ch : 0.0f);
+    const int nmax = (int)__reduce_max_sync(all, (unsigned)(hi - lo));
+    for (int j = 0; j < nmax; j += G) {
+      const int bs = lo + j + q;
+      bool acc = false, same = false;
+      int qx = 0;
+      if (bs < hi && bs != s) {
+        const float4 rb = D.srec[bs];
+        same = __float_as_int(rb.w) == ta;
+        if (!same || all_same || bs > s) {
+          qx = bs < b0 ? -1 : (bs < b1 ? 0 : 1);
+          const float cx = qx < 0 ? -cw : (qx > 0 ? cw : 0.0f);
+          if (g.uniform_h) {
+            const float fx = (xa - rb.x) - cx, fy = (ya - rb.y) - cy;
+            const float d2 = fx * fx + fy * fy;
+            acc = d2 < s2lo;
+            if (!acc && !(d2 > s2hi)) {
+              double r, dx, dy, mh;
+              acc = exact_test(D, a, D.sorted[bs], r, dx, dy, mh);
+            }
+          } else {
+            acc = gather_accept(D, a, xa, ya, ha, rb, bs, cx, cy, tau);
+          }
+        }
+      }
+      const unsigned mC = group(acc && !same), mS = group(acc && same);
+      nHalf += __popc(group(acc && bs > s));
+      const int code = bs | (((qy + 1) * 3 + (qx + 1)) << kHalfTypeShift);
+      if (acc) {
+        const int k = same ? nS + __popc(mS & below) : nC + __popc(mC & below);
+        if (!same && k < D.capC) bufC[k] = code;
+        if (SAME && same && k < D.capS) bufS[k] = code;
+      }
+      nC += __popc(mC);
+      nS += __popc(mS);
+    }
+  }
+  __syncwarp();
+  if (!act) return;
+  if (!all_same) nS = 0;
+  if (nHalf > D.capH || nC > D.capC || nS > D.capS) {
+    if (q == 0) {
+      if (nHalf > D.capH) atomicOr(D.err, ERR_HALF_CAP);
+      if (nC > D.capC || nS > D.capS) atomicOr(D.err, ERR_LIST_CAP);
+    }
+    nHalf = min(nHalf, D.capH);
+    nC = min(nC, D.capC);
+    nS = min(nS, D.capS);
+  }
+  const float xal = PLAIN ? 0.0f : D.xrl[a], yal = PLAIN ? 0.0f : D.yrl[a];
+  auto finish = [&](const int* buf, int n, int4* list, int2* compact, bool f32) {
+    for (int k = q; k < n; k += G) {
+      const unsigned v = (unsigned)buf[k];
+      const int code = (int)(v >> kHalfTypeShift);
+      const int4 e = gather_entry<PLAIN>(D, g, a, ta, xa, ya, ha, xal, yal, (int)(v & kHalfIdMask),
+                                         code % 3 - 1, code / 3 - 1, f32);
+      list[ell(k, col, D.N2)] = e;
+      if (compact) compact[(size_t)k * D.N2 + col] = make_int2(e.x, e.y);
+    }
+  };
+  finish(bufC, nC, D.cross, D.use_crossW ? D.crossW : nullptr, false);
+  if (SAME) finish(bufS, nS, D.same, nullptr, D.same_f32);
+  if (q == 0) {
+    D.degC[col] = nC;
+    D.degS[col] = nS;
+    D.half_cnt[s] = nHalf;
+  }
 }
 
 // every sorted position that is not a stress-point or node target: the half-list length
@@ -1141,16 +1246,33 @@ __device__ __forceinline__ void gather_rest(const Dev& D, int a) {
 }
 
 // the stress-point targets [0, bs blocks), the node targets [bs, bn), the dummies: one launch
-template <bool SAME, bool PLAIN>
+template <bool PLAIN>
 __global__ void __launch_bounds__(512, 2) k_fgather(Dev D, int bs, int bn) {
   extern __shared__ int gbuf[];
   const int ns = D.NT - D.NN, b = blockIdx.x;
   if (b < bs) {
     const int k = b * blockDim.x + threadIdx.x;
-    if (k < ns) gather_target<SAME, PLAIN>(D, D.tgtS[k], k, gbuf);
+    if (k < ns) gather_target<PLAIN>(D, D.tgtS[k], k, gbuf);
   } else if (b < bn) {
     const int k = (b - bs) * blockDim.x + threadIdx.x;
-    if (k < D.NN) gather_target<SAME, PLAIN>(D, D.tgtN[k], ns + k, gbuf);
+    if (k < D.NN) gather_target<PLAIN>(D, D.tgtN[k], ns + k, gbuf);
+  } else {
+    const int k = (b - bn) * blockDim.x + threadIdx.x;
+    if (D.NT + k < D.N2) gather_rest(D, D.NT + k);
+  }
+}
+
+template <bool SAME, bool PLAIN, int G>
+__global__ void __launch_bounds__(128) k_fgatherg(Dev D, int bs, int bn) {
+  extern __shared__ int gbuf[];
+  const int ns = D.NT - D.NN, b = blockIdx.x, per = blockDim.x / G, w = threadIdx.x / G;
+  int* buf = gbuf + (size_t)w * (D.capC + (SAME ? D.capS : 0));
+  if (b < bs) {
+    const int k = b * per + w, kk = k < ns ? k : 0;
+    gather_by_group<SAME, PLAIN, G>(D, D.tgtS[kk], kk, k < ns, buf);
+  } else if (b < bn) {
+    const int k = (b - bs) * per + w, kk = k < D.NN ? k : 0;
+    gather_by_group<SAME, PLAIN, G>(D, D.tgtN[kk], ns + kk, k < D.NN, buf);
   } else {
     const int k = (b - bn) * blockDim.x + threadIdx.x;
     if (D.NT + k < D.N2) gather_rest(D, D.NT + k);
@@ -1457,23 +1579,39 @@ void launch_lists(Ctx& c, bool keys, bool same = false) {
   else k_lists<false><<<nb, b, pend, c.stream>>>(D);
 }
 
-// FP32 form: the lists straight from the cell stencil and the remaining positions' counts; the
-// block size is the tuned pair-search size, lowered until each thread's candidate lists fit
-// 48 KB of shared memory and until two blocks an SM have work
+// The lists straight from the cell stencil and the remaining positions' counts.  Lanes a target:
+// fewer as the problem fills the chip by itself, since a group's ballots and partly filled
+// passes cost it two to three times the instructions a target (slopes of the FP32 form, no
+// same-kind lists, us with 8 / 4 / 2 lanes / 1: 17,000 targets 26 / - / - / 52; 29,000 30 / 24 /
+// 33 / 54; 80,000 57 / 50 / 57 / 58; 320,000 195 / 164 / 152 / 158; 2 million 1188 / 991 / 880 /
+// 762; with same-kind lists, 2 million, plain, 2082 / 1792 / 1728 / 2551: one lane's buffers
+// leave too few warps a multiprocessor, so that form is not built).  Dynamic shared memory: the
+// list capacity for each target of a block, blocks halved until it is within 48 KB.
 void launch_gather(Ctx& c, bool same, const Dev& D) {
-  const size_t per_thread = sizeof(int) * (size_t)(D.capC + (same ? D.capS : 0));
-  int b = Ctx::block_for(D.NT, std::min(c.blk[TK_HALF], 512));  // k_fgather's launch bounds
-  while (b > 32 && per_thread * (size_t)b > 49152) b >>= 1;
-  const size_t sm = per_thread * (size_t)b;
-  const int bs = (D.NT - D.NN + b - 1) / b, bn = bs + (D.NN + b - 1) / b;
-  const int nb = bn + (D.N2 - D.NT + b - 1) / b;
-  if (D.fast) {
-    if (same) k_fgather<true, false><<<nb, b, sm, c.stream>>>(D, bs, bn);
-    else k_fgather<false, false><<<nb, b, sm, c.stream>>>(D, bs, bn);
-  } else {
-    if (same) k_fgather<true, true><<<nb, b, sm, c.stream>>>(D, bs, bn);
-    else k_fgather<false, true><<<nb, b, sm, c.stream>>>(D, bs, bn);
+  const size_t per_target = sizeof(int) * (size_t)(D.capC + (same ? D.capS : 0));
+  const int G = D.NT <= 16000 ? 8 : (D.NT <= 100000 ? 4 : (same || D.NT <= 400000 ? 2 : 1));
+  if (G == 1) {
+    int b = std::min(c.blk[TK_HALF], 512);  // k_fgather's launch bounds
+    while (b > 32 && per_target * (size_t)b > 49152) b >>= 1;
+    const int bs = (D.NT - D.NN + b - 1) / b, bn = bs + (D.NN + b - 1) / b;
+    const int nb = bn + (D.N2 - D.NT + b - 1) / b;
+    auto k = D.fast ? k_fgather<false> : k_fgather<true>;
+    k<<<nb, b, per_target * b, c.stream>>>(D, bs, bn);
+    return;
   }
+  int b = Ctx::block_for((int64_t)D.NT * G, 128);
+  while (b > 32 && per_target * (b / G) > 49152) b >>= 1;
+  const int per = b / G;
+  const int bs = (D.NT - D.NN + per - 1) / per, bn = bs + (D.NN + per - 1) / per;
+  const int nb = bn + (D.N2 - D.NT + b - 1) / b;
+  auto form = [&](auto f, auto p) {
+    constexpr bool S = decltype(f)::value, P = decltype(p)::value;
+    return G == 8 ? k_fgatherg<S, P, 8> : (G == 4 ? k_fgatherg<S, P, 4> : k_fgatherg<S, P, 2>);
+  };
+  const std::true_type yes;
+  const std::false_type no;
+  auto k = same ? (D.fast ? form(yes, no) : form(yes, yes)) : (D.fast ? form(no, no) : form(no, yes));
+  k<<<nb, b, per_target * per, c.stream>>>(D, bs, bn);
 }
 
 int launch_pair_build(Ctx& c) {

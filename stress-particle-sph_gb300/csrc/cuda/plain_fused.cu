@@ -78,134 +78,177 @@ __device__ __forceinline__ void sp_publish(const Dev& D, const Real& M, const St
   }
 }
 
-// Once per step, per target: the constants of its list entries (file comment), the boundary
-// force of a node (boundary_forces, over its list's innermost dummies as k_bound), and the
-// state of stage 0.  Bound by the FP64 pipe (22 operations a stress-point entry, 8 a node's).
-__global__ void __launch_bounds__(128) k_pprep(Dev D) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= D.NT) return;
+// a stress-point's entry: its constants, and unless its partner is a wall (true) its terms of
+// the norm and of the CSPM moments
+struct Terms {
+  double norm, e[4];
+};
+template <bool CSPM>
+__device__ __forceinline__ bool sp_entry(const Dev& D, int k, int j, double xt, double yt,
+                                         Terms& T) {
   const int ns = D.NT - D.NN;
+  const int4 e = D.cross[ell(j, k, D.N2)];
+  const int u = e.x;
+  const double Gx = f64_of(__int_as_float(e.z)), Gy = f64_of(__int_as_float(e.w));
+  const double mu = D.mass[u], ru = D.rho[u], iu = D.rinv[u];
+  const bool wall = e.y < 0;
+  double h, h1, h2;
+  if (!wall) {
+    const double w = f64_of(__int_as_float(e.y));
+    h = D.vol[u] * w;
+    T.norm = div_rcp(w * mu, ru, iu);
+    h1 = div_rcp(Gx * mu, ru, iu);
+    h2 = div_rcp(Gy * mu, ru, iu);
+    if (CSPM) {
+      const double xu = D.px[u] - xt, yu = D.py[u] - yt;
+      T.e[0] = xu * h1;
+      T.e[1] = yu * h1;
+      T.e[2] = xu * h2;
+      T.e[3] = yu * h2;
+    }
+  } else {
+    const double wp = (double)D.wallpos[u];
+    double da, db;
+    if (D.horiz[u] == 1.0f) {
+      da = fabs(yt - wp);
+      db = fabs(D.py[u] - wp);
+    } else {
+      da = fabs(xt - wp);
+      db = fabs(D.px[u] - wp);
+    }
+    const double bq = 1.0 + db / da;
+    const double beta = 1.5 < bq ? 1.5 : bq;
+    h = 1.0 - beta;
+    h1 = div_rcp(-Gx * mu, ru, iu);
+    h2 = div_rcp(-Gy * mu, ru, iu);
+  }
+  D.hW[(size_t)j * D.NT + k] = h;
+  D.hG[(size_t)j * ns + k] = make_double2(h1, h2);
+  return wall;
+}
+// a node's entry: the same, and of a wall partner u the boundary force (fx, fy) if it has one
+// (push)
+template <bool CSPM>
+__device__ __forceinline__ bool node_entry(const Dev& D, const Real& M, int t, int k, int j,
+                                           double xt, double yt, Terms& T, int& u, bool& push,
+                                           float& fx, float& fy) {
+  const int4 e = D.cross[ell(j, k, D.N2)];
+  u = e.x;
+  push = false;
+  if (e.y < 0) {
+    push = D.inside && D.bound_from_lists && u >= M.dum0 && u < M.dum0 + M.ndum2 &&
+           bound_term(D, M, t, u, fx, fy);
+    return true;
+  }
+  const double w = f64_of(__int_as_float(e.y));
+  const double mu = D.mass[u], ru = D.rho[u], iu = D.rinv[u];
+  D.hW[(size_t)j * D.NT + k] = D.vol[u] * w;
+  T.norm = div_rcp(w * mu, ru, iu);
+  if (CSPM) {
+    const double dwx = -f64_of(__int_as_float(e.z)), dwy = -f64_of(__int_as_float(e.w));
+    const double h1b = -div_rcp(dwx * mu, ru, iu), h2b = -div_rcp(dwy * mu, ru, iu);
+    const double xu = D.px[u] - xt, yu = D.py[u] - yt;
+    T.e[0] = xu * h1b;
+    T.e[1] = yu * h1b;
+    T.e[2] = xu * h2b;
+    T.e[3] = yu * h2b;
+  }
+  return false;
+}
+
+// Once per step, per target: the constants of its list entries (file comment), the boundary
+// force of a node, and the state of stage 0.  Bound by the FP64 pipe (22 operations a
+// stress-point entry, 8 a node's; the terms of the CSPM moments are compiled out without them,
+// since FP64 instructions that a predicate switches off still occupy it: 1292 -> 1069 us at 2
+// million particles).  L = 8, for problems that cannot fill the chip with one lane a
+// target: eight lanes form eight entries' constants and terms together, and every one of them
+// adds the terms in list order (0.0 where an entry has none, which changes no sum: none of
+// them is ever -0.0); 58 -> 25 us at 600 particles, soil failure example 53 -> 18.
+template <int L, bool CSPM>
+__global__ void __launch_bounds__(128) k_pprep(Dev D) {
+  constexpr unsigned all = 0xffffffffu;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / L, q = threadIdx.x & (L - 1);
+  const bool act = i < D.NT;
+  if (L == 1 && !act) return;
+  const int k = act ? i : 0;
+  const int ns = D.NT - D.NN;
+  const bool sp = k < ns;
   const int t = D.colid[k];
   const Real* Mp;
   const StepScalars* scp;
   load_real(D, t, Mp, scp);
   const Real& M = *Mp;
-  const int deg = D.degC[k];
-  if (D.walk_order) put_target_walk_order(D, k, t, k >= ns);
+  const int deg = act ? D.degC[k] : 0;
+  if (D.walk_order && act && q == 0) put_target_walk_order(D, k, t, !sp);
+  if (L > 1) __syncwarp();
   const double xt = D.px[t], yt = D.py[t];
   double norm = 0.0;
   double AE[4] = {0.0, 0.0, 0.0, 0.0};
-  if (k < ns) {
-    for (int j = 0; j < deg; j++) {
-      const int4 e = D.cross[ell(j, k, D.N2)];
-      const int u = e.x;
-      const bool wall = e.y < 0;
-      const double Gx = f64_of(__int_as_float(e.z)), Gy = f64_of(__int_as_float(e.w));
-      const double mu = D.mass[u], ru = D.rho[u], iu = D.rinv[u];
-      double h, h1, h2;
-      if (!wall) {
-        const double w = f64_of(__int_as_float(e.y));
-        h = D.vol[u] * w;
-        norm = norm + div_rcp(w * mu, ru, iu);
-        h1 = div_rcp(Gx * mu, ru, iu);
-        h2 = div_rcp(Gy * mu, ru, iu);
-        if (D.cspm) {
-          const double xu = D.px[u] - xt, yu = D.py[u] - yt;
-          AE[0] = AE[0] + xu * h1;
-          AE[1] = AE[1] + yu * h1;
-          AE[2] = AE[2] + xu * h2;
-          AE[3] = AE[3] + yu * h2;
-        }
-      } else {
-        const double wp = (double)D.wallpos[u];
-        double da, db;
-        if (D.horiz[u] == 1.0f) {
-          da = fabs(yt - wp);
-          db = fabs(D.py[u] - wp);
-        } else {
-          da = fabs(xt - wp);
-          db = fabs(D.px[u] - wp);
-        }
-        const double bq = 1.0 + db / da;
-        const double beta = 1.5 < bq ? 1.5 : bq;
-        h = 1.0 - beta;
-        h1 = div_rcp(-Gx * mu, ru, iu);
-        h2 = div_rcp(-Gy * mu, ru, iu);
-      }
-      D.hW[(size_t)j * D.NT + k] = h;
-      D.hG[(size_t)j * ns + k] = make_double2(h1, h2);
-    }
-  } else {
-    constexpr int K = 8;
-    int ids[K];
-    float tx[K], ty[K];
-    int n = 0, bc_int = 0;
-    const int j0 = M.dum0, j1 = M.dum0 + M.ndum2;
-    for (int j = 0; j < deg; j++) {
-      const int4 e = D.cross[ell(j, k, D.N2)];
-      const int u = e.x;
-      if (e.y >= 0) {
-        const double w = f64_of(__int_as_float(e.y));
-        const double mu = D.mass[u], ru = D.rho[u], iu = D.rinv[u];
-        D.hW[(size_t)j * D.NT + k] = D.vol[u] * w;
-        norm = norm + div_rcp(w * mu, ru, iu);
-        if (D.cspm) {
-          const double dwx = -f64_of(__int_as_float(e.z)), dwy = -f64_of(__int_as_float(e.w));
-          const double h1b = -div_rcp(dwx * mu, ru, iu), h2b = -div_rcp(dwy * mu, ru, iu);
-          const double xu = D.px[u] - xt, yu = D.py[u] - yt;
-          AE[0] = AE[0] + xu * h1b;
-          AE[1] = AE[1] + yu * h1b;
-          AE[2] = AE[2] + xu * h2b;
-          AE[3] = AE[3] + yu * h2b;
-        }
-      } else {
-        bc_int = 1;
-        float fx, fy;
-        if (D.inside && D.bound_from_lists && u >= j0 && u < j1 && bound_term(D, M, t, u, fx, fy)) {
-          if (n < K) {
-            int p = n++;
-            while (p > 0 && ids[p - 1] > u) {
-              ids[p] = ids[p - 1];
-              tx[p] = tx[p - 1];
-              ty[p] = ty[p - 1];
-              p--;
-            }
-            ids[p] = u;
-            tx[p] = fx;
-            ty[p] = fy;
-          } else {
-            atomicOr(D.err, ERR_BOUND);
-          }
-        }
-      }
-    }
-    double bx = 0.0, by = 0.0;
-    if (D.inside && !D.bound_from_lists) {
-      for (int j = j0; j < j1; j++) {
-        float fx, fy;
-        if (!bound_term(D, M, t, j, fx, fy)) continue;
-        bx = bx + (double)fx;
-        by = by + (double)fy;
+  WallForce F;
+  if (L == 1) {
+    auto add = [&](const Terms& T) {
+      norm = norm + T.norm;
+      if (CSPM)
+        for (int p = 0; p < 4; p++) AE[p] = AE[p] + T.e[p];
+    };
+    if (sp) {
+      for (int j = 0; j < deg; j++) {
+        Terms T;
+        if (!sp_entry<CSPM>(D, k, j, xt, yt, T)) add(T);
       }
     } else {
-      for (int j = 0; j < n; j++) {
-        bx = bx + f64_of(tx[j]);
-        by = by + f64_of(ty[j]);
+      for (int j = 0; j < deg; j++) {
+        Terms T;
+        int u;
+        bool push;
+        float fx, fy;
+        const bool wall = node_entry<CSPM>(D, M, t, k, j, xt, yt, T, u, push, fx, fy);
+        if (!wall) add(T);
+        else F.met(D, push, u, fx, fy);
       }
     }
-    D.fbx[t] = bx;
-    D.fby[t] = by;
-    D.bc_int[t] = bc_int;
+  } else {
+    const int nmax = __reduce_max_sync(all, deg);
+    for (int j = 0; j < nmax; j += L) {
+      Terms T = {0.0, {0.0, 0.0, 0.0, 0.0}};
+      int u = 0;
+      bool wall = false, push = false;
+      float fx = 0.0f, fy = 0.0f;
+      if (j + q < deg) {
+        if (sp) sp_entry<CSPM>(D, k, j + q, xt, yt, T);
+        else wall = node_entry<CSPM>(D, M, t, k, j + q, xt, yt, T, u, push, fx, fy);
+      }
+#pragma unroll
+      for (int o = 0; o < L; o++) {
+        norm = norm + __shfl_sync(all, T.norm, o, L);
+        if (CSPM)
+          for (int p = 0; p < 4; p++) AE[p] = AE[p] + __shfl_sync(all, T.e[p], o, L);
+      }
+      if (__any_sync(all, wall)) {
+#pragma unroll
+        for (int o = 0; o < L; o++) {
+          const bool w = __shfl_sync(all, (int)wall, o, L), p = __shfl_sync(all, (int)push, o, L);
+          const int v = __shfl_sync(all, u, o, L);
+          const float x = __shfl_sync(all, fx, o, L), y = __shfl_sync(all, fy, o, L);
+          if (w) F.met(D, p, v, x, y);
+        }
+      }
+    }
+  }
+  if (q || !act) return;
+  if (!sp) {
+    F.store(D, M, t);
+    D.bc_int[t] = F.bc_int;
   }
   D.norm[k] = norm;
   D.rnorm[k] = norm != 0.0 ? 1.0 / norm : 0.0;
-  if (D.cspm) {
+  if (CSPM) {
     double A[5];
     cspm_moments<false>(D, AE, A);
-    for (int q = 0; q < 5; q++) D.AE[(size_t)q * D.NT + k] = A[q];
+    for (int p = 0; p < 5; p++) D.AE[(size_t)p * D.NT + k] = A[p];
   }
   // the state of stage 0 (RK4 starts from zero rates)
-  if (k < ns) {
+  if (sp) {
     const double a = D.s0[t], b = D.s1[t], c = D.s2[t], d = D.s3[t];
     st4(D.st0c + 4 * (size_t)k, a, b, c, d);
     sp_publish(D, M, *scp, t, 0, a + 0.0, b + 0.0, c + 0.0, d + 0.0, true, nullptr);
@@ -768,10 +811,13 @@ __global__ void __launch_bounds__(128) k_pfinish(Dev D) {
 }  // namespace
 
 void launch_pprep(Ctx& c) {
-  const int b = c.block_for(c.d.NT, 128);
   Dev D = c.d;
   D.same_entries = c.same_now();  // the lists to put in walk order
-  k_pprep<<<(D.NT + b - 1) / b, b, 0, c.stream>>>(D);
+  const bool group = D.NT <= c.group_max;
+  const int n = group ? 8 * D.NT : D.NT, b = c.block_for(n, 128), nb = (n + b - 1) / b;
+  auto k = D.cspm ? (group ? k_pprep<8, true> : k_pprep<1, true>)
+                  : (group ? k_pprep<8, false> : k_pprep<1, false>);
+  k<<<nb, b, 0, c.stream>>>(D);
 }
 
 // Lanes a target: split by component while one lane a target leaves most of the chip's 608

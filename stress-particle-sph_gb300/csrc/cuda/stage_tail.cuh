@@ -438,6 +438,51 @@ __device__ __forceinline__ bool bound_term(const Dev& D, const Real& M, int i, i
   return true;
 }
 
+// The wall force of a node (as k_bound): the terms of the innermost dummies met in its list, kept
+// in ascending id, or of every innermost dummy where the lists do not hold them all; and
+// whether the list holds a dummy at all
+struct WallForce {
+  static constexpr int K = 8;
+  int ids[K], n = 0, bc_int = 0;
+  float tx[K], ty[K];
+  __device__ __forceinline__ void met(const Dev& D, bool push, int u, float fx, float fy) {
+    bc_int = 1;
+    if (!push) return;
+    if (n < K) {
+      int p = n++;
+      while (p > 0 && ids[p - 1] > u) {
+        ids[p] = ids[p - 1];
+        tx[p] = tx[p - 1];
+        ty[p] = ty[p - 1];
+        p--;
+      }
+      ids[p] = u;
+      tx[p] = fx;
+      ty[p] = fy;
+    } else {
+      atomicOr(D.err, ERR_BOUND);
+    }
+  }
+  __device__ __forceinline__ void store(const Dev& D, const Real& M, int t) const {
+    double bx = 0.0, by = 0.0;
+    if (D.inside && !D.bound_from_lists) {
+      for (int j = M.dum0; j < M.dum0 + M.ndum2; j++) {
+        float fx, fy;
+        if (!bound_term(D, M, t, j, fx, fy)) continue;
+        bx = __dadd_rn(bx, f64_of(fx));
+        by = __dadd_rn(by, f64_of(fy));
+      }
+    } else {
+      for (int j = 0; j < n; j++) {
+        bx = __dadd_rn(bx, f64_of(tx[j]));
+        by = __dadd_rn(by, f64_of(ty[j]));
+      }
+    }
+    D.fbx[t] = bx;
+    D.fby[t] = by;
+  }
+};
+
 // The end of a step for particle t: its place in the step's pair build kept in x0x, x0y, then
 // the position update without XSPH (2_SPH_main_2018.f90:145-146): x = x0 + vel_half dt with
 // vel_half = 0.5 (v0 + v) rounded to FP32, and a node's displacement (:166-180).  With XSPH
