@@ -132,6 +132,9 @@ struct SurrGate {
   unsigned long long steps_on, steps_off;   // steps with and without the network
 };
 
+// elements a block of the exclusive scans (cells, pair counts): sizes of the block sums
+constexpr int kScan = 1024;
+
 struct Dev {
   // sizes (all realisations)
   int NN, NT, N2;  // nodes, nodes + stress-points, all particles

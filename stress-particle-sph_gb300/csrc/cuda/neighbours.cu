@@ -103,6 +103,13 @@ __device__ __forceinline__ double unkey(unsigned long long k) {
 }
 constexpr unsigned long long kNoKey = ~0ull;  // no active particle
 
+__device__ __forceinline__ unsigned long long warp_min(unsigned long long v) {
+  const unsigned hi = __reduce_min_sync(0xffffffffu, (unsigned)(v >> 32));
+  const unsigned lo =
+      __reduce_min_sync(0xffffffffu, (unsigned)(v >> 32) == hi ? (unsigned)v : 0xffffffffu);
+  return ((unsigned long long)hi << 32) | lo;
+}
+
 // true for every thread of the block that is the last of its grid to get here, once all
 // blocks' earlier global writes are visible to it (read them past L1: __ldcg); the ticket is
 // back at zero for the next launch
@@ -122,16 +129,20 @@ __device__ __forceinline__ bool last_block(unsigned* ticket) {
 }
 
 // Check_Out_Domain (2_SPH_main_2018.f90:1170) + the bounding box of the active particles of
-// every realisation: keys of (minx, miny, -maxx, -maxy, -maxh, minh), reduced over the warp
-// (or the block) when it holds one realisation, then atomicMin per realisation
+// every realisation: keys of (minx, miny, -maxx, -maxy, -maxh, minh).  A warp keeps the keys of
+// its stretch of consecutive particles in registers while they belong to one realisation,
+// and a block that holds one realisation combines its warps' before its atomicMin: one block's
+// worth of atomics for each 256 particles, to six addresses, took longer than the 29 bytes a
+// particle (2 million: 90 -> 37 us).
 // The step's first kernel: it also loads the step's scalars, clears the cell counts, and its
 // last block forms the grids (one launch instead of five: each of the small ones took about
 // 5 us of a step that lasts 300 at 10,000 particles).
 __device__ void grid_block(const Dev& D);
-__global__ void __launch_bounds__(kBlock) k_bbox(Dev D) {
+__global__ void __launch_bounds__(kBlock) k_bbox(Dev D, int per) {
   __shared__ unsigned long long sh[kBlock / 32][6];
   __shared__ int shr[kBlock / 32];
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (blockIdx.x == 0) {
     const int k = *D.step_idx;
     if (D.surr && threadIdx.x < 4) D.cand_count[threadIdx.x] = 0;  // the network's rows
@@ -140,77 +151,107 @@ __global__ void __launch_bounds__(kBlock) k_bbox(Dev D) {
     __syncthreads();
     if (threadIdx.x == 0) *D.step_idx = k + 1;
   }
-  for (int c = i; c < D.cell_cap + 2; c += gridDim.x * blockDim.x) {
+  for (int c = gid; c < D.cell_cap + 2; c += gridDim.x * blockDim.x) {
     D.cntK[c] = 0ull;
     D.cntD[c] = 0;
   }
-  unsigned long long v[6] = {kNoKey, kNoKey, kNoKey, kNoKey, kNoKey, kNoKey};
-  int r = -1;
-  if (i < D.N2) {
-    r = D.rid[i];
+  unsigned long long m[6] = {kNoKey, kNoKey, kNoKey, kNoKey, kNoKey, kNoKey};
+  int run = -1;  // the realisation that m is of
+  auto reduce = [&] {
+    for (int k = 0; k < 6; k++) m[k] = warp_min(m[k]);
+  };
+  // (x - xmin)(x - xmax) > 0 of the reference: both differences non-zero and of one sign, i.e.
+  // x outside [xmin, xmax] (the product of two such differences cannot underflow to zero for a
+  // domain of non-zero width; a NaN coordinate gives false), decided on the integer pipe
+  // with ordered keys
+  long long dom[4] = {0, 0, 0, 0};  // the realisation's domain: lowest and highest key by axis
+  auto domain = [&](int r) {
     const Real& M = D.real[r];
-    double x = D.px[i], y = D.py[i];
-    // (x - xmin)(x - xmax) > 0 of the reference: both differences non-zero and of one sign,
-    // i.e. x outside [xmin, xmax] (the product of two such differences cannot underflow to
-    // zero for a domain of non-zero width; a NaN coordinate gives false), decided on the
-    // integer pipe with ordered keys
-    auto outside = [](double v, double lo, double hi) {
-      if (f64_isnan(v)) return false;
-      const long long kv = f64_key(v), kl = f64_key(lo), kh = f64_key(hi);
-      return kv < min(kl, kh) || kv > max(kl, kh);
-    };
-    uint8_t o = D.out[i];
-    if (outside(x, M.xmin_dom[0], M.xmax_dom[0]) || outside(y, M.xmin_dom[1], M.xmax_dom[1]))
-      o = 1;
-    D.out[i] = o;
-    if (!o) {
-      double h = D.hsml[i];
-      v[0] = okey(x);
-      v[1] = okey(y);
-      v[2] = okey(-x);
-      v[3] = okey(-y);
-      v[4] = okey(-h);
-      v[5] = okey(h);
+    for (int d = 0; d < 2; d++) {
+      const long long a = f64_key(M.xmin_dom[d]), b = f64_key(M.xmax_dom[d]);
+      dom[2 * d] = min(a, b);
+      dom[2 * d + 1] = max(a, b);
+    }
+  };
+  auto outside = [](double v, long long lo, long long hi) {
+    const long long k = f64_key(v);
+    return !f64_isnan(v) && (k < lo || k > hi);
+  };
+  constexpr int U = 4;  // particles a lane whose loads are in flight together
+  const int i0 = (gid >> 5) * 32 * per + lane;
+  for (int q0 = 0; q0 < per; q0 += U) {
+    double X[U], Y[U], H[U];
+    int R[U];
+    uint8_t O[U];
+#pragma unroll
+    for (int q = 0; q < U; q++) {
+      const int i = i0 + 32 * (q0 + q);
+      const bool in = q0 + q < per && i < D.N2;
+      R[q] = in ? D.rid[i] : -1;
+      X[q] = in ? D.px[i] : 0.0;
+      Y[q] = in ? D.py[i] : 0.0;
+      H[q] = in ? D.hsml[i] : 0.0;
+      O[q] = in ? D.out[i] : 1;
+    }
+#pragma unroll
+    for (int q = 0; q < U; q++) {
+      const int r = R[q];
+      const int r0 = __reduce_max_sync(0xffffffffu, r);
+      if (r0 < 0) continue;  // past the end
+      // the 32 particles are of one realisation, or of several
+      const bool one = __all_sync(0xffffffffu, r < 0 || r == r0);
+      if (one && r0 != run) {
+        if (run >= 0) {
+          reduce();
+          if (lane == 0 && m[0] != kNoKey)
+            for (int k = 0; k < 6; k++) atomicMin(&D.bbox[6 * (size_t)run + k], m[k]);
+        }
+        for (int k = 0; k < 6; k++) m[k] = kNoKey;
+        run = r0;
+        domain(r0);
+      }
+      bool o = O[q];
+      if (r >= 0 && !o) {
+        if (!one) domain(r);
+        if (outside(X[q], dom[0], dom[1]) || outside(Y[q], dom[2], dom[3])) {
+          o = true;
+          D.out[i0 + 32 * (q0 + q)] = 1;
+        }
+      }
+      if (r >= 0 && !o) {
+        // the key of -x is the complement of x's
+        const unsigned long long kx = okey(X[q]), ky = okey(Y[q]), kh = okey(H[q]);
+        const unsigned long long v[6] = {kx, ky, ~kx, ~ky, ~kh, kh};
+        if (one) {
+          for (int k = 0; k < 6; k++) m[k] = v[k] < m[k] ? v[k] : m[k];
+        } else if (kx != kNoKey) {
+          for (int k = 0; k < 6; k++) atomicMin(&D.bbox[6 * (size_t)r + k], v[k]);
+        }
+      }
+      if (!one && run >= 0) domain(run);
     }
   }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  // the realisation of the warp (-1: several, or none active)
-  int r0 = __shfl_sync(0xffffffffu, r, 0);
-  for (int o = 16; o; o >>= 1) r0 = max(r0, __shfl_xor_sync(0xffffffffu, r0, o));
-  const bool uni = __all_sync(0xffffffffu, r < 0 || r == r0);
-  if (!uni) {
-    if (r >= 0 && v[0] != kNoKey)
-      for (int k = 0; k < 6; k++) atomicMin(&D.bbox[6 * (size_t)r + k], v[k]);
-    r0 = -1;
-  } else {
-    for (int k = 0; k < 6; k++)
-      for (int o = 16; o; o >>= 1) {
-        unsigned long long u = __shfl_xor_sync(0xffffffffu, v[k], o);
-        v[k] = u < v[k] ? u : v[k];
-      }
-  }
+  reduce();
   if (lane == 0) {
-    shr[wid] = r0;
-    for (int k = 0; k < 6; k++) sh[wid][k] = v[k];
+    shr[wid] = run;
+    for (int k = 0; k < 6; k++) sh[wid][k] = m[k];
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int rb = shr[0];
-    bool block_uni = rb >= 0;
-    for (int w = 1; w < kBlock / 32 && block_uni; w++) block_uni = shr[w] == rb;
-    if (block_uni) {
-      unsigned long long m[6];
-      for (int k = 0; k < 6; k++) {
-        m[k] = sh[0][k];
-        for (int w = 1; w < kBlock / 32; w++) m[k] = sh[w][k] < m[k] ? sh[w][k] : m[k];
-      }
-      if (m[0] != kNoKey)
-        for (int k = 0; k < 6; k++) atomicMin(&D.bbox[6 * (size_t)rb + k], m[k]);
-    } else {
-      for (int w = 0; w < kBlock / 32; w++)
-        if (shr[w] >= 0 && sh[w][0] != kNoKey)
-          for (int k = 0; k < 6; k++) atomicMin(&D.bbox[6 * (size_t)shr[w] + k], sh[w][k]);
+  int rb = -1;
+  bool one = true;  // the block's warps hold one realisation
+  for (int w = 0; w < kBlock / 32; w++) rb = max(rb, shr[w]);
+  for (int w = 0; w < kBlock / 32; w++) one = one && (shr[w] < 0 || shr[w] == rb);
+  const int t = threadIdx.x;
+  if (one) {
+    if (rb >= 0 && t < 6) {
+      unsigned long long u = sh[0][t];
+      for (int w = 1; w < kBlock / 32; w++) u = sh[w][t] < u ? sh[w][t] : u;
+      if (u != kNoKey) atomicMin(&D.bbox[6 * (size_t)rb + t], u);
     }
+  } else if (t < 6 * (kBlock / 32)) {
+    const int w = t / 6, k = t % 6;
+    if (shr[w] >= 0 && sh[w][k] != kNoKey)
+      atomicMin(&D.bbox[6 * (size_t)shr[w] + k], sh[w][k]);
   }
   if (last_block(D.tick)) grid_block(D);
 }
@@ -284,7 +325,7 @@ __device__ void grid_block(const Dev& D) {
     }
     sc[tid] = nc;
     __syncthreads();
-    for (int off = 1; off < kBlock; off <<= 1) {
+    for (int off = 1; off < kBlock && off < D.R; off <<= 1) {
       int add = tid >= off ? sc[tid - off] : 0;
       __syncthreads();
       sc[tid] += add;
@@ -296,7 +337,7 @@ __device__ void grid_block(const Dev& D) {
       D.grid[r] = g;
     }
     __syncthreads();
-    if (tid == kBlock - 1) carry += sc[tid];
+    if (tid == min(kBlock, D.R - base) - 1) carry += sc[tid];
     __syncthreads();
   }
   if (tid == 0) {
@@ -393,8 +434,10 @@ __global__ void k_cell_count(Dev D) {
 
 // Exclusive scans of the cells' counts (total and by kind), kScan cells a block: the scan
 // within the block (cell_loc, cell_locK) and, by the last block, of the blocks' sums (cell_bs,
-// cell_bsK); readers add the two.  Blocks past the last cell only take their ticket.
-constexpr int kScan = kBlock * 16;
+// cell_bsK); readers add the two.  Blocks past the last cell only take their ticket.  A chain of
+// latencies: four elements a thread, loaded together (16, one after the other, took 20 us at 10,000
+// particles where this takes 9, events included).
+constexpr int kPer = kScan / kBlock;
 template <typename T>
 __device__ __forceinline__ T block_exclusive(T v, T* sh, T& total) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -436,29 +479,34 @@ __global__ void __launch_bounds__(kBlock) k_scan_cells(Dev D) {
   const int n = D.gtot->ncells + 1;  // the out-of-domain bucket is the last
   const int base = blockIdx.x * kScan;
   if (base < n) {
-    const int i0 = base + threadIdx.x * 16;
-    int lt = 0;
-    unsigned long long lk = 0;
-    for (int q = 0; q < 16; q++) {
-      const int c = i0 + q;
-      if (c >= n) break;
-      const unsigned long long k = D.cntK[c];
-      const int t = (int)(k >> 32) + (int)(unsigned)k + D.cntD[c];
-      D.cell_cnt[c] = t;
-      lt += t;
-      lk += k;
+    const int i0 = base + threadIdx.x * kPer;
+    int t[kPer], lt = 0;
+    unsigned long long k[kPer], lk = 0;
+#pragma unroll
+    for (int q = 0; q < kPer; q++) {
+      k[q] = i0 + q < n ? D.cntK[i0 + q] : 0ull;
+      t[q] = i0 + q < n ? D.cntD[i0 + q] : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kPer; q++) {
+      t[q] += (int)(k[q] >> 32) + (int)(unsigned)k[q];
+      lt += t[q];
+      lk += k[q];
     }
     int totT;
     unsigned long long totK;
     int rt = block_exclusive(lt, shT, totT);
     unsigned long long rk = block_exclusive(lk, shK, totK);
-    for (int q = 0; q < 16; q++) {
+#pragma unroll
+    for (int q = 0; q < kPer; q++) {
       const int c = i0 + q;
-      if (c >= n) break;
-      D.cell_loc[c] = rt;
-      D.cell_locK[c] = rk;
-      rt += D.cell_cnt[c];
-      rk += D.cntK[c];
+      if (c < n) {
+        D.cell_cnt[c] = t[q];
+        D.cell_loc[c] = rt;
+        D.cell_locK[c] = rk;
+      }
+      rt += t[q];
+      rk += k[q];
     }
     if (threadIdx.x == 0) {
       D.cell_bs[blockIdx.x] = totT;
@@ -1311,17 +1359,20 @@ __device__ __forceinline__ int64_t half_first(const Dev& D, int s) {
 }
 __global__ void __launch_bounds__(kBlock) k_scan_half(Dev D) {
   __shared__ long long sh[kBlock / 32];
-  const int base = blockIdx.x * kScan, i0 = base + threadIdx.x * 16;
+  const int i0 = blockIdx.x * kScan + threadIdx.x * kPer;
+  int h[kPer];
   long long l = 0;
-  for (int q = 0; q < 16; q++)
-    if (i0 + q < D.N2) l += D.half_cnt[i0 + q];
+#pragma unroll
+  for (int q = 0; q < kPer; q++) h[q] = i0 + q < D.N2 ? D.half_cnt[i0 + q] : 0;
+#pragma unroll
+  for (int q = 0; q < kPer; q++) l += h[q];
   long long tot;
   long long run = block_exclusive(l, sh, tot);
-  for (int q = 0; q < 16; q++)
-    if (i0 + q <= D.N2) {  // one past the end: the total
-      D.half_off[i0 + q] = run;
-      if (i0 + q < D.N2) run += D.half_cnt[i0 + q];
-    }
+#pragma unroll
+  for (int q = 0; q < kPer; q++) {
+    if (i0 + q <= D.N2) D.half_off[i0 + q] = run;  // one past the end: the total
+    run += h[q];
+  }
   if (threadIdx.x == 0) D.half_bs[blockIdx.x] = tot;
   if (!last_block(D.tick + 2)) return;
   const long long all = scan_sums(reinterpret_cast<long long*>(D.half_bs), (int)gridDim.x, sh);
@@ -1620,7 +1671,9 @@ int launch_pair_build(Ctx& c) {
   const int nb = (D.N2 + kBlock - 1) / kBlock;
   const int b = Ctx::block_for(D.N2, kBlock), nbs = (D.N2 + b - 1) / b;
   c.mark("bbox");
-  k_bbox<<<nb, kBlock, 0, st>>>(D);
+  // 256 to 2048 particles a block: at least as many blocks as fit the chip while there are
+  const int per = std::min(8, std::max(1, nb / 608));
+  k_bbox<<<(nb + per - 1) / per, kBlock, 0, st>>>(D, per);
   c.mark("cell_count");
   k_cell_count<<<nbs, b, 0, st>>>(D);
   c.mark("scan_cells");

@@ -854,7 +854,7 @@ int sps_create_batch(int32_t nreal, const sps_params* ps, sps_ctx** out) {
     D.half_cnt = dalloc<int32_t>(c, N2);
     D.half_meta = dalloc<int4>(c, N2);
     D.half_off = dalloc<int64_t>(c, N2 + 1);
-    D.half_bs = dalloc<int64_t>(c, N2 / 4096 + 2);
+    D.half_bs = dalloc<int64_t>(c, N2 / sps::kScan + 2);
     D.degC = dalloc<int32_t>(c, N2);
     D.degS = dalloc<int32_t>(c, N2);
     D.meta = dalloc<sps::PairMeta>(c, nreal);
@@ -1045,8 +1045,8 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
       D.cell_loc = dalloc<int32_t>(c, (size_t)cap + 2);
       D.cntK = dalloc<unsigned long long>(c, (size_t)cap + 2);
       D.cell_locK = dalloc<unsigned long long>(c, (size_t)cap + 2);
-      D.cell_bs = dalloc<int32_t>(c, (size_t)cap / 4096 + 2);
-      D.cell_bsK = dalloc<unsigned long long>(c, (size_t)cap / 4096 + 2);
+      D.cell_bs = dalloc<int32_t>(c, (size_t)cap / sps::kScan + 2);
+      D.cell_bsK = dalloc<unsigned long long>(c, (size_t)cap / sps::kScan + 2);
       D.cell_cap = cap;
       drop_graphs(c);
     }

@@ -74,3 +74,24 @@ def test_gathered_lists_fp32(built_gpu, name):
         u, v = a[k][:n], b[k][:n]
         assert np.linalg.norm(u - v) <= 1e-5 * np.linalg.norm(v), k
     gpu.close()
+
+
+def test_batch_of_unequal_problems(built_gpu):
+    # realisations of 2,000 to 140,000 particles, so that the bounding boxes' stretches of
+    # consecutive particles (64 and more a warp at this total) lie in one realisation or
+    # span two; each equals its own run bit for bit
+    probs = [sps_gb300.Problem.slope(dx=0.045), sps_gb300.Problem.column(dx=0.0043),
+             sps_gb300.Problem.slope(dx=0.046), sps_gb300.Problem.column(dx=0.004),
+             sps_gb300.Problem.slope(dx=0.05)]
+    assert sum(p.ntotal for p in probs) > 320000
+    batch = sps_gb300.Batch(probs, precision=_abi.SPS_PREC_FP64_PLAIN)
+    batch.upload_all()
+    batch.step(2)
+    for r, p in enumerate(probs):
+        one = sps_gb300.StepContext(sps_gb300.gpu_lib(), "sps",
+                                    p.params_copy(precision=_abi.SPS_PREC_FP64_PLAIN))
+        one.upload_problem(p)
+        one.step(2, 0.0)
+        cases.assert_bitwise(batch.download(r), one.download(), p.ntotal)
+        one.close()
+    batch.close()
