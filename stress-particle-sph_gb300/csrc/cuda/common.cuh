@@ -328,22 +328,101 @@ __device__ __forceinline__ bool f64_isnan(double a) {
 // a >= b for non-NaN doubles, on the integer pipe
 __device__ __forceinline__ bool f64_ge(double a, double b) { return f64_key(a) >= f64_key(b); }
 
-// Correctly rounded a / b given y = RN(1/b), by Markstein's theorem (P. Markstein, "Computation
-// of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1),
-// 1990; see also Muller et al., Handbook of Floating-Point Arithmetic, the theorem on
+// ---- FP64 products and quotients on the integer pipes ------------------------------------
+// GB300 issues two FP64 lanes a clock on each SM: a warp's FP64 instruction holds its
+// scheduler's pipe for 64 cycles, and the sums of the plain form, which round every product and
+// every sum to FP64, are bound by that pipe.  The products, and the divisions by a density whose
+// reciprocal is known, leave it here: the exact product of the significands (or the exact
+// remainder) from 32 x 32 -> 64 bit multiply-adds, rounded to nearest even by the definition of
+// IEEE 754, in about 40 integer instructions; the additions stay on the FP64 pipe, which then
+// works beside the integer ones (2 million particles, us a step: stages 7170 -> 4650, list
+// constants 1069 -> 476, last interpolation 581 -> 416, cells of the particles 106 -> 63;
+// 115,000: stages 615 -> 362).  Operands or results outside the normal range (zeros,
+// subnormals, infinities, NaN) leave the line: inlined, the compiler may issue the FP64
+// instructions with their predicate off, which occupies the pipe as well.
+// sps_selftest compares both with the FP64 instructions, bit for bit.
+static __device__ __noinline__ double mul_rare(double a, double b) {
+  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  const unsigned long long u = (unsigned long long)x << 1, v = (unsigned long long)y << 1;
+  const unsigned long long inf = 0xffe0000000000000ull;  // without its sign
+  // a zero times a finite number, common where the material is still at rest
+  if ((u == 0 || v == 0) && u < inf && v < inf)
+    return __longlong_as_double((x ^ y) & (long long)0x8000000000000000ull);
+  return a * b;
+}
+__device__ __forceinline__ double mul_int(double a, double b) {
+  const unsigned ah = (unsigned)__double2hiint(a), al = (unsigned)__double2loint(a);
+  const unsigned bh = (unsigned)__double2hiint(b), bl = (unsigned)__double2loint(b);
+  // the significands as integers in [2^52, 2^53), b's times 2^11: the upper 64 bits of their
+  // product hold 52 or 53 bits
+  const unsigned a1 = (ah & 0xfffffu) | 0x100000u;
+  const unsigned b1 = __funnelshift_l(bl, (bh & 0xfffffu) | 0x100000u, 11), b0 = bl << 11;
+  const unsigned long long t0 = (unsigned long long)al * b0;
+  const unsigned long long t1 = (unsigned long long)a1 * b0 + (unsigned)(t0 >> 32);
+  const unsigned long long t2 = (unsigned long long)al * b1 + (unsigned)t1;
+  const unsigned long long t3 =
+      (unsigned long long)a1 * b1 + (unsigned)(t1 >> 32) + (unsigned)(t2 >> 32);
+  const unsigned w0 = (unsigned)t0, w1 = (unsigned)t2, w2 = (unsigned)t3, w3 = (unsigned)(t3 >> 32);
+  const unsigned n = w3 >> 20;  // 1: 53 bits (the significands' product is 2 or more)
+  const unsigned sh = 1u - n;
+  const unsigned h = __funnelshift_l(w2, w3, sh), l = __funnelshift_l(w1, w2, sh);
+  // the bits below the last place, the lowest of the 32 standing for all that follow
+  const unsigned f = __funnelshift_l(w0, w1, sh) | min(w0 << sh, 1u);
+  const unsigned up = f > 0x80000000u - (l & 1u);
+  const unsigned ea = ah & 0x7ff00000u, eb = bh & 0x7ff00000u;
+  const unsigned E = ea + eb - 0x40000000u + (n << 20);  // exponent - 1: h holds the leading 1
+  if (max(ea - 0x100000u, eb - 0x100000u) >= 0x7fe00000u || E >= 0x7fd00000u) return mul_rare(a, b);
+  const unsigned long long R = (((unsigned long long)(h + E) << 32) | l) + up;
+  return __hiloint2double((int)((unsigned)(R >> 32) | ((ah ^ bh) & 0x80000000u)), (int)(unsigned)R);
+}
+
+// Correctly rounded a / b given y = RN(1/b), outside the range of the integer form: by
+// Markstein's theorem (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34(1), 1990; see also Muller et al., Handbook of Floating-Point Arithmetic, the theorem on
 // FMA-based division): when y is within 1/2 ulp of 1/b and q within 1 ulp of a/b, the
 // corrected q' = RN(q + y * (a - b q)) equals RN(a/b).  q = RN(a y) can be up to 1.5 ulp
 // off, so one correction step brings it within 1 ulp and a second one rounds correctly.
 // Valid for normal operands without overflow or underflow (masses, densities and kernel
-// values here); a zero numerator returns a signed zero.  Bit-for-bit agreement with the
-// IEEE division is checked on the GPU by sps_selftest.
-__device__ __forceinline__ double div_rcp(double a, double b, double y) {
-  if ((__double_as_longlong(a) << 1) == 0) return a * y;  // a zero, tested on the integer pipe
+// values here); a zero numerator returns a signed zero.
+static __device__ __noinline__ double div_rcp_rare(double a, double b, double y) {
+  if ((__double_as_longlong(a) << 1) == 0) return mul_rare(a, y);
   double q = a * y;
   double r = fma(-b, q, a);
   q = fma(r, y, q);
   r = fma(-b, q, a);
   return fma(r, y, q);
+}
+// The integer form, in place of those five FP64 instructions: q, the product of a's and y's
+// significands rounded down, lies less than 2 below and less than 1 above the quotient X in
+// [2^52, 2^53), since y is off by half a place at most; the remainder R = a - q b, all of it
+// in the low 64 bits, tells the integer nearest to X (a quotient of two 53-bit numbers is
+// never half-way).  The reciprocal of a power of two takes one more place.
+__device__ __forceinline__ double div_rcp(double a, double b, double y) {
+  typedef unsigned long long u64;
+  const unsigned ah = (unsigned)__double2hiint(a), al = (unsigned)__double2loint(a);
+  const unsigned bh = (unsigned)__double2hiint(b), bl = (unsigned)__double2loint(b);
+  const unsigned yh = (unsigned)__double2hiint(y), yl = (unsigned)__double2loint(y);
+  const unsigned a1 = (ah & 0xfffffu) | 0x100000u, b1 = (bh & 0xfffffu) | 0x100000u;
+  const unsigned y1 = (yh & 0xfffffu) | 0x100000u;
+  const u64 mb = ((u64)b1 << 32) | bl;
+  const unsigned s = (((u64)a1 << 32) | al) < mb;  // 1: the significands' quotient is below 1
+  const unsigned ea = ah & 0x7ff00000u, eb = bh & 0x7ff00000u, ey = yh & 0x7ff00000u;
+  const unsigned p2 = eb + ey - 0x7fd00000u;  // 0; 0x100000 for a power of two b
+  const unsigned sh = s | (p2 >> 20);
+  const unsigned h1 = __funnelshift_l(al, a1, 11), h0 = al << 11;
+  const unsigned g1 = __funnelshift_l(yl, y1, sh), g0 = yl << (sh & 31u);
+  const u64 t0 = (u64)g0 * h0;
+  const u64 t1 = (u64)g1 * h0 + (unsigned)(t0 >> 32);
+  const u64 t2 = (u64)g0 * h1 + (unsigned)t1;
+  const u64 q = (u64)g1 * h1 + (unsigned)(t1 >> 32) + (unsigned)(t2 >> 32);
+  const u64 R = ((u64)(al << (20u + s)) << 32) - q * mb;
+  const long long R2 = (long long)(R << 1), B = (long long)mb;
+  const int d = (R2 > B) + (R2 > 3 * B) - (R2 < -B);
+  const unsigned E = ea - eb + 0x3fe00000u - (s << 20);  // exponent - 1
+  if (max(ea - 0x100000u, eb - 0x100000u) >= 0x7fc00000u || E >= 0x7fd00000u || p2 > 0x100000u)
+    return div_rcp_rare(a, b, y);
+  const u64 v = q + (long long)d + ((u64)E << 32);
+  return __hiloint2double((int)((unsigned)(v >> 32) | ((ah ^ bh) & 0x80000000u)), (int)(unsigned)v);
 }
 
 // ---- FP64 <-> FP32 conversions on the integer pipe --------------------------------------

@@ -9,7 +9,8 @@
 //   norm the sum of W m / rho of a target, and its reciprocal
 //   AE   the CSPM moments of a target
 // A stage then reads them instead of recomputing: 4 + 10 FP64 operations an entry on the
-// stress-point side and 8 + 21 on the node side, against 12 + 22 and 18 + 21.
+// stress-point side and 8 + 21 on the node side, against 12 + 22 and 18 + 21; the
+// multiplications among them (2 + 4 and 4 + 12) run on the integer pipes (mul_int).
 //
 // k_pstage runs a whole stage of both kinds (blocks of stress-points first, then blocks of
 // nodes): stress_point_update, adapt_stress2 and the BCs, get_derivatives, the rates, their
@@ -20,7 +21,7 @@
 // plain_step.cu, which remain for the options that change densities or node stresses between
 // the two halves of a stage (Ctx::fused).
 //
-// What bounds it: the FP64 pipe (2 lanes a clock and SM) at large sizes; at small ones the
+// What bounds it: the additions on the FP64 pipe (2 lanes a clock and SM) at large sizes; at small ones the
 // serial chain of a target's sums, which LS and LN lanes a target share by component (one
 // velocity component a lane, one stress component a lane), each component still summed in
 // list order by one lane.
@@ -95,10 +96,10 @@ __device__ __forceinline__ bool sp_entry(const Dev& D, int k, int j, double xt, 
   double h, h1, h2;
   if (!wall) {
     const double w = f64_of(__int_as_float(e.y));
-    h = D.vol[u] * w;
-    T.norm = div_rcp(w * mu, ru, iu);
-    h1 = div_rcp(Gx * mu, ru, iu);
-    h2 = div_rcp(Gy * mu, ru, iu);
+    h = mul_int(D.vol[u], w);
+    T.norm = div_rcp(mul_int(w, mu), ru, iu);
+    h1 = div_rcp(mul_int(Gx, mu), ru, iu);
+    h2 = div_rcp(mul_int(Gy, mu), ru, iu);
     if (CSPM) {
       const double xu = D.px[u] - xt, yu = D.py[u] - yt;
       T.e[0] = xu * h1;
@@ -142,8 +143,8 @@ __device__ __forceinline__ bool node_entry(const Dev& D, const Real& M, int t, i
   }
   const double w = f64_of(__int_as_float(e.y));
   const double mu = D.mass[u], ru = D.rho[u], iu = D.rinv[u];
-  D.hW[(size_t)j * D.NT + k] = D.vol[u] * w;
-  T.norm = div_rcp(w * mu, ru, iu);
+  D.hW[(size_t)j * D.NT + k] = mul_int(D.vol[u], w);
+  T.norm = div_rcp(mul_int(w, mu), ru, iu);
   if (CSPM) {
     const double dwx = -f64_of(__int_as_float(e.z)), dwy = -f64_of(__int_as_float(e.w));
     const double h1b = -div_rcp(dwx * mu, ru, iu), h2b = -div_rcp(dwy * mu, ru, iu);
@@ -272,7 +273,8 @@ __global__ void __launch_bounds__(128) k_pprep(Dev D) {
   }
 }
 
-// entries a pass whose list words and neighbour records are loaded before any is summed
+// entries a pass whose list words and neighbour records are loaded before any is summed: more
+// in flight where few warps are there to hide a latency, one where they are many (below)
 constexpr int kP = 4;
 
 // A wall's velocity seen by a stress-point: v - (v (1 - beta) + beta 0).  Rare, and out of line:
@@ -282,6 +284,7 @@ static __device__ __noinline__ double wall_du64(double v, double ob) { return v 
 // One stage of a stress-point; LS = 2: lane d of the pair sums velocity component d
 template <int LS>
 __device__ __forceinline__ void sp_stage(const Dev& D, int stage, int k, bool act, int q) {
+  constexpr int kP = LS == 1 ? 1 : 4;
   const int ns = D.NT - D.NN, cur = stage & 1, nxt = cur ^ 1;
   const int t = D.colid[k];
   const double2* __restrict__ pv = reinterpret_cast<const double2*>(D.pv[cur]);
@@ -307,8 +310,8 @@ __device__ __forceinline__ void sp_stage(const Dev& D, int stage, int k, bool ac
     for (int i = 0; i < kP; i++)
       if (e[i].y >= 0) {
         if (LS == 1) {
-          v0 = v0 + v[i].x * h[i];
-          v1 = v1 + v[i].y * h[i];
+          v0 = v0 + mul_int(v[i].x, h[i]);
+          v1 = v1 + mul_int(v[i].y, h[i]);
         } else {
           v0 = v0 + (q ? v[i].y : v[i].x) * h[i];
         }
@@ -357,11 +360,11 @@ __device__ __forceinline__ void sp_stage(const Dev& D, int stage, int k, bool ac
           du0 = wall_du64(vtq, v[i].x);
           if (LS == 1) du1 = wall_du64(vt1, v[i].x);
         }
-        g[0] = g[0] + du0 * h[i].x;
-        g[2] = g[2] + du0 * h[i].y;
+        g[0] = g[0] + mul_int(du0, h[i].x);
+        g[2] = g[2] + mul_int(du0, h[i].y);
         if (LS == 1) {
-          g[1] = g[1] + du1 * h[i].x;
-          g[3] = g[3] + du1 * h[i].y;
+          g[1] = g[1] + mul_int(du1, h[i].x);
+          g[3] = g[3] + mul_int(du1, h[i].y);
         }
       }
   }
@@ -457,6 +460,7 @@ static __device__ __noinline__ double wall_A(double s, double r2, double y) { re
 // derivative sums of component q (q < 3)
 template <int LN>
 __device__ __forceinline__ void node_stage(const Dev& D, int stage, int k, bool act, int q) {
+  constexpr int kP = LN == 1 ? 1 : 4;
   const int cur = stage & 1, nxt = cur ^ 1;
   const int t = D.colid[k];
   const double* __restrict__ ps = D.ps[cur];
@@ -490,10 +494,10 @@ __device__ __forceinline__ void node_stage(const Dev& D, int stage, int k, bool 
     for (int i = 0; i < kP; i++)
       if (e[i].y >= 0) {
         if (LN == 1) {
-          s[0] = s[0] + v[i].a * h[i];
-          s[1] = s[1] + v[i].b * h[i];
-          s[2] = s[2] + v[i].c * h[i];
-          s[3] = s[3] + v[i].d * h[i];
+          s[0] = s[0] + mul_int(v[i].a, h[i]);
+          s[1] = s[1] + mul_int(v[i].b, h[i]);
+          s[2] = s[2] + mul_int(v[i].c, h[i]);
+          s[3] = s[3] + mul_int(v[i].d, h[i]);
         } else {
           s[0] = s[0] + vq[i] * h[i];
         }
@@ -573,8 +577,8 @@ __device__ __forceinline__ void node_stage(const Dev& D, int stage, int k, bool 
 #pragma unroll
           for (int p = 0; p < 3; p++) {
             const double sum = at[p] + au[p];
-            g2[p] = g2[p] - mu[i] * (dwx * sum);
-            g2[p + 3] = g2[p + 3] - mu[i] * (dwy * sum);
+            g2[p] = g2[p] - mul_int(mu[i], mul_int(dwx, sum));
+            g2[p + 3] = g2[p + 3] - mul_int(mu[i], mul_int(dwy, sum));
           }
         } else {
           const double sum = at[0] + aq[i];
@@ -683,8 +687,12 @@ __device__ __forceinline__ void node_stage(const Dev& D, int stage, int k, bool 
 
 // RK4 stage (2_SPH_main_2018.f90:700-777): blocks [0, nbs) the stress-points, the rest the
 // nodes
+// One lane a target: 64 registers, eight blocks a multiprocessor, one entry in flight a lane; the
+// FP64 pipe and the integer pipes work for different warps at the same time, so many of them are
+// needed (2 million particles, us a step: four entries and 124 registers 6253, two and 5485,
+// one and 80 registers 5037, one and 64 registers 4903, spills included).
 template <int LS, int LN>
-__global__ void __launch_bounds__(128) k_pstage(Dev D, int stage, int nbs) {
+__global__ void __launch_bounds__(128, LS == 1 ? 8 : 1) k_pstage(Dev D, int stage, int nbs) {
   const int ns = D.NT - D.NN;
   if ((int)blockIdx.x < nbs) {
     const int g = (blockIdx.x * blockDim.x + threadIdx.x) / LS;
@@ -701,7 +709,12 @@ __global__ void __launch_bounds__(128) k_pstage(Dev D, int stage, int nbs) {
 
 // the final interpolation, return and BCs (2_SPH_main_2018.f90:130-135), then the position
 // update (:140-146, without XSPH) and the displacements (:166-180)
+// INT: the products on the integer pipes (large problems; below, where the chain of one warp's
+// latencies counts and not the FP64 pipe, the FP64 multiplication is shorter: 600 particles 24
+// us against 29; 2 million 581 against 430)
+template <bool INT>
 __global__ void __launch_bounds__(128) k_pfinish(Dev D) {
+  constexpr int kP = INT ? 2 : 4;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= D.N2) return;
   if (k >= D.NT) {  // dummies: their place in the step's pair build
@@ -735,8 +748,8 @@ __global__ void __launch_bounds__(128) k_pfinish(Dev D) {
 #pragma unroll
       for (int i = 0; i < kP; i++)
         if (e[i].y >= 0) {
-          v0 = v0 + v[i].x * h[i];
-          v1 = v1 + v[i].y * h[i];
+          v0 = v0 + (INT ? mul_int(v[i].x, h[i]) : v[i].x * h[i]);
+          v1 = v1 + (INT ? mul_int(v[i].y, h[i]) : v[i].y * h[i]);
         }
     }
     vx0 = D.vx[t];
@@ -771,10 +784,10 @@ __global__ void __launch_bounds__(128) k_pfinish(Dev D) {
 #pragma unroll
       for (int i = 0; i < kP; i++)
         if (e[i].y >= 0) {
-          s[0] = s[0] + v[i].a * h[i];
-          s[1] = s[1] + v[i].b * h[i];
-          s[2] = s[2] + v[i].c * h[i];
-          s[3] = s[3] + v[i].d * h[i];
+          s[0] = s[0] + (INT ? mul_int(v[i].a, h[i]) : v[i].a * h[i]);
+          s[1] = s[1] + (INT ? mul_int(v[i].b, h[i]) : v[i].b * h[i]);
+          s[2] = s[2] + (INT ? mul_int(v[i].c, h[i]) : v[i].c * h[i]);
+          s[3] = s[3] + (INT ? mul_int(v[i].d, h[i]) : v[i].d * h[i]);
           iv = iv + w[i] * h[i];
         }
     }
@@ -835,7 +848,8 @@ void launch_pstage(Ctx& c, int stage) {
 
 void launch_pfinish(Ctx& c) {
   const int b = c.block_for(c.d.N2, 128);
-  k_pfinish<<<(c.d.N2 + b - 1) / b, b, 0, c.stream>>>(c.d);
+  if (c.d.NT > c.split_max) k_pfinish<true><<<(c.d.N2 + b - 1) / b, b, 0, c.stream>>>(c.d);
+  else k_pfinish<false><<<(c.d.N2 + b - 1) / b, b, 0, c.stream>>>(c.d);
 }
 
 }  // namespace sps

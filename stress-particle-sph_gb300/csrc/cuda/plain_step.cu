@@ -773,6 +773,22 @@ __global__ void k_selftest_div(int64_t n, uint64_t seed, unsigned long long* bad
     double y = 1.0 / b;
     double q1 = div_rcp(a, b, y), q2 = a / b;
     if (__double_as_longlong(q1) != __double_as_longlong(q2)) nb++;
+    // products and quotients: of these, of numbers with few significand bits (exact results, ties,
+    // powers of two) and of any bits at all (zeros, subnormals, overflow, NaN)
+    auto same = [](double x, double y) {
+      return __double_as_longlong(x) == __double_as_longlong(y) || (x != x && y != y);
+    };
+    const double as = __longlong_as_double(__double_as_longlong(a) & ~((1ll << (r1 % 53)) - 1));
+    const double bs = __longlong_as_double(__double_as_longlong(b) & ~((1ll << (r2 % 53)) - 1));
+    const double ax = __longlong_as_double((long long)r2), bx = __longlong_as_double((long long)r3);
+    if (!same(mul_int(a, b), a * b) || !same(mul_int(as, b), as * b) ||
+        !same(mul_int(as, bs), as * bs) || !same(mul_int(ax, bx), ax * bx) ||
+        !same(mul_int(ax, b), ax * b) || !same(mul_int(a, 0.0), a * 0.0))
+      nb++;
+    const double ys = 1.0 / bs;
+    if (!same(div_rcp(as, b, y), as / b) || !same(div_rcp(a, bs, ys), a / bs) ||
+        !same(div_rcp(as, bs, ys), as / bs) || !same(div_rcp(as * bs, bs, ys), (as * bs) / bs))
+      nb++;
     // the float rounding of the quotient, also where the float boundary is near: a scaled
     // so that a / b sits within a few double ulps of a float or of a float half-way point
     if (__float_as_uint(div_rcp_f32(a, b, y)) != __float_as_uint((float)q2)) nb++;
