@@ -122,7 +122,12 @@ struct Ctx {
   // 52 / 41, of 40,000 64 / 51, of 80,000 86 / 91, biaxial sample of 40,000 with wall segments
   // 58 / 110; FP32 slope of 40,000 31 / 23, of 180,000 49 / 74)
   int group_max = 40000;
-  int split_max = 60000;  // largest NT whose stage kernels split a target's sums over lanes
+  // largest NT whose plain stages split a target's sums over lanes: few warps and a long chain
+  // each below it, the pipes busy with one lane a target above (us a step split / one lane:
+  // 600 particles 170 / 320, slopes of 17,000 135 / 244, 29,000 208 / 249, 40,000 257 / 249,
+  // 59,000 351 / 272, 87,000 458 / 325; biaxial sample of 40,000 418 / 385)
+  int split_max = 36000;
+  int surface_split_max = 60000;  // the same for the exact free-surface detection
   // the last pair build left the half lists unwritten (k_fgather): sps_dump_pairs and the
   // keyed lists of the exact detection build them first (set by enqueue_step for every
   // step, since a replayed graph runs no host code)

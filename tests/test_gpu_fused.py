@@ -1,6 +1,6 @@
 """GPU: the plain form's one-launch stages (plain_fused.cu) against the CPU oracle, bit for bit,
 at the sizes where their split matters: fewer targets than a warp, a ragged last warp, a
-target's sums shared by several lanes (below 60,000 particles) and by one lane (above), with
+target's sums shared by several lanes (small problems) and by one lane (large ones), with
 the list constants of walls, CSPM moments, artificial viscosity, several stress-points a cell
 and nodes without stress-points in reach."""
 import numpy as np
