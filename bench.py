@@ -547,6 +547,19 @@ def kernel_bytes(name, prob, deg, fast=False):
     ent = 16.0
     # the node-node list is read by the derivative sums only for artificial viscosity
     visc = prob.params.alpha > 0 or prob.params.beta > 0
+    # the one-launch stages, their preparation and the final interpolation: an entry is 8 B of
+    # partner and weight and 8 B of gradient (FP32 form), or 16 B of list entry, 8 B of
+    # weight and, on the stress-point side (half the entries), 16 B of gradient factors
+    if name == "stage":
+        state = ns * (32 + 64 + 80) + nn * (32 + 48)  # RK state, rates, the next stage's
+        if fast:
+            return 16.0 * deg["cross"] + 16 * nn + 32 * ns + state
+        return (ent + 8 + 8) * deg["cross"] + (ent * deg["same_nodes"] if visc else 0) + \
+            16 * nn + 64 * ns + state
+    if name == "prep":
+        return (ent + 16.0) * deg["cross"] + 16 * nn + 48 * ns
+    if name == "finish":
+        return (8.0 if fast else ent + 8) * deg["cross"] + 16 * nn + 32 * ns + 80 * n2
     if fast and name == "derivs":
         # entries + one 16 B record per neighbour-visible particle + per-particle FP64
         # state read/written once (SP: v, s, grad_u, RHS1, RKs, fdp, RKd; node: v, RHS2, RKv)
@@ -563,15 +576,13 @@ def kernel_bytes(name, prob, deg, fast=False):
         return ent * deg["cross"] + ns * (16 + 16) + nn * (40 + 16 + 16)
     if name == "half":
         return n2 * (4 * 8 + 8) + ent * deg["pairs"]
-    if fast and name == "gather":
-        # the FP32 form's direct lists: entries written (the same-kind lists' only when a
-        # step kernel reads them) and the compact {id, W} copy of the cross entries (8 B),
-        # and per particle its sorted record (16 + 8 B), its own offsets (20 B), ids, type,
-        # realisation and cell (16 B), counts (12 B), target (4 B)
+    if name == "gather":
+        # the direct lists: entries written (the same-kind lists' only when a step kernel
+        # reads them), and per particle its sorted record (16 + 8 B), its own offsets (20 B),
+        # ids, type, realisation and cell (16 B), counts (12 B), target (4 B)
         p = prob.params
         same_written = p.xsph or p.art_stress or p.alpha > 0 or p.beta > 0
-        return ent * (deg["cross"] + (deg["same"] if same_written else 0)) + \
-            8.0 * deg["cross"] + n2 * 76
+        return ent * (deg["cross"] + (deg["same"] if same_written else 0)) + n2 * 76
     if name == "lists":
         # entries written (the same-kind lists' only when a step kernel reads them: XSPH,
         # artificial viscosity or stress), and the creators' half-list entries read,
@@ -583,16 +594,16 @@ def kernel_bytes(name, prob, deg, fast=False):
     return None
 
 
-# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) per launch group of the FP32
-# form on the full-size slope (dx 0.012 m), from one ncu pass over the first timed stage
-# (profiles/dram_traffic_fp32_slope_2M.md); the neighbour sums' group is the stress-point
-# and the node launch of one stage, the gather's the two target kinds and the remaining
-# positions.  Valid for that workload and this code state only.
-NCU_TRAFFIC_FULL = {"derivs": 337793792 + 22539776 + 388249856 + 26990592,
-                    "interp": 176712704 + 8054784 + 178151168 + 22437632,
-                    "gather": 100680704 + 339088640 + 101198848 + 336080384 + 8663552}
+# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) per launch of the FP32 form on
+# the full-size slope (dx 0.012 m), from one ncu pass over a step
+# (profiles/one_launch_stages.md); the stages' figure is the mean of the four launches.
+# Valid for that workload and this code state only.
+NCU_TRAFFIC_FULL = {"stage": 825611328 + 224183168,
+                    "gather": 210693888 + 540843520,
+                    "prep": 649908736 + 707065856,
+                    "finish": 440041984 + 139260160}
 NCU_TRAFFIC_SOURCE = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum (1 pass), "
-                      "FP32 form, this slope at dx 0.012 m, first timed stage")
+                      "FP32 form, this slope at dx 0.012 m, the second step")
 
 
 def timed_steps(ctx, nsteps, t, dist, local, mark=False):
@@ -751,7 +762,9 @@ def run_ours(args):
         # for the stress-point targets and once for the node targets, back to back
         label = {"derivs": "k_fderivs<1> + k_fderivs<2>" if fast else "k_derivs (both kinds)",
                  "interp": "k_finterp<1> + k_finterp<2>" if fast else "k_interp (both kinds)",
-                 "gather": "k_fgather<1> + k_fgather<2> + k_fgather_rest"}
+                 "gather": "k_fgather", "prep": "k_fprep" if fast else "k_pprep",
+                 "stage": "k_fstage" if fast else "k_pstage",
+                 "finish": "k_ffinish" if fast else "k_pfinish"}
         roof = {"kernel": label.get(top, "k_" + top), "bound": "hbm", "achieved": round(ach, 1),
                 "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
                 "frac": round(ach / peaks.get("hbm_gbs"), 4),
@@ -762,7 +775,7 @@ def run_ours(args):
                 "peak_kind": peak_kind, "algorithmic_bytes_per_launch": int(b),
                 "per_launch_ms": round(per_launch_ms, 4), "launches_per_step": top_n / 2,
                 "launch": "one RK stage's stress-point and node launches together"
-                if top in label else "one launch",
+                if top in ("derivs", "interp") else "one launch",
                 "share_of_step": round(top_ms / sum(v[0] for v in prof.values()), 3)}
     alg_bytes = {k: int(v) for k in prof for v in [kernel_bytes(k, prob, deg, fast)]
                  if v is not None}
