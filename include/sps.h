@@ -217,8 +217,11 @@ int sps_selftest_cone(sps_ctx* ctx, int64_t n, uint64_t seed, int64_t* mismatche
    kernels, XSPH) at block sizes 64, 128, 256 and 512 over nsteps profiled steps of the
    uploaded state, keep the fastest size per kernel, and restore the state, so the results
    of later steps are the same as without tuning.  blocks (may be NULL) receives the 8
-   chosen sizes in that order.  The FP32 form then tunes its neighbour sums' look-ahead
-   the same way (sps_tuned_lookahead), then their L2 prefetch (sps_tuned_prefetch).  The cell size is not tuned: the reference's pair
+   chosen sizes in that order; where a stage is one launch (every option but the continuity
+   equation, artificial stress and the traction-free BC) the derivative sums' size is the
+   stage's, and the sizes of kernels that do not run keep their defaults.  The FP32 form
+   then tunes its neighbour sums' look-ahead the same way (sps_tuned_lookahead), then their
+   L2 prefetch (sps_tuned_prefetch).  The cell size is not tuned: the reference's pair
    order depends on it. */
 int sps_autotune(sps_ctx* ctx, int32_t nsteps, int32_t* blocks);
 
@@ -232,7 +235,7 @@ int sps_tuned_lookahead(sps_ctx* ctx, int32_t* ahead);
 /* Whether the FP32 form's neighbour sums request their list entries into L2 ahead of use
    (no reference counterpart): *flags bit 0 for the interpolation, bit 1 for the
    derivative sums.  One lane of each warp issues a bulk L2 prefetch of the warp's entries;
-   a hint that changes no result.  sps_autotune times both settings after the look-ahead
+   a hint that changes no result (and that the one-launch stages do not take).  sps_autotune times both settings after the look-ahead
    and keeps the faster per group; the default before tuning is 0 (off). */
 int sps_tuned_prefetch(sps_ctx* ctx, int32_t* flags);
 

@@ -980,7 +980,7 @@ __device__ __forceinline__ void store_pair(int4* dst, int4 a, int4 b) {
 // negated exactly (double-float additions and the cell shift are sign-symmetric), so W is
 // the same bits as the creator's evaluation and the gradient its exact negation.  Every
 // target also counts the partners after it, which is its half-list length (half_cnt), for
-// the pair count bookkeeping; dummies and inactive positions are counted by k_fgather_rest.
+// the pair count bookkeeping; dummies and inactive positions are counted by gather_rest.
 
 // the list entry of partner bs (cell offset qx, qy) of a target of type ta with FP32
 // cell-relative offsets (xa, xal), (ya, yal) and smoothing length ha: {partner id, W (sign

@@ -1,6 +1,9 @@
-// plain_step.cu -- FP64 "plain" step of the SPS hot path (compiled with -fmad=false).
+// plain_step.cu -- FP64 "plain" step of the SPS hot path (compiled with -fmad=false), and the
+// launch sequence of both forms' steps.
 //
-// One launch sequence per step restates time_integration
+// Where the densities are constant within a step and nothing couples the two halves of a stage
+// (Ctx::fused) a stage is one launch: plain_fused.cu, fast_fused.cu.  Otherwise one launch
+// sequence per step restates time_integration
 // (example_problems/soil_failure_bui_et_al_2008/2_SPH_main_2018.f90:78-184) and RK4
 // (:653-802).  The reference scatters every pair into both of its particles while it walks
 // the pair linked list; here every target gathers its own terms from its neighbour list,
