@@ -40,7 +40,7 @@ namespace {
 __device__ __forceinline__ void ret(const Real& M, double& a, double& b, double& c, double& d) {
   if (M.ncrit != 12) return;
   if (inside_cone_f32(M.alpha2f, M.kcf, a, b, c, d)) return;
-  adapt_stress(M.alpha2, M.kc, a, b, c, d);
+  adapt_stress(M.alpha2, M.kc, M.kc_shift, a, b, c, d);
 }
 
 // a / b with y = RN(1/b): the corrected product for a numerator of ordinary exponent (the

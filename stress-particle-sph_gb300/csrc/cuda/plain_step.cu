@@ -40,7 +40,7 @@ __device__ __forceinline__ void stress_return(const Dev& D, const Real& M, doubl
                                               double& b, double& c, double& d) {
   if (inside_cone_f32(M.alpha2f, M.kcf, a, b, c, d)) return;
   if (D.fast) adapt_stress_fast(M.alpha2, M.kc, M.kc_shift, a, b, c, d);
-  else adapt_stress(M.alpha2, M.kc, a, b, c, d);
+  else adapt_stress(M.alpha2, M.kc, M.kc_shift, a, b, c, d);
 }
 
 // FP32-form neighbour records of particle i (velocity, volume, stress, internal variable)
@@ -884,7 +884,7 @@ __global__ void k_selftest_cone(int64_t n, uint64_t seed, unsigned long long* ba
       nc++;
       // both returns must leave a certified stress exactly as it is
       double p0 = a, p1 = b, p2 = c, p3 = d, f0 = a, f1 = b, f2 = c, f3 = d;
-      adapt_stress(alpha2, kc, p0, p1, p2, p3);
+      adapt_stress(alpha2, kc, alpha2 > 0.0 ? kc / (3.0 * alpha2) : 0.0, p0, p1, p2, p3);
       adapt_stress_fast(alpha2, kc, alpha2 > 0.0 ? kc / (3.0 * alpha2) : 0.0, f0, f1, f2, f3);
       auto same = [](double x, double y) { return __double_as_longlong(x) == __double_as_longlong(y); };
       if (!(same(p0, a) && same(p1, b) && same(p2, c) && same(p3, d) && same(f0, a) &&

@@ -176,6 +176,11 @@ __device__ __forceinline__ void tail_sp_grad(const Dev& D, int t, double* g, con
     gu[3] = g[3];
 }
 
+// Get_derivative_intvars: the plastic strain rate's norm
+static __device__ __noinline__ double plastic_rate(double v0, double v1, double v2, double v3) {
+  return sqrt(third_of(2.0 * ((v0 * v0 + v1 * v1) + v3 * v3) + v2 * v2));
+}
+
 // stress-point rates of the plain form from the gradient g and the stage stress st: D : grad(v),
 // plastic_terms / drucker_prager (updates f_drucker), Jaumann spin; rhs(4) and the plastic
 // strain rate
@@ -205,9 +210,10 @@ __device__ __forceinline__ void sp_rates_f64(const Dev& D, const Real& M, const 
       if (D.cap_buf && (G2[0] != 0.0 || G2[1] != 0.0 || G2[2] != 0.0 || G2[3] != 0.0))
         capture_tuple(D, t, s2v, g, Gs);
     }
-    der = sqrt((2.0 * ((vivel[0] * vivel[0] + vivel[1] * vivel[1]) + vivel[3] * vivel[3]) +
-                vivel[2] * vivel[2]) /
-               3.0);
+    // zero for the points that do not flow, whose FP64 square root is left out
+    if ((__double_as_longlong(vivel[0]) | __double_as_longlong(vivel[1]) |
+         __double_as_longlong(vivel[2]) | __double_as_longlong(vivel[3])) << 1)
+      der = plastic_rate(vivel[0], vivel[1], vivel[2], vivel[3]);
   }
   double spin[4] = {0.0, 0.0, 0.0, 0.0};
   if (D.update_x) {
