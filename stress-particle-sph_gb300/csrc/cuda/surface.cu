@@ -5,7 +5,8 @@
 // FP32 accumulation with an FP64 operand is evaluated in FP64 and rounded once.  Steps 1 and
 // 4 accumulate over node--stress-point and same-type pairs in the order of the reference's
 // linked list: a particle merges its two neighbour lists by their walk-order keys (written
-// by k_lists), which restores that order.  Step 3 (is a neighbour inside the particle's scan
+// by k_lists, or the partner's sorted position where the lists were gathered directly), which
+// restores that order.  Step 3 (is a neighbour inside the particle's scan
 // region?) does not depend on the order.
 //   k_fs_normal0  steps 1-2 (:1180-1253): renormalisation matrix, kernel-gradient sums,
 //                 first normal
