@@ -1044,8 +1044,7 @@ __device__ __forceinline__ bool gather_accept(const Dev& D, int a, float xa, flo
 // kernel values, so that a warp's lanes evaluate together.  Dynamic shared memory:
 // capC ints per thread, entry k of thread j at k * blockDim + j.
 template <bool PLAIN>
-__device__ __forceinline__ void gather_target(const Dev& D, int s, int col,
-                                              unsigned short* buf) {
+__device__ __forceinline__ void gather_target(const Dev& D, int s, int col, int* buf) {
   const int bd = blockDim.x, tid = threadIdx.x;
   int nC = 0, nS = 0, nHalf = 0;
   if (s < D.gtot->nactive) {
@@ -1073,7 +1072,6 @@ __device__ __forceinline__ void gather_target(const Dev& D, int s, int col,
     }
     // the stencil row by row: a row's three cells are one contiguous run of sorted
     // positions; a candidate's cell follows from the run's cell boundaries
-#pragma unroll 1
     for (int qy = -1; qy <= 1; qy++) {
       const int jy = iy + qy;
       if (jy < 0 || jy >= ny) continue;
@@ -1110,8 +1108,7 @@ __device__ __forceinline__ void gather_target(const Dev& D, int s, int col,
         if (same) {
           nS++;
         } else {
-          if (nC < D.capC) buf[(size_t)nC * bd + tid] =
-                             (unsigned short)(min(bs - lo, 4095) | code << 12);
+          if (nC < D.capC) buf[(size_t)nC * bd + tid] = bs | (code << kHalfTypeShift);
           nC++;
         }
       }
@@ -1130,12 +1127,10 @@ __device__ __forceinline__ void gather_target(const Dev& D, int s, int col,
     // phase 2: the entries, stored in pairs (whole 32-byte sectors)
     int4 pend = make_int4(0, 0, 0, 0);
     for (int k = 0; k < nC; k++) {
-      const unsigned v = buf[(size_t)k * bd + tid];
-      const int code = (int)(v >> 12);
-      const int bs = D.cell_start[g.cell0 + (iy + code / 3 - 1) * nx + (ix > 0 ? ix - 1 : 0)] +
-                     (int)(v & 4095u);
-      const int4 e = gather_entry<PLAIN>(D, g, a, ta, xa, ya, ha, xal, yal,
-                                         bs, code % 3 - 1, code / 3 - 1, false);
+      const unsigned v = (unsigned)buf[(size_t)k * bd + tid];
+      const int code = (int)(v >> kHalfTypeShift);
+      const int4 e = gather_entry<PLAIN>(D, g, a, ta, xa, ya, ha, xal, yal, (int)(v & kHalfIdMask),
+                                         code % 3 - 1, code / 3 - 1, false);
       if (k & 1) store_pair(D.cross + ell(k - 1, col, D.N2), pend, e);
       else pend = e;
       // the lanes of a warp write entry k of adjacent columns together: whole sectors
@@ -1300,15 +1295,15 @@ __device__ __forceinline__ void gather_rest(const Dev& D, int a) {
 
 // the stress-point targets [0, bs blocks), the node targets [bs, bn), the dummies: one launch
 template <bool PLAIN>
-__global__ void __launch_bounds__(256, PLAIN ? 4 : 5) k_fgather(Dev D, int bs, int bn) {
-  extern __shared__ unsigned short gbuf16[];
+__global__ void __launch_bounds__(512, 2) k_fgather(Dev D, int bs, int bn) {
+  extern __shared__ int gbuf[];
   const int ns = D.NT - D.NN, b = blockIdx.x;
   if (b < bs) {
     const int k = b * blockDim.x + threadIdx.x;
-    if (k < ns) gather_target<PLAIN>(D, D.tgtS[k], k, gbuf16);
+    if (k < ns) gather_target<PLAIN>(D, D.tgtS[k], k, gbuf);
   } else if (b < bn) {
     const int k = (b - bs) * blockDim.x + threadIdx.x;
-    if (k < D.NN) gather_target<PLAIN>(D, D.tgtN[k], ns + k, gbuf16);
+    if (k < D.NN) gather_target<PLAIN>(D, D.tgtN[k], ns + k, gbuf);
   } else {
     const int k = (b - bn) * blockDim.x + threadIdx.x;
     if (D.NT + k < D.N2) gather_rest(D, D.NT + k);
@@ -1649,8 +1644,7 @@ void launch_gather(Ctx& c, bool same, Dev D) {
   const size_t per_target = sizeof(int) * (size_t)(D.capC + (same ? D.capS : 0));
   const int G = D.NT <= 16000 ? 8 : (D.NT <= 100000 ? 4 : (same || D.NT <= 400000 ? 2 : 1));
   if (G == 1) {
-    int b = std::min(c.blk[TK_HALF], 256);  // k_fgather's launch bounds
-    const size_t per_target = sizeof(short) * (size_t)D.capC;
+    int b = std::min(c.blk[TK_HALF], 512);  // k_fgather's launch bounds
     while (b > 32 && per_target * (size_t)b > 49152) b >>= 1;
     const int bs = (D.NT - D.NN + b - 1) / b, bn = bs + (D.NN + b - 1) / b;
     const int nb = bn + (D.N2 - D.NT + b - 1) / b;
