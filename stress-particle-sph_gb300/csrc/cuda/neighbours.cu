@@ -1638,9 +1638,7 @@ void launch_lists(Ctx& c, bool keys, bool same = false) {
 // 762; with same-kind lists, 2 million, plain, 2082 / 1792 / 1728 / 2551: one lane's buffers
 // leave too few warps a multiprocessor, so that form is not built).  Dynamic shared memory: the
 // list capacity for each target of a block, blocks halved until it is within 48 KB.
-void launch_gather(Ctx& c, bool same, Dev D) {
-  // the one-launch stages' preparation writes the compact entries itself, weighted
-  if (c.fused()) D.use_crossW = 0;
+void launch_gather(Ctx& c, bool same, const Dev& D) {
   const size_t per_target = sizeof(int) * (size_t)(D.capC + (same ? D.capS : 0));
   const int G = D.NT <= 16000 ? 8 : (D.NT <= 100000 ? 4 : (same || D.NT <= 400000 ? 2 : 1));
   if (G == 1) {

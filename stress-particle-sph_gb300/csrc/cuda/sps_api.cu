@@ -1092,13 +1092,14 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
       if (q.uploaded && !((double)D.scale_k * q.hmin_nd > 0.76 * q.p.dx)) bfl = 0;
     if (bfl != D.bound_from_lists) drop_graphs(c);
     D.bound_from_lists = bfl;
-    // the FP32 form's interpolation reads the compact {id, W} entries that the gathered
-    // lists also write
     const int wo = c.lists_direct() && c.walks() ? 1 : 0;
     if (wo != D.walk_order) drop_graphs(c);
     D.walk_order = wo;
     D.same_f32 = D.fast && !D.same_entries && !c.surf_every;
-    const int uw = c.lists_direct() && D.crossW ? 1 : 0;
+    // the separate kernels read the compact {id, W} entries that the gathered lists also
+    // write; the one-launch stages' preparation writes them itself, weighted, so that what
+    // runs before it (the re-interpolation of the outside approach) reads the full entries
+    const int uw = c.lists_direct() && D.crossW && !c.fused() ? 1 : 0;
     if (uw != D.use_crossW) drop_graphs(c);
     D.use_crossW = uw;
   } catch (const std::exception& e) {
