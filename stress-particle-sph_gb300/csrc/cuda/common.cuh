@@ -1039,7 +1039,9 @@ int launch_pair_build(Ctx& c);
 int launch_plain_step(Ctx& c);
 int launch_fast_step(Ctx& c);
 void launch_vol(Ctx& c, int lo, int hi);
-void launch_pprep(Ctx& c);  // (both preparations put the lists in walk order)
+void launch_walk_order(Ctx& c);
+// both preparations put the lists in walk order, unless the re-interpolation needed it before
+void launch_pprep(Ctx& c);
 void launch_pstage(Ctx& c, int stage);
 void launch_pfinish(Ctx& c);
 void launch_fprep(Ctx& c);

@@ -102,6 +102,8 @@ struct Ctx {
     return !(d.sle == 2 && d.cont_density) && (!walks() || fused()) &&
            2 * d.capC * 32 * 4 <= 49152;
   }
+  // whether this step begins with the outside approach's re-interpolation
+  bool reinterpolates() const { return (step_variant & 1) != 0; }
   // whether this step writes the same-kind lists
   bool same_now() const { return d.same_entries || surf_every || (step_variant & 4); }
   // one launch per RK4 stage: the positions, lists and densities do not change within a step

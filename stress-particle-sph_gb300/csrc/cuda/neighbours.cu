@@ -1705,12 +1705,19 @@ int launch_pair_build(Ctx& c) {
   return 0;
 }
 
-// both lists of every target from creation order to walk order (a rebuild after the step; in
-// the step the fused stages' preparation does it)
+// both lists of every target from creation order to walk order: in a step that re-interpolates
+// before the one-launch stages' preparation, which does it otherwise, and after a rebuild.  Once
+// for each gather: it reverses the new pairs of a list.
 __global__ void k_walk_order(Dev D) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < D.NT) put_target_walk_order(D, k, D.colid[k], k >= D.NT - D.NN);
 }
+static void walk_order(Ctx& c, Dev D, bool same) {
+  D.same_entries = same;
+  const int b = Ctx::block_for(D.NT, kBlock);
+  k_walk_order<<<(D.NT + b - 1) / b, b, 0, c.stream>>>(D);
+}
+void launch_walk_order(Ctx& c) { walk_order(c, c.d, c.same_now()); }
 
 // The device view of the last pair build for a rebuild after the step: the FP64 positions
 // the build's exact band test read (x0x, x0y hold them from the step's start, before
@@ -1744,10 +1751,9 @@ void launch_lists_keys(Ctx& c) {
 // the lists of the last step again with the same-kind entries (the FP32 detection)
 void launch_lists_same(Ctx& c) {
   if (c.lists_direct()) {
-    Dev D = build_view(c);
+    const Dev D = build_view(c);
     launch_gather(c, true, D);
-    D.same_entries = 1;
-    if (D.walk_order) k_walk_order<<<(D.NT + kBlock - 1) / kBlock, kBlock, 0, c.stream>>>(D);
+    if (D.walk_order) walk_order(c, D, true);
   } else {
     launch_lists(c, false, true);
   }

@@ -825,6 +825,7 @@ __global__ void __launch_bounds__(128) k_pfinish(Dev D) {
 
 void launch_pprep(Ctx& c) {
   Dev D = c.d;
+  if (c.reinterpolates()) D.walk_order = 0;  // done
   D.same_entries = c.same_now();  // the lists to put in walk order
   const bool group = D.NT <= c.group_max;
   const int n = group ? 8 * D.NT : D.NT, b = c.block_for(n, 128), nb = (n + b - 1) / b;

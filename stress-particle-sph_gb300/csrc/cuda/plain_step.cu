@@ -1000,9 +1000,13 @@ int launch_plain_step(Ctx& c) {
   cudaStream_t st = c.stream;
   int nbN = (D.NN + kBlock - 1) / kBlock;
   launch_pair_build(c);
-  if (c.step_variant & 1) {
+  if (c.reinterpolates()) {
     // the outside approach re-interpolates after a shift: stress_point_update and
     // adapt_stress2 (2_SPH_main_2018.f90:99-108)
+    if (D.walk_order) {
+      c.mark("walk_order");
+      launch_walk_order(c);
+    }
     c.mark("interp");
     if (D.fast) launch_finterp(c);
     else launch_pinterp(c);

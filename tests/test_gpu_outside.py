@@ -60,3 +60,32 @@ def test_reinterpolation_with_moving_particles_fp32(built_gpu):
                     ("intvars1", a["intvars1"][:nt], b["intvars1"][:nt])):
         assert np.abs(u - w).max() <= 1e-5 * np.abs(w).max(), (k, np.abs(u - w).max())
     gpu.close()
+
+
+def test_reinterpolation_in_a_step_that_grows_the_list(built_gpu):
+    # Plain form, bit for bit.  The stress-points start 1.5 times as far apart as their nodes;
+    # the shift at the end of step 2 puts them at their nodes, so the re-interpolating step 3
+    # meets 8% more pairs than any step before and takes the new ones first.  The nodes' large
+    # velocities, antisymmetric about the diagonal, cancel in the sums of the stress-points on
+    # it: what is left shows the order.  One of those lies at the origin, so that its position
+    # shows the last bits of its velocity.
+    dx = 0.05
+    p = cases.bui_like(width=0.5, height=0.5, dx=dx, outside=OUTSIDE, npoints=1, dt=1e-13,
+                       coh=1e9, alpha=0.0, beta=0.0, xsph=False)
+    s, nn = p.state(), p.nnode
+    x, v = s["x"].reshape(-1, 2), s["vel"].reshape(-1, 2)
+    i, j = np.rint((x[:nn] - x[:nn].min(axis=0)) / dx).T
+    x -= x[np.flatnonzero((i == 8) & (j == 8))[0]] + dx / 3
+    x[nn:2 * nn] = 1.5 * (x[:nn] - x[:nn].mean(axis=0)) + x[:nn].mean(axis=0)
+    v[:nn] = np.random.default_rng(5).uniform(0.5e-3, 1.5e-3, (nn, 2))
+    v[:nn] += 1e8 * np.sign(i - j)[:, None] * [1.0, -1.0]
+    v[nn:2 * nn] = v[:nn]
+    gpu, ref = pair(p, s, _abi.SPS_PREC_FP64_PLAIN)
+    n = []
+    for _ in range(3):
+        gpu.step(1, 0.0)
+        ref.step(1, 0.0)
+        n.append(len(ref.dump_pairs()["pair_i"]))
+    assert n[2] > 1.05 * max(n[:2])
+    cases.assert_bitwise(gpu.download(), ref.download(), p.ntotal)
+    gpu.close()
