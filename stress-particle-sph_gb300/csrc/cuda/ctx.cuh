@@ -102,6 +102,11 @@ struct Ctx {
     return !(d.sle == 2 && d.cont_density) && (!walks() || fused()) &&
            2 * d.capC * 32 * 4 <= 49152;
   }
+  // whether the FP32 detection is all that reads the gathered same-kind entries (Dev::same_f32);
+  // the exact one reads them where they are in walk order, and keyed lists of its own elsewhere
+  bool same_for_f32() const {
+    return d.fast && !d.same_entries && !surf_every && !(surface_exact && d.walk_order);
+  }
   // whether this step begins with the outside approach's re-interpolation
   bool reinterpolates() const { return (step_variant & 1) != 0; }
   // whether this step writes the same-kind lists

@@ -1095,7 +1095,7 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
     const int wo = c.lists_direct() && c.walks() ? 1 : 0;
     if (wo != D.walk_order) drop_graphs(c);
     D.walk_order = wo;
-    D.same_f32 = D.fast && !D.same_entries && !c.surf_every;
+    D.same_f32 = c.same_for_f32();
     // the separate kernels read the compact {id, W} entries that the gathered lists also
     // write; the one-launch stages' preparation writes them itself, weighted, so that what
     // runs before it (the re-interpolation of the outside approach) reads the full entries
@@ -1560,6 +1560,7 @@ int sps_set_surface_detection(sps_ctx* h, int32_t exact) {
     c.surface_exact = exact != 0;
     // the step graphs that write the lists for a download differ between the two
     c.keys_written = c.same_written = false;
+    c.d.same_f32 = c.same_for_f32();
     drop_graphs(c);
   } catch (const std::exception& e) {
     return fail(&c, SPS_ERR_CUDA, e.what());
