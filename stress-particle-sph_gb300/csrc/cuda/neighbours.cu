@@ -718,12 +718,12 @@ __device__ __forceinline__ bool rounds_to_hi(dfl v, float rel) {
 // polynomials lose at most a factor 8 to cancellation.  The FP64 evaluation's own error is below
 // 2^-49 (1 + 1 / t).  E = 2^-41 (1 + 1 / t), 2^-41 for q <= 1; the largest errors met in 2.4e7
 // random pairs (h 3e-4 .. 3, all directions) were 2^-43.1 (1 + 1 / t) and 2^-44.  q within
-// 2^-36 of 1 and t below 2^-9 stay undecided.
+// 2^-36 of 1 and t below 2^-9 stay undecided, and so does a separation component below 2^-74
+// that is not zero (below about 2^-106 its low part is subnormal and no longer exact to 2^-47).
 __device__ __forceinline__ bool cubic_certified(const Grid& g, double dxd, double dyd, float* w,
                                                 float* dw0, float* dw1) {
   dfl dx, dy;
-  f32_split(dxd, dx.hi, dx.lo);
-  f32_split(dyd, dy.hi, dy.lo);
+  if (!f32_split_int(dxd, dx.hi, dx.lo) || !f32_split_int(dyd, dy.hi, dy.lo)) return false;
   const dfl r2 = df_sumsq(dx, dy);
   if (!(r2.hi > 1e-25f && r2.hi < 1e25f)) return false;
   const dfl r = df_sqrt_rn(r2);
