@@ -45,7 +45,9 @@ constexpr int kBlock = 256;
 
 // n elements of device memory for the life of the context.  Small requests are cut from a
 // chunk (a context holds about ninety arrays, and an allocation call costs about 10 us); one
-// that would waste much of a chunk is an allocation of its own.
+// that would waste much of a chunk is an allocation of its own.  The first chunk is sized for a
+// context's creation; those opened when it is used up are small, since little follows.
+constexpr size_t kLaterChunk = 4 << 20;
 template <typename T>
 T* dalloc(sps::Ctx& c, size_t n) {
   const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~(size_t)255;
@@ -55,6 +57,7 @@ T* dalloc(sps::Ctx& c, size_t n) {
     c.allocs.push_back(p);
     c.arena = static_cast<char*>(p);
     c.arena_left = c.arena_chunk;
+    c.arena_chunk = std::min(c.arena_chunk, kLaterChunk);
   }
   if (bytes <= c.arena_left) {
     p = c.arena;
