@@ -224,7 +224,7 @@ struct Dev {
   GridTotal* gtot;
   unsigned long long* bbox;  // per realisation: ordered keys of minx, miny, -maxx, -maxy, -maxh, minh
   // pairs
-  int4* half;
+  int4* half;  // (fused: its place is the list constants' too)
   int32_t* half_cnt;
   int4* half_meta;    // per creator (sorted position): group starts 1-4 (16 bits each),
                       // pair count, id
@@ -238,7 +238,7 @@ struct Dev {
   int use_crossW;
   // per-target lists, entries in pairs: entries 2j and 2j+1 of list column c side by side
   // at (j * N2 + c) * 2 (ell()), one 32-byte sector; keys flat at k * N2 + c
-  int32_t *keyC, *keyS;  // per entry: 2 x (position in the reference's walk order) + (target is pair_i)
+  int32_t *keyC, *keyS;  // (Ctx::keyed_lists) per entry: 2 x (position in the reference's walk order) + (target is pair_i)
   int32_t *degC, *degS;  // by list column
   int l2_prefetch;  // FP32 form: bulk L2 prefetch of list entries (bit 0 interp, bit 1 derivs)
   // sorted positions of the stress-point and of the node targets (each in sorted order), so

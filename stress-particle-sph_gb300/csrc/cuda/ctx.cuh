@@ -102,6 +102,11 @@ struct Ctx {
     return !(d.sle == 2 && d.cont_density) && (!walks() || fused()) &&
            2 * d.capC * 32 * 4 <= 49152;
   }
+  // whether a detection reads the lists' walk-order keys
+  bool keyed_lists() const {
+    return !(lists_direct() && walks()) &&
+           (precision == SPS_PREC_FP64_PLAIN || surf_every || surface_exact);
+  }
   // whether the FP32 detection is all that reads the gathered same-kind entries (Dev::same_f32);
   // the exact one reads them where they are in walk order, and keyed lists of its own elsewhere
   bool same_for_f32() const {
@@ -135,9 +140,9 @@ struct Ctx {
   // 59,000 351 / 272, 87,000 458 / 325; biaxial sample of 40,000 418 / 385)
   int split_max = 36000;
   int surface_split_max = 60000;  // the same for the exact free-surface detection
-  // the last pair build left the half lists unwritten (k_fgather): sps_dump_pairs and the
-  // keyed lists of the exact detection build them first (set by enqueue_step for every
-  // step, since a replayed graph runs no host code)
+  // the last step left the half lists unwritten (k_fgather) or overwrote them with its list
+  // constants: sps_dump_pairs and the lists of a detection build them first (set by enqueue_step
+  // for every step, since a replayed graph runs no host code)
   bool half_stale = false;
   int step_variant = 0;    // the variant launch_*_step enqueues
   int64_t itimestep = 0;   // itimestep_sph of the last step (0 after an upload)

@@ -1701,7 +1701,7 @@ int launch_pair_build(Ctx& c) {
     c.mark("lists");
     launch_lists(c, c.surf_every || (want && !c.surface_f32()), want);
   }
-  c.half_stale = direct;
+  c.half_stale = direct || c.fused();
   return 0;
 }
 
@@ -1755,6 +1755,7 @@ void launch_lists_same(Ctx& c) {
     launch_gather(c, true, D);
     if (D.walk_order) walk_order(c, D, true);
   } else {
+    ensure_half_lists(c);
     launch_lists(c, false, true);
   }
 }

@@ -70,6 +70,15 @@ T* dalloc(sps::Ctx& c, size_t n) {
   return static_cast<T*>(p);
 }
 
+// the walk-order keys of the lists, for a context whose detection reads them
+void ensure_keys(sps::Ctx& c) {
+  sps::Dev& D = c.d;
+  if (!c.keyed_lists() || D.keyS || D.capH <= 0) return;
+  const size_t n = (size_t)D.N2 * (size_t)D.capH;
+  if (!D.keyC) D.keyC = dalloc<int32_t>(c, n);
+  D.keyS = dalloc<int32_t>(c, n);
+}
+
 // realisations whose packed fields are at most this long cross the bus as one copy through
 // pinned memory: eight copies into the caller's pageable arrays cost about 8 us each, the host
 // copy of 1 MB about 60
@@ -409,7 +418,7 @@ void enqueue_step(sps::Ctx& c) {
   c.keys_written = !c.d.walk_order && ((c.keys_in_step && !c.surface_f32() && !c.lists_direct()) || c.surf_every);
   c.same_written = c.keys_in_step || c.surf_every || c.d.same_entries;
   // set here, on the host, for every step: a replayed graph runs no host code
-  c.half_stale = c.lists_direct();
+  c.half_stale = c.lists_direct() || c.fused();
   if (c.use_graph && !c.profiling) {
     if (!c.graphs[c.step_variant]) build_graph(c);
     SPS_CUDA_CHECK(cudaGraphLaunch(c.graphs[c.step_variant], c.stream));
@@ -1068,23 +1077,30 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
       int capn = c.p.max_neighbours > 0 ? std::max(4, c.p.max_neighbours / 2) : std::max(48, est);
       capn = std::min(capn, 65535);  // half-list positions are kept in 16 bits
       if (capn > D.capH || (c.p.max_neighbours > 0 && capn != D.capH)) {
-        D.half = dalloc<int4>(c, (size_t)D.N2 * (size_t)capn);
+        // the one-launch stages' list constants take the place of the half lists, which are
+        // of no use once the lists are built (and rebuilt when they are wanted)
+        const size_t cap = (size_t)capn, ns = (size_t)(D.NT - D.NN);
+        const size_t first = D.fast ? 8 * D.NT * cap : ns * cap * 16;
+        const size_t second = D.fast ? 8 * ns * cap : 8 * D.NT * cap;
+        const size_t consts = c.fused() ? first + second : 0;
+        char* half = dalloc<char>(c, std::max(sizeof(int4) * (size_t)D.N2 * cap, consts));
+        D.half = reinterpret_cast<int4*>(half);
+        if (c.fused() && D.fast) {
+          D.hGf = reinterpret_cast<float2*>(half);
+          D.hB = reinterpret_cast<double*>(half + first);
+        } else if (c.fused()) {
+          D.hG = reinterpret_cast<double2*>(half);
+          D.hW = reinterpret_cast<double*>(half + first);
+        }
         // the lists hold their entries in pairs (ell()): an even number of rows
         const size_t rows = (size_t)capn + (capn & 1);
         D.cross = dalloc<int4>(c, (size_t)D.N2 * rows);
         D.same = dalloc<int4>(c, (size_t)D.N2 * rows);
         D.crossW = c.precision == SPS_PREC_FP32_FAST ? dalloc<int2>(c, (size_t)D.N2 * rows)
                                                      : nullptr;
-        if (c.fused() && D.fast) {
-          D.hGf = dalloc<float2>(c, (size_t)D.NT * (size_t)capn);
-          D.hB = dalloc<double>(c, (size_t)(D.NT - D.NN) * (size_t)capn);
-        } else if (c.fused()) {
-          D.hW = dalloc<double>(c, (size_t)D.NT * (size_t)capn);
-          D.hG = dalloc<double2>(c, (size_t)(D.NT - D.NN) * (size_t)capn);
-        }
-        D.keyC = dalloc<int32_t>(c, (size_t)D.N2 * (size_t)capn);
-        D.keyS = dalloc<int32_t>(c, (size_t)D.N2 * (size_t)capn);
+        D.keyC = D.keyS = nullptr;
         D.capH = D.capC = D.capS = capn;
+        ensure_keys(c);
         drop_graphs(c);
       }
     }
@@ -1561,6 +1577,12 @@ int sps_set_surface_detection(sps_ctx* h, int32_t exact) {
   try {
     SPS_CUDA_CHECK(cudaStreamSynchronize(c.stream));
     c.surface_exact = exact != 0;
+    try {
+      ensure_keys(c);
+    } catch (...) {  // out of memory: the detection stays as it was
+      c.surface_exact = !c.surface_exact;
+      throw;
+    }
     // the step graphs that write the lists for a download differ between the two
     c.keys_written = c.same_written = false;
     c.d.same_f32 = c.same_for_f32();
