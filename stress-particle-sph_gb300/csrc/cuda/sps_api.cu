@@ -1048,9 +1048,17 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
     hr.hmin_nd = hmin_nd;
     hr.uploaded = true;
     double nc = 0.0;
-    for (const sps::HostReal& q : c.hr) nc += q.ncells_est;
+    int known = 0;
+    for (const sps::HostReal& q : c.hr) {
+      nc += q.ncells_est;
+      known += q.uploaded;
+    }
     int cap = (int)std::min(4.0 * nc + 1024.0, 2.0e9 / 4.0);
     if (cap > D.cell_cap) {
+      // a batch's uploads come one after the other: room for those to come, as large as the ones
+      // known, but no more than twice what there was
+      const double all = std::min(4.0 * nc * D.R / known + 1024.0, 2.0e9 / 4.0);
+      cap = std::max(cap, (int)std::min(all, 2.0 * D.cell_cap));
       D.cell_cnt = dalloc<int32_t>(c, (size_t)cap + 2);
       D.cell_start = dalloc<int32_t>(c, (size_t)cap + 2);
       D.cntD = dalloc<int32_t>(c, (size_t)cap + 2);

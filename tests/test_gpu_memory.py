@@ -87,3 +87,21 @@ def test_pairs_and_detection_after_steps(built_gpu, max_neighbours):
         np.testing.assert_array_equal(na.view(np.int64), nb.view(np.int64))
     for c in (gpu, fast):
         c.close()
+
+
+def test_a_batch_takes_its_cells_once(built_gpu):
+    # 64 uploads one after the other: the cells' arrays (40 bytes a cell, four times the cells of
+    # the uploaded realisations) grow by doubling, so what they left behind is no more than what
+    # they are
+    torch = pytest.importorskip("torch")
+    probs = [sps_gb300.Problem.column(dx=0.004 + 1e-5 * i) for i in range(64)]
+    torch.zeros(1, device="cuda")
+    b = sps_gb300.Batch(probs, precision=_abi.SPS_PREC_FP32_FAST)
+    torch.cuda.synchronize()
+    a = torch.cuda.mem_get_info()[0]
+    b.upload_all()
+    torch.cuda.synchronize()
+    took = a - torch.cuda.mem_get_info()[0]
+    n = sum(len(p.mass) for p in probs)
+    b.close()
+    assert took <= n * 64 * SLOTS + (32 << 20), took / n
