@@ -697,6 +697,7 @@ int sps_create_batch(int32_t nreal, const sps_params* ps, sps_ctx** out) {
     D.xsph = p->xsph;
     D.update_x = p->update_x;
     D.cont_density = p->cont_density;
+    D.art_stress = p->art_stress ? 1 : 0;
     D.sle = p->sle;
     D.sp_sph = p->sp_sph;
     D.inside = p->inside_approach;
@@ -711,7 +712,8 @@ int sps_create_batch(int32_t nreal, const sps_params* ps, sps_ctx** out) {
     D.pi = p->pi;
     for (int b = 0; b < p->no_bcs; b++) D.bcvar[b] = (int)p->bc_list[8 * (size_t)b + 1];
     const size_t N2 = D.N2, NT = D.NT, NN_ = D.NN;
-    c.arena_chunk = N2 * 1200 + (size_t)nreal * 1024 + (1 << 16);  // about what follows
+    // what follows: 700 to 830 bytes a particle
+    c.arena_chunk = N2 * 820 + (size_t)nreal * 1024 + (1 << 16);
     {
       sps::Real* rd = dalloc<sps::Real>(c, nreal);
       SPS_CUDA_CHECK(cudaMemcpyAsync(rd, c.real.data(), sizeof(sps::Real) * nreal,
@@ -768,24 +770,24 @@ int sps_create_batch(int32_t nreal, const sps_params* ps, sps_ctx** out) {
     D.x0y = dalloc<double>(c, N2);
     D.vx0 = dalloc<double>(c, NT);
     D.vy0 = dalloc<double>(c, NT);
-    for (int k = 0; k < 4; k++) {
-      D.st0[k] = dalloc<double>(c, NT);
-      D.RKs[k] = dalloc<double>(c, NT);
-      D.RHS1[k] = dalloc<double>(c, NT);
-    }
-    for (int k = 0; k < 2; k++) {
-      D.RKv[k] = dalloc<double>(c, NT);
-      D.RHS2[k] = dalloc<double>(c, NT);
-    }
-    D.rho0 = dalloc<double>(c, NT);
-    D.hsml0 = dalloc<double>(c, NT);
-    D.RKr = dalloc<double>(c, NT);
-    D.RKh = dalloc<double>(c, NT);
+    for (int k = 0; k < 2; k++) D.RKv[k] = dalloc<double>(c, NT);
     D.RKd = dalloc<double>(c, NT);
-    D.RHSr = dalloc<double>(c, NT);
-    D.RHSh = dalloc<double>(c, NT);
+    if (!c.fused()) {  // the separate kernels' state between their launches
+      for (int k = 0; k < 4; k++) {
+        D.st0[k] = dalloc<double>(c, NT);
+        D.RKs[k] = dalloc<double>(c, NT);
+        D.RHS1[k] = dalloc<double>(c, NT);
+      }
+      for (int k = 0; k < 2; k++) D.RHS2[k] = dalloc<double>(c, NT);
+      for (int k = 0; k < 3; k++) D.A[k] = dalloc<double>(c, NT);
+      D.rho0 = dalloc<double>(c, NT);
+      D.hsml0 = dalloc<double>(c, NT);
+      D.RKr = dalloc<double>(c, NT);
+      D.RKh = dalloc<double>(c, NT);
+      D.RHSr = dalloc<double>(c, NT);
+      D.RHSh = dalloc<double>(c, NT);
+    }
     D.fbx = dalloc<double>(c, NN_);
-    D.art_stress = p->art_stress ? 1 : 0;
     // the same-kind lists (node-node, stress-point-stress-point) are read within a step only
     // by XSPH, artificial viscosity and artificial stress; the free-surface detection
     // builds its own lists with walk-order keys, which always carry them
@@ -806,7 +808,6 @@ int sps_create_batch(int32_t nreal, const sps_params* ps, sps_ctx** out) {
     D.Ddev = dalloc<double>(c, NT);
     D.vol = dalloc<double>(c, N2);
     D.rinv = dalloc<double>(c, N2);
-    for (int k = 0; k < 3; k++) D.A[k] = dalloc<double>(c, NT);
     D.fast = (p->precision == SPS_PREC_FP32_FAST) ? 1 : 0;
     D.l2_prefetch = 0;  // off until the autotuner finds it faster
     // stress-point and node targets in sorted order (both forms)

@@ -105,3 +105,12 @@ def test_a_batch_takes_its_cells_once(built_gpu):
     n = sum(len(p.mass) for p in probs)
     b.close()
     assert took <= n * 64 * SLOTS + (32 << 20), took / n
+
+
+@pytest.mark.parametrize("precision", [_abi.SPS_PREC_FP64_PLAIN, _abi.SPS_PREC_FP32_FAST],
+                         ids=["plain", "fp32"])
+def test_a_context_has_one_form_of_stages(built_gpu, precision):
+    # its arrays come to 700 bytes a particle (plain) and 760 (FP32) where a stage is one
+    # launch; the separate kernels' would be 184 more
+    create, _, n = used(precision)
+    assert create <= n * 850 + (32 << 20), create / n
