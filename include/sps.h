@@ -229,14 +229,17 @@ int sps_autotune(sps_ctx* ctx, int32_t nsteps, int32_t* blocks);
    block sizes (no reference counterpart): ahead[0] neighbours a pass in the interpolation
    (2, 4 or 8), ahead[1] in the node derivative sums (1, 2 or 4); a pass loads its
    neighbours' list entries and records before it sums any of them, in the same order, so
-   the results do not depend on these.  Defaults before tuning: 4 and 2. */
+   the results do not depend on these.  Defaults before tuning: 4 and 2.  A one-launch stage
+   (sps_autotune) is built for the pairs (2, 1), (2, 2), (4, 2) and (8, 4), which are the ones
+   that sps_autotune times; of another pair it takes the one with the same ahead[0], of (2, 4) (2, 2). */
 int sps_tuned_lookahead(sps_ctx* ctx, int32_t* ahead);
 
 /* Whether the FP32 form's neighbour sums request their list entries into L2 ahead of use
    (no reference counterpart): *flags bit 0 for the interpolation, bit 1 for the
    derivative sums.  One lane of each warp issues a bulk L2 prefetch of the warp's entries;
-   a hint that changes no result (and that the one-launch stages do not take).  sps_autotune times both settings after the look-ahead
-   and keeps the faster per group; the default before tuning is 0 (off). */
+   a hint that changes no result.  sps_autotune times both settings after the look-ahead and
+   keeps the faster per group; the default before tuning is 0 (off).  One-launch stages do
+   not take it, and where no other kernel does sps_autotune leaves the flags as they are. */
 int sps_tuned_prefetch(sps_ctx* ctx, int32_t* flags);
 
 /* Sets those flags directly (0 .. 3). */

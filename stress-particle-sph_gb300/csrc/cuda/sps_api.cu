@@ -1859,17 +1859,20 @@ int sps_autotune(sps_ctx* h, int32_t nsteps, int32_t* blocks) {
         copy(false);
         for (int g = 0; g < 2; g++)
           for (size_t q = 0; q < kn.size(); q++)
-            if ((kn[q] == names[g] || (c.fused() && kn[q] == "stage")) && kms[q] < best_la_ms[g]) {
+            if (kn[q] == (c.fused() ? "stage" : names[g]) && kms[q] < best_la_ms[g]) {
               best_la_ms[g] = kms[q];
               best_la[g] = v[g];
             }
       }
       c.ahead[0] = best_la[0];
       c.ahead[1] = best_la[1];
-      // then the bulk L2 prefetch of the list entries, off and on for both groups
+      // then the bulk L2 prefetch of the list entries, off and on for both groups, where a kernel
+      // takes it: one-launch stages do not, the re-interpolation of the outside approach does
       double best_pf_ms[2] = {1e300, 1e300};
-      int best_pf = 0;
+      const bool timed = !c.fused() || c.d.outside;
+      int best_pf = timed ? 0 : c.d.l2_prefetch;
       for (int pf : {0, 3}) {
+        if (!timed) break;
         c.d.l2_prefetch = pf;
         std::vector<std::string> kn;
         std::vector<double> kms;
