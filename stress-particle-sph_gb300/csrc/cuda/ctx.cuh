@@ -130,16 +130,22 @@ struct Ctx {
     return b;
   }
   // largest NT whose preparation takes eight lanes a target: every lane of a group repeats the
-  // sums, which pays while lanes are idle (us with one / eight lanes: plain slope of 29,000
-  // 52 / 41, of 40,000 64 / 51, of 80,000 86 / 91, biaxial sample of 40,000 with wall segments
-  // 58 / 110; FP32 slope of 40,000 31 / 23, of 180,000 49 / 74)
+  // sums and one of them does the rest, which pays while lanes are idle.  The rest is longer for
+  // material that flows (stress returned twice, flow rule), so the sizes at which both are equal
+  // lie apart, and the line between them (us with one / eight lanes: plain slopes of 29,000
+  // 49 / 30, 39,000 56 / 35, 59,000 58 / 42, 86,000 62 / 55; plain biaxial samples of 16,000
+  // 37 / 29, 28,000 41 / 42, 40,300 37 / 58, 63,000 49 / 78; FP32 slopes of 39,000 37 / 23, 59,000
+  // 38 / 29, 116,000 38 / 47; FP32 biaxial samples of 28,000 25 / 28, 40,300 18 / 37)
   int group_max = 40000;
   // largest NT whose plain stages split a target's sums over lanes: few warps and a long chain
   // each below it, the pipes busy with one lane a target above (us a step split / one lane:
-  // 600 particles 170 / 320, slopes of 17,000 135 / 244, 29,000 208 / 249, 40,000 257 / 249,
-  // 59,000 351 / 272, 87,000 458 / 325; biaxial sample of 40,000 418 / 385)
+  // 638 particles 120 / 257, slopes of 20,000 173 / 247, 29,000 197 / 249, 39,000 232 / 267,
+  // 59,000 318 / 273, 86,000 425 / 320; biaxial samples of 28,000 236 / 301, 40,300 338 / 343,
+  // 63,000 448 / 383).  The exact free-surface detection splits its sums up to the same size: it
+  // gains 52 us at 638 particles, 34 at 12,000, 20 at 29,000 and 14 to 30 at 28,000 of the biaxial
+  // sample, and loses 14 to 25 at 39,000, 7 to 37 at 40,300 of the biaxial sample, 70 to 106 at
+  // 59,000.
   int split_max = 36000;
-  int surface_split_max = 60000;  // the same for the exact free-surface detection
   // the last step left the half lists unwritten (k_fgather) or overwrote them with its list
   // constants: sps_dump_pairs and the lists of a detection build them first (set by enqueue_step
   // for every step, since a replayed graph runs no host code)

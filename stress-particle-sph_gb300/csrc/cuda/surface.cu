@@ -466,7 +466,7 @@ void launch_surface(Ctx& c) {
   const int b = Ctx::block_for(D.N2, kBlock), nb = (D.N2 + b - 1) / b;
   const bool direct = D.walk_order;  // lists gathered directly, in walk order
   c.mark("surface", 3);
-  if (D.NT <= c.surface_split_max) {
+  if (D.NT <= c.split_max) {
     const int b4 = Ctx::block_for(4 * (int64_t)D.N2, kBlock);
     const int n4 = (int)((4 * (int64_t)D.N2 + b4 - 1) / b4), n8 = (int)((8 * (int64_t)D.N2 + b4 - 1) / b4);
     if (direct) k_fs_normal0<true, 4><<<n4, b4, 0, c.stream>>>(D);
