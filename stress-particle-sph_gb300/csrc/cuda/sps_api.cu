@@ -1088,9 +1088,9 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
       if (capn > D.capH || (c.p.max_neighbours > 0 && capn != D.capH)) {
         // the one-launch stages' list constants take the place of the half lists, which are
         // of no use once the lists are built (and rebuilt when they are wanted)
-        const size_t cap = (size_t)capn, ns = (size_t)(D.NT - D.NN);
-        const size_t first = D.fast ? 8 * D.NT * cap : ns * cap * 16;
-        const size_t second = D.fast ? 8 * ns * cap : 8 * D.NT * cap;
+        const size_t cap = (size_t)capn, nt = (size_t)D.NT, ns = nt - (size_t)D.NN;
+        const size_t first = D.fast ? nt * cap * sizeof(float2) : ns * cap * sizeof(double2);
+        const size_t second = (D.fast ? ns : nt) * cap * sizeof(double);
         const size_t consts = c.fused() ? first + second : 0;
         char* half = dalloc<char>(c, std::max(sizeof(int4) * (size_t)D.N2 * cap, consts));
         D.half = reinterpret_cast<int4*>(half);
