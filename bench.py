@@ -595,8 +595,8 @@ def kernel_bytes(name, prob, deg, fast=False):
 
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) per launch of the FP32 form on
-# the full-size slope (dx 0.012 m), from one ncu pass over a step
-# (profiles/one_launch_stages.md); the stages' figure is the mean of the four launches.
+# the full-size slope (dx 0.012 m), from one ncu pass over a step; the stages' figure is the mean
+# of the four launches.
 # Valid for that workload and this code state only.
 NCU_TRAFFIC_FULL = {"stage": 825611328 + 224183168,
                     "gather": 210693888 + 540843520,

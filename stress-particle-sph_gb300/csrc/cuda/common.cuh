@@ -218,7 +218,7 @@ struct Dev {
   unsigned* tick;  // tickets of the kernels whose last block finishes the work
   float *xr, *yr, *hr;
   float *xrl, *yrl;  // FP32 form: low parts of the cell-relative offsets
-  float4* srec;       // by sorted position: (xr, yr, hr, 0) of the particle there
+  float4* srec;       // by sorted position: (xr, yr, hr, type) of the particle there
   float2* srecl;      // by sorted position, FP32 form: (xrl, yrl)
   Grid* grid;                // per realisation
   GridTotal* gtot;
@@ -336,7 +336,7 @@ __device__ __forceinline__ bool f64_ge(double a, double b) { return f64_key(a) >
 // remainder) from 32 x 32 -> 64 bit multiply-adds, rounded to nearest even by the definition of
 // IEEE 754, in about 40 integer instructions; the additions stay on the FP64 pipe, which then
 // works beside the integer ones (2 million particles, us a step: stages 7170 -> 4650, list
-// constants 1069 -> 476, last interpolation 581 -> 416, cells of the particles 106 -> 63;
+// constants 1069 -> 494, last interpolation 581 -> 396, cells of the particles 106 -> 64;
 // 115,000: stages 615 -> 362).  Operands or results outside the normal range (zeros,
 // subnormals, infinities, NaN) leave the line: inlined, the compiler may issue the FP64
 // instructions with their predicate off, which occupies the pipe as well.

@@ -540,7 +540,7 @@ __global__ void k_fxsph(Dev D) {
 
 }  // namespace
 
-// the targets split by kind (k_split_targets) after the pair build; one launch per kind
+// one launch per kind of target (tgtS, tgtN of the pair build)
 template <int KP>
 void launch_finterp_kp(Ctx& c) {
   const Dev& D = c.d;

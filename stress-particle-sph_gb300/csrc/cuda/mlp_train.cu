@@ -14,8 +14,11 @@
 //             into partial products
 //   k_update  the partial products summed in a fixed order, Adam, the next forward pass's
 //             rounded weights, the loss sums
-// Every sum is one FP32 multiply-add chain in ascending index, so training is deterministic
-// and does not depend on the tiling.
+// Training is deterministic: the sums of Z and dA are single FP32 multiply-add chains in
+// ascending index, whatever the tiling; a weight gradient is at most kSplit such chains over
+// consecutive rows, added in order; a loss is a tree over 256 rows at a time, added in order on the host.
+// An epoch's order (Fisher-Yates over all rows) is drawn on the host before an epoch's first
+// launch: 0.37 ms of the 1.54 that an epoch of 65,536 rows takes.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 

@@ -1035,8 +1035,8 @@ __device__ __forceinline__ bool gather_accept(const Dev& D, int a, float xa, flo
   return true;
 }
 
-// FP32 form: Task 3 of grid_find_NEW (2_SPH_main_2018.f90:1307-1403), kernel (:1440-1538)
-// and Pint_Update (3_SPH_material_2018.f90:1574-1634) per target, gathering its entries
+// Task 3 of grid_find_NEW (2_SPH_main_2018.f90:1307-1403), kernel (:1440-1538) and
+// Pint_Update (3_SPH_material_2018.f90:1574-1634) per target of either form, gathering its entries
 // from the 3 x 3 cell stencil directly in creation order.
 // No same-kind lists (gather_by_group writes them): degS holds 0 unless the outside approach
 // reads the counts.  Phase 1 tests the stencil's candidates and keeps the

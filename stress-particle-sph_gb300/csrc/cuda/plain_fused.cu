@@ -158,13 +158,13 @@ __device__ __forceinline__ bool node_entry(const Dev& D, const Real& M, int t, i
 }
 
 // Once per step, per target: the constants of its list entries (file comment), the boundary
-// force of a node, and the state of stage 0.  Bound by the FP64 pipe (22 operations a
-// stress-point entry, 8 a node's; the terms of the CSPM moments are compiled out without them,
-// since FP64 instructions that a predicate switches off still occupy it: 1292 -> 1069 us at 2
-// million particles).  L = 8, for problems that cannot fill the chip with one lane a
+// force of a node, and the state of stage 0.  Bound by the integer pipes, which form the
+// products and quotients, and by memory (494 us at 2 million particles, 1069 with FP64 products;
+// the terms of the CSPM moments are compiled out without them, since FP64 instructions that a
+// predicate switches off still occupy their pipe: 1292 -> 1069 then).  L = 8, for problems that cannot fill the chip with one lane a
 // target: eight lanes form eight entries' constants and terms together, and every one of them
 // adds the terms in list order (0.0 where an entry has none, which changes no sum: none of
-// them is ever -0.0); 58 -> 25 us at 600 particles, soil failure example 53 -> 18.
+// them is ever -0.0); 49 -> 18 us at 600 particles, soil failure example 53 -> 16.
 template <int L, bool CSPM>
 __global__ void __launch_bounds__(128) k_pprep(Dev D) {
   constexpr unsigned all = 0xffffffffu;
@@ -273,9 +273,9 @@ __global__ void __launch_bounds__(128) k_pprep(Dev D) {
   }
 }
 
-// entries a pass whose list words and neighbour records are loaded before any is summed: more
-// in flight where few warps are there to hide a latency, one where they are many (below)
-constexpr int kP = 4;
+// In the kernels below kP is the number of entries a pass whose list words and neighbour records
+// are loaded before any is summed: more in flight where few warps are there to hide a
+// latency, one where they are many.
 
 // A wall's velocity seen by a stress-point: v - (v (1 - beta) + beta 0).  Rare, and out of line:
 // as predicated instructions it would take the FP64 pipe for every entry.
@@ -690,7 +690,8 @@ __device__ __forceinline__ void node_stage(const Dev& D, int stage, int k, bool 
 // One lane a target: 64 registers, eight blocks a multiprocessor, one entry in flight a lane; the
 // FP64 pipe and the integer pipes work for different warps at the same time, so many of them are
 // needed (2 million particles, us a step: four entries and 124 registers 6253, two and 5485,
-// one and 80 registers 5037, one and 64 registers 4903, spills included).
+// one and 80 registers 5037, one and 64 registers 4903, spills included; 4234 since the stress
+// return and the flow rule repeat no FP64 work).
 template <int LS, int LN>
 __global__ void __launch_bounds__(128, LS == 1 ? 8 : 1) k_pstage(Dev D, int stage, int nbs) {
   const int ns = D.NT - D.NN;
@@ -711,7 +712,7 @@ __global__ void __launch_bounds__(128, LS == 1 ? 8 : 1) k_pstage(Dev D, int stag
 // update (:140-146, without XSPH) and the displacements (:166-180)
 // INT: the products on the integer pipes (large problems; below, where the chain of one warp's
 // latencies counts and not the FP64 pipe, the FP64 multiplication is shorter: 600 particles 24
-// us against 29; 2 million 581 against 430)
+// us against 29; 2 million 581 against 396)
 template <bool INT>
 __global__ void __launch_bounds__(128) k_pfinish(Dev D) {
   constexpr int kP = INT ? 2 : 4;
