@@ -486,10 +486,8 @@ __device__ __forceinline__ float i2f_rn(int r) {
 }
 
 // hi = (float)x, lo = (float)(x - (double)hi): the exact remainder x - hi is the dropped
-// significand bits (minus one float ulp when hi was rounded up), scaled by 2^(E-1075).
-// f32_split_int returns false, without a result, for |x| below 2^-74 but not zero and for
-// |x| of 2^128 and above, infinities and NaN.
-__device__ __forceinline__ bool f32_split_int(double x, float& hi, float& lo) {
+// significand bits (minus one float ulp when hi was rounded up), scaled by 2^(E-1075)
+__device__ __forceinline__ void f32_split(double x, float& hi, float& lo) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x);
   const unsigned h32 = (unsigned)(u >> 32), l32 = (unsigned)u;
   const int E = (int)((h32 >> 20) & 0x7FFu);
@@ -497,9 +495,12 @@ __device__ __forceinline__ bool f32_split_int(double x, float& hi, float& lo) {
     if ((u << 1) == 0ull) {  // +-0: hi keeps the sign, x - hi = +0
       hi = __uint_as_float(h32 & 0x80000000u);
       lo = 0.0f;
-      return true;
+      return;
     }
-    return false;
+    const float2 v = f32_split_hw(x);  // returned by value: no local escapes to memory
+    hi = v.x;
+    lo = v.y;
+    return;
   }
   const unsigned f23 = ((h32 & 0xFFFFFu) << 3) | (l32 >> 29);
   const unsigned rem = l32 & 0x1FFFFFFFu;
@@ -508,13 +509,25 @@ __device__ __forceinline__ bool f32_split_int(double x, float& hi, float& lo) {
   int r = (int)rem - (up ? 0x20000000 : 0);
   if (h32 & 0x80000000u) r = -r;
   lo = i2f_rn(r) * __uint_as_float((unsigned)(E - 948) << 23);
-  return true;
 }
-__device__ __forceinline__ void f32_split(double x, float& hi, float& lo) {
-  if (f32_split_int(x, hi, lo)) return;
-  const float2 v = f32_split_hw(x);  // returned by value: no local escapes to memory
-  hi = v.x;
-  lo = v.y;
+// the same where x is zero or |x| in [2^-74, 2^128) (returns whether it is): without a branch
+// for a zero, which is common among the separations on a lattice (a branch there: the two-lane
+// gather of 2 million particles on one 2074 us, without 1735; off one 1724 and 1732)
+__device__ __forceinline__ bool f32_split_int(double x, float& hi, float& lo) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  const unsigned h32 = (unsigned)(u >> 32), l32 = (unsigned)u;
+  const int E = (int)((h32 >> 20) & 0x7FFu);
+  const unsigned s = h32 & 0x80000000u;
+  const bool zero = ((h32 ^ s) | l32) == 0u;
+  const unsigned f23 = ((h32 & 0xFFFFFu) << 3) | (l32 >> 29);
+  const unsigned rem = l32 & 0x1FFFFFFFu;
+  const unsigned up = (rem > 0x10000000u) || (rem == 0x10000000u && (f23 & 1u));
+  hi = __uint_as_float(zero ? s : ((s | ((unsigned)(E - 896) << 23) | f23) + up));
+  int r = (int)rem - (up ? 0x20000000 : 0);
+  if (s) r = -r;
+  // a zero has r = 0; its scale is a number all the same
+  lo = i2f_rn(r) * __uint_as_float(zero ? 0u : (unsigned)(E - 948) << 23);
+  return zero || (unsigned)(E - 949) <= 201u;
 }
 
 // exact float -> double, identical to (double)f

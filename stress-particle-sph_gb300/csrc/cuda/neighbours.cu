@@ -723,7 +723,8 @@ __device__ __forceinline__ bool rounds_to_hi(dfl v, float rel) {
 __device__ __forceinline__ bool cubic_certified(const Grid& g, double dxd, double dyd, float* w,
                                                 float* dw0, float* dw1) {
   dfl dx, dy;
-  if (!f32_split_int(dxd, dx.hi, dx.lo) || !f32_split_int(dyd, dy.hi, dy.lo)) return false;
+  const bool okx = f32_split_int(dxd, dx.hi, dx.lo), oky = f32_split_int(dyd, dy.hi, dy.lo);
+  if (!(okx && oky)) return false;
   const dfl r2 = df_sumsq(dx, dy);
   if (!(r2.hi > 1e-25f && r2.hi < 1e25f)) return false;
   const dfl r = df_sqrt_rn(r2);
