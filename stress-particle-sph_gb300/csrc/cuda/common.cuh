@@ -175,7 +175,7 @@ struct Dev {
   int same_entries;    // k_lists writes the same-kind lists' entries only when a step kernel
                       // reads them (XSPH, artificial viscosity or stress) or with keys;
                       // their lengths (degS) always
-  int same_f32;    // the gathered same-kind entries serve the FP32 detection only
+  int same_f32;    // the gathered same-kind entries are evaluated in FP32 (Ctx::same_for_f32)
   int walk_order;  // directly gathered lists are put in walk order (put_walk_order)
   double* artR;        // its per-node rotated tensile stresses R(3) of the stage, (3, NN)
   double *vol, *rinv;  // m / rho and 1 / rho per particle (refreshed when rho changes)

@@ -107,10 +107,11 @@ struct Ctx {
     return !(lists_direct() && walks()) &&
            (precision == SPS_PREC_FP64_PLAIN || surf_every || surface_exact);
   }
-  // whether the FP32 detection is all that reads the gathered same-kind entries (Dev::same_f32);
-  // the exact one reads them where they are in walk order, and keyed lists of its own elsewhere
+  // whether the gathered same-kind entries are evaluated in FP32 (Dev::same_f32): where only the
+  // FP32 detection reads them and the lists are in creation order.  Lists in walk order keep
+  // their accuracy for either detection, as they had before they were gathered.
   bool same_for_f32() const {
-    return d.fast && !d.same_entries && !surf_every && !(surface_exact && d.walk_order);
+    return d.fast && !d.same_entries && !surf_every && !d.walk_order;
   }
   // whether this step begins with the outside approach's re-interpolation
   bool reinterpolates() const { return (step_variant & 1) != 0; }

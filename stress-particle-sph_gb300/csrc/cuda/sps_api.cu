@@ -1594,7 +1594,6 @@ int sps_set_surface_detection(sps_ctx* h, int32_t exact) {
     }
     // the step graphs that write the lists for a download differ between the two
     c.keys_written = c.same_written = false;
-    c.d.same_f32 = c.same_for_f32();
     drop_graphs(c);
   } catch (const std::exception& e) {
     return fail(&c, SPS_ERR_CUDA, e.what());
