@@ -288,8 +288,12 @@ __global__ void k_snap_pack(sps::Dev D, char* out, const int64_t* roff) {
     s[2 * l + 1] = make_double2(0.0, 0.0);
   }
 }
-// realisation r's fields, one thread a local particle, in the layout of snap_block
-__global__ void k_pack_real(sps::Dev D, int r, char* base) {
+// realisation r's fields, one thread a local particle, in the layout of snap_block; only the
+// fields of `want` (bits in the order of sps_download's arguments), since a caller that wants
+// one of them need not wait for the others
+enum { kWantX = 1, kWantVel = 2, kWantStress = 4, kWantRho = 8, kWantIv1 = 16, kWantDispl = 32,
+       kWantBc = 64, kWantFdp = 128 };
+__global__ void k_pack_real(sps::Dev D, int r, char* base, unsigned want) {
   const sps::Real& M = D.real[r];
   const int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t nn = M.nnode, nt = nn + M.nsp, n2 = nt + M.ndum;
@@ -297,20 +301,23 @@ __global__ void k_pack_real(sps::Dev D, int r, char* base) {
   const int g = (int)(l < nn ? M.node0 + l : l < nt ? M.sp0 + (l - nn) : M.dum0 + (l - nt));
   const SnapBlock b = snap_block(nn, nt, n2);
   double2* s = reinterpret_cast<double2*>(base + b.stress);
-  reinterpret_cast<double2*>(base + b.x)[l] = make_double2(D.px[g], D.py[g]);
-  reinterpret_cast<double2*>(base + b.vel)[l] = make_double2(D.vx[g], D.vy[g]);
-  reinterpret_cast<double*>(base + b.rho)[l] = D.rho[g];
+  if (want & kWantX) reinterpret_cast<double2*>(base + b.x)[l] = make_double2(D.px[g], D.py[g]);
+  if (want & kWantVel) reinterpret_cast<double2*>(base + b.vel)[l] = make_double2(D.vx[g], D.vy[g]);
+  if (want & kWantRho) reinterpret_cast<double*>(base + b.rho)[l] = D.rho[g];
   if (l >= nt) {
     // dummy stress is pair-local in the reference; report zero like its RK4 clear (:690)
-    s[2 * l] = s[2 * l + 1] = make_double2(0.0, 0.0);
+    if (want & kWantStress) s[2 * l] = s[2 * l + 1] = make_double2(0.0, 0.0);
     return;
   }
-  s[2 * l] = make_double2(D.s0[g], D.s1[g]);
-  s[2 * l + 1] = make_double2(D.s2[g], D.s3[g]);
-  reinterpret_cast<double*>(base + b.iv1)[l] = D.iv1[g];
-  reinterpret_cast<double*>(base + b.fdp)[l] = D.fdp[g];
-  reinterpret_cast<int32_t*>(base + b.bc)[l] = D.bc_or_not[g];
-  if (l < nn) reinterpret_cast<double2*>(base + b.displ)[l] = make_double2(D.dispx[g], D.dispy[g]);
+  if (want & kWantStress) {
+    s[2 * l] = make_double2(D.s0[g], D.s1[g]);
+    s[2 * l + 1] = make_double2(D.s2[g], D.s3[g]);
+  }
+  if (want & kWantIv1) reinterpret_cast<double*>(base + b.iv1)[l] = D.iv1[g];
+  if (want & kWantFdp) reinterpret_cast<double*>(base + b.fdp)[l] = D.fdp[g];
+  if (want & kWantBc) reinterpret_cast<int32_t*>(base + b.bc)[l] = D.bc_or_not[g];
+  if (l < nn && (want & kWantDispl))
+    reinterpret_cast<double2*>(base + b.displ)[l] = make_double2(D.dispx[g], D.dispy[g]);
 }
 
 // an uploaded realisation: x(2,n2) vel(2,n2) x00(2,n2) stress(4,n2) mass rho hsml(n2)
@@ -1227,25 +1234,44 @@ int sps_download_real(sps_ctx* h, int32_t r, double* x, double* vel, double* str
   const size_t nn = M.nnode, nt = (size_t)M.nnode + M.nsp, n2 = nt + M.ndum;
   try {
     if (bc_or_not) refresh_surface(c, false);
-    // the fields are packed side by side in the staging buffer; a small realisation crosses
-    // as one copy through pinned memory, a larger one field by field into the caller's arrays
+    // the wanted fields are packed side by side in the staging buffer; those of a small
+    // realisation cross as one copy through pinned memory (from the first to the last of them),
+    // those of a larger one field by field into the caller's arrays (of a single problem the
+    // fields of one value a particle as they lie, unpacked)
     const SnapBlock b = snap_block((int64_t)nn, (int64_t)nt, (int64_t)n2);
     char* st = reinterpret_cast<char*>(c.stage);
-    if (n2 > 0)
-      k_pack_real<<<(int)((n2 + kBlock - 1) / kBlock), kBlock, 0, c.stream>>>(D, r, st);
-    const bool packed = b.bytes <= c.pack_cap;
-    if (packed)
-      SPS_CUDA_CHECK(cudaMemcpyAsync(c.h_pack, st, b.bytes, cudaMemcpyDeviceToHost, c.stream));
+    const bool packed = b.bytes <= c.pack_cap, whole = !packed && D.R == 1;
     struct Field {
       void* dst;
       size_t off, bytes;
-    } fields[] = {{x, b.x, 16 * n2},          {vel, b.vel, 16 * n2},  {stress, b.stress, 32 * n2},
-                  {rho, b.rho, 8 * n2},       {intvars1, b.iv1, 8 * nt}, {f_drucker, b.fdp, 8 * nt},
-                  {displ, b.displ, 16 * nn},  {bc_or_not, b.bc, 4 * nt}};
+      unsigned bit;
+      const void* whole;  // the state's own array, where it is the field
+    } fields[] = {{x, b.x, 16 * n2, kWantX, nullptr},
+                  {vel, b.vel, 16 * n2, kWantVel, nullptr},
+                  {stress, b.stress, 32 * n2, kWantStress, nullptr},
+                  {rho, b.rho, 8 * n2, kWantRho, whole ? D.rho : nullptr},
+                  {intvars1, b.iv1, 8 * nt, kWantIv1, whole ? D.iv1 : nullptr},
+                  {f_drucker, b.fdp, 8 * nt, kWantFdp, whole ? D.fdp : nullptr},
+                  {displ, b.displ, 16 * nn, kWantDispl, nullptr},
+                  {bc_or_not, b.bc, 4 * nt, kWantBc, whole ? D.bc_or_not : nullptr}};
+    unsigned want = 0;
+    for (const Field& f : fields)
+      if (f.dst && !f.whole) want |= f.bit;
+    if (n2 > 0 && want)
+      k_pack_real<<<(int)((n2 + kBlock - 1) / kBlock), kBlock, 0, c.stream>>>(D, r, st, want);
+    size_t lo = b.bytes, hi = 0;
+    for (const Field& f : fields)
+      if (f.dst && f.bytes) {
+        lo = std::min(lo, f.off);
+        hi = std::max(hi, f.off + f.bytes);
+      }
+    if (packed && lo < hi)
+      SPS_CUDA_CHECK(cudaMemcpyAsync(c.h_pack + lo, st + lo, hi - lo, cudaMemcpyDeviceToHost, c.stream));
     if (!packed)
       for (const Field& f : fields)
         if (f.dst && f.bytes)
-          SPS_CUDA_CHECK(cudaMemcpyAsync(f.dst, st + f.off, f.bytes, cudaMemcpyDeviceToHost, c.stream));
+          SPS_CUDA_CHECK(cudaMemcpyAsync(f.dst, f.whole ? f.whole : st + f.off, f.bytes,
+                                         cudaMemcpyDeviceToHost, c.stream));
     SPS_CUDA_CHECK(cudaGetLastError());
     SPS_CUDA_CHECK(cudaStreamSynchronize(c.stream));
     if (packed)

@@ -82,3 +82,25 @@ def test_nonfinite_state_after_a_step(built_gpu):
     cases.assert_bitwise(ctx.download(), ref.download(), prob.ntotal)
     ctx.close()
     ref.close()
+
+
+@pytest.mark.parametrize("dx", [0.05, 0.02, 0.01])  # 0.09 and 0.36 MB as one copy; 1.2 MB by field
+def test_download_of_some_fields(built_gpu, dx):
+    """A null pointer skips its field: every single field, the first and the last, all but
+    one and none, against the whole download."""
+    prob = cases.bui_like(width=1.0, height=0.5, dx=dx)
+    ctx = _ctx(prob)
+    ctx.upload_problem(prob)
+    ctx.step(2, 0.0)
+    names = ("x", "vel", "stress", "rho", "intvars1", "displ", "bc_or_not", "f_drucker")
+    full = ctx.download()
+    sets = [(k,) for k in names] + [("x", "f_drucker"), ("displ", "bc_or_not"), names[1:], names[:-1], ()]
+    for want in sets:
+        out = {k: np.full_like(full[k], 77) for k in names}
+        ctx._call("download", ctx._h, *[sps_gb300.context._ip(out[k]) if k in want and k == "bc_or_not"
+                                        else sps_gb300.context._dp(out[k]) if k in want else None
+                                        for k in names])
+        for k in names:
+            want_k = full[k] if k in want else np.full_like(full[k], 77)
+            assert np.array_equal(out[k], want_k, equal_nan=True), (want, k)
+    ctx.close()
