@@ -28,6 +28,7 @@ struct HostReal {
   // extent and smoothing lengths of the uploaded state (capacity sizing)
   double ncells_est = 0.0, hmax = 0.0, hmin_nd = 1e300;
   bool uploaded = false;
+  int64_t kept = 0;  // Ctx::builds when its smoothing lengths went to Ctx::hbuilt
   // get_nodes_on_free_surface: every step when a later step reads its output (the
   // traction-free BC, or XSPH's marks next to BC particles, or standard SPH's position
   // copy after it); otherwise on demand when the state is downloaded, which gives the same
@@ -151,6 +152,12 @@ struct Ctx {
   // constants: sps_dump_pairs and the lists of a detection build them first (set by enqueue_step
   // for every step, since a replayed graph runs no host code)
   bool half_stale = false;
+  // the smoothing lengths of the last pair build, which those rebuilds read, once an upload has
+  // replaced them (hbuilt_of == builds): in the place of the same-kind lists, which nothing reads
+  // from an upload to the next step
+  int64_t builds = 0;  // steps enqueued
+  double* hbuilt = nullptr;
+  int64_t hbuilt_of = 0;
   int step_variant = 0;    // the variant launch_*_step enqueues
   int64_t itimestep = 0;   // itimestep_sph of the last step (0 after an upload)
   bool use_graph = true;

@@ -1722,13 +1722,27 @@ void launch_walk_order(Ctx& c) { walk_order(c, c.d, c.same_now()); }
 
 // The device view of the last pair build for a rebuild after the step: the FP64 positions
 // the build's exact band test read (x0x, x0y hold them from the step's start, before
-// anything moved; the smoothing lengths are constant when the lists are gathered), so the
-// rebuild decides every pair as the build did.  The cell-frame offsets and sorted records
-// are the build's own.
-Dev build_view(const Ctx& c) {
+// anything moved; the smoothing lengths are constant when the lists are gathered, and an upload
+// keeps the ones that it replaces), so the rebuild decides every pair as the build did.  The
+// cell-frame offsets and sorted records are the build's own.
+Dev build_view(Ctx& c) {
   Dev D = c.d;
   D.px = D.x0x;
   D.py = D.x0y;
+  if (c.builds > 0 && c.hbuilt_of == c.builds) {
+    // (of a batch, the realisations that no upload has replaced)
+    for (size_t r = 0; r < c.hr.size(); r++) {
+      if (c.hr[r].kept == c.builds) continue;
+      c.hr[r].kept = c.builds;
+      const Real& M = c.real[r];
+      const int64_t seg[3][2] = {{M.node0, M.nnode}, {M.sp0, M.nsp}, {M.dum0, M.ndum}};
+      for (const auto& q : seg)
+        if (q[1] > 0)
+          SPS_CUDA_CHECK(cudaMemcpyAsync(c.hbuilt + q[0], D.hsml + q[0], sizeof(double) * q[1],
+                                         cudaMemcpyDeviceToDevice, c.stream));
+    }
+    D.hsml = c.hbuilt;
+  }
   return D;
 }
 

@@ -344,7 +344,7 @@ __host__ __device__ inline UpBlock up_block(int64_t nt, int64_t n2) {
 // an upload's fields into the state of realisation r (one pass instead of about thirty copies,
 // transposes and clears), and the start values of its checks
 __global__ void k_unpack_real(sps::Dev D, int r, const char* base, bool iv, bool fdp,
-                              unsigned long long* chk) {
+                              unsigned long long* chk, double* hbuilt) {
   const sps::Real& M = D.real[r];
   const int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (l < 8) chk[l] = l < 6 ? ~0ull : 0ull;
@@ -370,6 +370,7 @@ __global__ void k_unpack_real(sps::Dev D, int r, const char* base, bool iv, bool
   D.s3[g] = s23.y;
   D.mass[g] = reinterpret_cast<const double*>(base + b.mass)[l];
   D.rho[g] = rho;
+  if (hbuilt) hbuilt[g] = D.hsml[g];  // (Ctx::hbuilt)
   D.hsml[g] = reinterpret_cast<const double*>(base + b.hsml)[l];
   D.itype[g] = reinterpret_cast<const int32_t*>(base + b.itype)[l];
   D.out[g] = 0;
@@ -421,6 +422,7 @@ int variant_of(const sps::Ctx& c, int64_t it) {
 // enqueue one step (itimestep_sph advanced first) as its variant's graph, or directly
 void enqueue_step(sps::Ctx& c) {
   c.itimestep += 1;
+  c.builds += 1;
   c.step_variant = variant_of(c, c.itimestep) | (c.keys_in_step ? 4 : 0);
   c.keys_written = !c.d.walk_order && ((c.keys_in_step && !c.surface_f32() && !c.lists_direct()) || c.surf_every);
   c.same_written = c.keys_in_step || c.surf_every || c.d.same_entries;
@@ -1017,8 +1019,19 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
       SPS_CUDA_CHECK(cudaMemcpyAsync(st, c.h_pack, ub.bytes, cudaMemcpyHostToDevice, c.up_stream));
     SPS_CUDA_CHECK(cudaEventRecord(c.up_ready, c.up_stream));
     SPS_CUDA_CHECK(cudaStreamWaitEvent(c.stream, c.up_ready, 0));
+    // the first upload of r since a step keeps the smoothing lengths of that step's pairs
+    double* keep = nullptr;
+    if (c.builds > 0 && c.hr[r].kept != c.builds) {
+      if (c.hbuilt_of != c.builds) {
+        c.hbuilt = reinterpret_cast<double*>(D.same);
+        c.hbuilt_of = c.builds;
+      }
+      c.hr[r].kept = c.builds;
+      keep = c.hbuilt;
+      c.surf_stale = false;  // the step's positions go, whether the upload is accepted or not
+    }
     k_unpack_real<<<nbk(std::max<int64_t>((int64_t)n2, 8)), kBlock, 0, c.stream>>>(
-        D, r, st, intvars1 != nullptr, f_drucker != nullptr, c.d_chk);
+        D, r, st, intvars1 != nullptr, f_drucker != nullptr, c.d_chk, keep);
     for (const Seg& q : sg)
       if (q.n > 0) sps::launch_vol(c, (int)q.g, (int)(q.g + q.n));
     if (n2 > 0)
@@ -1067,8 +1080,14 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
       // known, but no more than twice what there was
       const double all = std::min(4.0 * nc * D.R / known + 1024.0, 2.0e9 / 4.0);
       cap = std::max(cap, (int)std::min(all, 2.0 * D.cell_cap));
-      D.cell_cnt = dalloc<int32_t>(c, (size_t)cap + 2);
-      D.cell_start = dalloc<int32_t>(c, (size_t)cap + 2);
+      // (the cells of the last pair build go along: a rebuild of its half lists reads them)
+      for (int32_t** a : {&D.cell_cnt, &D.cell_start}) {
+        int32_t* grown = dalloc<int32_t>(c, (size_t)cap + 2);
+        if (c.builds > 0)
+          SPS_CUDA_CHECK(cudaMemcpyAsync(grown, *a, sizeof(int32_t) * ((size_t)D.cell_cap + 2),
+                                         cudaMemcpyDeviceToDevice, c.stream));
+        *a = grown;
+      }
       D.cntD = dalloc<int32_t>(c, (size_t)cap + 2);
       D.cell_loc = dalloc<int32_t>(c, (size_t)cap + 2);
       D.cntK = dalloc<unsigned long long>(c, (size_t)cap + 2);
@@ -1100,6 +1119,12 @@ int sps_upload_real(sps_ctx* h, int32_t r, const double* x, const double* vel,
         const size_t second = (D.fast ? ns : nt) * cap * sizeof(double);
         const size_t consts = c.fused() ? first + second : 0;
         char* half = dalloc<char>(c, std::max(sizeof(int4) * (size_t)D.N2 * cap, consts));
+        // half lists that cannot be built again go along
+        if (c.builds > 0 && !c.half_stale && D.N2 > 0)
+          SPS_CUDA_CHECK(cudaMemcpy2DAsync(half, sizeof(int4) * cap, D.half,
+                                           sizeof(int4) * (size_t)D.capH,
+                                           sizeof(int4) * std::min(cap, (size_t)D.capH),
+                                           (size_t)D.N2, cudaMemcpyDeviceToDevice, c.stream));
         D.half = reinterpret_cast<int4*>(half);
         if (c.fused() && D.fast) {
           D.hGf = reinterpret_cast<float2*>(half);
@@ -1455,7 +1480,7 @@ int sps_dump_pairs_real(sps_ctx* h, int32_t r, int32_t* pair_i, int32_t* pair_j,
     sps::Grid g;
     sps::GridTotal gt;
     SPS_CUDA_CHECK(cudaMemcpy(&meta, D.meta + r, sizeof(meta), cudaMemcpyDeviceToHost));
-    if (!pair_i) {
+    if (!pair_i || meta.n <= 0) {  // (none before the first step)
       *npairs = meta.n;
       return SPS_OK;
     }
@@ -1516,6 +1541,7 @@ int sps_dump_pairs_real(sps_ctx* h, int32_t r, int32_t* pair_i, int32_t* pair_j,
         cy.push_back(gy);
       }
     int64_t n = (int64_t)ci.size(), m = meta.m_prev, k = 0;
+    if (n > *npairs) return fail(&c, SPS_ERR_CAPACITY, "sps_dump_pairs: buffer too small");
     auto put = [&](int64_t q) {
       pair_i[k] = ci[q];
       pair_j[k] = cj[q];
