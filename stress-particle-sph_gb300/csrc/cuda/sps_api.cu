@@ -1830,6 +1830,23 @@ std::vector<std::pair<void*, size_t>> carried_state(sps::Ctx& c) {
   return v;
 }
 
+// the last step's pair build: what its half lists are built from again, or the lists themselves
+void add_pair_build(sps::Ctx& c, std::vector<std::pair<void*, size_t>>& v) {
+  sps::Dev& D = c.d;
+  const size_t N2 = D.N2, cells = sizeof(int32_t) * ((size_t)D.cell_cap + 2);
+  for (void* p : {(void*)D.cell_of, (void*)D.sorted, (void*)D.xr, (void*)D.yr, (void*)D.hr,
+                  (void*)D.xrl, (void*)D.yrl, (void*)D.half_cnt})
+    v.push_back({p, 4 * N2});
+  for (void* p : {(void*)D.x0x, (void*)D.x0y, (void*)D.srecl}) v.push_back({p, 8 * N2});
+  v.push_back({D.srec, 16 * N2});
+  v.push_back({D.cell_start, cells});
+  v.push_back({D.cell_cnt, cells});
+  v.push_back({D.grid, sizeof(sps::Grid) * D.R});
+  v.push_back({D.gtot, sizeof(sps::GridTotal)});
+  if (!c.half_stale) v.push_back({D.half, sizeof(int4) * N2 * (size_t)D.capH});
+  if (c.hbuilt_of == c.builds) v.push_back({c.hbuilt, 8 * N2});
+}
+
 }  // namespace
 
 int sps_autotune(sps_ctx* h, int32_t nsteps, int32_t* blocks) {
@@ -1839,7 +1856,11 @@ int sps_autotune(sps_ctx* h, int32_t nsteps, int32_t* blocks) {
   void* snap = nullptr;
   try {
     SPS_CUDA_CHECK(cudaStreamSynchronize(c.stream));
+    // the profiled steps overwrite the pair tables: detect a pending free surface first, and keep
+    // the pairs of the last step
+    refresh_surface(c);
     auto st = carried_state(c);
+    if (c.builds > 0) add_pair_build(c, st);
     size_t total = 0;
     for (auto& a : st) total += (a.second + 255) & ~size_t(255);
     SPS_CUDA_CHECK(cudaMalloc(&snap, total));
@@ -1854,10 +1875,9 @@ int sps_autotune(sps_ctx* h, int32_t nsteps, int32_t* blocks) {
       SPS_CUDA_CHECK(cudaStreamSynchronize(c.stream));
     };
     copy(true);
-    // the profiled steps overwrite the pair tables: detect a pending free surface first
-    refresh_surface(c);
     const bool stale = c.surf_stale;
-    const int64_t it0 = c.itimestep;
+    const int64_t it0 = c.itimestep, builds = c.builds;
+    const bool hs = c.half_stale;
     const bool kin = c.keys_in_step, kw = c.keys_written, sw = c.same_written;
     const int cand[] = {64, 128, 256, 512};
     int best[sps::TK_N];
@@ -1943,6 +1963,8 @@ int sps_autotune(sps_ctx* h, int32_t nsteps, int32_t* blocks) {
     }
     c.surf_stale = stale;
     c.itimestep = it0;
+    c.builds = builds;
+    c.half_stale = hs;
     c.keys_in_step = kin;
     c.keys_written = kw;
     c.same_written = sw;

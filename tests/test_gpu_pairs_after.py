@@ -1,5 +1,6 @@
 """GPU: sps_dump_pairs reports the last step's pairs also after calls that replace what their
-rebuild reads: an upload of other smoothing lengths, which may move the list and cell capacities."""
+rebuild reads: an upload of other smoothing lengths, which may move the list and cell capacities,
+and the autotuner's steps, which also leave the free surface as it was."""
 import numpy as np
 import pytest
 
@@ -72,3 +73,31 @@ def test_pairs_of_a_batch_after_one_upload(built_gpu, form):
         _same(ref.dump_pairs(r), b.dump_pairs(r))
     ref.close()
     b.close()
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("option", OPTIONS)
+@pytest.mark.parametrize("upload", [False, True])
+def test_pairs_and_surface_after_tuning(built_gpu, form, option, upload):
+    # the block falls apart at 20 m/s: the autotuner's steps meet other pairs than the last one
+    p = cases.bui_like(width=1.0, height=0.5, dx=0.05, coh=1e9, dt=6e-4, **OPTIONS[option])
+    s = p.state()
+    x, v = s["x"].reshape(-1, 2), s["vel"].reshape(-1, 2)
+    v[:p.ntotal] = 20.0 * (x[:p.ntotal] + 0.1)
+    ref, ctx = _ctx(p, form), _ctx(p, form)
+    for c in (ref, ctx):
+        c.upload(**s)
+        c.step(3, 0.0)
+        if upload:
+            s2 = p.state()
+            s2["hsml"] *= 0.9
+            c.upload(**s2)
+    sps_gb300.autotune(ctx, 4)
+    a, b = ctx.download(), ref.download()
+    cases.assert_bitwise(a, b, p.ntotal)
+    assert np.array_equal(a["bc_or_not"], b["bc_or_not"])
+    for u, w in zip(ctx.download_surface(0), ref.download_surface(0)):
+        assert np.array_equal(u, w, equal_nan=True)
+    _same(ref.dump_pairs(), ctx.dump_pairs())
+    ref.close()
+    ctx.close()
